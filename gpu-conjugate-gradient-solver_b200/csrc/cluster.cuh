@@ -1,0 +1,368 @@
+// Whole Gauss-Seidel smoothing steps of a small level in one thread-block
+// cluster, the iterate in distributed shared memory.
+//
+// What bounds such a level. A multicolour sweep is one dependent step per
+// colour, and a Galerkin level of a few thousand rows has 15-45 colours of a
+// few hundred rows: launched one kernel per colour, a pass is one or two
+// blocks whose warps wait on row pointer -> column -> gather -> store -> next
+// launch, about 3 us a pass with the GPU idle (ncu: 0.1 % of DRAM, 8-11 % of
+// the warps of the SMs in use). Here the step is latency only:
+//   * one cluster of up to 16 CTAs owns the level. Each colour's rows are cut
+//     into one contiguous piece per CTA, and a CTA keeps in shared memory the
+//     entries of x that its rows own or read ("slots", numbered per CTA);
+//   * the thread group that updates a row sends the new value straight into
+//     the slots of every CTA that reads it (st.async), which also counts the
+//     bytes on that CTA's mbarrier of the pass: there is one mbarrier per
+//     pass, armed once with the bytes the CTA will receive, so a CTA starts
+//     pass p + 1 as soon as the values it reads have arrived: one one-way
+//     message, no barrier round trip;
+//   * the matrix is stored in the order in which each CTA's threads read it
+//     (values and 16-bit slot numbers, slot pairs, threads contiguous), and
+//     every thread loads its next row's operands before it waits.
+// Measured (one B200, FP64, level 2 of a 61 x 47 x 83 Poisson: 5,103 rows, 37
+// colours, 361 k entries): a symmetric step of 73 passes 183 -> 86 us, 1.0 us
+// a pass. What is left of a pass: 0.78 us with next to no rows (message,
+// mbarrier wake-up, shuffles, quotient), the rest shared memory gathers (bank
+// conflicts) and the issue of the 16 warps.
+//
+// No race. Row j of colour c' is overwritten in CTA B's slots only after the
+// owner A of j has waited for every earlier pass of the sweep, and A receives
+// every row i that reads j (checked when the layout is built): B's read of j
+// for i happened before B sent i. Two writes of one row to one slot are
+// separated by a direction change or a step's end, where every CTA first
+// waits for all its passes and then meets the others at the cluster barrier,
+// so the earlier write has landed. Rows of one colour do not read each other
+// (or, on a level whose colouring is of the strong couplings only, read the
+// copy of x taken where the sweep starts: slot numbers with bit 15 set).
+// All CTAs meet at the cluster barrier before any of them exits.
+//
+// Each row is updated with the arithmetic of csrv_gs_kernel with the same
+// lanes per row (bsrv_gs_kernel for 3x3 blocks): same sums in the same order,
+// same shuffles, same division, so the iterates are the same bits.
+//
+// Waits on mbarriers are bounded: a wait that gives up records
+// CgState::sync_fault and stops the solve; the kernel then runs to its end
+// without waiting.
+#pragma once
+
+#include "bulk.cuh"
+#include "kernels.cuh"
+
+namespace gsb {
+
+constexpr int kClusterThreads = 512;    // at most; a layout may use fewer
+constexpr int kClusterPairs = 4;        // slot pairs per lane loaded ahead
+constexpr int kClusterMaxPasses = 512;  // mbarriers
+constexpr int kClusterMaxSlots = 32760; // two copies of the slots in 16 bits
+constexpr int kClusterMaxColors = 128;
+
+// One CTA's piece of one colour.
+struct __align__(16) ClusterSeg {
+  int row0, rows;  // global rows [row0, row0 + rows) (nodes of a block level)
+  int trips;       // rows per thread group, at least 1
+  int base;        // first slot pair (block slot) of trip 0
+  int pairs;       // slot pairs (block slots) per lane and trip
+  int stride;      // threads that take part (a multiple of 32; 0: no rows)
+  int sbase;       // first send entry
+  int schunks;     // send entries per lane and trip
+};
+
+template <typename T>
+struct ClusterView {
+  int ncta, ncolors, threads;
+  int max_slots;                               // slots of the widest CTA, without the zero slot
+  const ClusterSeg *__restrict__ seg;          // [cta][colour]
+  const unsigned *__restrict__ expect;         // [cta][colour]: rows of the colour that the CTA receives
+  const int *__restrict__ slot_ptr;            // ncta + 1
+  const int *__restrict__ slot_row;            // global row of each slot
+  const typename Pair<T>::type *__restrict__ val;
+  const unsigned *__restrict__ col;            // two slots; + max_slots + 1: the copy taken at the sweep's start
+  const unsigned *__restrict__ send;           // cta << 16 | slot, or kNoSend
+  const unsigned short *__restrict__ own;      // slot of each row in its owner
+  const typename Pair<T>::type *__restrict__ diag;  // per row {d, 1 / d}; the latter 0 where it is not safe to use
+  int relaxed;                                 // own-colour reads from the sweep's start
+};
+
+constexpr unsigned kNoSend = 0xffffffffu;
+
+// The passes of one call: dir 0 symmetric steps, 1 forward sweeps, 2
+// backward sweeps; skip drops the colour repeated where a sweep turns.
+struct ClusterPasses {
+  int ncolors, steps, dir, skip;
+  // sweep s of the call: its first colour, direction (+1 / -1) and passes
+  __host__ __device__ int sweeps() const { return dir == 0 ? 2 * steps : steps; }
+  __host__ __device__ int direction(int s) const { return dir == 1 || (dir == 0 && (s & 1) == 0) ? 1 : -1; }
+  __host__ __device__ int first(int s) const {
+    const int drop = dir == 0 && skip != 0 && s > 0 ? 1 : 0;
+    return direction(s) > 0 ? drop : ncolors - 1 - drop;
+  }
+  __host__ __device__ int count(int s) const { return ncolors - (dir == 0 && skip != 0 && s > 0 ? 1 : 0); }
+  __host__ __device__ int total() const {
+    int t = 0;
+    for (int s = 0; s < sweeps(); ++s) t += count(s);
+    return t;
+  }
+};
+
+namespace cluster_detail {
+
+__device__ __forceinline__ unsigned cta_rank() {
+  unsigned r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire;" ::: "memory");
+}
+__device__ __forceinline__ unsigned remote(unsigned addr, unsigned cta) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
+  return r;
+}
+__device__ __forceinline__ void send_value(unsigned addr, double v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void send_value(unsigned addr, float v, unsigned bar) {
+  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
+               "r"(__float_as_uint(v)), "r"(bar)
+               : "memory");
+}
+// Read-only loads that keep their place: the operands of the next row are
+// requested before the wait on the current pass (a plain load is moved down to
+// its first use, which exposes its latency: 770 of 3000 cycles a pass).
+__device__ __forceinline__ double2 load_early(const double2 *p) {
+  double2 v;
+  asm volatile("ld.global.nc.v2.f64 {%0, %1}, [%2];" : "=d"(v.x), "=d"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float2 load_early(const float2 *p) {
+  float2 v;
+  asm volatile("ld.global.nc.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ double load_early(const double *p) {
+  double v;
+  asm volatile("ld.global.nc.f64 %0, [%1];" : "=d"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ float load_early(const float *p) {
+  float v;
+  asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned load_early(const unsigned *p) {
+  unsigned v;
+  asm volatile("ld.global.nc.u32 %0, [%1];" : "=r"(v) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ unsigned short load_early(const unsigned short *p) {
+  unsigned short v;
+  asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));
+  return v;
+}
+
+// The quotient n / d from r = 1 / d: two residual corrections of n r
+// (Markstein, IBM J. Res. Dev. 34, 1990), after which it is correctly rounded.
+// The plain division (370 cycles in FP64 on the critical path of every pass)
+// where r is 0 (1 / d may not be a normal number) or the result not finite.
+template <typename T>
+__device__ __forceinline__ T quotient(T n, T d, T r) {
+  T q = n * r;
+  q = fma(fma(-q, d, n), r, q);
+  q = fma(fma(-q, d, n), r, q);
+  if (r == T(0) || !isfinite(q)) q = n / d;
+  return q;
+}
+
+// Bounded wait for the values of a pass (written by other CTAs: acquire at
+// cluster scope); false after about a second of clocks.
+constexpr long long kClusterWaitClocks = 2000000000LL;
+
+__device__ __forceinline__ bool pass_ready(unsigned bar) {
+  unsigned ok;
+  asm volatile(
+      "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], 0;\n"
+      " selp.u32 %0, 1, 0, p;\n}"
+      : "=r"(ok)
+      : "r"(bar)
+      : "memory");
+  return ok != 0;
+}
+__device__ __forceinline__ bool pass_wait(unsigned bar) {
+  if (pass_ready(bar)) return true;
+  const long long t0 = clock64();
+  while (clock64() - t0 < kClusterWaitClocks)
+    if (pass_ready(bar)) return true;
+  return false;
+}
+
+}  // namespace cluster_detail
+
+// What one thread needs of one row before the iterate.
+template <typename T, typename BT>
+struct ClusterUnit {
+  typename Pair<T>::type v[kClusterPairs];
+  unsigned c[kClusterPairs];  // two slots
+  unsigned send;
+  typename Pair<T>::type d;
+  BT b;
+};
+
+// The matrix part of a unit: trip t of piece sg.
+template <typename T, typename BT>
+__device__ __forceinline__ void cluster_load(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid, int local,
+                                             ClusterUnit<T, BT> &u) {
+  using cluster_detail::load_early;
+  const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
+#pragma unroll
+  for (int q = 0; q < kClusterPairs; ++q)
+    if (q < sg.pairs) {
+      u.v[q] = load_early(A.val + e0 + q * sg.stride);
+      u.c[q] = load_early(A.col + e0 + q * sg.stride);
+    }
+  u.send = load_early(A.send + sg.sbase + t * sg.schunks * sg.stride + tid);
+  u.d = load_early(A.diag + sg.row0 + min(local, sg.rows - 1));
+}
+
+// Smoothing steps of a scalar level; grid = one cluster of A.ncta CTAs.
+template <typename T, typename BT, int G>
+__global__ void __launch_bounds__(kClusterThreads, 1)
+    cluster_gs_kernel(ClusterView<T> A, ClusterPasses P, const BT *__restrict__ b, T *__restrict__ x, int zero,
+                      const T *__restrict__ wts, T omega, CgState *st) {
+  using namespace cluster_detail;
+  extern __shared__ __align__(16) unsigned char cluster_smem[];
+  __shared__ ClusterSeg seg[kClusterMaxColors];
+  __shared__ unsigned long long bars[kClusterMaxPasses];
+  // colour of each pass, bit 15 on the last one of a sweep; 0xffff at the end
+  __shared__ unsigned short plist[kClusterMaxPasses + 1];
+  T *xs = reinterpret_cast<T *>(cluster_smem);  // max_slots + 1, the last one zero (then the sweep's start)
+  const int tid = threadIdx.x, nthr = A.threads;
+  const unsigned me = cta_rank();
+  const int s0 = __ldg(A.slot_ptr + me), nslots = __ldg(A.slot_ptr + me + 1) - s0;
+  T *xp = xs + A.max_slots + 1;
+  for (int c = tid; c < A.ncolors; c += nthr) seg[c] = A.seg[me * A.ncolors + c];
+  const int npass = P.total();
+  for (int p = tid; p < npass; p += nthr)
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bars + p)) : "memory");
+  asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  __syncthreads();
+  // arm every pass once with the bytes this CTA receives in it
+  for (int s = 0, p = 0; s < P.sweeps(); ++s) {
+    const int n = P.count(s), f = P.first(s), dr = P.direction(s);
+    for (int i = tid; i < n; i += nthr) {
+      const int c = f + dr * i;
+      mbar_expect_tx(bars + p + i, __ldg(A.expect + me * A.ncolors + c) * static_cast<unsigned>(sizeof(T)));
+      plist[p + i] = static_cast<unsigned short>(c | (i + 1 == n ? 0x8000 : 0));
+    }
+    p += n;
+  }
+  if (tid == 0) plist[npass] = 0xffff;
+  __syncthreads();
+  // the first row's matrix operands do not change during a solve
+  constexpr int kLog = G == 4 ? 2 : (G == 8 ? 3 : (G == 16 ? 4 : 5));
+  const int grp = tid >> kLog, groups = nthr >> kLog;
+  ClusterUnit<T, BT> cur, nxt;
+  unsigned code = plist[0];
+  ClusterSeg sg = seg[code & 0x7fffu];
+  if (tid < sg.stride) cluster_load<T, BT>(A, sg, 0, tid, grp, cur);
+  const bool stop = pass_entry(&st->done);  // the same in every CTA: only a finished kernel writes it
+  if (!stop) {
+    if (tid < sg.stride) cur.b = load_early(b + sg.row0 + min(grp, sg.rows - 1));
+    for (int i = tid; i <= A.max_slots; i += nthr) {
+      const T v = zero || i >= nslots ? T(0) : x[__ldg(A.slot_row + s0 + i)];
+      xs[i] = v;
+      if (A.relaxed) xp[i] = v;
+    }
+  }
+  cluster_barrier();
+  if (stop) return;
+  const unsigned xs_addr = smem_addr(xs), bar_addr = smem_addr(bars);
+  // passes from here on write x back to the level (the last step's)
+  const int keep = npass - (P.dir == 0 ? P.count(P.sweeps() - 1) + P.count(P.sweeps() - 2) : A.ncolors);
+  int p = 0, t = 0;
+  bool fresh = true, dead = false;  // first pass of a sweep; a wait gave up
+  for (;;) {
+    // the next unit's operands, before this one waits
+    const bool last_trip = t + 1 == sg.trips;
+    const int tn = last_trip ? 0 : t + 1;
+    const unsigned next_code = plist[last_trip ? p + 1 : p];
+    ClusterSeg sn;
+    sn.stride = 0;
+    if (next_code != 0xffffu) {
+      sn = seg[next_code & 0x7fffu];
+      if (tid < sn.stride) {
+        const int local = tn * groups + grp;
+        cluster_load<T, BT>(A, sn, tn, tid, local, nxt);
+        nxt.b = load_early(b + sn.row0 + min(local, sn.rows - 1));
+      }
+    }
+    const unsigned to_cta = (cur.send >> 16) & 15u;
+    const unsigned to_x = remote(xs_addr + static_cast<unsigned>(sizeof(T)) * (cur.send & 0xffffu), to_cta);
+    const unsigned to_bar = remote(bar_addr + 8 * p, to_cta);
+    if (t == 0 && !fresh && !dead) dead = !pass_wait(bar_addr + 8 * (p - 1));
+    if (tid < sg.stride) {
+      T sum = T(0);
+#pragma unroll
+      for (int q = 0; q < kClusterPairs; ++q)
+        if (q < sg.pairs) {
+          sum = fma(cur.v[q].x, xs[cur.c[q] & 0xffffu], sum);
+          sum = fma(cur.v[q].y, xs[cur.c[q] >> 16], sum);
+        }
+      if (sg.pairs > kClusterPairs) {
+        const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
+#pragma unroll 4
+        for (int q = kClusterPairs; q < sg.pairs; ++q) {
+          const typename Pair<T>::type v = __ldg(A.val + e0 + q * sg.stride);
+          const unsigned c = __ldg(A.col + e0 + q * sg.stride);
+          sum = fma(v.x, xs[c & 0xffffu], sum);
+          sum = fma(v.y, xs[c >> 16], sum);
+        }
+      }
+#pragma unroll
+      for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
+      const int local = t * groups + grp;
+      if (local < sg.rows) {
+        T xn = quotient(T(cur.b) - sum, cur.d.x, cur.d.y);
+        const T w = wts != nullptr ? __ldg(wts + (code & 0x7fffu)) : omega;
+        if (w != T(1)) xn = fma(T(1) - w, xs[__ldg(A.own + sg.row0 + local)], w * xn);
+        if (cur.send != kNoSend) send_value(to_x, xn, to_bar);
+        for (int q = 1; q < sg.schunks; ++q) {
+          const unsigned to = __ldg(A.send + sg.sbase + (t * sg.schunks + q) * sg.stride + tid);
+          if (to != kNoSend)
+            send_value(remote(xs_addr + static_cast<unsigned>(sizeof(T)) * (to & 0xffffu), to >> 16), xn,
+                       remote(bar_addr + 8 * p, to >> 16));
+        }
+        if (p >= keep && (tid & (G - 1)) == 0) x[sg.row0 + local] = xn;
+      }
+    }
+    fresh = false;
+    if (last_trip) {
+      if (code & 0x8000u) {
+        // every value of this sweep has arrived before the next one starts
+        // (or before the CTAs leave)
+        if (!dead) dead = !pass_wait(bar_addr + 8 * p);
+        if (A.relaxed) {
+          __syncthreads();
+          for (int k = tid; k < nslots; k += nthr) xp[k] = xs[k];
+        }
+        cluster_barrier();
+        if (next_code == 0xffffu) break;
+        fresh = true;
+      }
+      ++p;
+    }
+    code = next_code;
+    t = tn;
+    sg = sn;
+    cur = nxt;
+  }
+  if (dead) {
+    st->sync_fault = 1;
+    st->done = 1;
+  }
+}
+
+}  // namespace gsb

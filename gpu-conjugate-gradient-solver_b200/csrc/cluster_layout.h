@@ -1,0 +1,214 @@
+// Host construction of the cluster-resident smoothing layout (cluster.cuh):
+// which CTA owns which rows, the slots of x each CTA keeps, the matrix in the
+// order its threads read it, and where every updated row is sent.
+#pragma once
+
+#include <algorithm>
+#include <vector>
+
+#include "cluster.cuh"
+#include "formats.cuh"
+
+namespace gsb {
+
+template <typename T>
+struct HostCluster {
+  int ncta = 0, ncolors = 0, g = 0, threads = 0, max_slots = 0, relaxed = 0;
+  std::vector<ClusterSeg> seg;
+  std::vector<unsigned> expect;
+  std::vector<int> slot_ptr, slot_row;
+  std::vector<T> val;                // two per pair
+  std::vector<unsigned short> col;   // two per pair
+  std::vector<unsigned> send;
+  std::vector<unsigned short> own;
+  std::vector<T> diag;               // {d, 1 / d} per row
+};
+
+// Rows [lo, hi) of colour piece q of ncta over [r0, r1).
+inline int cluster_cut(int r0, int r1, int q, int ncta) {
+  return r0 + static_cast<int>(static_cast<long long>(r1 - r0) * q / ncta);
+}
+
+// {d, 1 / d} of every row; the reciprocal is 0 where d or 1 / d is too close
+// to the ends of T's range for the kernel's quotient.
+template <typename T>
+void cluster_diag(const Csr &a, HostCluster<T> &h) {
+  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p60f);
+  h.diag.assign(2 * static_cast<size_t>(a.rows), T(0));
+  for (int r = 0; r < a.rows; ++r)
+    for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
+      if (a.ci[k] == r) {
+        const T d = T(a.v[k]);
+        h.diag[2 * static_cast<size_t>(r)] = d;
+        h.diag[2 * static_cast<size_t>(r) + 1] = std::fabs(d) < big && std::fabs(d) > T(1) / big ? T(1) / d : T(0);
+      }
+}
+
+// Layout of the square scalar matrix `a` (rows in colour-contiguous order,
+// colour c = rows [first[c], first[c + 1]), sorted columns) for ncta CTAs and
+// g lanes per row, with the k-th off-diagonal entry of a row on lane k % g as
+// the CSR-vector kernels read it. False when the level does not qualify: a
+// CTA needs more than `slot_limit` slots, a single colour, too many colours,
+// or a row is read by a row that its own owner does not read (the pattern is
+// not structurally symmetric; see the race argument in cluster.cuh).
+template <typename T>
+bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, int threads, bool relaxed,
+                  int slot_limit, HostCluster<T> &h) {
+  const int n = a.rows, nc = static_cast<int>(first.size()) - 1;
+  if (nc < 2 || nc > kClusterMaxColors || n < 1) return false;
+  const int limit = std::min(slot_limit, kClusterMaxSlots);
+  if (static_cast<long long>(n) > static_cast<long long>(limit) * ncta) return false;
+  h.ncta = ncta, h.ncolors = nc, h.g = g, h.threads = threads, h.relaxed = relaxed ? 1 : 0;
+  std::vector<unsigned char> owner(n);
+  std::vector<int> colour(n);
+  for (int c = 0; c < nc; ++c)
+    for (int q = 0; q < ncta; ++q)
+      for (int r = cluster_cut(first[c], first[c + 1], q, ncta); r < cluster_cut(first[c], first[c + 1], q + 1, ncta); ++r)
+        owner[r] = static_cast<unsigned char>(q), colour[r] = c;
+  // slots: the rows a CTA owns or reads, ascending
+  std::vector<std::vector<int>> rows_of(ncta);
+  std::vector<std::vector<unsigned short>> slot(ncta);
+  const unsigned short none = 0xffff;
+  std::vector<int> over(ncta, 0);
+  parallel_for(ncta, [&](long long q0, long long q1) {
+    for (long long q = q0; q < q1; ++q) {
+      std::vector<unsigned char> need(n, 0);
+      for (int c = 0; c < nc; ++c)
+        for (int r = cluster_cut(first[c], first[c + 1], q, ncta); r < cluster_cut(first[c], first[c + 1], q + 1, ncta); ++r) {
+          need[r] = 1;
+          for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) need[a.ci[k]] = 1;
+        }
+      slot[q].assign(n, none);
+      for (int r = 0; r < n; ++r)
+        if (need[r]) {
+          if (static_cast<int>(rows_of[q].size()) >= limit) {
+            over[q] = 1;
+            break;
+          }
+          slot[q][r] = static_cast<unsigned short>(rows_of[q].size());
+          rows_of[q].push_back(r);
+        }
+    }
+  }, 1);
+  for (int q = 0; q < ncta; ++q)
+    if (over[q]) return false;
+  h.max_slots = 0;
+  h.slot_ptr.assign(1, 0);
+  h.slot_row.clear();
+  for (int q = 0; q < ncta; ++q) {
+    h.max_slots = std::max(h.max_slots, static_cast<int>(rows_of[q].size()));
+    h.slot_row.insert(h.slot_row.end(), rows_of[q].begin(), rows_of[q].end());
+    h.slot_ptr.push_back(static_cast<int>(h.slot_row.size()));
+  }
+  const unsigned short zero_slot = static_cast<unsigned short>(h.max_slots);
+  h.own.resize(n);
+  for (int r = 0; r < n; ++r) h.own[r] = slot[owner[r]][r];
+  // pieces: sizes and offsets
+  const int groups = threads / g;
+  h.seg.assign(static_cast<size_t>(ncta) * nc, ClusterSeg{});
+  h.expect.assign(h.seg.size(), 0u);
+  std::vector<unsigned> dests(n, 0);  // CTAs that keep row r
+  for (int q = 0; q < ncta; ++q)
+    for (int r : rows_of[q]) dests[r] |= 1u << q;
+  long long pairs_total = 0, send_total = 0;
+  std::vector<int> ok(ncta, 1);
+  for (int q = 0; q < ncta; ++q)
+    for (int c = 0; c < nc; ++c) {
+      ClusterSeg &s = h.seg[static_cast<size_t>(q) * nc + c];
+      s.row0 = cluster_cut(first[c], first[c + 1], q, ncta);
+      s.rows = cluster_cut(first[c], first[c + 1], q + 1, ncta) - s.row0;
+      int len = 0, deg = 1;
+      for (int r = s.row0; r < s.row0 + s.rows; ++r) {
+        int off = 0;
+        for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) off += a.ci[k] != r ? 1 : 0;
+        len = std::max(len, off);
+        deg = std::max(deg, __builtin_popcount(dests[r]));
+      }
+      s.pairs = ((len + g - 1) / g + 1) / 2;
+      s.stride = std::min(threads, (s.rows * g + 31) / 32 * 32);
+      s.schunks = (deg + g - 1) / g;
+      const int trips = (s.rows + groups - 1) / groups;
+      s.trips = std::max(1, trips);
+      s.base = static_cast<int>(pairs_total);
+      s.sbase = static_cast<int>(send_total);
+      pairs_total += static_cast<long long>(trips) * s.pairs * s.stride;
+      send_total += static_cast<long long>(trips) * s.schunks * s.stride;
+      if (pairs_total > (1LL << 27) || send_total > (1LL << 28)) return false;  // 32-bit offsets in the kernel
+      // rows of colour c among CTA q's slots
+      const auto &rq = rows_of[q];
+      h.expect[static_cast<size_t>(q) * nc + c] = static_cast<unsigned>(std::lower_bound(rq.begin(), rq.end(), first[c + 1]) -
+                                       std::lower_bound(rq.begin(), rq.end(), first[c]));
+    }
+  h.val.assign(2 * static_cast<size_t>(pairs_total), T(0));
+  h.col.assign(2 * static_cast<size_t>(pairs_total), zero_slot);
+  h.send.assign(static_cast<size_t>(send_total), kNoSend);
+  parallel_for(ncta, [&](long long q0, long long q1) {
+    for (long long q = q0; q < q1; ++q)
+      for (int c = 0; c < nc; ++c) {
+        const ClusterSeg &s = h.seg[static_cast<size_t>(q) * nc + c];
+        for (int i = 0; i < s.rows; ++i) {
+          const int r = s.row0 + i, t = i / groups, lane0 = (i % groups) * g;
+          int k = 0;
+          for (int e = a.rp[r]; e < a.rp[r + 1]; ++e) {
+            const int j = a.ci[e];
+            if (j == r) continue;
+            const int lane = k % g, kk = k / g;
+            const size_t at = 2 * (static_cast<size_t>(s.base) + (static_cast<size_t>(t) * s.pairs + kk / 2) * s.stride +
+                                   lane0 + lane) + (kk & 1);
+            unsigned short sl = slot[q][j];
+            if (colour[j] == c) {
+              if (!relaxed) ok[q] = 0;  // two coupled rows of one colour
+              sl = static_cast<unsigned short>(sl + h.max_slots + 1);
+            }
+            if (slot[owner[j]][r] == none) ok[q] = 0;  // j's owner does not receive r
+            h.col[at] = sl;
+            h.val[at] = T(a.v[e]);
+            ++k;
+          }
+          int d = 0;
+          for (int to = 0; to < ncta; ++to) {
+            if ((dests[r] >> to & 1u) == 0) continue;
+            h.send[s.sbase + (static_cast<size_t>(t) * s.schunks + d / g) * s.stride + lane0 + d % g] =
+                static_cast<unsigned>(to) << 16 | slot[to][r];
+            ++d;
+          }
+        }
+      }
+  }, 1);
+  for (int q = 0; q < ncta; ++q)
+    if (!ok[q]) return false;
+  cluster_diag(a, h);
+  return true;
+}
+
+template <typename T>
+struct DevCluster {
+  int g = 0, ncta = 0, threads = 0, max_slots = 0;
+  T *val = nullptr, *diag = nullptr;  // what a value refresh overwrites
+  size_t values = 0;
+  ClusterView<T> v{};
+  size_t smem() const { return (static_cast<size_t>(max_slots) + 1) * sizeof(T) * (v.relaxed ? 2 : 1); }
+};
+
+template <typename T>
+DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h) {
+  DevCluster<T> d;
+  d.g = h.g, d.ncta = h.ncta, d.threads = h.threads, d.max_slots = h.max_slots;
+  d.values = h.val.size();
+  d.v.ncta = h.ncta, d.v.ncolors = h.ncolors, d.v.threads = h.threads, d.v.max_slots = h.max_slots;
+  d.v.relaxed = h.relaxed;
+  d.v.seg = ar.upload(h.seg);
+  d.v.expect = ar.upload(h.expect);
+  d.v.slot_ptr = ar.upload(h.slot_ptr);
+  d.v.slot_row = ar.upload(h.slot_row);
+  d.val = ar.upload(h.val);
+  d.v.val = reinterpret_cast<const typename Pair<T>::type *>(d.val);
+  d.v.col = reinterpret_cast<const unsigned *>(ar.upload(h.col));
+  d.v.send = ar.upload(h.send);
+  d.v.own = ar.upload(h.own);
+  d.diag = ar.upload(h.diag);
+  d.v.diag = reinterpret_cast<const typename Pair<T>::type *>(d.diag);
+  return d;
+}
+
+}  // namespace gsb

@@ -27,6 +27,7 @@
 #include <unordered_map>
 
 #include "amg_setup.h"
+#include "cluster_layout.h"
 #include "dense.h"
 #include "dense_mma.cuh"
 #include "formats.cuh"
@@ -353,6 +354,16 @@ void refresh_sell(const DevSell<T> &d, const Csr &a, const std::vector<int> &bou
 }
 
 template <typename T>
+void refresh_cluster(const DevCluster<T> &d, const Csr &a, const std::vector<int> &bounds) {
+  HostCluster<T> h;
+  if (!make_cluster<T>(a, bounds, d.g, d.ncta, d.threads, d.v.relaxed != 0, kClusterMaxSlots, h) ||
+      h.val.size() != d.values || h.max_slots != d.max_slots)
+    throw std::runtime_error("update_values: the matrix sparsity changed");
+  GSB_CK(cudaMemcpy(d.val, h.val.data(), sizeof(T) * h.val.size(), cudaMemcpyHostToDevice));
+  GSB_CK(cudaMemcpy(d.diag, h.diag.data(), sizeof(T) * h.diag.size(), cudaMemcpyHostToDevice));
+}
+
+template <typename T>
 void refresh_csrv(const DevCsrv<T> &d, const Csr &a, bool split_diag) {
   if (d.v == nullptr) return;
   std::vector<T> v, diag;
@@ -473,6 +484,8 @@ class AmgPcg final : public Solver {
     float *ainv_scale = nullptr;
     std::vector<VT *> wts;  // per colour: device pointer to the weight, or nullptr
     bool coop = false;      // symmetric sweeps as one cooperative launch (scalar SGS levels)
+    bool cluster = false;   // smoothing steps in one thread-block cluster (cluster.cuh), layout K
+    DevCluster<VT> K;
     // colouring of the strong couplings only (coloring 2): a pass reads its
     // own colour's neighbours from `xprev`, the iterate its sweep started with
     bool relaxed = false;
@@ -491,6 +504,18 @@ class AmgPcg final : public Solver {
   void gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaStream_t s);
   template <typename BT>
   void coop_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero, bool forward_only, cudaStream_t s);
+  template <typename BT>
+  void cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero, int dir, cudaStream_t s);
+  ClusterPasses cluster_passes(const Level &L, int steps, int dir) const {
+    return ClusterPasses{L.ncolors, steps, dir, skip_repeats(L) ? 1 : 0};
+  }
+  bool in_cluster(const Level &L, int steps, int dir) const {
+    return L.cluster && cluster_passes(L, steps, dir).total() <= kClusterMaxPasses;
+  }
+  int cluster_limit(bool relaxed);
+  int cluster_ctas(int g, size_t smem);
+  bool build_cluster(Level &L, int k, Arena &where);
+  void tune_cluster(Level &L, int k);
   // omega 1 and no learned weight: the update of a row does not depend on
   // its own value, so a colour pass repeated right after itself (where the
   // sweep turns) reproduces its input bit for bit and is skipped
@@ -869,7 +894,7 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
     info_[k].tail_ctas = info_[k].in_tail ? tail_cluster_ : 0;
     info_[k].lanes = lv_[k].g;
     info_[k].sliced = lv_[k].sliced ? 1 : 0;
-    info_[k].launch = lv_[k].coop ? 1 : (lv_[k].staged ? 2 : 0);
+    info_[k].launch = lv_[k].coop || lv_[k].cluster ? 1 : (lv_[k].staged ? 2 : 0);
     info_[k].p_lanes = lv_[k].pg;
     info_[k].r_lanes = lv_[k].rg;
   }
@@ -983,6 +1008,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
       refresh_sell(lv.A1, Ai, lv.color_first, true);
       if (lv.A.val != lv.A1.val) refresh_sell(lv.A, Ai, lv.color_first, true);
       refresh_csrv(lv.C, Ai, true);
+      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first);
       if (k == 0) refresh_sell(cgA_, Ai, lv.color_first, true);
       if (lv.kind == 2) {
         std::vector<VT> jd(Ai.rows, VT(0));
@@ -1217,8 +1243,12 @@ void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cu
     }
     return;
   }
+  if (dir == 2 && zero) throw std::runtime_error("smoother: a backward sweep from a zero iterate is not supported");
+  if (in_cluster(L, steps, dir)) {
+    cluster_sweep(L, rhs, x, steps, zero, dir, s);
+    return;
+  }
   if (dir != 0) {
-    if (zero && dir == 2) throw std::runtime_error("smoother: a backward sweep from a zero iterate is not supported");
     // one direction per step: consecutive passes never repeat a colour
     for (int step = 0; step < steps; ++step) {
       const bool zs = zero && step == 0 && dir == 1;
@@ -1322,9 +1352,101 @@ void AmgPcg<VT>::coop_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero
   CKL("cooperative Gauss-Seidel sweep");
 }
 
+// Lanes per row of the cluster layout's kernels.
+template <typename F>
+void with_lanes(int g, F &&f) {
+  switch (g) {
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    case 16: f(std::integral_constant<int, 16>()); break;
+    default: f(std::integral_constant<int, 32>()); break;
+  }
+}
+
+// Launch of one cluster of ncta CTAs, with programmatic stream serialization
+// when `overlap` (launch_pass).
+struct ClusterLaunch {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  ClusterLaunch(int ncta, int threads, size_t smem, bool overlap, cudaStream_t s) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ncta;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(ncta));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 2 : 1;
+  }
+  ClusterLaunch(const ClusterLaunch &) = delete;
+};
+
+// Smoothing steps of a level in one cluster (cluster.cuh); the same iterate
+// as the per-colour passes with the same lanes per row, bit for bit.
+template <typename VT>
+template <typename BT>
+void AmgPcg<VT>::cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero, int dir, cudaStream_t s) {
+  ClusterLaunch l(L.K.ncta, L.K.threads, L.K.smem(), pdl_, s);
+  const VT *w = L.wts.empty() ? nullptr : L.wts[0];
+  with_lanes(L.K.g, [&](auto G) {
+    CK(cudaLaunchKernelEx(&l.cfg, cluster_gs_kernel<VT, BT, decltype(G)::value>, L.K.v, cluster_passes(L, steps, dir),
+                          rhs, x, zero ? 1 : 0, w, VT(opt_.omega), st_));
+  });
+  CKL("cluster Gauss-Seidel step");
+}
+
+// Slots of x that one CTA's shared memory holds.
+template <typename VT>
+int AmgPcg<VT>::cluster_limit(bool relaxed) {
+  int optin = 0;
+  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+  cudaFuncAttributes fa{};
+  CK(cudaFuncGetAttributes(&fa, cluster_gs_kernel<VT, VT, 8>));
+  const long long bytes = optin - static_cast<long long>(fa.sharedSizeBytes) - 1024;
+  return static_cast<int>(std::min<long long>(kClusterMaxSlots, bytes / static_cast<long long>(sizeof(VT) * (relaxed ? 2 : 1)) - 1));
+}
+
+// Largest cluster (16 or 8 CTAs) the device co-schedules with `smem` bytes per
+// CTA, or 0. Raises the kernels' shared memory limit to the device's maximum
+// (a limit only, the same for every solver of the process).
+template <typename VT>
+int AmgPcg<VT>::cluster_ctas(int g, size_t smem) {
+  int best = 0;
+  with_lanes(g, [&](auto G) {
+    auto setup = [&](auto kernel) {
+      int optin = 0;
+      CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
+      cudaFuncAttributes fa{};
+      CK(cudaFuncGetAttributes(&fa, kernel));
+      const int most = optin - static_cast<int>(fa.sharedSizeBytes);
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
+      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+      if (smem > static_cast<size_t>(most)) return 0;
+      for (int want : {16, 8}) {
+        ClusterLaunch l(want, kClusterThreads, smem, false, nullptr);
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) return want;
+        cudaGetLastError();
+      }
+      return 0;
+    };
+    best = std::min(setup(cluster_gs_kernel<VT, VT, decltype(G)::value>),
+                    setup(cluster_gs_kernel<VT, double, decltype(G)::value>));
+  });
+  return best;
+}
+
 // One forward sweep over all colours of a level (the timing helpers).
 template <typename VT>
 void AmgPcg<VT>::forward_sweep(Level &L, cudaStream_t s) {
+  if (in_cluster(L, 1, 1)) {
+    cluster_sweep<VT>(L, L.b, L.x, 1, false, 1, s);
+    return;
+  }
   if (L.coop && L.kind == 0 && !block_ && !L.relaxed) {
     coop_sweep<VT>(L, L.b, L.x, 1, false, true, s);
     return;
@@ -1548,7 +1670,7 @@ void AmgPcg<VT>::set_layout(Level &L, int k, bool sliced, int g, Arena &where) {
 template <typename VT>
 void AmgPcg<VT>::autotune() {
   static const int cands[] = {1, 4, 8, 16, 32};
-  const std::string sig = "v4:" + signature();
+  const std::string sig = "v5:" + signature();
   if (!opt_.tune_cache.empty()) {
     std::ifstream in(opt_.tune_cache);
     std::string key, line;
@@ -1556,17 +1678,19 @@ void AmgPcg<VT>::autotune() {
       std::istringstream ls(line);
       ls >> key;
       if (key != sig) continue;
-      std::vector<int> v(6 * lv_.size() + 1);
+      std::vector<int> v(7 * lv_.size() + 1);
       for (int &t : v) ls >> t;
       if (!ls) continue;
       set_outer_lanes(v.back());
       for (size_t k = 0; k < lv_.size(); ++k) {
         Level &L = lv_[k];
-        L.rg = v[6 * k + 2];
-        L.pg = v[6 * k + 3];
-        set_layout(L, static_cast<int>(k), v[6 * k] != 0, v[6 * k + 1], ar_);
-        L.coop = v[6 * k + 4] != 0 && opt_.sweep_launch != 0 && !L.relaxed && !opt_.half_sweeps;
-        L.staged = v[6 * k + 5] != 0 && opt_.sweep_launch != 0 && block_ && L.sliced && L.g == 1 &&
+        L.rg = v[7 * k + 2];
+        L.pg = v[7 * k + 3];
+        set_layout(L, static_cast<int>(k), v[7 * k] != 0, v[7 * k + 1], ar_);
+        L.coop = v[7 * k + 4] != 0 && opt_.sweep_launch != 0 && !L.relaxed && !opt_.half_sweeps;
+        L.cluster = v[7 * k + 6] != 0 && opt_.sweep_launch == 1 && L.kind == 0 && !block_ &&
+                    build_cluster(L, static_cast<int>(k), ar_);
+        L.staged = v[7 * k + 5] != 0 && opt_.sweep_launch != 0 && block_ && L.sliced && L.g == 1 &&
                    prepare_staged<VT>(L.B.max_slots, device_);
       }
       return;
@@ -1656,6 +1780,7 @@ void AmgPcg<VT>::autotune() {
         }
         L.coop = t_coop < t_pass;
       }
+      if (L.kind == 0 && !block_ && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k));
     }
     if (k + 1 < lv_.size()) {
       Level &Cn = lv_[k + 1];
@@ -1683,9 +1808,61 @@ void AmgPcg<VT>::autotune() {
     out << sig;
     for (const Level &L : lv_)
       out << " " << (L.sliced ? 1 : 0) << " " << L.g << " " << L.rg << " " << L.pg << " " << (L.coop ? 1 : 0) << " "
-          << (L.staged ? 1 : 0);
+          << (L.staged ? 1 : 0) << " " << (L.cluster ? 1 : 0);
     out << " " << (block_ ? cgB_.g : 1) << "\n";
   }
+}
+
+// Entries per colour pass up to which a level is tried in one cluster, and
+// the lanes per row there. One cluster's 16 SMs beat a launch per pass while a
+// pass is latency: FP64 symmetric steps, cluster / launches: 9.8 k entries a
+// pass (5,103 rows, 37 colours) 86 / 183 us, 8.2 k (4,143, 23) 53 / 108,
+// 13.5 k (4,096, 2) 7.7 / 9.4; above, the 16 SMs' gathers bound it: 58 k
+// (32,768, 8) 58 / 37, 66 k (37,505, 18) 120 / 95. About five entries a lane:
+// fewer lanes leave the loaded-ahead slots (5,103 rows, 70 entries a row: 125
+// us with 8 lanes, 86 with 16, 90 with 32).
+constexpr long long kClusterPassEntries = 40000;
+inline int cluster_lanes(const Csr &a) {
+  const double len = static_cast<double>(a.nnz()) / std::max(1, a.rows) - 1.0;
+  int g = 4;
+  while (g < 32 && g * 5.0 < len) g *= 2;
+  return g;
+}
+
+// The cluster layout of level k (cluster_layout.h), built into `where`; false
+// when the level or the device does not qualify.
+template <typename VT>
+bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
+  const Csr &a = host_A_.at(k);
+  const int g = cluster_lanes(a), ncta = cluster_ctas(g, 0);
+  HostCluster<VT> h;
+  if (ncta == 0 || !make_cluster<VT>(a, L.color_first, g, ncta, kClusterThreads, L.relaxed, cluster_limit(L.relaxed), h))
+    return false;
+  L.K = upload_cluster<VT>(where, h);
+  return cluster_ctas(g, L.K.smem()) >= ncta;
+}
+
+// One smoothing step of the level as the solve runs it, per-colour (or
+// cooperative) launches against one cluster; the faster is kept.
+template <typename VT>
+void AmgPcg<VT>::tune_cluster(Level &L, int k) {
+  L.cluster = false;
+  if (host_A_.at(k).nnz() > kClusterPassEntries * L.ncolors) return;
+  auto step = [&] {
+    if (opt_.half_sweeps) {
+      smooth<VT>(L, L.b, L.x, 1, true, stream_, 1);
+      smooth<VT>(L, L.b, L.x, 1, false, stream_, 2);
+    } else {
+      smooth<VT>(L, L.b, L.x, 1, false, stream_);
+    }
+  };
+  std::unique_ptr<Arena> arena(new Arena);
+  if (!build_cluster(L, k, *arena)) return;
+  const float t_pass = time_segment(step, 10, 2);
+  L.cluster = true;
+  L.cluster = time_segment(step, 10, 2) < t_pass;
+  CK(cudaStreamSynchronize(stream_));
+  if (L.cluster) kept_layouts_.push_back(std::move(arena));
 }
 
 template <typename VT>
@@ -2163,12 +2340,13 @@ double AmgPcg<VT>::time_level(int level, int op, int lanes, int reps, cudaStream
   Level &L = lv_[level];
   Level &C = lv_[level + 1];
   const int sg = L.g, spg = L.pg, srg = L.rg;
-  const bool ssl = L.sliced, scoop = L.coop, sstaged = L.staged;
+  const bool ssl = L.sliced, scoop = L.coop, sstaged = L.staged, scluster = L.cluster;
   const DevSell<VT> sA = L.A;
   const DevBell<VT> sB = L.B;
   const std::vector<int> scs = L.color_slice;
   auto restore = [&] {
     L.g = sg, L.pg = spg, L.rg = srg, L.sliced = ssl, L.A = sA, L.B = sB, L.coop = scoop, L.staged = sstaged;
+    L.cluster = scluster;
     if (L.color_slice != scs) {
       L.color_slice = scs;
       CK(cudaMemcpy(L.d_color_slice, scs.data(), sizeof(int) * scs.size(), cudaMemcpyHostToDevice));
@@ -2177,6 +2355,7 @@ double AmgPcg<VT>::time_level(int level, int op, int lanes, int reps, cudaStream
   if (lanes != 0) {
     if (op <= 1) {
       L.coop = false;  // a forced layout runs its per-colour passes
+      L.cluster = false;
       L.staged = false;
       L.sliced = lanes == 1;
       L.g = lanes;

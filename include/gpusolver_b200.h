@@ -274,8 +274,9 @@ typedef struct {
                          level 1) */
   int sweep_launch;   /* symmetric Gauss-Seidel steps of a scalar level: 0 one launch per
                          colour pass (the reference's structure); 1 (default) one cooperative
-                         launch per smoothing step, grid barriers between colours, where timed
-                         faster at setup; 2 cooperative on every such level. Colour passes of
+                         launch per smoothing step (grid barriers between colours, or one
+                         thread-block cluster) where timed faster at setup; 2 cooperative with
+                         grid barriers on every such level. Colour passes of
                          a 3x3 block level in the BELL-1 layout: 1 with each slice's blocks
                          bulk-copied to shared memory where timed faster, 2 on every such
                          level whose widest slice fits, 0 never. Same iterates bit for bit
@@ -341,8 +342,8 @@ int gs_solver_level_in_tail(const gs_solver *s, int level);
  * `lanes` lanes per row; -1 on a bad argument. No reference counterpart. */
 int gs_solver_level_layout(const gs_solver *s, int level);
 /* How `level`'s colour passes are launched: 0 one kernel per colour pass,
- * 1 one cooperative kernel per smoothing step (grid barriers between the
- * colours), 2 one kernel per colour pass that bulk-copies each BELL-1
+ * 1 one kernel per smoothing step (grid barriers between the colours, or one
+ * thread-block cluster), 2 one kernel per colour pass that bulk-copies each BELL-1
  * slice's blocks to shared memory (gs_solver_options.sweep_launch chooses);
  * -1 on a bad argument. No reference counterpart. */
 int gs_solver_level_launch(const gs_solver *s, int level);
