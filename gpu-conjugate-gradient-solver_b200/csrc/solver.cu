@@ -1024,6 +1024,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
   }
   features_ = features;
   node_features_ = node_features;
+  CK(cudaDeviceSynchronize());  // the new values have landed before the next solve reads them
 }
 
 template <typename VT>
@@ -1971,6 +1972,11 @@ void AmgPcg<VT>::upload_tail_table(int k0) {
 // in graph mode, launched on the stream otherwise.
 template <typename VT>
 float AmgPcg<VT>::time_segment(const std::function<void()> &f, int reps, int trials) {
+  // A pass reads its matrix before it waits on the launch ahead of it: the
+  // uploads of a new layout have landed, and the first launch follows an
+  // operation of the stream that is not a kernel, so it starts in plain order
+  CK(cudaDeviceSynchronize());
+  CK(cudaMemsetAsync(sync_, 0, sizeof(SweepSync), stream_));
   if (!opt_.graph) {
     float t = time_ms(f, reps);
     for (int i = 1; i < trials; ++i) t = std::min(t, time_ms(f, reps));
