@@ -32,9 +32,8 @@ namespace {
 
 #define BCK(x) cuda_check((x), #x)
 
-constexpr int kSellItemSlices = 8;  // GS / SpMV items: one slice per warp of a 256-thread block
+constexpr int kSellItemSlices = 8;  // GS / SpMV items: one slice per warp of a 256-thread block (CSR-vector: 256 / G rows)
 constexpr int kCgItemSlices = 32;   // CG items: up to 1024 rows, one partial sum each
-constexpr int kCsrvTrips = 1;       // CSR-vector items: 256 / G rows, one trip (coarse passes are latency-bound)
 constexpr int kDenseItemRows = 32;  // coarsest-level items: 32 rows of one system
 
 // Rows [r0, r1) of one system on one batch level; c0 = first row of their colour.
@@ -245,7 +244,7 @@ void row_items(const std::vector<Seg> &segs, int per, std::vector<BItem> &out) {
 
 void items_for(const std::vector<Seg> &segs, int g, const std::vector<int> &srow, std::vector<BItem> &out) {
   if (g == 1) sell_items(segs, srow, kSellItemSlices, out);
-  else row_items(segs, (256 / g) * kCsrvTrips, out);
+  else row_items(segs, 256 / g, out);
 }
 
 // Block-diagonal concatenation: part i occupies rows [roff[i], ...) and its
@@ -378,6 +377,7 @@ class Batch final : public BatchSolver {
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaGraph_t graph_[2] = {nullptr, nullptr};
   cudaGraphExec_t exec_[2] = {nullptr, nullptr};
+  bool pdl_ = true;  // programmatic stream serialization (SolverOptions::overlap_launch)
   long long launches_ = 0, graph_kernels_ = 0;
 };
 
@@ -398,6 +398,7 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
   if (opt.lanes != 0 && opt.lanes != 1 && opt.lanes != 2 && opt.lanes != 4 && opt.lanes != 8 && opt.lanes != 16 &&
       opt.lanes != 32)
     throw std::runtime_error("lanes must be 1, 2, 4, 8, 16 or 32");
+  pdl_ = opt.overlap_launch >= 1;
   S_ = static_cast<int>(h.size());
   nrhs_ = nrhs;
   BCK(cudaSetDevice(device_));
@@ -547,12 +548,14 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
     cg_range_ = Range{0, static_cast<int>(cgi.size())};
   }
 
+  BCK(cudaDeviceSynchronize());  // uploads precede the kernels of stream_
   if (opt_.lanes > 0) {
     for (BLevel &L : lv_) L.g = L.pg = L.rg = opt_.lanes;
   } else if (opt_.autotune) {
     autotune();
   }
   build_items();
+  BCK(cudaDeviceSynchronize());  // every upload has landed
   for (int k = 0; k < K_; ++k) {
     info_[k].lanes = lv_[k].g;
     info_[k].p_lanes = lv_[k].pg;
@@ -625,13 +628,13 @@ void Batch<VT, R>::gs_pass(const BLevel &L, const BItem *it, int cnt, const Rv<B
   const VT w = VT(opt_.omega);
   const int gb = grid(cnt);
   if (L.g == 1) {
-    if (zero) bsell_gs_kernel<VT, BT, R, true><<<gb, 256, 0, s>>>(L.A.view(), it, cnt, b, x, w, sys_done_);
-    else bsell_gs_kernel<VT, BT, R, false><<<gb, 256, 0, s>>>(L.A.view(), it, cnt, b, x, w, sys_done_);
+    if (zero) launch_pass(pdl_, bsell_gs_kernel<VT, BT, R, true>, gb, s, L.A.view(), it, cnt, b, x, w, sys_done_);
+    else launch_pass(pdl_, bsell_gs_kernel<VT, BT, R, false>, gb, s, L.A.view(), it, cnt, b, x, w, sys_done_);
   } else {
     const CsrvView<VT> v = L.C.view();
 #define BGS(G)                                                                                       \
-  if (zero) bcsrv_gs_kernel<VT, BT, R, true, G><<<gb, 256, 0, s>>>(v, it, cnt, b, x, w, sys_done_);  \
-  else bcsrv_gs_kernel<VT, BT, R, false, G><<<gb, 256, 0, s>>>(v, it, cnt, b, x, w, sys_done_);
+  if (zero) launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, true, G>, gb, s, v, it, cnt, b, x, w, sys_done_);  \
+  else launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, false, G>, gb, s, v, it, cnt, b, x, w, sys_done_);
     switch (L.g) {
       case 2: BGS(2) break;
       case 4: BGS(4) break;
@@ -651,15 +654,15 @@ void Batch<VT, R>::spmv(const DevSell<VT> &Sm, const DevCsrv<VT> &Cm, int g, con
   if (cnt <= 0) return;
   const int gb = grid(cnt);
   if (g == 1) {
-    bsell_spmv_kernel<VT, BT, R, kMode><<<gb, 256, 0, s>>>(Sm.view(), it, cnt, x, y, b, sys_done_);
+    launch_pass(pdl_, bsell_spmv_kernel<VT, BT, R, kMode>, gb, s, Sm.view(), it, cnt, x, y, b, sys_done_);
   } else {
     const CsrvView<VT> v = Cm.view();
     switch (g) {
-      case 2: bcsrv_spmv_kernel<VT, BT, R, kMode, 2><<<gb, 256, 0, s>>>(v, it, cnt, x, y, b, sys_done_); break;
-      case 4: bcsrv_spmv_kernel<VT, BT, R, kMode, 4><<<gb, 256, 0, s>>>(v, it, cnt, x, y, b, sys_done_); break;
-      case 8: bcsrv_spmv_kernel<VT, BT, R, kMode, 8><<<gb, 256, 0, s>>>(v, it, cnt, x, y, b, sys_done_); break;
-      case 16: bcsrv_spmv_kernel<VT, BT, R, kMode, 16><<<gb, 256, 0, s>>>(v, it, cnt, x, y, b, sys_done_); break;
-      default: bcsrv_spmv_kernel<VT, BT, R, kMode, 32><<<gb, 256, 0, s>>>(v, it, cnt, x, y, b, sys_done_); break;
+      case 2: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 2>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 4: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 4>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 8: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 8>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 16: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 16>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      default: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 32>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
     }
   }
   BKL("batched spmv");
@@ -667,14 +670,22 @@ void Batch<VT, R>::spmv(const DevSell<VT> &Sm, const DevCsrv<VT> &Cm, int g, con
 
 // SymmetricGaussSeidelSmoother::smooth on every smoothed system of level k:
 // forward pass j is colour j of each system, backward pass j its colour
-// C_s - 1 - j.
+// C_s - 1 - j. With omega 1 a row's update does not depend on its own value,
+// so the pass repeated where a sweep turns -- backward pass 0 (every system's
+// last colour, updated last by the forward sweep) and forward pass 0 of a
+// further step (colour 0, updated last by the backward sweep) -- reproduces
+// its input bit for bit and is not launched: 3 instead of 4 passes on a
+// two-colour level.
 template <typename VT, int R>
 template <typename BT>
 void Batch<VT, R>::smooth(int k, const Rv<BT, R> *b, RV *x, int steps, bool zero, cudaStream_t s) {
   const BLevel &L = lv_[k];
+  const bool skip = VT(opt_.omega) == VT(1);
   for (int step = 0; step < steps; ++step) {
-    for (const Range &r : L.fwd) gs_pass<BT>(L, items_ + r.off, r.count, b, x, zero && step == 0, s);
-    for (const Range &r : L.bwd) gs_pass<BT>(L, items_ + r.off, r.count, b, x, false, s);
+    for (size_t j = skip && step > 0 ? 1 : 0; j < L.fwd.size(); ++j)
+      gs_pass<BT>(L, items_ + L.fwd[j].off, L.fwd[j].count, b, x, zero && step == 0, s);
+    for (size_t j = skip ? 1 : 0; j < L.bwd.size(); ++j)
+      gs_pass<BT>(L, items_ + L.bwd[j].off, L.bwd[j].count, b, x, false, s);
   }
 }
 
@@ -692,7 +703,7 @@ void Batch<VT, R>::vcycle(const RD *r0, RV *z, bool zero0, cudaStream_t s) {
     spmv<kSpmvSet, VT>(L.Rs, L.Rc, L.rg, items_ + L.below_r.off, L.below_r.count, L.r, lv_[k + 1].b,
                        static_cast<const RV *>(nullptr), s);
   }
-  bdense_kernel<VT, R><<<grid(dense_range_.count), 256, 0, s>>>(items_ + dense_range_.off, dense_range_.count,
+  launch_pass(pdl_, bdense_kernel<VT, R>, grid(dense_range_.count), s, items_ + dense_range_.off, dense_range_.count,
                                                                  ainv_, ainv_off_, crow0_, cn_, xl_, bl_,
                                                                  sys_done_);
   BKL("batched coarsest solve");
@@ -749,7 +760,11 @@ float Batch<VT, R>::time_level_op(int k, int op, int g, int reps) {
     BCK(cudaMalloc(&tmp_, sizeof(BItem) * v.size()));
     tmp_cap_ = v.size();
   }
-  if (!v.empty()) BCK(cudaMemcpy(tmp_, v.data(), sizeof(BItem) * v.size(), cudaMemcpyHostToDevice));
+  // in stream order: the passes read their items before they wait on the
+  // launch ahead of them, so the copy has to be a predecessor of the first one
+  // (a plain cudaMemcpy may return with its last bytes still on their way)
+  if (!v.empty())
+    BCK(cudaMemcpyAsync(tmp_, v.data(), sizeof(BItem) * v.size(), cudaMemcpyHostToDevice, stream_));
   const int c = static_cast<int>(v.size());
   const int saved_g = L.g;
   L.g = g;
@@ -834,21 +849,21 @@ void Batch<VT, R>::cg_iteration(int parity, cudaStream_t s) {
   RV *z_old = z_[parity], *z_new = z_[parity ^ 1];
   const BItem *ci = items_ + cg_range_.off;
   const int nc = cg_range_.count, gb = grid(nc);
-  bcg_spmv_pap_kernel<R><<<gb, 256, 0, s>>>(cgA_.view(), ci, nc, p_, ap_, sys_done_, partials_);
+  launch_pass(pdl_, bcg_spmv_pap_kernel<R>, gb, s, cgA_.view(), ci, nc, p_, ap_, sys_done_, partials_);
   BKL("batched cg spmv");
   bcg_finalize_kernel<R, kBFinPap><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
   BKL("batched cg alpha");
-  bcg_update_xr_kernel<R><<<gb, 256, 0, s>>>(cgA_.srow, ci, nc, x_, r_, p_, ap_, pairs_, sys_done_, partials_);
+  launch_pass(pdl_, bcg_update_xr_kernel<R>, gb, s, cgA_.srow, ci, nc, x_, r_, p_, ap_, pairs_, sys_done_, partials_);
   BKL("batched cg update");
   bcg_finalize_kernel<R, kBFinXr><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
   BKL("batched cg convergence");
   precondition(r_, z_new, s);
-  bcg_dot_rz_kernel<VT, R><<<gb, 256, 0, s>>>(cgA_.srow, ci, nc, r_, z_new, opt_.flexible ? z_old : nullptr,
+  launch_pass(pdl_, bcg_dot_rz_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, r_, z_new, opt_.flexible ? z_old : nullptr,
                                               sys_done_, partials_);
   BKL("batched cg dot");
   bcg_finalize_kernel<R, kBFinRz><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
   BKL("batched cg beta");
-  bcg_update_p_kernel<VT, R><<<gb, 256, 0, s>>>(cgA_.srow, ci, nc, z_new, p_, pairs_, sys_done_);
+  launch_pass(pdl_, bcg_update_p_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, z_new, p_, pairs_, sys_done_);
   BKL("batched cg p update");
 }
 
@@ -879,9 +894,12 @@ void Batch<VT, R>::ensure_graphs() {
   if (exec_[0] != nullptr) return;
   for (int par = 0; par < 2; ++par) {
     const long long before = launches_;
+    const bool eager = pdl_;
+    pdl_ = opt_.overlap_launch == 2;  // programmatic edges inside the graph
     BCK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
     cg_iteration(par, stream_);
     BCK(cudaStreamEndCapture(stream_, &graph_[par]));
+    pdl_ = eager;
     BCK(cudaGraphInstantiate(&exec_[par], graph_[par], 0));
     graph_kernels_ = launches_ - before;
     launches_ = before;  // captured, not executed
