@@ -146,14 +146,14 @@ __global__ void __launch_bounds__(256) bsell_gs_kernel(SellView<T> A, const BIte
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   BItem q = __ldg(items + blockIdx.x);
   SellHead<T> h;
-  if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h);
+  if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
   bpass_entry();
   b = after_wait(b);
   x = after_wait(x);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     if (it != static_cast<int>(blockIdx.x)) {
       q = __ldg(items + it);
-      if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h);
+      if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
     }
     if (item_skipped(sys_done, q.x) || q.y + warp >= q.z) continue;
     const int row = h.r0 + lane;

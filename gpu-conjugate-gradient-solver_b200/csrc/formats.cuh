@@ -56,6 +56,7 @@ template <typename T>
 struct HostSell {
   int rows = 0, cols = 0, g = 1;
   std::vector<int> srow, sptr, col;
+  std::vector<int> first, lo, up;  // colour split of each slice (square level matrices)
   std::vector<T> val, diag;
 };
 
@@ -72,7 +73,10 @@ HostSell<T> make_sell(const Csr &a, const std::vector<int> &bounds, bool split_d
   h.g = g;
   const int per = 32 / g;
   for (size_t b = 0; b + 1 < bounds.size(); ++b)
-    for (int r = bounds[b]; r < bounds[b + 1]; r += per) h.srow.push_back(r);
+    for (int r = bounds[b]; r < bounds[b + 1]; r += per) {
+      h.srow.push_back(r);
+      if (split_diag) h.first.push_back(bounds[b]);
+    }
   h.srow.push_back(a.rows);
   const int ns = static_cast<int>(h.srow.size()) - 1;
   std::vector<int> width(ns, 0);  // slots per lane, even
@@ -96,7 +100,11 @@ HostSell<T> make_sell(const Csr &a, const std::vector<int> &bounds, bool split_d
   }
   h.col.assign(h.sptr[ns], 0);
   h.val.assign(h.sptr[ns], T(0));
-  if (split_diag) h.diag.assign(a.rows, T(0));
+  if (split_diag) {
+    h.diag.assign(a.rows, T(0));
+    h.lo.assign(h.sptr.begin(), h.sptr.end() - 1);
+    h.up.assign(h.sptr.begin() + 1, h.sptr.end());
+  }
   parallel_for(ns, [&](long long s0, long long s1) {
     for (long long s = s0; s < s1; ++s) {
       // Padding gathers x[pad] * 0. Square level matrices pad with the slice's
@@ -123,6 +131,11 @@ HostSell<T> make_sell(const Csr &a, const std::vector<int> &bounds, bool split_d
           const int idx = h.sptr[s] + (kk >> 1) * 64 + 2 * lane + (kk & 1);
           h.col[idx] = a.ci[e];
           h.val[idx] = T(a.v[e]);
+          if (split_diag) {
+            const int pair = h.sptr[s] + (kk >> 1) * 64;
+            if (a.ci[e] < h.first[s]) h.lo[s] = std::max(h.lo[s], pair + 64);
+            else h.up[s] = std::min(h.up[s], pair);
+          }
           ++k;
         }
       }
@@ -136,9 +149,14 @@ struct DevSell {
   int rows = 0, cols = 0, nslices = 0, g = 1;
   long long stored = 0;
   int *srow = nullptr, *sptr = nullptr, *col = nullptr;
+  int *first = nullptr, *lo = nullptr, *up = nullptr;
   T *val = nullptr, *diag = nullptr;
   std::vector<int> h_srow;  // slice -> first row, kept on the host for launch ranges
-  SellView<T> view() const { return SellView<T>{rows, cols, nslices, srow, sptr, col, val, diag}; }
+  SellView<T> view() const { return SellView<T>{rows, cols, nslices, srow, sptr, col, val, diag, first, lo, up}; }
+  // slice that starts at `row` (a bound of the layout)
+  int slice_of(int row) const {
+    return static_cast<int>(std::lower_bound(h_srow.begin(), h_srow.end(), row) - h_srow.begin());
+  }
 };
 
 template <typename T>
@@ -154,6 +172,11 @@ DevSell<T> upload_sell(Arena &ar, const HostSell<T> &h) {
   d.col = ar.upload(h.col);
   d.val = ar.upload(h.val);
   d.diag = h.diag.empty() ? nullptr : ar.upload(h.diag);
+  if (!h.first.empty()) {
+    d.first = ar.upload(h.first);
+    d.lo = ar.upload(h.lo);
+    d.up = ar.upload(h.up);
+  }
   d.h_srow = h.srow;
   return d;
 }
@@ -162,14 +185,18 @@ template <typename T>
 struct DevCsrv {
   int rows = 0;
   int *rp = nullptr, *ci = nullptr;
+  int *mid = nullptr;  // first entry of each row whose column is at or past the row's cut, or nullptr
   T *v = nullptr, *diag = nullptr;
-  CsrvView<T> view() const { return CsrvView<T>{rows, rp, ci, v, diag}; }
+  CsrvView<T> view() const { return CsrvView<T>{rows, rp, ci, v, diag, rp + 1}; }
+  CsrvView<T> below() const { return CsrvView<T>{rows, rp, ci, v, diag, mid}; }    // columns below the cut
+  CsrvView<T> past() const { return CsrvView<T>{rows, mid, ci, v, nullptr, rp + 1}; }  // the rest, no diagonal
 };
 
 // CSR with the diagonal split off (square level matrices) or kept (transfer
-// operators), columns in stored order.
+// operators), columns in stored order. `cut`: the column at which row r's
+// entries are divided (ascending columns), or nullptr.
 template <typename T>
-DevCsrv<T> upload_csrv(Arena &ar, const Csr &a, bool split_diag) {
+DevCsrv<T> upload_csrv(Arena &ar, const Csr &a, bool split_diag, const std::vector<int> *cut = nullptr) {
   std::vector<int> rp(a.rows + 1, 0);
   std::vector<T> diag;
   if (split_diag) diag.assign(a.rows, T(0));
@@ -179,7 +206,8 @@ DevCsrv<T> upload_csrv(Arena &ar, const Csr &a, bool split_diag) {
       for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) c -= a.ci[k] == r ? 1 : 0;
     rp[r + 1] = rp[r] + c;
   }
-  std::vector<int> ci(rp[a.rows]);
+  std::vector<int> ci(rp[a.rows]), mid;
+  if (cut != nullptr) mid.resize(a.rows);
   std::vector<T> v(rp[a.rows]);
   parallel_for(a.rows, [&](long long r0, long long r1) {
     for (long long r = r0; r < r1; ++r) {
@@ -193,6 +221,8 @@ DevCsrv<T> upload_csrv(Arena &ar, const Csr &a, bool split_diag) {
         v[dst] = T(a.v[k]);
         ++dst;
       }
+      if (cut != nullptr)
+        mid[r] = static_cast<int>(std::lower_bound(ci.begin() + rp[r], ci.begin() + dst, (*cut)[r]) - ci.begin());
     }
   }, row_grain(a.rows, a.nnz()));
   DevCsrv<T> d;
@@ -201,6 +231,7 @@ DevCsrv<T> upload_csrv(Arena &ar, const Csr &a, bool split_diag) {
   d.ci = ar.upload(ci);
   d.v = ar.upload(v);
   d.diag = split_diag ? ar.upload(diag) : nullptr;
+  if (cut != nullptr) d.mid = ar.upload(mid);
   return d;
 }
 

@@ -33,6 +33,13 @@ struct SellView {
   const int *__restrict__ col;
   const T *__restrict__ val;
   const T *__restrict__ diag;    // rows, or nullptr (transfer operators)
+  // Colour split of a level's slices, or nullptr: first row of the slice's
+  // colour, end of the slot pairs that hold a column below it, start of those
+  // that hold one at or past it (a row's columns ascend, so these are a prefix
+  // and a suffix of its slots, cut at the slice's widest and narrowest lane).
+  const int *__restrict__ first;
+  const int *__restrict__ lo;
+  const int *__restrict__ up;
 };
 
 template <typename T>
@@ -44,6 +51,9 @@ struct BellView {
   const T *__restrict__ val;     // 9 per block slot, component-major per slice
   const T *__restrict__ diag;    // 9 per node
   const T *__restrict__ dinv;    // 9 per node
+  const int *__restrict__ first; // colour split, as SellView (block slots)
+  const int *__restrict__ lo;
+  const int *__restrict__ up;
 };
 
 // State of one preconditioned CG solve, resident on the device. Scalars are
@@ -68,7 +78,9 @@ enum CgStatus : int {
 
 // kSpmvTwice writes y = (A x) + (A x): the reference's prolongation on a
 // level below the finest, whose correction buffer is the solution itself.
-enum SpmvMode : int { kSpmvSet = 0, kSpmvResid = 1, kSpmvAdd = 2, kSpmvTwice = 3 };
+// kSpmvNeg writes y = -A x: the residual of a level right after one forward
+// sweep from zero, with A the entries that the sweep had not used (below).
+enum SpmvMode : int { kSpmvSet = 0, kSpmvResid = 1, kSpmvAdd = 2, kSpmvTwice = 3, kSpmvNeg = 4 };
 
 template <typename T> struct Pair;
 template <> struct Pair<double> { using type = double2; };
@@ -126,14 +138,17 @@ struct SellHead {
   int2 c[kPairs];
 };
 
-// Loads the head of slice s (bounds and the lane's first slot pairs).
+// Loads the head of slice s (bounds and the lane's first slot pairs). `zero`:
+// for a sweep from a zero iterate, which uses only the slots that hold a
+// column below the slice's colour (none in the first colour).
 template <typename T>
-__device__ __forceinline__ void sell_head_ops(const SellView<T> &A, int s, int lane, SellHead<T> &h) {
+__device__ __forceinline__ void sell_head_ops(const SellView<T> &A, int s, int lane, SellHead<T> &h,
+                                              bool zero = false) {
   using P2 = typename Pair<T>::type;
   h.r0 = __ldg(A.srow + s);
   h.r1 = __ldg(A.srow + s + 1);
   h.p0 = __ldg(A.sptr + s);
-  h.p1 = __ldg(A.sptr + s + 1);
+  h.p1 = zero && A.lo != nullptr ? __ldg(A.lo + s) : __ldg(A.sptr + s + 1);
 #pragma unroll
   for (int q = 0; q < SellHead<T>::kPairs; ++q) {
     const int p = h.p0 + 2 * lane + 64 * q;
@@ -150,8 +165,8 @@ __device__ __forceinline__ void sell_head_ops(const SellView<T> &A, int s, int l
 // Loads the head of slice s; returns the diagonal of the lane's row (1 for
 // lanes that hold no row start).
 template <typename T, int G>
-__device__ __forceinline__ T sell_head(const SellView<T> &A, int s, int lane, SellHead<T> &h) {
-  sell_head_ops(A, s, lane, h);
+__device__ __forceinline__ T sell_head(const SellView<T> &A, int s, int lane, SellHead<T> &h, bool zero = false) {
+  sell_head_ops(A, s, lane, h, zero);
   const int row = h.r0 + lane / G;
   return ((lane & (G - 1)) == 0 && row < h.r1) ? __ldg(A.diag + row) : T(1);
 }
@@ -224,13 +239,13 @@ template <typename T, typename BT, int kMode, int G = 1>
 __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done) {
+                                                        const int *done, int s_begin, int s_end) {
   if (pass_entry(done)) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   // Bandwidth-bound on the big levels: no head held across trips (it costs
   // occupancy, measured slower on the fine-level residual and prolongation)
-  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < A.nslices; s += warps) {
+  for (int s = s_begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); s < s_end; s += warps) {
     T sum = sell_offdiag<T, false>(A, s, lane, x, 0);
 #pragma unroll
     for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
@@ -242,6 +257,37 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
       else y[row] += sum;
     }
+  }
+}
+
+// Residual of a level right after one forward Gauss-Seidel sweep from zero
+// with omega 1, slices [s_begin, s_end). Row i of colour c was set to
+// x_i = (b_i - sum over the columns below c) / a_ii, so b_i and those columns
+// cancel and r_i = -(sum over the columns at or past c's rows): neither b, nor
+// the diagonal, nor the first half of the matrix is read (P128 level 0, whose
+// last colour has no such columns and is left out by the caller: 28.9 -> 11
+// us).
+template <typename T, int G>
+__global__ void __launch_bounds__(256) sell_upper_kernel(SellView<T> A, const T *__restrict__ x, T *__restrict__ r,
+                                                         const int *done, int s_begin, int s_end) {
+  using P2 = typename Pair<T>::type;
+  if (pass_entry(done)) return;
+  const int lane = threadIdx.x & 31;
+  const int warps = (gridDim.x * blockDim.x) >> 5;
+  for (int s = s_begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); s < s_end; s += warps) {
+    const int p1 = A.sptr[s + 1], from = A.first[s];
+    T sum = T(0);
+#pragma unroll 4
+    for (int p = A.up[s] + 2 * lane; p < p1; p += 64) {
+      const P2 v = __ldg(reinterpret_cast<const P2 *>(A.val + p));
+      const int2 c = __ldg(reinterpret_cast<const int2 *>(A.col + p));
+      if (c.x >= from) sum = fma(v.x, __ldg(x + c.x), sum);
+      if (c.y >= from) sum = fma(v.y, __ldg(x + c.y), sum);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    const int row = A.srow[s] + lane / G;
+    if ((lane & (G - 1)) == 0 && row < A.srow[s + 1]) r[row] = -sum;
   }
 }
 
@@ -267,13 +313,13 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 1) sell_gs_kernel(Se
   // programmatic dependent launch they arrive while that pass drains.
   SellHead<T> h;
   T di = T(1);
-  if (first < s_end) di = sell_head<T, G>(A, first, lane, h);
+  if (first < s_end) di = sell_head<T, G>(A, first, lane, h, kZero);
   if (pass_entry(done)) return;
   const T w = wts != nullptr ? wts[0] : omega;
   // grid-stride over the colour's slices: resident warps stay busy instead
   // of the grid running in partial waves
   for (int s = first; s < s_end; s += warps) {
-    if (s != first) di = sell_head<T, G>(A, s, lane, h);
+    if (s != first) di = sell_head<T, G>(A, s, lane, h, kZero);
     // the row's own operands do not depend on the neighbour sum: issue their
     // loads first so they overlap the gathers
     const int row = h.r0 + lane / G;
@@ -303,10 +349,11 @@ __global__ void __launch_bounds__(256, sizeof(T) == 4 ? 8 : 1) sell_gs_kernel(Se
 template <typename T>
 struct CsrvView {
   int rows;
-  const int *__restrict__ rp;
+  const int *__restrict__ rp;  // first entry of each row
   const int *__restrict__ ci;
   const T *__restrict__ v;
   const T *__restrict__ diag;  // rows, or nullptr
+  const int *__restrict__ re;  // end of each row (rp + 1 for whole rows)
 };
 
 template <typename T, bool kSkip, int G>
@@ -314,7 +361,7 @@ __device__ __forceinline__ T csrv_offdiag(const CsrvView<T> &A, int row, bool va
                                           const T *__restrict__ x, int skip_from) {
   T sum = T(0);
   if (valid) {
-    const int k1 = A.rp[row + 1];
+    const int k1 = A.re[row];
     // chunks of 4 entries per lane: the 4 column loads, then their 4 gathers
     // and values, then the FMAs, so a chunk costs two dependent round trips
     for (int k0 = A.rp[row] + sub; k0 < k1; k0 += 4 * G) {
@@ -355,7 +402,7 @@ __device__ __forceinline__ void csrv_head(const CsrvView<T> &A, int row, bool va
   h.k1 = 0;
   if (valid) {
     h.k0 = __ldg(A.rp + row) + sub;
-    h.k1 = __ldg(A.rp + row + 1);
+    h.k1 = __ldg(A.re + row);
   }
 #pragma unroll
   for (int u = 0; u < kE; ++u) {
@@ -405,25 +452,25 @@ template <typename T, typename BT, int kMode, int G>
 __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done) {
+                                                        const int *done, int row_begin, int row_end) {
   const int sub = threadIdx.x & (G - 1);
   const int groups = (gridDim.x * blockDim.x) / G;
   // every lane of a warp runs the same number of trips so the shuffles
   // inside csrv_offdiag_head see full warps
-  const int first = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int trips = (A.rows + groups - 1) / groups;
+  const int first = row_begin + (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int trips = (row_end - row_begin + groups - 1) / groups;
   // The first row's head (64 entries per row from 8 lanes up) is loaded
   // before the wait on the predecessor, and every trip loads the next row's
   // while its own gathers are in flight. Same sums as csrv_offdiag.
   CsrvHead<T, (G >= 8 ? 8 : 64 / G)> h;
-  csrv_head<T, G>(A, first, first < A.rows, sub, h);
+  csrv_head<T, G>(A, first, first < row_end, sub, h);
   if (pass_entry(done)) return;
   for (int t = 0; t < trips; ++t) {
     const int row = first + t * groups;
-    const bool valid = row < A.rows;
+    const bool valid = row < row_end;
     CsrvHead<T, (G >= 8 ? 8 : 64 / G)> hn;
     const bool more = t + 1 < trips;
-    if (more) csrv_head<T, G>(A, row + groups, row + groups < A.rows, sub, hn);
+    if (more) csrv_head<T, G>(A, row + groups, row + groups < row_end, sub, hn);
     T sum = csrv_offdiag_head<T, false, G>(A, h, sub, x, 0);
     if (more) h = hn;
     if (valid && sub == 0) {
@@ -431,6 +478,7 @@ __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *
       if (kMode == kSpmvSet) y[row] = sum;
       else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
+      else if (kMode == kSpmvNeg) y[row] = -sum;
       else y[row] += sum;
     }
   }
@@ -461,10 +509,11 @@ __global__ void __launch_bounds__(256) csrv_gs_kernel(CsrvView<T> A, int row_beg
 }
 
 // ---- 3x3 block kernels ----------------------------------------------------
-template <typename T, bool kSkip>
-__device__ __forceinline__ void bell_offdiag(const BellView<T> &A, int s, int lane,
-                                             const T *__restrict__ x, int skip_from, T acc[3]) {
-  const int q0 = A.bptr[s], q1 = A.bptr[s + 1];
+// Block slots [q0, q1) of slice s. kUpper: only the columns at or past
+// `from` (the rest of a sweep from zero, see sell_upper_kernel).
+template <typename T, bool kUpper>
+__device__ __forceinline__ void bell_offdiag(const BellView<T> &A, int q0, int q1, int lane,
+                                             const T *__restrict__ x, int from, T acc[3]) {
   acc[0] = acc[1] = acc[2] = T(0);
   // kSlots block slots per step: all column loads, then all gathers and value
   // loads, then the FMAs in slot order (the same sums as one slot at a time)
@@ -488,7 +537,7 @@ __device__ __forceinline__ void bell_offdiag(const BellView<T> &A, int s, int la
     }
 #pragma unroll
     for (int u = 0; u < kSlots; ++u) {
-      use[u] = in[u] && (!kSkip || bc[u] < skip_from);
+      use[u] = in[u] && (!kUpper || bc[u] >= from);
 #pragma unroll
       for (int c = 0; c < 3; ++c) xv[u][c] = use[u] ? __ldg(x + 3 * bc[u] + c) : T(0);
     }
@@ -515,10 +564,10 @@ struct BellHead {
 };
 
 template <typename T>
-__device__ __forceinline__ void bell_head(const BellView<T> &A, int s, int lane, BellHead<T> &h) {
+__device__ __forceinline__ void bell_head(const BellView<T> &A, int s, int lane, BellHead<T> &h, bool zero = false) {
   constexpr int kSlots = BellHead<T>::kSlots;
   h.q0 = __ldg(A.bptr + s);
-  h.q1 = __ldg(A.bptr + s + 1);
+  h.q1 = zero && A.lo != nullptr ? __ldg(A.lo + s) : __ldg(A.bptr + s + 1);
   const T *va = A.val + 9 * static_cast<size_t>(h.q0) + lane;
 #pragma unroll
   for (int u = 0; u < kSlots; ++u) {
@@ -631,18 +680,27 @@ template <typename T, typename BT, int kMode, int G = 1>
 __global__ void __launch_bounds__(256, 2) bell_spmv_kernel(BellView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done) {
+                                                        const int *done, int s_begin, int s_end) {
   __shared__ T sdiag[8][288];
   if (pass_entry(done)) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   T *sd = sdiag[threadIdx.x >> 5];
-  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < A.nslices; s += warps) {
+  for (int s = s_begin + ((blockIdx.x * blockDim.x + threadIdx.x) >> 5); s < s_end; s += warps) {
     const int n0 = A.srow[s], n1 = A.srow[s + 1];
+    if constexpr (kMode == kSpmvNeg) {  // as sell_upper_kernel
+      T acc[3];
+      bell_offdiag<T, true>(A, A.up[s], A.bptr[s + 1], lane, x, A.first[s], acc);
+      reduce3<G>(acc);
+      const int node = n0 + lane / G;
+      if ((lane & (G - 1)) == 0 && node < n1)
+        for (int r = 0; r < 3; ++r) y[3 * node + r] = -acc[r];
+      continue;
+    }
     NodeBlocks<T> nb;
     fetch_node_blocks(A.diag, n0, n1, lane, nb);
     T acc[3];
-    bell_offdiag<T, false>(A, s, lane, x, 0, acc);
+    bell_offdiag<T, false>(A, A.bptr[s], A.bptr[s + 1], lane, x, 0, acc);
     reduce3<G>(acc);
     stage_node_blocks(nb, lane, sd);
     const int node = n0 + lane / G;
@@ -681,7 +739,7 @@ __global__ void __launch_bounds__(256, 2) bell_gs_kernel(BellView<T> A, int s_be
   int n0 = 0, n1 = 0;
   if (s < s_end) {
     n0 = __ldg(A.srow + s), n1 = __ldg(A.srow + s + 1);
-    bell_head(A, s, lane, h);
+    bell_head(A, s, lane, h, kZero);
     fetch_node_blocks(A.dinv, n0, n1, lane, nb);
   }
   if (pass_entry(done)) return;
@@ -722,6 +780,7 @@ struct BsrvView {
   const T *__restrict__ v;       // 9 per block, row-major
   const T *__restrict__ diag;    // 9 per node
   const T *__restrict__ dinv;    // 9 per node
+  const int *__restrict__ re;    // end of each node row (rp + 1 for whole rows)
 };
 
 template <typename T, bool kSkip, int G>
@@ -729,7 +788,7 @@ __device__ __forceinline__ void bsrv_offdiag(const BsrvView<T> &A, int node, boo
                                              const T *__restrict__ x, int skip_from, T acc[3]) {
   acc[0] = acc[1] = acc[2] = T(0);
   if (valid) {
-    const int k1 = A.rp[node + 1];
+    const int k1 = A.re[node];
     // chunks of 4 blocks per lane: the 4 block-column loads, then the 12
     // gathers, then values and FMAs (two dependent round trips per chunk)
     for (int k0 = A.rp[node] + sub; k0 < k1; k0 += 4 * G) {
@@ -778,7 +837,7 @@ __device__ __forceinline__ void bsrv_head(const BsrvView<T> &A, int node, bool v
   h.k0 = h.k1 = 0;
   if (valid) {
     h.k0 = __ldg(A.rp + node) + sub;
-    h.k1 = __ldg(A.rp + node + 1);
+    h.k1 = __ldg(A.re + node);
   }
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
@@ -881,17 +940,22 @@ template <typename T, typename BT, int kMode, int G>
 __global__ void __launch_bounds__(256) bsrv_spmv_kernel(BsrvView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done) {
+                                                        const int *done, int node_begin, int node_end) {
   if (pass_entry(done)) return;
   const int sub = threadIdx.x & (G - 1);
   const int groups = (gridDim.x * blockDim.x) / G;
-  const int first = (blockIdx.x * blockDim.x + threadIdx.x) / G;
-  const int trips = (A.nodes + groups - 1) / groups;
+  const int first = node_begin + (blockIdx.x * blockDim.x + threadIdx.x) / G;
+  const int trips = (node_end - node_begin + groups - 1) / groups;
   for (int t = 0; t < trips; ++t) {
     const int node = first + t * groups;
-    const bool valid = node < A.nodes;
+    const bool valid = node < node_end;
     T acc[3];
     bsrv_offdiag<T, false, G>(A, node, valid, sub, x, 0, acc);
+    if (kMode == kSpmvNeg) {
+      if (valid && sub == 0)
+        for (int r = 0; r < 3; ++r) y[3 * node + r] = -acc[r];
+      continue;
+    }
     if (valid && sub == 0) {
       const T *d = A.diag + 9 * static_cast<size_t>(node);
       const T x0 = x[3 * node], x1 = x[3 * node + 1], x2 = x[3 * node + 2];
@@ -1017,7 +1081,7 @@ __global__ void __launch_bounds__(256, 2) cg_bell_spmv_pap_kernel(BellView<doubl
     NodeBlocks<double> nb;
     fetch_node_blocks(A.diag, n0, n1, lane, nb);
     double o[3];
-    bell_offdiag<double, false>(A, s, lane, p, 0, o);
+    bell_offdiag<double, false>(A, A.bptr[s], A.bptr[s + 1], lane, p, 0, o);
     reduce3<G>(o);
     stage_node_blocks(nb, lane, sd);
     const int node = n0 + lane / G;

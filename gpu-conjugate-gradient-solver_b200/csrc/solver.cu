@@ -90,6 +90,7 @@ template <typename T>
 struct HostBell {
   int nodes = 0, g = 1;
   std::vector<int> srow, bptr, col;
+  std::vector<int> first, lo, up;  // colour split of each slice (SellView)
   std::vector<T> val, diag, dinv;
 };
 
@@ -116,7 +117,10 @@ HostBell<T> make_bell(const Csr &a, const std::vector<int> &node_bounds, int g =
     }
   }, row_grain(nn, a.nnz()));
   for (size_t b = 0; b + 1 < node_bounds.size(); ++b)
-    for (int r = node_bounds[b]; r < node_bounds[b + 1]; r += 32 / g) h.srow.push_back(r);
+    for (int r = node_bounds[b]; r < node_bounds[b + 1]; r += 32 / g) {
+      h.srow.push_back(r);
+      h.first.push_back(node_bounds[b]);
+    }
   h.srow.push_back(nn);
   const int ns = static_cast<int>(h.srow.size()) - 1;
   h.bptr.assign(ns + 1, 0);
@@ -129,14 +133,20 @@ HostBell<T> make_bell(const Csr &a, const std::vector<int> &node_bounds, int g =
   h.col.assign(h.bptr[ns], 0);
   h.val.assign(9 * static_cast<size_t>(h.bptr[ns]), T(0));
   h.diag.assign(9 * static_cast<size_t>(nn), T(0));
+  h.lo.assign(h.bptr.begin(), h.bptr.end() - 1);
+  h.up.assign(h.bptr.begin() + 1, h.bptr.end());
   parallel_for(ns, [&](long long s0, long long s1) {  // slices write disjoint ranges
     for (long long s = s0; s < s1; ++s) {
       for (int p = h.bptr[s]; p < h.bptr[s + 1]; ++p) h.col[p] = h.srow[s];
       for (int I = h.srow[s]; I < h.srow[s + 1]; ++I) {
         const int local = I - h.srow[s];
         const auto &bc = bcols[I];
-        for (size_t q = 0; q < bc.size(); ++q)
-          h.col[h.bptr[s] + (q / g) * 32 + local * g + q % g] = bc[q];
+        for (size_t q = 0; q < bc.size(); ++q) {
+          const int slot = h.bptr[s] + static_cast<int>(q / g) * 32;
+          h.col[slot + local * g + q % g] = bc[q];
+          if (bc[q] < h.first[s]) h.lo[s] = std::max(h.lo[s], slot + 32);
+          else h.up[s] = std::min(h.up[s], slot);
+        }
         for (int r = 0; r < 3; ++r) {
           const int row = 3 * I + r;
           for (int k = a.rp[row]; k < a.rp[row + 1]; ++k) {
@@ -168,9 +178,10 @@ struct DevBell {
   int max_slots = 0;  // block slots per lane of the widest slice
   long long stored = 0;
   int *srow = nullptr, *bptr = nullptr, *col = nullptr;
+  int *first = nullptr, *lo = nullptr, *up = nullptr;
   T *val = nullptr, *diag = nullptr, *dinv = nullptr;
   std::vector<int> h_srow;
-  BellView<T> view() const { return BellView<T>{nodes, nslices, srow, bptr, col, val, diag, dinv}; }
+  BellView<T> view() const { return BellView<T>{nodes, nslices, srow, bptr, col, val, diag, dinv, first, lo, up}; }
 };
 
 template <typename T>
@@ -186,6 +197,9 @@ DevBell<T> upload_bell(Arena &ar, const HostBell<T> &h) {
   d.val = ar.upload(h.val);
   d.diag = ar.upload(h.diag);
   d.dinv = ar.upload(h.dinv);
+  d.first = ar.upload(h.first);
+  d.lo = ar.upload(h.lo);
+  d.up = ar.upload(h.up);
   d.h_srow = h.srow;
   for (size_t q = 0; q + 1 < h.bptr.size(); ++q) d.max_slots = std::max(d.max_slots, (h.bptr[q + 1] - h.bptr[q]) / 32);
   return d;
@@ -195,16 +209,20 @@ template <typename T>
 struct DevBsrv {
   int nodes = 0;
   int *rp = nullptr, *bc = nullptr;
+  int *mid = nullptr;  // first block of each node row at or past its colour's nodes
   T *v = nullptr, *diag = nullptr, *dinv = nullptr;
-  BsrvView<T> view() const { return BsrvView<T>{nodes, rp, bc, v, diag, dinv}; }
+  BsrvView<T> view() const { return BsrvView<T>{nodes, rp, bc, v, diag, dinv, rp + 1}; }
+  BsrvView<T> below() const { return BsrvView<T>{nodes, rp, bc, v, diag, dinv, mid}; }
+  BsrvView<T> past() const { return BsrvView<T>{nodes, mid, bc, v, diag, dinv, rp + 1}; }
 };
 
 // Block CSR of the off-diagonal 3x3 blocks (row-major), diagonal blocks and
 // their inverses apart; diag / dinv shared with the BELL copy.
 template <typename T>
-DevBsrv<T> upload_bsrv(Arena &ar, const Csr &a, const DevBell<T> &bell) {
+DevBsrv<T> upload_bsrv(Arena &ar, const Csr &a, const DevBell<T> &bell, const std::vector<int> &node_bounds) {
   const int nn = a.rows / 3;
-  std::vector<int> rp(nn + 1, 0), bc;
+  std::vector<int> rp(nn + 1, 0), bc, mid(nn, 0);
+  size_t colour = 0;
   std::vector<T> v;
   std::vector<int> cols;
   for (int I = 0; I < nn; ++I) {
@@ -223,6 +241,8 @@ DevBsrv<T> upload_bsrv(Arena &ar, const Csr &a, const DevBell<T> &bell) {
         const size_t q = std::lower_bound(cols.begin(), cols.end(), J) - cols.begin();
         v[base + 9 * q + 3 * r + a.ci[k] % 3] = T(a.v[k]);
       }
+    while (node_bounds[colour + 1] <= I) ++colour;
+    mid[I] = rp[I] + static_cast<int>(std::lower_bound(cols.begin(), cols.end(), node_bounds[colour]) - cols.begin());
     bc.insert(bc.end(), cols.begin(), cols.end());
     rp[I + 1] = static_cast<int>(bc.size());
   }
@@ -230,6 +250,7 @@ DevBsrv<T> upload_bsrv(Arena &ar, const Csr &a, const DevBell<T> &bell) {
   d.nodes = nn;
   d.rp = ar.upload(rp);
   d.bc = ar.upload(bc);
+  d.mid = ar.upload(mid);
   d.v = ar.upload(v);
   d.diag = bell.diag;
   d.dinv = bell.dinv;
@@ -533,12 +554,33 @@ class AmgPcg final : public Solver {
   void dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s);
   template <typename BT>
   void vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s);
+  // Colours [c0, c1) of a level; upper: only the entries at or past each
+  // row's colour count (sell_upper_kernel).
+  struct Part {
+    int c0, c1;
+    bool upper;
+  };
+  // With omega 1 and no learned weight other than 1 a colour pass solves its
+  // rows exactly, whatever their old values.
+  bool exact_passes(const Level &L) const {
+    return VT(opt_.omega) == VT(1) && (L.wts.empty() || L.wts[0] == nullptr || unit_weights_) && L.nwts == nullptr &&
+           (L.kind == 0 || L.kind == 1);
+  }
+  Part resid_part(const Level &L, bool zero) const;
+  Part swept_part(const Level &L) const;
   template <typename BT>
-  void level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, cudaStream_t s);
+  void level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, cudaStream_t s) {
+    level_spmv_resid(L, rhs, x, r, Part{0, L.ncolors, false}, s);
+  }
+  template <typename BT>
+  void level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, Part part, cudaStream_t s);
+  void restrict_residual(Level &L, Part part, VT *y, cudaStream_t s);
+  template <int kMode>
+  void prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s);
   void precondition(const double *r, VT *z, cudaStream_t s);
   template <int kMode, typename BT>
-  void transfer(const DevSell<VT> &S, const DevCsrv<VT> &Cm, int g, const VT *x, VT *y, const BT *b,
-                cudaStream_t s);
+  void transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g, const VT *x, VT *y,
+                const BT *b, cudaStream_t s);
   void autotune();
   float time_ms(const std::function<void()> &f, int reps);
   void cg_iteration(int parity, cudaStream_t s);
@@ -585,6 +627,7 @@ class AmgPcg final : public Solver {
   CgState *host_st_ = nullptr;                  // pinned, two slots
   SweepSync *sync_ = nullptr;                   // grid-barrier state of the cooperative sweeps
   VT *wbuf_ = nullptr;
+  bool unit_weights_ = false;  // installed colour weights are all 1
   cudaStream_t stream_ = nullptr;
   cudaEvent_t ev_[4] = {nullptr, nullptr, nullptr, nullptr};
   cudaGraph_t graph_[2] = {nullptr, nullptr};
@@ -751,7 +794,7 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
     if (block_) {
       const HostBell<VT> hb = make_bell<VT>(Ai, offs);
       lv.B = upload_bell(ar_, hb);
-      lv.Bv = upload_bsrv<VT>(ar_, Ai, lv.B);
+      lv.Bv = upload_bsrv<VT>(ar_, Ai, lv.B, offs);
       info_[k].slices = lv.B.nslices;
       info_[k].stored = lv.B.stored;
       if (k == 0) {
@@ -773,7 +816,9 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
         lv.jdinv = ar_.upload(jd);
       }
       lv.A = upload_sell(ar_, hs);
-      lv.C = upload_csrv<VT>(ar_, Ai, true);
+      std::vector<int> cut(n);
+      for (int c = 0; c < nc; ++c) std::fill(cut.begin() + offs[c], cut.begin() + offs[c + 1], offs[c]);
+      lv.C = upload_csrv<VT>(ar_, Ai, true, &cut);
       info_[k].slices = lv.A.nslices;
       info_[k].stored = lv.A.stored;
       if (k == 0) cgA_ = upload_sell(ar_, make_sell<double>(Ai, offs, true));
@@ -797,10 +842,18 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
       const Csr Ri = permute_matrix(h.R[k - 1], Q[k].data(), Q[k - 1].data());
       if (Pi.rows != lv_[k - 1].n || Pi.cols != n || Ri.rows != n || Ri.cols != lv_[k - 1].n)
         throw std::runtime_error("MultigridSmoother: transfer operator shape mismatch.");
-      lv_[k - 1].P = upload_sell(ar_, make_sell<VT>(Pi, {0, Pi.rows}, false));
-      lv_[k - 1].R = upload_sell(ar_, make_sell<VT>(Ri, {0, Ri.rows}, false));
-      lv_[k - 1].Pc = upload_csrv<VT>(ar_, Pi, false);
-      lv_[k - 1].Rc = upload_csrv<VT>(ar_, Ri, false);
+      Level &f = lv_[k - 1];
+      // P's slices and R's rows are cut where the first and the last colour
+      // of the fine level begin (swept_rows)
+      const int u = block_ ? 3 : 1, lo = u * f.color_first[std::min(1, f.ncolors)],
+                hi = u * f.color_first[std::max(0, f.ncolors - 1)];
+      std::vector<int> pb = {0, std::min(lo, hi), std::max(lo, hi), Pi.rows};
+      pb.erase(std::unique(pb.begin(), pb.end()), pb.end());
+      const std::vector<int> rcut(Ri.rows, opt_.half_sweeps ? hi : lo);
+      f.P = upload_sell(ar_, make_sell<VT>(Pi, pb, false));
+      f.R = upload_sell(ar_, make_sell<VT>(Ri, {0, Ri.rows}, false));
+      f.Pc = upload_csrv<VT>(ar_, Pi, false);
+      f.Rc = upload_csrv<VT>(ar_, Ri, false, &rcut);
     }
     lap(8);
     if (k == L - 1 && opt_.coarse == 1) {
@@ -1052,6 +1105,7 @@ void AmgPcg<VT>::set_weights(const ColourWeights &w) {
     wbuf_ = ar_.alloc<VT>(total);
   }
   CK(cudaMemcpy(wbuf_, hv.data(), hv.size() * sizeof(VT), cudaMemcpyHostToDevice));
+  unit_weights_ = std::all_of(hv.begin(), hv.end(), [](VT v) { return v == VT(1); });
   for (int k = 0; k < L; ++k)
     for (int c = 0; c < lv_[k].ncolors; ++c) lv_[k].wts[c] = wbuf_ + w.level_offset[k] + c;
   if (tail_on_) upload_tail_table(tail_k0_);  // the table carries the weight pointers
@@ -1164,7 +1218,7 @@ void AmgPcg<VT>::gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaS
   } else if (block_) {
     const int n0 = L.color_first[c], n1 = L.color_first[c + 1];
     const int gb = static_cast<int>((static_cast<long long>(n1 - n0) * L.g + 255) / 256);
-    const BsrvView<VT> v = L.Bv.view();
+    const BsrvView<VT> v = zero ? L.Bv.below() : L.Bv.view();
 #define GS_BSRV(G)                                                                                   \
   if (zero) launch_pass(pdl_, bsrv_gs_kernel<VT, BT, true, G>, gb, s, v, n0, n1, rhs, x, w, om, done, nw, xp);     \
   else if (xp) launch_pass(pdl_, bsrv_gs_kernel<VT, BT, false, G, true>, gb, s, v, n0, n1, rhs, x, w, om, done, nw, xp); \
@@ -1196,7 +1250,7 @@ void AmgPcg<VT>::gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaS
   } else {
     const int r0 = L.color_first[c], r1 = L.color_first[c + 1];
     const int gb = static_cast<int>((static_cast<long long>(r1 - r0) * L.g + 255) / 256);
-    const CsrvView<VT> v = L.C.view();
+    const CsrvView<VT> v = zero ? L.C.below() : L.C.view();
 #define GS_CSRV(G)                                                                                   \
   if (zero) launch_pass(pdl_, csrv_gs_kernel<VT, BT, true, G>, gb, s, v, r0, r1, rhs, x, w, om, done, xp);     \
   else if (xp) launch_pass(pdl_, csrv_gs_kernel<VT, BT, false, G, true>, gb, s, v, r0, r1, rhs, x, w, om, done, xp); \
@@ -1466,38 +1520,109 @@ void AmgPcg<VT>::check_sync_fault(const CgState &hs) {
   throw CudaError("cooperative Gauss-Seidel sweep: a grid-barrier wait timed out");
 }
 
+// Rows whose residual is not zero after pre-smoothing. The colour updated
+// last was solved exactly, so its rows' residual is 0 (up to the rounding of
+// their update): the last colour after forward half sweeps, the first after
+// symmetric steps. Their rows are left out, and so are their columns of the
+// restriction (cut at the same colour, in the CSR-vector layout: SELL has no
+// cut, and a level whose autotuner chose it keeps the whole residual). After
+// one forward sweep from zero the others need only half of the matrix.
+// A level coloured by its strong couplings keeps all rows: same-colour
+// couplings leave a residual.
+template <typename VT>
+typename AmgPcg<VT>::Part AmgPcg<VT>::resid_part(const Level &L, bool zero) const {
+  Part p{0, L.ncolors, false};
+  if (!exact_passes(L)) return p;
+  p.upper = opt_.half_sweeps && opt_.pre == 1 && zero;
+  if (L.relaxed || L.ncolors < 2 || L.rg == 1) return p;
+  if (opt_.half_sweeps) p.c1 = L.ncolors - 1;
+  else p.c0 = 1;
+  return p;
+}
+
+// Rows that the prolongation has to correct: post-smoothing starts with the
+// last colour (backward half sweeps) or the first (symmetric steps) and
+// overwrites it from its neighbours alone, so its rows are left out. Not in
+// the reference's aliased V-cycle, nor where same-colour couplings read them.
+template <typename VT>
+typename AmgPcg<VT>::Part AmgPcg<VT>::swept_part(const Level &L) const {
+  Part p{0, L.ncolors, false};
+  if (!exact_passes(L) || L.relaxed || L.ncolors < 2 || opt_.reference_vcycle) return p;
+  if (opt_.half_sweeps) p.c1 = L.ncolors - 1;
+  else p.c0 = 1;
+  return p;
+}
+
 template <typename VT>
 template <typename BT>
-void AmgPcg<VT>::level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, cudaStream_t s) {
+void AmgPcg<VT>::level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, Part part, cudaStream_t s) {
   const int *done = &st_->done;
+  const int n0 = L.color_first[part.c0], n1 = L.color_first[part.c1];  // rows, or nodes
+  if (n1 <= n0) return;
+  const int s0 = L.sliced ? L.color_slice[part.c0] : 0, s1 = L.sliced ? L.color_slice[part.c1] : 0;
   if (block_ && L.sliced) {
-    const int gb = blocks_for(32LL * L.B.nslices, cap_blocks_);
+    const int gb = blocks_for(32LL * (s1 - s0), cap_blocks_);
+#define RES_BELL(G)                                                                                                 \
+  if (part.upper) launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvNeg, G>, gb, s, L.B.view(), x, r, rhs, done, s0, s1); \
+  else launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.B.view(), x, r, rhs, done, s0, s1);
     switch (L.g) {
-      case 1: launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvResid, 1>, gb, s, L.B.view(), x, r, rhs, done); break;
-      case 2: launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvResid, 2>, gb, s, L.B.view(), x, r, rhs, done); break;
-      case 4: launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvResid, 4>, gb, s, L.B.view(), x, r, rhs, done); break;
-      default: launch_pass(pdl_, bell_spmv_kernel<VT, BT, kSpmvResid, 8>, gb, s, L.B.view(), x, r, rhs, done); break;
+      case 1: RES_BELL(1) break;
+      case 2: RES_BELL(2) break;
+      case 4: RES_BELL(4) break;
+      default: RES_BELL(8) break;
     }
+#undef RES_BELL
   } else if (block_) {
-    const int gb = blocks_for(static_cast<long long>(L.Bv.nodes) * L.g, cap_blocks_);
+    const int gb = blocks_for(static_cast<long long>(n1 - n0) * L.g, cap_blocks_);
+#define RES_BSRV(G)                                                                                                    \
+  if (part.upper) launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvNeg, G>, gb, s, L.Bv.past(), x, r, rhs, done, n0, n1); \
+  else launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.Bv.view(), x, r, rhs, done, n0, n1);
     switch (L.g) {
-      case 4: launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvResid, 4>, gb, s, L.Bv.view(), x, r, rhs, done); break;
-      case 8: launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvResid, 8>, gb, s, L.Bv.view(), x, r, rhs, done); break;
-      case 16: launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvResid, 16>, gb, s, L.Bv.view(), x, r, rhs, done); break;
-      default: launch_pass(pdl_, bsrv_spmv_kernel<VT, BT, kSpmvResid, 32>, gb, s, L.Bv.view(), x, r, rhs, done); break;
+      case 4: RES_BSRV(4) break;
+      case 8: RES_BSRV(8) break;
+      case 16: RES_BSRV(16) break;
+      default: RES_BSRV(32) break;
     }
+#undef RES_BSRV
   } else if (L.sliced) {
-    const int gb = blocks_for(32LL * L.A.nslices, cap_blocks_);
+    const int gb = blocks_for(32LL * (s1 - s0), cap_blocks_);
+#define RES_SELL(G)                                                                                      \
+  if (part.upper) launch_pass(pdl_, sell_upper_kernel<VT, G>, gb, s, L.A.view(), x, r, done, s0, s1);     \
+  else launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.A.view(), x, r, rhs, done, s0, s1);
     switch (L.g) {
-      case 1: launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, 1>, gb, s, L.A.view(), x, r, rhs, done); break;
-      case 2: launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, 2>, gb, s, L.A.view(), x, r, rhs, done); break;
-      case 4: launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, 4>, gb, s, L.A.view(), x, r, rhs, done); break;
-      default: launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, 8>, gb, s, L.A.view(), x, r, rhs, done); break;
+      case 1: RES_SELL(1) break;
+      case 2: RES_SELL(2) break;
+      case 4: RES_SELL(4) break;
+      default: RES_SELL(8) break;
     }
+#undef RES_SELL
+  } else if (part.upper) {
+    transfer<kSpmvNeg, BT>(L.A1.view(), 0, 0, L.C.past(), n0, n1, L.g, x, r, rhs, s);
   } else {
-    transfer<kSpmvResid, BT>(L.A1, L.C, L.g, x, r, rhs, s);
+    transfer<kSpmvResid, BT>(L.A1.view(), 0, 0, L.C.view(), n0, n1, L.g, x, r, rhs, s);
   }
   CKL("residual");
+}
+
+// y = R r, with the columns of `part`'s rows only.
+template <typename VT>
+void AmgPcg<VT>::restrict_residual(Level &L, Part part, VT *y, cudaStream_t s) {
+  CsrvView<VT> v = L.Rc.view();
+  if (part.c1 < L.ncolors) v = L.Rc.below();
+  else if (part.c0 > 0) v = L.Rc.past();
+  transfer<kSpmvSet, VT>(L.R.view(), 0, L.R.nslices, v, 0, L.Rc.rows, L.rg, L.r, y, (const VT *)nullptr, s);
+  CKL("restriction");
+}
+
+// x += P xc (kSpmvAdd; kSpmvTwice as the mode says) on the rows of `part`.
+template <typename VT>
+template <int kMode>
+void AmgPcg<VT>::prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s) {
+  const int u = block_ ? 3 : 1, r0 = u * L.color_first[part.c0], r1 = u * L.color_first[part.c1];
+  if (r1 <= r0) return;
+  transfer<kMode, VT>(L.P.view(), L.P.slice_of(r0), L.P.slice_of(r1), L.Pc.view(), r0, r1, L.pg, xc, x,
+                      (const VT *)nullptr, s);
+  CKL("prolongation");
 }
 
 // x = A^-1 rhs on the dense coarsest level: full row-major inverse, or the
@@ -1566,35 +1691,34 @@ void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s) 
     return;
   }
   smooth(L, rhs, x, opt_.pre, zero, s, opt_.half_sweeps ? 1 : 0);
-  level_spmv_resid(L, rhs, x, L.r, s);
+  const Part part = resid_part(L, zero);
+  level_spmv_resid(L, rhs, x, L.r, part, s);
   Level &C = lv_[k + 1];
-  transfer<kSpmvSet, VT>(L.R, L.Rc, L.rg, L.r, C.b, (const VT *)nullptr, s);
-  CKL("restriction");
+  restrict_residual(L, part, C.b, s);
   vcycle<VT>(k + 1, C.b, C.x, true, s);
-  if (opt_.reference_vcycle && k > 0)
-    transfer<kSpmvTwice, VT>(L.P, L.Pc, L.pg, C.x, x, (const VT *)nullptr, s);
-  else
-    transfer<kSpmvAdd, VT>(L.P, L.Pc, L.pg, C.x, x, (const VT *)nullptr, s);
-  CKL("prolongation");
+  if (opt_.reference_vcycle && k > 0) prolong<kSpmvTwice>(L, swept_part(L), C.x, x, s);
+  else prolong<kSpmvAdd>(L, swept_part(L), C.x, x, s);
   smooth(L, rhs, x, opt_.post, false, s, opt_.half_sweeps ? 2 : 0);
 }
 
-// y (op)= M x with M in SELL-32 (g == 1) or CSR-vector with g lanes per row.
+// y (op)= M x on rows [r0, r1) of M in SELL-32 (g == 1, slices [s0, s1)) or
+// CSR-vector with g lanes per row.
 template <typename VT>
 template <int kMode, typename BT>
-void AmgPcg<VT>::transfer(const DevSell<VT> &S, const DevCsrv<VT> &Cm, int g, const VT *x, VT *y,
-                          const BT *b, cudaStream_t s) {
+void AmgPcg<VT>::transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g,
+                          const VT *x, VT *y, const BT *b, cudaStream_t s) {
   const int *done = &st_->done;
   if (g == 1) {
-    launch_pass(pdl_, sell_spmv_kernel<VT, BT, kMode>, blocks_for(32LL * S.nslices, cap_blocks_), s, S.view(), x, y, b, done);
+    launch_pass(pdl_, sell_spmv_kernel<VT, BT, kMode>, blocks_for(32LL * (s1 - s0), cap_blocks_), s, S, x, y, b, done, s0,
+                s1);
     return;
   }
-  const int gb = blocks_for(static_cast<long long>(Cm.rows) * g, cap_blocks_);
+  const int gb = blocks_for(static_cast<long long>(r1 - r0) * g, cap_blocks_);
   switch (g) {
-    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm.view(), x, y, b, done); break;
-    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm.view(), x, y, b, done); break;
-    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm.view(), x, y, b, done); break;
-    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm.view(), x, y, b, done); break;
+    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm, x, y, b, done, r0, r1); break;
+    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm, x, y, b, done, r0, r1); break;
+    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm, x, y, b, done, r0, r1); break;
+    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm, x, y, b, done, r0, r1); break;
   }
 }
 
@@ -1791,8 +1915,14 @@ void AmgPcg<VT>::autotune() {
       float bp = 1e30f, br = 1e30f;
       int gp = 1, gr = 1;
       for (int g : cands) {
-        const float tr = time_segment([&] { transfer<kSpmvSet, VT>(L.R, L.Rc, g, L.x, Cn.b, (const VT *)nullptr, stream_); }, 10, 2);
-        const float tp = time_segment([&] { transfer<kSpmvAdd, VT>(L.P, L.Pc, g, Cn.x, L.r, (const VT *)nullptr, stream_); }, 10, 2);
+        L.rg = L.pg = g;
+        const Part rpart = resid_part(L, true);
+        // without the column cut (SELL) the whole residual is paid for too
+        const float tr = time_segment([&] {
+          level_spmv_resid<VT>(L, L.b, L.x, L.r, rpart, stream_);
+          restrict_residual(L, rpart, Cn.b, stream_);
+        }, 10, 2);
+        const float tp = time_segment([&] { prolong<kSpmvAdd>(L, swept_part(L), Cn.x, L.x, stream_); }, 10, 2);
         if (tr < br) br = tr, gr = g;
         if (tp < bp) bp = tp, gp = g;
       }
@@ -2156,15 +2286,15 @@ template <typename VT>
 void AmgPcg<VT>::outer_resid(cudaStream_t s) {
   if (!block_) {
     sell_spmv_kernel<double, double, kSpmvResid>
-        <<<blocks_for(32LL * cgA_.nslices, cap_blocks_), 256, 0, s>>>(cgA_.view(), x_, r_, b_, nullptr);
+        <<<blocks_for(32LL * cgA_.nslices, cap_blocks_), 256, 0, s>>>(cgA_.view(), x_, r_, b_, nullptr, 0, cgA_.nslices);
     return;
   }
   const int blocks = blocks_for(32LL * cgB_.nslices, cap_blocks_);
   switch (cgB_.g) {
-    case 1: bell_spmv_kernel<double, double, kSpmvResid, 1><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr); break;
-    case 2: bell_spmv_kernel<double, double, kSpmvResid, 2><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr); break;
-    case 4: bell_spmv_kernel<double, double, kSpmvResid, 4><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr); break;
-    default: bell_spmv_kernel<double, double, kSpmvResid, 8><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr); break;
+    case 1: bell_spmv_kernel<double, double, kSpmvResid, 1><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr, 0, cgB_.nslices); break;
+    case 2: bell_spmv_kernel<double, double, kSpmvResid, 2><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr, 0, cgB_.nslices); break;
+    case 4: bell_spmv_kernel<double, double, kSpmvResid, 4><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr, 0, cgB_.nslices); break;
+    default: bell_spmv_kernel<double, double, kSpmvResid, 8><<<blocks, 256, 0, s>>>(cgB_.view(), x_, r_, b_, nullptr, 0, cgB_.nslices); break;
   }
 }
 
@@ -2381,11 +2511,11 @@ double AmgPcg<VT>::time_level(int level, int op, int lanes, int reps, cudaStream
     if (op == 0) {
       forward_sweep(L, stream);
     } else if (op == 1) {
-      level_spmv_resid<VT>(L, L.b, L.x, L.r, stream);
+      level_spmv_resid<VT>(L, L.b, L.x, L.r, resid_part(L, true), stream);
     } else if (op == 2) {
-      transfer<kSpmvSet, VT>(L.R, L.Rc, L.rg, L.r, C.b, (const VT *)nullptr, stream);
+      restrict_residual(L, resid_part(L, true), C.b, stream);
     } else {
-      transfer<kSpmvAdd, VT>(L.P, L.Pc, L.pg, C.x, L.x, (const VT *)nullptr, stream);
+      prolong<kSpmvAdd>(L, swept_part(L), C.x, L.x, stream);
     }
   };
   // defined inputs: x = 0, b = 1 on both levels; the stop flag cleared
