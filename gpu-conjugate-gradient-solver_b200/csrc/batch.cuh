@@ -74,13 +74,6 @@ __device__ __forceinline__ void bpass_entry() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// A pointer whose loads stay behind the wait.
-template <typename T>
-__device__ __forceinline__ T *after_wait(T *p) {
-  asm volatile("" : "+l"(p)::"memory");
-  return p;
-}
-
 __device__ __forceinline__ bool item_skipped(const int *sys_done, int sys) {
   return sys_done != nullptr && reinterpret_cast<const volatile int *>(sys_done)[sys] != 0;
 }

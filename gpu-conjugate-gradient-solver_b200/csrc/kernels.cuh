@@ -104,6 +104,13 @@ __device__ __forceinline__ bool pass_entry(const int *done) {
   return stop_requested(done);
 }
 
+// A pointer whose loads stay behind the wait.
+template <typename T>
+__device__ __forceinline__ T *after_wait(T *p) {
+  asm volatile("" : "+l"(p)::"memory");
+  return p;
+}
+
 // Off-diagonal row sum of lane `lane` of slice s: sum_k val * x[col].
 // With kSkipFrom >= 0 (zero initial guess, first forward sweep), columns at
 // or above `skip_from` are known to hold zero and are not gathered.
@@ -232,6 +239,25 @@ __device__ __forceinline__ T sell_offdiag_head(const SellView<T> &A, const SellH
   return sum;
 }
 
+// First pass of a forward Gauss-Seidel sweep from zero: no neighbour counts,
+// so a row of the first colour is x_i = w b_i / a_ii, formed where b_i is
+// (the update of r on the finest level, the restriction below it).
+template <typename T>
+struct FirstColour {
+  T *x;                        // nullptr: no such pass
+  const T *__restrict__ diag;
+  int rows;                    // rows [0, rows)
+  const T *wts;                // the colour's learned weight, or nullptr
+  T omega;
+  template <typename BT>
+  __device__ __forceinline__ void operator()(int row, BT b) const {
+    if (row < rows) {
+      const T w = wts != nullptr ? wts[0] : omega;
+      x[row] = w * (T(b) / __ldg(diag + row));
+    }
+  }
+};
+
 // y = A x (kSpmvSet), y = b - A x (kSpmvResid), y += A x (kSpmvAdd).
 // One warp per slice, grid-stride over slices. G lanes per row: a slice holds
 // 32 / G rows, lane l serves row l / G and the group adds its partial sums.
@@ -239,7 +265,8 @@ template <typename T, typename BT, int kMode, int G = 1>
 __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done, int s_begin, int s_end) {
+                                                        const int *done, int s_begin, int s_end,
+                                                        FirstColour<T> fc = FirstColour<T>{}) {
   if (pass_entry(done)) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -252,8 +279,10 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *
     const int row = A.srow[s] + lane / G;
     if ((lane & (G - 1)) == 0 && row < A.srow[s + 1]) {
       if (A.diag != nullptr) sum = fma(A.diag[row], x[row], sum);
-      if (kMode == kSpmvSet) y[row] = sum;
-      else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
+      if (kMode == kSpmvSet) {
+        y[row] = sum;
+        if (fc.x != nullptr) fc(row, sum);
+      } else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
       else y[row] += sum;
     }
@@ -452,7 +481,8 @@ template <typename T, typename BT, int kMode, int G>
 __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *__restrict__ x,
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
-                                                        const int *done, int row_begin, int row_end) {
+                                                        const int *done, int row_begin, int row_end,
+                                                        FirstColour<T> fc = FirstColour<T>{}) {
   const int sub = threadIdx.x & (G - 1);
   const int groups = (gridDim.x * blockDim.x) / G;
   // every lane of a warp runs the same number of trips so the shuffles
@@ -475,8 +505,10 @@ __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *
     if (more) h = hn;
     if (valid && sub == 0) {
       if (A.diag != nullptr) sum = fma(A.diag[row], x[row], sum);
-      if (kMode == kSpmvSet) y[row] = sum;
-      else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
+      if (kMode == kSpmvSet) {
+        y[row] = sum;
+        if (fc.x != nullptr) fc(row, sum);
+      } else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
       else if (kMode == kSpmvNeg) y[row] = -sum;
       else y[row] += sum;
@@ -1029,18 +1061,31 @@ __device__ __forceinline__ bool grid_sum(double (&v)[kN], double *partials, unsi
 // ---- CG kernels (FP64 outer iteration) --------------------------------------
 __device__ __forceinline__ bool finite_d(double v) { return isfinite(v); }
 
-// Ap = A p and pAp = p . Ap; the last block sets alpha = rho / pAp.
-static __global__ void __launch_bounds__(256) cg_spmv_pap_kernel(SellView<double> A,
+// The CG kernels enter through pass_entry like the V-cycle's and are launched
+// with programmatic serialization: what a kernel's predecessor does not write
+// (matrix operands, vectors completed two launches earlier) is loaded before
+// the wait, so that a launch costs one dependent round trip instead of a cold
+// start. The early vector loads go through L2 (ld.global.cg).
+
+// Ap = A p and pAp = p . Ap; the last block sets alpha = rho / pAp. kHead:
+// every warp has at most one slice, whose first slot pairs are loaded before
+// the wait (small problems; on large ones the registers cost bandwidth).
+template <bool kHead>
+__global__ void __launch_bounds__(256) cg_spmv_pap_kernel(SellView<double> A,
                                                           const double *__restrict__ p,
                                                           double *__restrict__ ap, CgState *st,
                                                           double *partials) {
   __shared__ double smem[32];
-  if (st->done) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
+  const int s0 = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  SellHead<double> h;
+  if (kHead && s0 < A.nslices) sell_head_ops(A, s0, lane, h);
+  if (pass_entry(&st->done)) return;
+  p = after_wait(p);
   double acc[1] = {0.0};
-  for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < A.nslices; s += warps) {
-    double sum = sell_offdiag<double, false>(A, s, lane, p, 0);
+  for (int s = s0; s < A.nslices; s += warps) {
+    double sum = kHead ? sell_offdiag_head<double, false>(A, h, lane, p, 0) : sell_offdiag<double, false>(A, s, lane, p, 0);
     const int row = A.srow[s] + lane;
     if (row < A.srow[s + 1]) {
       const double pr = p[row];
@@ -1071,7 +1116,7 @@ __global__ void __launch_bounds__(256, 2) cg_bell_spmv_pap_kernel(BellView<doubl
                                                                double *partials) {
   __shared__ double smem[32];
   __shared__ double sdiag[8][288];
-  if (st->done) return;
+  if (pass_entry(&st->done)) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
   double *sd = sdiag[threadIdx.x >> 5];
@@ -1110,22 +1155,42 @@ __global__ void __launch_bounds__(256, 2) cg_bell_spmv_pap_kernel(BellView<doubl
   }
 }
 
-// x += alpha p; r -= alpha Ap; rr = r . r; convergence test on rr / bb.
-static __global__ void __launch_bounds__(256) cg_update_xr_kernel(int n, double *__restrict__ x,
+// What the host polls: 2 * (iterations whose convergence test has run) + stop
+// flag, in pinned memory.
+__device__ __forceinline__ void publish_state(const CgState *st, volatile unsigned *host) {
+  *host = 2u * static_cast<unsigned>(st->iter) + (st->done != 0 ? 1u : 0u);
+}
+
+// x += alpha p; r -= alpha Ap; rr = r . r; convergence test on rr / bb, its
+// outcome published to the host. z's first colour from the new r.
+template <typename ZT>
+__global__ void __launch_bounds__(256) cg_update_xr_kernel(int n, double *__restrict__ x,
                                                            double *__restrict__ r,
                                                            const double *__restrict__ p,
                                                            const double *__restrict__ ap,
-                                                           CgState *st, double *partials) {
+                                                           CgState *st, double *partials, FirstColour<ZT> z,
+                                                           volatile unsigned *host) {
   __shared__ double smem[32];
-  if (st->done) return;
-  const double alpha = st->alpha;
-  double acc[1] = {0.0};
   const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    x[i] = fma(alpha, p[i], x[i]);
-    const double ri = fma(-alpha, ap[i], r[i]);
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double xi = 0.0, pi = 0.0, ri = 0.0;
+  if (i < n) xi = __ldcg(x + i), pi = __ldcg(p + i), ri = __ldcg(r + i);
+  if (pass_entry(&st->done)) {
+    // the product broke down: the host learns of it here
+    if (blockIdx.x == 0 && threadIdx.x == 0) publish_state(st, host);
+    return;
+  }
+  ap = after_wait(ap);
+  const double alpha = *reinterpret_cast<volatile double *>(&st->alpha);
+  double acc[1] = {0.0};
+  while (i < n) {
+    x[i] = fma(alpha, pi, xi);
+    ri = fma(-alpha, ap[i], ri);
     r[i] = ri;
+    if (z.x != nullptr) z(i, ri);
     acc[0] = fma(ri, ri, acc[0]);
+    i += stride;
+    if (i < n) xi = x[i], pi = p[i], ri = r[i];
   }
   if (grid_sum<1>(acc, partials, &st->ticket, smem) && threadIdx.x == 0) {
     st->rr = acc[0];
@@ -1145,6 +1210,7 @@ static __global__ void __launch_bounds__(256) cg_update_xr_kernel(int n, double 
       st->iterations = st->max_iter;
     }
     st->iter += 1;
+    publish_state(st, host);
   }
 }
 
@@ -1152,18 +1218,28 @@ static __global__ void __launch_bounds__(256) cg_update_xr_kernel(int n, double 
 // sets beta = (rho_new - r.z_old) / rho (Polak-Ribiere) or rho_new / rho.
 template <typename ZT>
 __global__ void __launch_bounds__(256) cg_dot_rz_kernel(int n, const double *__restrict__ r,
-                                                        const ZT *__restrict__ z,
+                                                        const ZT *z,
                                                         const ZT *__restrict__ z_old, CgState *st,
                                                         double *partials) {
   __shared__ double smem[64];
-  if (st->done) return;
-  double acc[2] = {0.0, 0.0};
   const int stride = gridDim.x * blockDim.x;
   const bool flex = z_old != nullptr;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
-    const double ri = r[i];
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double ri = 0.0, zo = 0.0;
+  if (i < n) {
+    ri = __ldcg(r + i);
+    if (flex) zo = double(__ldcg(z_old + i));
+  }
+  if (pass_entry(&st->done)) return;
+  double acc[2] = {0.0, 0.0};
+  while (i < n) {
     acc[0] = fma(ri, double(z[i]), acc[0]);
-    if (flex) acc[1] = fma(ri, double(z_old[i]), acc[1]);
+    if (flex) acc[1] = fma(ri, zo, acc[1]);
+    i += stride;
+    if (i < n) {
+      ri = r[i];
+      if (flex) zo = double(z_old[i]);
+    }
   }
   if (grid_sum<2>(acc, partials, &st->ticket, smem) && threadIdx.x == 0) {
     st->rho_new = acc[0];
@@ -1178,11 +1254,17 @@ template <typename ZT>
 __global__ void __launch_bounds__(256) cg_update_p_kernel(int n, const ZT *__restrict__ z,
                                                           double *__restrict__ p,
                                                           const CgState *st) {
-  if (st->done) return;
-  const double beta = st->beta;
   const int stride = gridDim.x * blockDim.x;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
-    p[i] = fma(beta, p[i], double(z[i]));
+  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  double zi = 0.0, pi = 0.0;
+  if (i < n) zi = double(__ldcg(z + i)), pi = __ldcg(p + i);
+  if (pass_entry(&st->done)) return;
+  const double beta = *reinterpret_cast<const volatile double *>(&st->beta);
+  while (i < n) {
+    p[i] = fma(beta, pi, zi);
+    i += stride;
+    if (i < n) zi = double(z[i]), pi = p[i];
+  }
 }
 
 // Start of the solve: p = z; bb = b.b, rho = r.z, rr = r.r.

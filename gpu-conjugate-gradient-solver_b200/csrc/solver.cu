@@ -519,8 +519,10 @@ class AmgPcg final : public Solver {
 
   // dir: 0 symmetric steps (forward then backward colours), 1 forward
   // sweeps only, 2 backward sweeps only (half_sweeps pre / post smoothing)
+  // first_done: the first colour of a sweep from zero is already in x
   template <typename BT>
-  void smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir = 0);
+  void smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir = 0, bool first_done = false);
+  FirstColour<VT> first_colour(int k, VT *x);
   template <typename BT>
   void gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaStream_t s);
   template <typename BT>
@@ -553,7 +555,7 @@ class AmgPcg final : public Solver {
   template <typename BT>
   void dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s);
   template <typename BT>
-  void vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s);
+  void vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s, bool first_done = false);
   // Colours [c0, c1) of a level; upper: only the entries at or past each
   // row's colour count (sell_upper_kernel).
   struct Part {
@@ -574,13 +576,13 @@ class AmgPcg final : public Solver {
   }
   template <typename BT>
   void level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, Part part, cudaStream_t s);
-  void restrict_residual(Level &L, Part part, VT *y, cudaStream_t s);
+  void restrict_residual(Level &L, Part part, VT *y, cudaStream_t s, FirstColour<VT> fc = FirstColour<VT>{});
   template <int kMode>
   void prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s);
-  void precondition(const double *r, VT *z, cudaStream_t s);
+  void precondition(const double *r, VT *z, cudaStream_t s, bool first_done = false);
   template <int kMode, typename BT>
   void transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g, const VT *x, VT *y,
-                const BT *b, cudaStream_t s);
+                const BT *b, cudaStream_t s, FirstColour<VT> fc = FirstColour<VT>{});
   void autotune();
   float time_ms(const std::function<void()> &f, int reps);
   void cg_iteration(int parity, cudaStream_t s);
@@ -624,7 +626,9 @@ class AmgPcg final : public Solver {
   int *q0_ = nullptr;                           // internal index of caller row i
   CgState *st_ = nullptr, *scratch_st_ = nullptr;
   double *partials_ = nullptr;
-  CgState *host_st_ = nullptr;                  // pinned, two slots
+  CgState *host_st_ = nullptr;                  // pinned
+  volatile unsigned *host_seq_ = nullptr;       // pinned, written by the convergence test (publish_state)
+  bool wait_published(int it);
   SweepSync *sync_ = nullptr;                   // grid-barrier state of the cooperative sweeps
   VT *wbuf_ = nullptr;
   bool unit_weights_ = false;  // installed colour weights are all 1
@@ -902,8 +906,9 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
   sync_ = ar_.alloc<SweepSync>(1);
   CK(cudaMemset(sync_, 0, sizeof(SweepSync)));
   partials_ = ar_.alloc<double>(3 * static_cast<size_t>(cap_blocks_) + 8);
-  CK(cudaMallocHost(&host_st_, 2 * sizeof(CgState)));
-  std::memset(host_st_, 0, 2 * sizeof(CgState));
+  CK(cudaMallocHost(&host_st_, sizeof(CgState) + 16));
+  std::memset(host_st_, 0, sizeof(CgState) + 16);
+  host_seq_ = reinterpret_cast<volatile unsigned *>(host_st_ + 1);
   CK(cudaDeviceSynchronize());
   setup_ms_[0] = ms_since(t_setup);
   const auto t_tune = clock::now();
@@ -1270,7 +1275,7 @@ void AmgPcg<VT>::gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaS
 // each step is a forward sweep over colours 0..C-1 then a backward sweep.
 template <typename VT>
 template <typename BT>
-void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir) {
+void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir, bool first_done) {
   const int *done = &st_->done;
   if (L.kind == 4) {  // IdentityPreconditioner::apply
     launch_pass(pdl_, convert_kernel<VT, BT>, blocks_for(L.n, cap_blocks_), s, L.n, rhs, x, done);
@@ -1310,6 +1315,7 @@ void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cu
       if (!zs) sweep_start(L, x, s);  // from zero the own colour is skipped anyway
       for (int i = 0; i < L.ncolors; ++i) {
         const int c = dir == 1 ? i : L.ncolors - 1 - i;
+        if (first_done && step == 0 && i == 0) continue;
         // from a zero iterate the first forward sweep skips the later colours'
         // gathers; a backward sweep from zero has no such shortcut
         gs_pass(L, c, rhs, x, zs, s);
@@ -1326,6 +1332,7 @@ void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cu
     if (!(zero && step == 0)) sweep_start(L, x, s);
     for (int c = 0; c < L.ncolors; ++c) {
       if (skip && step > 0 && c == 0) continue;  // the backward sweep just ended with colour 0
+      if (first_done && step == 0 && c == 0) continue;
       gs_pass(L, c, rhs, x, zero && step == 0, s);
     }
     sweep_start(L, x, s);
@@ -1588,7 +1595,7 @@ void AmgPcg<VT>::level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, P
     const int gb = blocks_for(32LL * (s1 - s0), cap_blocks_);
 #define RES_SELL(G)                                                                                      \
   if (part.upper) launch_pass(pdl_, sell_upper_kernel<VT, G>, gb, s, L.A.view(), x, r, done, s0, s1);     \
-  else launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.A.view(), x, r, rhs, done, s0, s1);
+  else launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.A.view(), x, r, rhs, done, s0, s1, FirstColour<VT>{});
     switch (L.g) {
       case 1: RES_SELL(1) break;
       case 2: RES_SELL(2) break;
@@ -1606,11 +1613,11 @@ void AmgPcg<VT>::level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, P
 
 // y = R r, with the columns of `part`'s rows only.
 template <typename VT>
-void AmgPcg<VT>::restrict_residual(Level &L, Part part, VT *y, cudaStream_t s) {
+void AmgPcg<VT>::restrict_residual(Level &L, Part part, VT *y, cudaStream_t s, FirstColour<VT> fc) {
   CsrvView<VT> v = L.Rc.view();
   if (part.c1 < L.ncolors) v = L.Rc.below();
   else if (part.c0 > 0) v = L.Rc.past();
-  transfer<kSpmvSet, VT>(L.R.view(), 0, L.R.nslices, v, 0, L.Rc.rows, L.rg, L.r, y, (const VT *)nullptr, s);
+  transfer<kSpmvSet, VT>(L.R.view(), 0, L.R.nslices, v, 0, L.Rc.rows, L.rg, L.r, y, (const VT *)nullptr, s, fc);
   CKL("restriction");
 }
 
@@ -1670,12 +1677,27 @@ void AmgPcg<VT>::dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s) {
   }
 }
 
+// The first pass of level k's pre-smoothing from zero, for the kernel that
+// writes its right-hand side; none where the level is not smoothed by
+// per-colour launches of scalar Gauss-Seidel passes.
+template <typename VT>
+FirstColour<VT> AmgPcg<VT>::first_colour(int k, VT *x) {
+  const Level &L = lv_[k];
+  const bool smoothed = k + 1 < static_cast<int>(lv_.size()) || opt_.coarse == 0;
+  const int steps = k + 1 < static_cast<int>(lv_.size()) ? opt_.pre : opt_.coarse_steps;
+  const int dir = k + 1 < static_cast<int>(lv_.size()) && opt_.half_sweeps ? 1 : 0;
+  if (!smoothed || L.kind != 0 || block_ || (tail_on_ && k >= tail_k0_) || in_cluster(L, steps, dir) ||
+      (L.coop && dir == 0 && !L.relaxed))
+    return FirstColour<VT>{};
+  return FirstColour<VT>{x, L.C.diag, L.color_first[1], L.wts[0], VT(opt_.omega)};
+}
+
 // MultigridSmoother::vCycle (src/Smoothers/MultigridSmoother.cc:337-412).
 // `zero`: x is an implicit zero vector on entry (the preconditioner zeroes z,
 // and every coarse correction starts from zero).
 template <typename VT>
 template <typename BT>
-void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s) {
+void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s, bool first_done) {
   Level &L = lv_[k];
   if (tail_on_ && k == tail_k0_) {
     launch_tail(s);  // the whole V-cycle of levels k..L-1, x_k from a zero guess
@@ -1686,16 +1708,17 @@ void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s) 
     if (opt_.coarse == 1) {
       dense_coarse<BT>(L, rhs, x, s);
     } else {
-      smooth(L, rhs, x, opt_.coarse_steps, zero, s);
+      smooth(L, rhs, x, opt_.coarse_steps, zero, s, 0, first_done);
     }
     return;
   }
-  smooth(L, rhs, x, opt_.pre, zero, s, opt_.half_sweeps ? 1 : 0);
+  smooth(L, rhs, x, opt_.pre, zero, s, opt_.half_sweeps ? 1 : 0, first_done);
   const Part part = resid_part(L, zero);
   level_spmv_resid(L, rhs, x, L.r, part, s);
   Level &C = lv_[k + 1];
-  restrict_residual(L, part, C.b, s);
-  vcycle<VT>(k + 1, C.b, C.x, true, s);
+  const FirstColour<VT> fc = first_colour(k + 1, C.x);
+  restrict_residual(L, part, C.b, s, fc);
+  vcycle<VT>(k + 1, C.b, C.x, true, s, fc.x != nullptr);
   if (opt_.reference_vcycle && k > 0) prolong<kSpmvTwice>(L, swept_part(L), C.x, x, s);
   else prolong<kSpmvAdd>(L, swept_part(L), C.x, x, s);
   smooth(L, rhs, x, opt_.post, false, s, opt_.half_sweeps ? 2 : 0);
@@ -1706,19 +1729,19 @@ void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s) 
 template <typename VT>
 template <int kMode, typename BT>
 void AmgPcg<VT>::transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g,
-                          const VT *x, VT *y, const BT *b, cudaStream_t s) {
+                          const VT *x, VT *y, const BT *b, cudaStream_t s, FirstColour<VT> fc) {
   const int *done = &st_->done;
   if (g == 1) {
     launch_pass(pdl_, sell_spmv_kernel<VT, BT, kMode>, blocks_for(32LL * (s1 - s0), cap_blocks_), s, S, x, y, b, done, s0,
-                s1);
+                s1, fc);
     return;
   }
   const int gb = blocks_for(static_cast<long long>(r1 - r0) * g, cap_blocks_);
   switch (g) {
-    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm, x, y, b, done, r0, r1); break;
-    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm, x, y, b, done, r0, r1); break;
-    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm, x, y, b, done, r0, r1); break;
-    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm, x, y, b, done, r0, r1); break;
+    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
+    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
+    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
+    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
   }
 }
 
@@ -2215,8 +2238,8 @@ void AmgPcg<VT>::setup_tail() {
 
 // Multigrid*Preconditioner::apply: z = 0, then `vcycles` V-cycles.
 template <typename VT>
-void AmgPcg<VT>::precondition(const double *r, VT *z, cudaStream_t s) {
-  for (int v = 0; v < opt_.vcycles; ++v) vcycle<double>(0, r, z, v == 0, s);
+void AmgPcg<VT>::precondition(const double *r, VT *z, cudaStream_t s, bool first_done) {
+  for (int v = 0; v < opt_.vcycles; ++v) vcycle<double>(0, r, z, v == 0, s, first_done && v == 0);
 }
 
 // The outer 3x3 block operator in BELL-32 with g lanes per node (rebuilt
@@ -2269,15 +2292,20 @@ void AmgPcg<VT>::tune_outer() {
 template <typename VT>
 void AmgPcg<VT>::outer_spmv(const double *v, CgState *st, cudaStream_t s) {
   if (!block_) {
-    cg_spmv_pap_kernel<<<blocks_for(32LL * cgA_.nslices, cap_blocks_), 256, 0, s>>>(cgA_.view(), v, ap_, st, partials_);
+    const int blocks = blocks_for(32LL * cgA_.nslices, cap_blocks_);
+    // small: one slice per warp, all of them resident at once
+    if (blocks * 8 >= cgA_.nslices)
+      launch_pass(pdl_, cg_spmv_pap_kernel<true>, blocks, s, cgA_.view(), v, ap_, st, partials_);
+    else
+      launch_pass(pdl_, cg_spmv_pap_kernel<false>, blocks, s, cgA_.view(), v, ap_, st, partials_);
     return;
   }
   const int blocks = blocks_for(32LL * cgB_.nslices, cap_blocks_);
   switch (cgB_.g) {
-    case 1: cg_bell_spmv_pap_kernel<1><<<blocks, 256, 0, s>>>(cgB_.view(), v, ap_, st, partials_); break;
-    case 2: cg_bell_spmv_pap_kernel<2><<<blocks, 256, 0, s>>>(cgB_.view(), v, ap_, st, partials_); break;
-    case 4: cg_bell_spmv_pap_kernel<4><<<blocks, 256, 0, s>>>(cgB_.view(), v, ap_, st, partials_); break;
-    default: cg_bell_spmv_pap_kernel<8><<<blocks, 256, 0, s>>>(cgB_.view(), v, ap_, st, partials_); break;
+    case 1: launch_pass(pdl_, cg_bell_spmv_pap_kernel<1>, blocks, s, cgB_.view(), v, ap_, st, partials_); break;
+    case 2: launch_pass(pdl_, cg_bell_spmv_pap_kernel<2>, blocks, s, cgB_.view(), v, ap_, st, partials_); break;
+    case 4: launch_pass(pdl_, cg_bell_spmv_pap_kernel<4>, blocks, s, cgB_.view(), v, ap_, st, partials_); break;
+    default: launch_pass(pdl_, cg_bell_spmv_pap_kernel<8>, blocks, s, cgB_.view(), v, ap_, st, partials_); break;
   }
 }
 
@@ -2303,12 +2331,14 @@ void AmgPcg<VT>::cg_iteration(int parity, cudaStream_t s) {
   VT *z_old = z_[parity], *z_new = z_[parity ^ 1];
   outer_spmv(p_, st_, s);
   CKL("cg spmv");
-  cg_update_xr_kernel<<<blocks_for(n0_, cap_blocks_), 256, 0, s>>>(n0_, x_, r_, p_, ap_, st_, partials_);
+  const int blocks = blocks_for(n0_, cap_blocks_);
+  const FirstColour<VT> fc = first_colour(0, z_new);
+  launch_pass(pdl_, cg_update_xr_kernel<VT>, blocks, s, n0_, x_, r_, p_, ap_, st_, partials_, fc, host_seq_);
   CKL("cg update");
-  precondition(r_, z_new, s);
-  cg_dot_rz_kernel<VT><<<blocks_for(n0_, cap_blocks_), 256, 0, s>>>(n0_, r_, z_new, opt_.flexible ? z_old : nullptr, st_, partials_);
+  precondition(r_, z_new, s, fc.x != nullptr);
+  launch_pass(pdl_, cg_dot_rz_kernel<VT>, blocks, s, n0_, r_, z_new, opt_.flexible ? z_old : nullptr, st_, partials_);
   CKL("cg dot");
-  cg_update_p_kernel<VT><<<blocks_for(n0_, cap_blocks_), 256, 0, s>>>(n0_, z_new, p_, st_);
+  launch_pass(pdl_, cg_update_p_kernel<VT>, blocks, s, n0_, z_new, p_, st_);
   CKL("cg p update");
 }
 
@@ -2345,6 +2375,23 @@ void AmgPcg<VT>::ensure_graphs() {
   }
 }
 
+// Waits until iteration `it`'s convergence test has run; whether the solve
+// stopped there (or before, on a breakdown or a fault).
+template <typename VT>
+bool AmgPcg<VT>::wait_published(int it) {
+  for (unsigned spins = 0;; ++spins) {
+    const unsigned v = *host_seq_;
+    if (v & 1u) return true;
+    if (v >= 2u * static_cast<unsigned>(it + 1)) return false;
+    if ((spins & 1023u) == 1023u) {
+      // an idle stream that published nothing: the solve was stopped elsewhere
+      const cudaError_t e = cudaStreamQuery(stream_);
+      if (e == cudaSuccess) return *host_seq_ < 2u * static_cast<unsigned>(it + 1) || (*host_seq_ & 1u) != 0;
+      if (e != cudaErrorNotReady) CK(e);
+    }
+  }
+}
+
 template <typename VT>
 void AmgPcg<VT>::run(cudaStream_t user, SolveStats *out) {
   // Order after the caller's stream, work on the solver's own stream.
@@ -2364,34 +2411,24 @@ void AmgPcg<VT>::run(cudaStream_t user, SolveStats *out) {
       hs.iterations = 0;
     }
   } else if (!hs.done) {
-    if (opt_.graph) {
-      ensure_graphs();
-      // Keep one iteration queued ahead of the host check; kernels of an
-      // iteration queued after the stop flag was set return immediately.
-      int it = 0;
-      for (; it < opt_.max_iter; ++it) {
+    // One iteration at a time, as CGSolver::solve; its convergence test runs
+    // before its V-cycle and tells the host through pinned memory, so the next
+    // iteration is queued while the V-cycle runs (and the V-cycle of the last
+    // one returns at once: its kernels see the stop flag).
+    if (opt_.graph) ensure_graphs();
+    *host_seq_ = 0u;
+    for (int it = 0; it < opt_.max_iter; ++it) {
+      if (opt_.graph) {
         CK(cudaGraphLaunch(exec_[it & 1], stream_));
         launches_ += graph_kernels_;
-        CK(cudaMemcpyAsync(&host_st_[it & 1], st_, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
-        CK(cudaEventRecord(ev_[it & 1], stream_));
-        if (it >= 1) {
-          CK(cudaEventSynchronize(ev_[(it - 1) & 1]));
-          if (host_st_[(it - 1) & 1].done) break;
-        }
-      }
-      CK(cudaStreamSynchronize(stream_));
-      CK(cudaMemcpy(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost));
-      hs = host_st_[0];
-    } else {
-      // CGSolver::solve: one submitAndWait and one scalar read per iteration.
-      for (int it = 0; it < opt_.max_iter; ++it) {
+      } else {
         cg_iteration(it & 1, stream_);
-        CK(cudaMemcpyAsync(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
-        CK(cudaStreamSynchronize(stream_));
-        if (host_st_[0].done) break;
       }
-      hs = host_st_[0];
+      if (wait_published(it)) break;
     }
+    CK(cudaMemcpyAsync(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
+    CK(cudaStreamSynchronize(stream_));
+    hs = host_st_[0];
     spmv = hs.iter;
   }
   CK(cudaEventRecord(ev_[3], stream_));
