@@ -50,8 +50,10 @@
 
 namespace gsb {
 
-constexpr int kClusterThreads = 512;    // at most; a layout may use fewer
+constexpr int kClusterThreads = 512;    // scalar levels
+constexpr int kClusterBlockThreads = 256;  // 3x3 levels: two units of 18 block values a thread
 constexpr int kClusterPairs = 4;        // slot pairs per lane loaded ahead
+constexpr int kClusterBlocks = 2;       // 3x3 blocks per lane loaded ahead
 constexpr int kClusterMaxPasses = 512;  // mbarriers
 constexpr int kClusterMaxSlots = 32760; // two copies of the slots in 16 bits
 constexpr int kClusterMaxColors = 128;
@@ -75,12 +77,15 @@ struct ClusterView {
   const unsigned *__restrict__ expect;         // [cta][colour]: rows of the colour that the CTA receives
   const int *__restrict__ slot_ptr;            // ncta + 1
   const int *__restrict__ slot_row;            // global row of each slot
-  const typename Pair<T>::type *__restrict__ val;
-  const unsigned *__restrict__ col;            // two slots; + max_slots + 1: the copy taken at the sweep's start
+  const T *__restrict__ val;                   // slot pairs (scalar), or 9 per block slot, component-major
+  const unsigned *__restrict__ col;            // two slots a pair; block slots: 16 bits each. + max_slots + 1: the
+                                               // copy taken at the sweep's start
   const unsigned *__restrict__ send;           // cta << 16 | slot, or kNoSend
   const unsigned short *__restrict__ own;      // slot of each row in its owner
-  const typename Pair<T>::type *__restrict__ diag;  // per row {d, 1 / d}; the latter 0 where it is not safe to use
+  const T *__restrict__ diag;                  // scalar: {d, 1 / d} per row, the latter 0 where it is not safe to
+                                               // use; 3x3: the inverse diagonal block per node
   int relaxed;                                 // own-colour reads from the sweep's start
+  int row0;                                    // first row of this system in the level's vectors (batches)
 };
 
 constexpr unsigned kNoSend = 0xffffffffu;
@@ -201,48 +206,173 @@ __device__ __forceinline__ bool pass_wait(unsigned bar) {
 
 }  // namespace cluster_detail
 
-// What one thread needs of one row before the iterate.
-template <typename T, typename BT>
-struct ClusterUnit {
-  typename Pair<T>::type v[kClusterPairs];
-  unsigned c[kClusterPairs];  // two slots
-  unsigned send;
-  typename Pair<T>::type d;
-  BT b;
+// Rows of a scalar level with R right-hand sides, vectors row-interleaved
+// ([row][R]): the arithmetic of csrv_gs_kernel (bcsrv_gs_kernel) with G lanes.
+template <typename T, typename BT, int G, int R>
+struct ClusterScalar {
+  using V = T;
+  using B = BT;
+  static constexpr int kLanes = G, kW = R, kThreads = kClusterThreads;
+  using P2 = typename Pair<T>::type;
+  // what one thread needs of one row before the iterate
+  struct Unit {
+    P2 v[kClusterPairs];
+    unsigned c[kClusterPairs];  // two slots
+    unsigned send;
+    P2 d;
+    BT b[R];
+  };
+
+  static __device__ __forceinline__ void load(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid, int row,
+                                              Unit &u) {
+    using cluster_detail::load_early;
+    const P2 *val = reinterpret_cast<const P2 *>(A.val);
+    const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
+#pragma unroll
+    for (int q = 0; q < kClusterPairs; ++q)
+      if (q < sg.pairs) {
+        u.v[q] = load_early(val + e0 + q * sg.stride);
+        u.c[q] = load_early(A.col + e0 + q * sg.stride);
+      }
+    u.d = load_early(reinterpret_cast<const P2 *>(A.diag) + row);
+  }
+  static __device__ __forceinline__ void load_b(const BT *b, int row, Unit &u) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) u.b[j] = cluster_detail::load_early(b + static_cast<size_t>(row) * R + j);
+  }
+  static __device__ __forceinline__ void add(T v, const T *xs, unsigned slot, T (&sum)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) sum[j] = fma(v, xs[slot * R + j], sum[j]);
+  }
+  // neighbour sums of the row (in every lane of its group)
+  static __device__ __forceinline__ void sums(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid,
+                                              const T *xs, const Unit &u, T (&sum)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) sum[j] = T(0);
+#pragma unroll
+    for (int q = 0; q < kClusterPairs; ++q)
+      if (q < sg.pairs) {
+        add(u.v[q].x, xs, u.c[q] & 0xffffu, sum);
+        add(u.v[q].y, xs, u.c[q] >> 16, sum);
+      }
+    if (sg.pairs > kClusterPairs) {
+      const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
+#pragma unroll 4
+      for (int q = kClusterPairs; q < sg.pairs; ++q) {
+        const P2 v = __ldg(reinterpret_cast<const P2 *>(A.val) + e0 + q * sg.stride);
+        const unsigned c = __ldg(A.col + e0 + q * sg.stride);
+        add(v.x, xs, c & 0xffffu, sum);
+        add(v.y, xs, c >> 16, sum);
+      }
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int j = 0; j < R; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o, G);
+  }
+  static __device__ __forceinline__ void update(const Unit &u, const T (&sum)[R], T (&xn)[R]) {
+#pragma unroll
+    for (int j = 0; j < R; ++j) xn[j] = cluster_detail::quotient(T(u.b[j]) - sum[j], u.d.x, u.d.y);
+  }
 };
 
-// The matrix part of a unit: trip t of piece sg.
-template <typename T, typename BT>
-__device__ __forceinline__ void cluster_load(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid, int local,
-                                             ClusterUnit<T, BT> &u) {
-  using cluster_detail::load_early;
-  const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
-#pragma unroll
-  for (int q = 0; q < kClusterPairs; ++q)
-    if (q < sg.pairs) {
-      u.v[q] = load_early(A.val + e0 + q * sg.stride);
-      u.c[q] = load_early(A.col + e0 + q * sg.stride);
-    }
-  u.send = load_early(A.send + sg.sbase + t * sg.schunks * sg.stride + tid);
-  u.d = load_early(A.diag + sg.row0 + min(local, sg.rows - 1));
-}
-
-// Smoothing steps of a scalar level; grid = one cluster of A.ncta CTAs.
+// Node rows of a 3x3 level: the arithmetic of bsrv_gs_kernel with G lanes.
 template <typename T, typename BT, int G>
-__global__ void __launch_bounds__(kClusterThreads, 1)
-    cluster_gs_kernel(ClusterView<T> A, ClusterPasses P, const BT *__restrict__ b, T *__restrict__ x, int zero,
-                      const T *__restrict__ wts, T omega, CgState *st) {
+struct ClusterBlock {
+  using V = T;
+  using B = BT;
+  static constexpr int kLanes = G, kW = 3, kThreads = kClusterBlockThreads;
+  struct Unit {
+    T v[kClusterBlocks][9];
+    unsigned short c[kClusterBlocks];
+    unsigned send;
+    T d[9];
+    BT b[3];
+  };
+
+  static __device__ __forceinline__ void load(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid, int row,
+                                              Unit &u) {
+    using cluster_detail::load_early;
+    const unsigned short *col = reinterpret_cast<const unsigned short *>(A.col);
+#pragma unroll
+    for (int q = 0; q < kClusterBlocks; ++q)
+      if (q < sg.pairs) {
+        const int e = t * sg.pairs + q;
+        u.c[q] = load_early(col + sg.base + e * sg.stride + tid);
+#pragma unroll
+        for (int k = 0; k < 9; ++k) u.v[q][k] = load_early(A.val + 9 * sg.base + (9 * e + k) * sg.stride + tid);
+      }
+#pragma unroll
+    for (int k = 0; k < 9; ++k) u.d[k] = load_early(A.diag + 9 * static_cast<size_t>(row) + k);
+  }
+  static __device__ __forceinline__ void load_b(const BT *b, int row, Unit &u) {
+#pragma unroll
+    for (int j = 0; j < 3; ++j) u.b[j] = cluster_detail::load_early(b + 3 * static_cast<size_t>(row) + j);
+  }
+  static __device__ __forceinline__ void add(const T (&v)[9], const T *x, T (&sum)[3]) {
+    const T x0 = x[0], x1 = x[1], x2 = x[2];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) sum[r] = fma(v[3 * r], x0, fma(v[3 * r + 1], x1, fma(v[3 * r + 2], x2, sum[r])));
+  }
+  static __device__ __forceinline__ void sums(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid,
+                                              const T *xs, const Unit &u, T (&sum)[3]) {
+    sum[0] = sum[1] = sum[2] = T(0);
+#pragma unroll
+    for (int q = 0; q < kClusterBlocks; ++q)
+      if (q < sg.pairs) add(u.v[q], xs + 3 * static_cast<unsigned>(u.c[q]), sum);
+    const unsigned short *col = reinterpret_cast<const unsigned short *>(A.col);
+#pragma unroll 2
+    for (int q = kClusterBlocks; q < sg.pairs; ++q) {
+      const int e = t * sg.pairs + q;
+      T v[9];
+#pragma unroll
+      for (int k = 0; k < 9; ++k) v[k] = __ldg(A.val + 9 * sg.base + (9 * e + k) * sg.stride + tid);
+      add(v, xs + 3 * static_cast<unsigned>(__ldg(col + sg.base + e * sg.stride + tid)), sum);
+    }
+#pragma unroll
+    for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+      for (int r = 0; r < 3; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o, G);
+  }
+  static __device__ __forceinline__ void update(const Unit &u, const T (&sum)[3], T (&xn)[3]) {
+    const T r0 = T(u.b[0]) - sum[0], r1 = T(u.b[1]) - sum[1], r2 = T(u.b[2]) - sum[2];
+#pragma unroll
+    for (int r = 0; r < 3; ++r) {
+      T nv = u.d[3 * r] * r0;
+      nv = fma(u.d[3 * r + 1], r1, nv);
+      xn[r] = fma(u.d[3 * r + 2], r2, nv);
+    }
+  }
+};
+
+// Where a launch reads its stop flag and records a fault.
+struct ClusterStatus {
+  int *stop;   // nonzero: nothing to do
+  int *fault;  // set when a wait gave up (and *stop with it)
+};
+
+// Smoothing steps of the level (or, in a batch, of one system of the level)
+// that A describes; called by every thread of its cluster.
+template <typename Row>
+__device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V> &A, const ClusterPasses &P,
+                                              const typename Row::B *__restrict__ b, typename Row::V *__restrict__ x,
+                                              int zero, const typename Row::V *__restrict__ wts,
+                                              const typename Row::V *__restrict__ nw, typename Row::V omega,
+                                              ClusterStatus status) {
   using namespace cluster_detail;
+  using T = typename Row::V;
+  constexpr int W = Row::kW, G = Row::kLanes;
   extern __shared__ __align__(16) unsigned char cluster_smem[];
   __shared__ ClusterSeg seg[kClusterMaxColors];
   __shared__ unsigned long long bars[kClusterMaxPasses];
   // colour of each pass, bit 15 on the last one of a sweep; 0xffff at the end
   __shared__ unsigned short plist[kClusterMaxPasses + 1];
-  T *xs = reinterpret_cast<T *>(cluster_smem);  // max_slots + 1, the last one zero (then the sweep's start)
+  // max_slots + 1 slots of W values, the last one zero (then the sweep's start)
+  T *xs = reinterpret_cast<T *>(cluster_smem);
   const int tid = threadIdx.x, nthr = A.threads;
   const unsigned me = cta_rank();
   const int s0 = __ldg(A.slot_ptr + me), nslots = __ldg(A.slot_ptr + me + 1) - s0;
-  T *xp = xs + A.max_slots + 1;
+  T *xp = xs + (A.max_slots + 1) * W;
   for (int c = tid; c < A.ncolors; c += nthr) seg[c] = A.seg[me * A.ncolors + c];
   const int npass = P.total();
   for (int p = tid; p < npass; p += nthr)
@@ -254,7 +384,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     const int n = P.count(s), f = P.first(s), dr = P.direction(s);
     for (int i = tid; i < n; i += nthr) {
       const int c = f + dr * i;
-      mbar_expect_tx(bars + p + i, __ldg(A.expect + me * A.ncolors + c) * static_cast<unsigned>(sizeof(T)));
+      mbar_expect_tx(bars + p + i, __ldg(A.expect + me * A.ncolors + c) * static_cast<unsigned>(W * sizeof(T)));
       plist[p + i] = static_cast<unsigned short>(c | (i + 1 == n ? 0x8000 : 0));
     }
     p += n;
@@ -264,15 +394,19 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   // the first row's matrix operands do not change during a solve
   constexpr int kLog = G == 4 ? 2 : (G == 8 ? 3 : (G == 16 ? 4 : 5));
   const int grp = tid >> kLog, groups = nthr >> kLog;
-  ClusterUnit<T, BT> cur, nxt;
+  typename Row::Unit cur, nxt;
   unsigned code = plist[0];
   ClusterSeg sg = seg[code & 0x7fffu];
-  if (tid < sg.stride) cluster_load<T, BT>(A, sg, 0, tid, grp, cur);
-  const bool stop = pass_entry(&st->done);  // the same in every CTA: only a finished kernel writes it
+  if (tid < sg.stride) {
+    Row::load(A, sg, 0, tid, sg.row0 + min(grp, sg.rows - 1), cur);
+    cur.send = load_early(A.send + sg.sbase + tid);
+  }
+  const bool stop = pass_entry(status.stop);  // the same in every CTA: only a finished kernel writes it
   if (!stop) {
-    if (tid < sg.stride) cur.b = load_early(b + sg.row0 + min(grp, sg.rows - 1));
-    for (int i = tid; i <= A.max_slots; i += nthr) {
-      const T v = zero || i >= nslots ? T(0) : x[__ldg(A.slot_row + s0 + i)];
+    if (tid < sg.stride) Row::load_b(b, sg.row0 + min(grp, sg.rows - 1), cur);
+    for (int i = tid; i < (A.max_slots + 1) * W; i += nthr) {
+      const int slot = i / W;
+      const T v = zero || slot >= nslots ? T(0) : x[static_cast<size_t>(__ldg(A.slot_row + s0 + slot)) * W + i % W];
       xs[i] = v;
       if (A.relaxed) xp[i] = v;
     }
@@ -294,48 +428,44 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     if (next_code != 0xffffu) {
       sn = seg[next_code & 0x7fffu];
       if (tid < sn.stride) {
-        const int local = tn * groups + grp;
-        cluster_load<T, BT>(A, sn, tn, tid, local, nxt);
-        nxt.b = load_early(b + sn.row0 + min(local, sn.rows - 1));
+        const int row = sn.row0 + min(tn * groups + grp, sn.rows - 1);
+        Row::load(A, sn, tn, tid, row, nxt);
+        nxt.send = load_early(A.send + sn.sbase + tn * sn.schunks * sn.stride + tid);
+        Row::load_b(b, row, nxt);
       }
     }
     const unsigned to_cta = (cur.send >> 16) & 15u;
-    const unsigned to_x = remote(xs_addr + static_cast<unsigned>(sizeof(T)) * (cur.send & 0xffffu), to_cta);
+    const unsigned to_x = remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (cur.send & 0xffffu), to_cta);
     const unsigned to_bar = remote(bar_addr + 8 * p, to_cta);
     if (t == 0 && !fresh && !dead) dead = !pass_wait(bar_addr + 8 * (p - 1));
     if (tid < sg.stride) {
-      T sum = T(0);
-#pragma unroll
-      for (int q = 0; q < kClusterPairs; ++q)
-        if (q < sg.pairs) {
-          sum = fma(cur.v[q].x, xs[cur.c[q] & 0xffffu], sum);
-          sum = fma(cur.v[q].y, xs[cur.c[q] >> 16], sum);
-        }
-      if (sg.pairs > kClusterPairs) {
-        const int e0 = sg.base + t * sg.pairs * sg.stride + tid;
-#pragma unroll 4
-        for (int q = kClusterPairs; q < sg.pairs; ++q) {
-          const typename Pair<T>::type v = __ldg(A.val + e0 + q * sg.stride);
-          const unsigned c = __ldg(A.col + e0 + q * sg.stride);
-          sum = fma(v.x, xs[c & 0xffffu], sum);
-          sum = fma(v.y, xs[c >> 16], sum);
-        }
-      }
-#pragma unroll
-      for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
+      T sum[W], xn[W];
+      Row::sums(A, sg, t, tid, xs, cur, sum);
       const int local = t * groups + grp;
       if (local < sg.rows) {
-        T xn = quotient(T(cur.b) - sum, cur.d.x, cur.d.y);
-        const T w = wts != nullptr ? __ldg(wts + (code & 0x7fffu)) : omega;
-        if (w != T(1)) xn = fma(T(1) - w, xs[__ldg(A.own + sg.row0 + local)], w * xn);
-        if (cur.send != kNoSend) send_value(to_x, xn, to_bar);
+        Row::update(cur, sum, xn);
+        const T w = nw != nullptr ? __ldg(nw + sg.row0 + local)
+                                  : (wts != nullptr ? __ldg(wts + (code & 0x7fffu)) : omega);
+        if (w != T(1)) {
+          const unsigned own = W * __ldg(A.own + sg.row0 + local);
+#pragma unroll
+          for (int j = 0; j < W; ++j) xn[j] = fma(T(1) - w, xs[own + j], w * xn[j]);
+        }
+        if (cur.send != kNoSend)
+#pragma unroll
+          for (int j = 0; j < W; ++j) send_value(to_x + j * static_cast<unsigned>(sizeof(T)), xn[j], to_bar);
         for (int q = 1; q < sg.schunks; ++q) {
           const unsigned to = __ldg(A.send + sg.sbase + (t * sg.schunks + q) * sg.stride + tid);
-          if (to != kNoSend)
-            send_value(remote(xs_addr + static_cast<unsigned>(sizeof(T)) * (to & 0xffffu), to >> 16), xn,
-                       remote(bar_addr + 8 * p, to >> 16));
+          if (to != kNoSend) {
+            const unsigned rx = remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (to & 0xffffu), to >> 16);
+            const unsigned rb = remote(bar_addr + 8 * p, to >> 16);
+#pragma unroll
+            for (int j = 0; j < W; ++j) send_value(rx + j * static_cast<unsigned>(sizeof(T)), xn[j], rb);
+          }
         }
-        if (p >= keep && (tid & (G - 1)) == 0) x[sg.row0 + local] = xn;
+        if (p >= keep && (tid & (G - 1)) == 0)
+#pragma unroll
+          for (int j = 0; j < W; ++j) x[static_cast<size_t>(sg.row0 + local) * W + j] = xn[j];
       }
     }
     fresh = false;
@@ -346,7 +476,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         if (!dead) dead = !pass_wait(bar_addr + 8 * p);
         if (A.relaxed) {
           __syncthreads();
-          for (int k = tid; k < nslots; k += nthr) xp[k] = xs[k];
+          for (int k = tid; k < nslots * W; k += nthr) xp[k] = xs[k];
         }
         cluster_barrier();
         if (next_code == 0xffffu) break;
@@ -360,9 +490,19 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     cur = nxt;
   }
   if (dead) {
-    st->sync_fault = 1;
-    st->done = 1;
+    *status.fault = 1;
+    *status.stop = 1;
   }
+}
+
+// Grid = one cluster of A.ncta CTAs. wts: per colour, nw: per node (or
+// nullptr).
+template <typename Row>
+__global__ void __launch_bounds__(Row::kThreads, 1)
+    cluster_gs_kernel(ClusterView<typename Row::V> A, ClusterPasses P, const typename Row::B *__restrict__ b,
+                      typename Row::V *__restrict__ x, int zero, const typename Row::V *__restrict__ wts,
+                      const typename Row::V *__restrict__ nw, typename Row::V omega, CgState *st) {
+  cluster_steps<Row>(A, P, b, x, zero, wts, nw, omega, ClusterStatus{&st->done, &st->sync_fault});
 }
 
 }  // namespace gsb

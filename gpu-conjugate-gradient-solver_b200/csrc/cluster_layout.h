@@ -17,11 +17,11 @@ struct HostCluster {
   std::vector<ClusterSeg> seg;
   std::vector<unsigned> expect;
   std::vector<int> slot_ptr, slot_row;
-  std::vector<T> val;                // two per pair
-  std::vector<unsigned short> col;   // two per pair
+  std::vector<T> val;                // two per pair, or nine per block slot
+  std::vector<unsigned short> col;   // two per pair, or one per block slot
   std::vector<unsigned> send;
   std::vector<unsigned short> own;
-  std::vector<T> diag;               // {d, 1 / d} per row
+  std::vector<T> diag;               // scalar levels: {d, 1 / d} per row
 };
 
 // Rows [lo, hi) of colour piece q of ncta over [r0, r1).
@@ -29,32 +29,21 @@ inline int cluster_cut(int r0, int r1, int q, int ncta) {
   return r0 + static_cast<int>(static_cast<long long>(r1 - r0) * q / ncta);
 }
 
-// {d, 1 / d} of every row; the reciprocal is 0 where d or 1 / d is too close
-// to the ends of T's range for the kernel's quotient.
-template <typename T>
-void cluster_diag(const Csr &a, HostCluster<T> &h) {
-  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p60f);
-  h.diag.assign(2 * static_cast<size_t>(a.rows), T(0));
-  for (int r = 0; r < a.rows; ++r)
-    for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
-      if (a.ci[k] == r) {
-        const T d = T(a.v[k]);
-        h.diag[2 * static_cast<size_t>(r)] = d;
-        h.diag[2 * static_cast<size_t>(r) + 1] = std::fabs(d) < big && std::fabs(d) > T(1) / big ? T(1) / d : T(0);
-      }
-}
-
-// Layout of the square scalar matrix `a` (rows in colour-contiguous order,
-// colour c = rows [first[c], first[c + 1]), sorted columns) for ncta CTAs and
-// g lanes per row, with the k-th off-diagonal entry of a row on lane k % g as
-// the CSR-vector kernels read it. False when the level does not qualify: a
-// CTA needs more than `slot_limit` slots, a single colour, too many colours,
-// or a row is read by a row that its own owner does not read (the pattern is
-// not structurally symmetric; see the race argument in cluster.cuh).
-template <typename T>
-bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, int threads, bool relaxed,
-                  int slot_limit, HostCluster<T> &h) {
-  const int n = a.rows, nc = static_cast<int>(first.size()) - 1;
+// Layout of a level with n rows (or 3x3 nodes) in colour-contiguous order,
+// colour c = rows [first[c], first[c + 1]), whose off-diagonal pattern is
+// (rp, ci), columns ascending, for ncta CTAs of `threads` threads and g lanes
+// per row: the k-th entry of a row goes to lane k % g, as the CSR-vector
+// kernels read it, as that lane's entry k / g; `per` entries share a slot word
+// (2 on scalar levels, 1 on 3x3 ones). put(e, at, step) stores entry e's values
+// (scalar: at `at`; 3x3: component c at at + c * step). False when the level
+// does not qualify: a CTA needs more than `slot_limit` slots, a single colour,
+// too many colours, or a row is read by a row that its own owner does not
+// read (the pattern is not structurally symmetric; see the race argument in
+// cluster.cuh).
+template <typename T, typename F>
+bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &first, int per,
+                   int g, int ncta, int threads, bool relaxed, int slot_limit, HostCluster<T> &h, F put) {
+  const int nc = static_cast<int>(first.size()) - 1, values = per == 2 ? 2 : 9;  // values per slot word
   if (nc < 2 || nc > kClusterMaxColors || n < 1) return false;
   const int limit = std::min(slot_limit, kClusterMaxSlots);
   if (static_cast<long long>(n) > static_cast<long long>(limit) * ncta) return false;
@@ -76,7 +65,7 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
       for (int c = 0; c < nc; ++c)
         for (int r = cluster_cut(first[c], first[c + 1], q, ncta); r < cluster_cut(first[c], first[c + 1], q + 1, ncta); ++r) {
           need[r] = 1;
-          for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) need[a.ci[k]] = 1;
+          for (int k = rp[r]; k < rp[r + 1]; ++k) need[ci[k]] = 1;
         }
       slot[q].assign(n, none);
       for (int r = 0; r < n; ++r)
@@ -110,7 +99,7 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
   std::vector<unsigned> dests(n, 0);  // CTAs that keep row r
   for (int q = 0; q < ncta; ++q)
     for (int r : rows_of[q]) dests[r] |= 1u << q;
-  long long pairs_total = 0, send_total = 0;
+  long long words = 0, send_total = 0;
   std::vector<int> ok(ncta, 1);
   for (int q = 0; q < ncta; ++q)
     for (int c = 0; c < nc; ++c) {
@@ -119,28 +108,26 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
       s.rows = cluster_cut(first[c], first[c + 1], q + 1, ncta) - s.row0;
       int len = 0, deg = 1;
       for (int r = s.row0; r < s.row0 + s.rows; ++r) {
-        int off = 0;
-        for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) off += a.ci[k] != r ? 1 : 0;
-        len = std::max(len, off);
+        len = std::max(len, rp[r + 1] - rp[r]);
         deg = std::max(deg, __builtin_popcount(dests[r]));
       }
-      s.pairs = ((len + g - 1) / g + 1) / 2;
+      s.pairs = ((len + g - 1) / g + per - 1) / per;
       s.stride = std::min(threads, (s.rows * g + 31) / 32 * 32);
       s.schunks = (deg + g - 1) / g;
       const int trips = (s.rows + groups - 1) / groups;
       s.trips = std::max(1, trips);
-      s.base = static_cast<int>(pairs_total);
+      s.base = static_cast<int>(words);
       s.sbase = static_cast<int>(send_total);
-      pairs_total += static_cast<long long>(trips) * s.pairs * s.stride;
+      words += static_cast<long long>(trips) * s.pairs * s.stride;
       send_total += static_cast<long long>(trips) * s.schunks * s.stride;
-      if (pairs_total > (1LL << 27) || send_total > (1LL << 28)) return false;  // 32-bit offsets in the kernel
+      if (words * values > (1LL << 28) || send_total > (1LL << 28)) return false;  // 32-bit offsets in the kernel
       // rows of colour c among CTA q's slots
       const auto &rq = rows_of[q];
-      h.expect[static_cast<size_t>(q) * nc + c] = static_cast<unsigned>(std::lower_bound(rq.begin(), rq.end(), first[c + 1]) -
-                                       std::lower_bound(rq.begin(), rq.end(), first[c]));
+      h.expect[static_cast<size_t>(q) * nc + c] = static_cast<unsigned>(
+          std::lower_bound(rq.begin(), rq.end(), first[c + 1]) - std::lower_bound(rq.begin(), rq.end(), first[c]));
     }
-  h.val.assign(2 * static_cast<size_t>(pairs_total), T(0));
-  h.col.assign(2 * static_cast<size_t>(pairs_total), zero_slot);
+  h.val.assign(static_cast<size_t>(values) * words, T(0));
+  h.col.assign(static_cast<size_t>(per) * words, zero_slot);
   h.send.assign(static_cast<size_t>(send_total), kNoSend);
   parallel_for(ncta, [&](long long q0, long long q1) {
     for (long long q = q0; q < q1; ++q)
@@ -148,22 +135,23 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
         const ClusterSeg &s = h.seg[static_cast<size_t>(q) * nc + c];
         for (int i = 0; i < s.rows; ++i) {
           const int r = s.row0 + i, t = i / groups, lane0 = (i % groups) * g;
-          int k = 0;
-          for (int e = a.rp[r]; e < a.rp[r + 1]; ++e) {
-            const int j = a.ci[e];
-            if (j == r) continue;
-            const int lane = k % g, kk = k / g;
-            const size_t at = 2 * (static_cast<size_t>(s.base) + (static_cast<size_t>(t) * s.pairs + kk / 2) * s.stride +
-                                   lane0 + lane) + (kk & 1);
+          for (int e = rp[r]; e < rp[r + 1]; ++e) {
+            const int j = ci[e], k = e - rp[r], lane = lane0 + k % g, kk = k / g;
             unsigned short sl = slot[q][j];
             if (colour[j] == c) {
               if (!relaxed) ok[q] = 0;  // two coupled rows of one colour
               sl = static_cast<unsigned short>(sl + h.max_slots + 1);
             }
             if (slot[owner[j]][r] == none) ok[q] = 0;  // j's owner does not receive r
-            h.col[at] = sl;
-            h.val[at] = T(a.v[e]);
-            ++k;
+            const size_t word = static_cast<size_t>(t) * s.pairs + kk / per;  // of the lane, within the piece
+            if (per == 2) {
+              const size_t at = 2 * (s.base + word * s.stride + lane) + (kk & 1);
+              h.col[at] = sl;
+              put(e, at, 0);
+            } else {
+              h.col[s.base + word * s.stride + lane] = sl;
+              put(e, 9 * static_cast<size_t>(s.base) + 9 * word * s.stride + lane, s.stride);
+            }
           }
           int d = 0;
           for (int to = 0; to < ncta; ++to) {
@@ -177,8 +165,69 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
   }, 1);
   for (int q = 0; q < ncta; ++q)
     if (!ok[q]) return false;
-  cluster_diag(a, h);
   return true;
+}
+
+// The layout of a square scalar matrix (sorted columns), with {d, 1 / d} of
+// every row; the reciprocal is 0 where d or 1 / d is too close to the ends of
+// T's range for the kernel's quotient.
+template <typename T>
+bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, bool relaxed, int slot_limit,
+                  HostCluster<T> &h) {
+  std::vector<int> rp(a.rows + 1, 0), ci, from;
+  ci.reserve(a.ci.size());
+  from.reserve(a.ci.size());
+  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p60f);
+  h.diag.assign(2 * static_cast<size_t>(a.rows), T(0));
+  for (int r = 0; r < a.rows; ++r) {
+    for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) {
+      if (a.ci[k] != r) {
+        ci.push_back(a.ci[k]);
+        from.push_back(k);
+        continue;
+      }
+      const T d = T(a.v[k]);
+      h.diag[2 * static_cast<size_t>(r)] = d;
+      h.diag[2 * static_cast<size_t>(r) + 1] = std::fabs(d) < big && std::fabs(d) > T(1) / big ? T(1) / d : T(0);
+    }
+    rp[r + 1] = static_cast<int>(ci.size());
+  }
+  return cluster_build<T>(a.rows, rp, ci, first, 2, g, ncta, kClusterThreads, relaxed, slot_limit, h,
+                          [&](int e, size_t at, int) { h.val[at] = T(a.v[from[e]]); });
+}
+
+// The layout of a 3x3-blocked matrix, `first` in nodes; the inverse diagonal
+// blocks stay where the level has them (upload_cluster).
+template <typename T>
+bool make_cluster_blocks(const Csr &a, const std::vector<int> &first, int g, int ncta, bool relaxed, int slot_limit,
+                         HostCluster<T> &h) {
+  const int nn = a.rows / 3;
+  std::vector<int> rp(nn + 1, 0), ci, cols;
+  std::vector<T> v;  // 9 per block, row-major
+  for (int I = 0; I < nn; ++I) {
+    cols.clear();
+    for (int r = 3 * I; r < 3 * I + 3; ++r)
+      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
+        if (a.ci[k] / 3 != I) cols.push_back(a.ci[k] / 3);
+    std::sort(cols.begin(), cols.end());
+    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
+    const size_t base = v.size();
+    v.resize(base + 9 * cols.size(), T(0));
+    for (int r = 0; r < 3; ++r)
+      for (int k = a.rp[3 * I + r]; k < a.rp[3 * I + r + 1]; ++k) {
+        const int J = a.ci[k] / 3;
+        if (J == I) continue;
+        const size_t q = std::lower_bound(cols.begin(), cols.end(), J) - cols.begin();
+        v[base + 9 * q + 3 * r + a.ci[k] % 3] = T(a.v[k]);
+      }
+    ci.insert(ci.end(), cols.begin(), cols.end());
+    rp[I + 1] = static_cast<int>(ci.size());
+  }
+  return cluster_build<T>(nn, rp, ci, first, 1, g, ncta, kClusterBlockThreads, relaxed, slot_limit, h,
+                          [&](int e, size_t at, int step) {
+                            for (int c = 0; c < 9; ++c)
+                              h.val[at + static_cast<size_t>(c) * step] = v[9 * static_cast<size_t>(e) + c];
+                          });
 }
 
 template <typename T>
@@ -187,27 +236,31 @@ struct DevCluster {
   T *val = nullptr, *diag = nullptr;  // what a value refresh overwrites
   size_t values = 0;
   ClusterView<T> v{};
-  size_t smem() const { return (static_cast<size_t>(max_slots) + 1) * sizeof(T) * (v.relaxed ? 2 : 1); }
+  // dynamic shared memory of a CTA, `width` values a slot
+  size_t smem(int width) const {
+    return (static_cast<size_t>(max_slots) + 1) * width * sizeof(T) * (v.relaxed ? 2 : 1);
+  }
 };
 
+// `diag`: the level's inverse diagonal blocks (3x3 levels), else nullptr.
 template <typename T>
-DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h) {
+DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, int row0 = 0) {
   DevCluster<T> d;
   d.g = h.g, d.ncta = h.ncta, d.threads = h.threads, d.max_slots = h.max_slots;
   d.values = h.val.size();
   d.v.ncta = h.ncta, d.v.ncolors = h.ncolors, d.v.threads = h.threads, d.v.max_slots = h.max_slots;
   d.v.relaxed = h.relaxed;
+  d.v.row0 = row0;
   d.v.seg = ar.upload(h.seg);
   d.v.expect = ar.upload(h.expect);
   d.v.slot_ptr = ar.upload(h.slot_ptr);
   d.v.slot_row = ar.upload(h.slot_row);
-  d.val = ar.upload(h.val);
-  d.v.val = reinterpret_cast<const typename Pair<T>::type *>(d.val);
+  d.v.val = d.val = ar.upload(h.val);
   d.v.col = reinterpret_cast<const unsigned *>(ar.upload(h.col));
   d.v.send = ar.upload(h.send);
   d.v.own = ar.upload(h.own);
-  d.diag = ar.upload(h.diag);
-  d.v.diag = reinterpret_cast<const typename Pair<T>::type *>(d.diag);
+  if (diag == nullptr) diag = d.diag = ar.upload(h.diag);
+  d.v.diag = diag;
   return d;
 }
 

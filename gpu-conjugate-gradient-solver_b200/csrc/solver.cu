@@ -375,13 +375,16 @@ void refresh_sell(const DevSell<T> &d, const Csr &a, const std::vector<int> &bou
 }
 
 template <typename T>
-void refresh_cluster(const DevCluster<T> &d, const Csr &a, const std::vector<int> &bounds) {
+void refresh_cluster(const DevCluster<T> &d, const Csr &a, const std::vector<int> &bounds, bool block) {
   HostCluster<T> h;
-  if (!make_cluster<T>(a, bounds, d.g, d.ncta, d.threads, d.v.relaxed != 0, kClusterMaxSlots, h) ||
-      h.val.size() != d.values || h.max_slots != d.max_slots)
+  const bool relaxed = d.v.relaxed != 0;
+  const bool built = block ? make_cluster_blocks<T>(a, bounds, d.g, d.ncta, relaxed, kClusterMaxSlots, h)
+                           : make_cluster<T>(a, bounds, d.g, d.ncta, relaxed, kClusterMaxSlots, h);
+  if (!built || h.val.size() != d.values || h.max_slots != d.max_slots)
     throw std::runtime_error("update_values: the matrix sparsity changed");
   GSB_CK(cudaMemcpy(d.val, h.val.data(), sizeof(T) * h.val.size(), cudaMemcpyHostToDevice));
-  GSB_CK(cudaMemcpy(d.diag, h.diag.data(), sizeof(T) * h.diag.size(), cudaMemcpyHostToDevice));
+  if (d.diag != nullptr)  // scalar levels; the inverse blocks are the level's own
+    GSB_CK(cudaMemcpy(d.diag, h.diag.data(), sizeof(T) * h.diag.size(), cudaMemcpyHostToDevice));
 }
 
 template <typename T>
@@ -1055,6 +1058,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
       refresh_bell(lv.B1, Ai, lv.color_first);
       if (lv.B.val != lv.B1.val) refresh_bell(lv.B, Ai, lv.color_first);
       refresh_bsrv(lv.Bv, Ai);
+      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first, true);
       if (k == 0) refresh_bell(cgB_, Ai, lv.color_first);
     } else {
       for (int r = 0; r < Ai.rows; ++r) {
@@ -1066,7 +1070,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
       refresh_sell(lv.A1, Ai, lv.color_first, true);
       if (lv.A.val != lv.A1.val) refresh_sell(lv.A, Ai, lv.color_first, true);
       refresh_csrv(lv.C, Ai, true);
-      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first);
+      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first, false);
       if (k == 0) refresh_sell(cgA_, Ai, lv.color_first, true);
       if (lv.kind == 2) {
         std::vector<VT> jd(Ai.rows, VT(0));
@@ -1452,11 +1456,17 @@ struct ClusterLaunch {
 template <typename VT>
 template <typename BT>
 void AmgPcg<VT>::cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero, int dir, cudaStream_t s) {
-  ClusterLaunch l(L.K.ncta, L.K.threads, L.K.smem(), pdl_, s);
+  ClusterLaunch l(L.K.ncta, L.K.threads, L.K.smem(block_ ? 3 : 1), pdl_, s);
   const VT *w = L.wts.empty() ? nullptr : L.wts[0];
+  const VT *nw = L.nwts;
   with_lanes(L.K.g, [&](auto G) {
-    CK(cudaLaunchKernelEx(&l.cfg, cluster_gs_kernel<VT, BT, decltype(G)::value>, L.K.v, cluster_passes(L, steps, dir),
-                          rhs, x, zero ? 1 : 0, w, VT(opt_.omega), st_));
+    constexpr int g = decltype(G)::value;
+    auto go = [&](auto kernel) {
+      CK(cudaLaunchKernelEx(&l.cfg, kernel, L.K.v, cluster_passes(L, steps, dir), rhs, x, zero ? 1 : 0, w, nw,
+                            VT(opt_.omega), st_));
+    };
+    if (block_) go(cluster_gs_kernel<ClusterBlock<VT, BT, g>>);
+    else go(cluster_gs_kernel<ClusterScalar<VT, BT, g, 1>>);
   });
   CKL("cluster Gauss-Seidel step");
 }
@@ -1467,9 +1477,10 @@ int AmgPcg<VT>::cluster_limit(bool relaxed) {
   int optin = 0;
   CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
   cudaFuncAttributes fa{};
-  CK(cudaFuncGetAttributes(&fa, cluster_gs_kernel<VT, VT, 8>));
+  CK(cudaFuncGetAttributes(&fa, cluster_gs_kernel<ClusterScalar<VT, VT, 8, 1>>));
   const long long bytes = optin - static_cast<long long>(fa.sharedSizeBytes) - 1024;
-  return static_cast<int>(std::min<long long>(kClusterMaxSlots, bytes / static_cast<long long>(sizeof(VT) * (relaxed ? 2 : 1)) - 1));
+  const long long slot = static_cast<long long>(sizeof(VT)) * (block_ ? 3 : 1) * (relaxed ? 2 : 1);
+  return static_cast<int>(std::min<long long>(kClusterMaxSlots, bytes / slot - 1));
 }
 
 // Largest cluster (16 or 8 CTAs) the device co-schedules with `smem` bytes per
@@ -1489,15 +1500,19 @@ int AmgPcg<VT>::cluster_ctas(int g, size_t smem) {
       CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
       if (smem > static_cast<size_t>(most)) return 0;
       for (int want : {16, 8}) {
-        ClusterLaunch l(want, kClusterThreads, smem, false, nullptr);
+        ClusterLaunch l(want, block_ ? kClusterBlockThreads : kClusterThreads, smem, false, nullptr);
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) return want;
         cudaGetLastError();
       }
       return 0;
     };
-    best = std::min(setup(cluster_gs_kernel<VT, VT, decltype(G)::value>),
-                    setup(cluster_gs_kernel<VT, double, decltype(G)::value>));
+    constexpr int g = decltype(G)::value;
+    if (block_)
+      best = std::min(setup(cluster_gs_kernel<ClusterBlock<VT, VT, g>>), setup(cluster_gs_kernel<ClusterBlock<VT, double, g>>));
+    else
+      best = std::min(setup(cluster_gs_kernel<ClusterScalar<VT, VT, g, 1>>),
+                      setup(cluster_gs_kernel<ClusterScalar<VT, double, g, 1>>));
   });
   return best;
 }
@@ -1836,7 +1851,7 @@ void AmgPcg<VT>::autotune() {
         L.pg = v[7 * k + 3];
         set_layout(L, static_cast<int>(k), v[7 * k] != 0, v[7 * k + 1], ar_);
         L.coop = v[7 * k + 4] != 0 && opt_.sweep_launch != 0 && !L.relaxed && !opt_.half_sweeps;
-        L.cluster = v[7 * k + 6] != 0 && opt_.sweep_launch == 1 && L.kind == 0 && !block_ &&
+        L.cluster = v[7 * k + 6] != 0 && opt_.sweep_launch == 1 && L.kind == (block_ ? 1 : 0) &&
                     build_cluster(L, static_cast<int>(k), ar_);
         L.staged = v[7 * k + 5] != 0 && opt_.sweep_launch != 0 && block_ && L.sliced && L.g == 1 &&
                    prepare_staged<VT>(L.B.max_slots, device_);
@@ -1928,7 +1943,7 @@ void AmgPcg<VT>::autotune() {
         }
         L.coop = t_coop < t_pass;
       }
-      if (L.kind == 0 && !block_ && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k));
+      if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k));
     }
     if (k + 1 < lv_.size()) {
       Level &Cn = lv_[k + 1];
@@ -1976,10 +1991,14 @@ void AmgPcg<VT>::autotune() {
 // fewer lanes leave the loaded-ahead slots (5,103 rows, 70 entries a row: 125
 // us with 8 lanes, 86 with 16, 90 with 32).
 constexpr long long kClusterPassEntries = 40000;
-inline int cluster_lanes(const Csr &a) {
-  const double len = static_cast<double>(a.nnz()) / std::max(1, a.rows) - 1.0;
+// 3x3 levels stream nine values per gathered slot: they are tried up to three
+// times as many entries.
+constexpr long long kClusterPassBlockEntries = 120000;
+inline int cluster_lanes(const Csr &a, bool block) {
+  // blocks: two a lane, what a thread loads ahead
+  const double len = static_cast<double>(a.nnz()) / std::max(1, a.rows) / (block ? 3.0 : 1.0) - 1.0;
   int g = 4;
-  while (g < 32 && g * 5.0 < len) g *= 2;
+  while (g < 32 && g * (block ? 2.0 : 5.0) < len) g *= 2;
   return g;
 }
 
@@ -1988,12 +2007,16 @@ inline int cluster_lanes(const Csr &a) {
 template <typename VT>
 bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
   const Csr &a = host_A_.at(k);
-  const int g = cluster_lanes(a), ncta = cluster_ctas(g, 0);
+  const int g = cluster_lanes(a, block_), ncta = cluster_ctas(g, 0);
   HostCluster<VT> h;
-  if (ncta == 0 || !make_cluster<VT>(a, L.color_first, g, ncta, kClusterThreads, L.relaxed, cluster_limit(L.relaxed), h))
-    return false;
-  L.K = upload_cluster<VT>(where, h);
-  return cluster_ctas(g, L.K.smem()) >= ncta;
+  if (ncta == 0) return false;
+  if (block_) {
+    if (!make_cluster_blocks<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_limit(L.relaxed), h)) return false;
+  } else {
+    if (!make_cluster<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_limit(L.relaxed), h)) return false;
+  }
+  L.K = upload_cluster<VT>(where, h, block_ ? L.B1.dinv : nullptr);
+  return cluster_ctas(g, L.K.smem(block_ ? 3 : 1)) >= ncta;
 }
 
 // One smoothing step of the level as the solve runs it, per-colour (or
@@ -2001,7 +2024,7 @@ bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
 template <typename VT>
 void AmgPcg<VT>::tune_cluster(Level &L, int k) {
   L.cluster = false;
-  if (host_A_.at(k).nnz() > kClusterPassEntries * L.ncolors) return;
+  if (host_A_.at(k).nnz() > (block_ ? kClusterPassBlockEntries : kClusterPassEntries) * L.ncolors) return;
   auto step = [&] {
     if (opt_.half_sweeps) {
       smooth<VT>(L, L.b, L.x, 1, true, stream_, 1);

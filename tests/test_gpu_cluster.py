@@ -9,10 +9,10 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
-def lanes_of(a):
-    """Lanes per row of a level in the cluster (about five entries a lane)."""
-    length, g = a.nnz / a.rows - 1.0, 4
-    while g < 32 and g * 5.0 < length:
+def lanes_of(a, block=1):
+    """Lanes per row of a level in the cluster (about five entries, or two 3x3 blocks, a lane)."""
+    length, g = a.nnz / a.rows / block - 1.0, 4
+    while g < 32 and g * (2.0 if block == 3 else 5.0) < length:
         g *= 2
     return g
 
@@ -29,7 +29,7 @@ def solver_with(gs, device, tmp_path, H, opts, cluster, mask=None):
         fields = []
         for k in range(levels):
             on = cluster and (mask is None or mask[k])
-            fields += [0, lanes_of(H.A(k)), 8, 4, 0, 0, int(on)]
+            fields += [0, lanes_of(H.A(k), 3 if opts.smoother == 1 else 1), 8, 4, 0, 0, int(on)]
         path.write_text(key + " " + " ".join(map(str, fields)) + " 1\n")
         return gs.Solver(H, opts, device=device)
     finally:
@@ -72,6 +72,34 @@ def test_cluster_steps_are_bit_identical(gs, device, tmp_path, probs, name, kw):
         assert st.status == gs.STATUS_CONVERGED and np.array_equal(x, again)
         out.append((x, st.iterations))
     assert out[0][1] == out[1][1] and np.array_equal(out[0][0], out[1][0])
+
+
+@pytest.mark.parametrize("side,min_dofs", [(4, 20), (9, 60)])
+@pytest.mark.parametrize("kw", [
+    dict(),
+    dict(use_graph=1, flexible=1, precision=1),
+    dict(omega=0.9, pre_steps=2, post_steps=1),
+    dict(half_sweeps=1, coloring=2, precision=1, flexible=1),
+    dict(half_sweeps=1, coloring=2, pre_steps=2, post_steps=2),
+], ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()) or "default")
+def test_block_cluster_steps_are_bit_identical(gs, device, tmp_path, kw, side, min_dofs):
+    """3x3 block levels; also with a weight per node and with new values."""
+    a = gs.elasticity(side)
+    H = gs.Hierarchy.build(a, 3, 0.1, 10, min_dofs)
+    out = []
+    for cluster in (False, True):
+        s = solver_with(gs, device, tmp_path, H, gs.SolverOptions(smoother=1, tol=1e-9, coarse_tail=0, **kw), cluster)
+        assert any(lv["launch"] for lv in s.level_info()) == cluster
+        runs = [s.solve(a.rhs)[0]]
+        n = len(s.node_features())
+        s.set_node_weights(np.linspace(0.9, 1.1, n))
+        runs.append(s.solve(a.rhs)[0])
+        s.set_node_weights(None)
+        s.update_matrix(a.val * 3.0)
+        runs.append(s.solve(a.rhs)[0])
+        out.append(runs)
+    for p, q in zip(*out):
+        assert np.array_equal(p, q)
 
 
 def test_cluster_steps_with_weights_and_refresh(gs, device, tmp_path, probs):
