@@ -19,10 +19,12 @@
 #include <cmath>
 #include <cstring>
 #include <functional>
+#include <numeric>
 #include <string>
 #include <thread>
 
 #include "batch.cuh"
+#include "cluster_layout.h"
 #include "dense.h"
 #include "formats.cuh"
 
@@ -293,6 +295,12 @@ class Batch final : public BatchSolver {
     DevCsrv<VT> C, Pc, Rc;
     int g = 1, pg = 1, rg = 1;
     RV *x = nullptr, *b = nullptr, *r = nullptr;
+    // smoothing steps in one thread-block cluster per system (cluster.cuh)
+    bool cluster = false;
+    int cncta = 0, cg = 0, csystems = 0, ccolors = 0;
+    size_t csmem = 0;
+    const ClusterView<VT> *views = nullptr;
+    const int *csys = nullptr;
     std::vector<Range> fwd, bwd;
     Range whole_a, whole_p, below_r;
   };
@@ -326,6 +334,12 @@ class Batch final : public BatchSolver {
             const Rv<BT, R> *b, cudaStream_t s);
   template <typename BT>
   void smooth(int k, const Rv<BT, R> *b, RV *x, int steps, bool zero, cudaStream_t s);
+  ClusterPasses cluster_passes(const BLevel &L, int steps, int dir) const {
+    return ClusterPasses{L.ccolors, steps, dir, VT(opt_.omega) == VT(1) ? 1 : 0};
+  }
+  void cluster_smooth(const BLevel &L, const VT *b, VT *x, int steps, bool zero, int dir, cudaStream_t s);
+  void tune_cluster(int k, const std::vector<SysPrep> &sp);
+  void check_fault();
   void vcycle(const RD *r0, RV *z, bool zero0, cudaStream_t s);
   void precondition(const RD *r, RV *z, cudaStream_t s) {
     for (int v = 0; v < opt_.vcycles; ++v) vcycle(r, z, v == 0, s);
@@ -335,6 +349,7 @@ class Batch final : public BatchSolver {
   void ensure_graphs();
   void run(std::vector<SolveStats> &st);
   void build_items();
+  std::vector<std::unique_ptr<Arena>> kept_;  // cluster layouts in use
   void autotune();
   float time_ms(const std::function<void()> &f, int reps);
 
@@ -556,6 +571,17 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
   }
   build_items();
   BCK(cudaDeviceSynchronize());  // every upload has landed
+  if (opt_.lanes == 0 && opt_.autotune && opt_.sweep_launch == 1) {
+    const long long saved = launches_;
+    BCK(cudaMemset(sh_, 0, sizeof(BCgShared)));
+    for (int k = 1; k + 1 < K_; ++k) tune_cluster(k, sp);
+    for (BLevel &L : lv_) {  // the timed steps left values in the level vectors
+      BCK(cudaMemset(L.x, 0, sizeof(RV) * L.n));
+      BCK(cudaMemset(L.b, 0, sizeof(RV) * L.n));
+    }
+    BCK(cudaDeviceSynchronize());
+    launches_ = saved;
+  }
   for (int k = 0; k < K_; ++k) {
     info_[k].lanes = lv_[k].g;
     info_[k].p_lanes = lv_[k].pg;
@@ -680,6 +706,12 @@ template <typename VT, int R>
 template <typename BT>
 void Batch<VT, R>::smooth(int k, const Rv<BT, R> *b, RV *x, int steps, bool zero, cudaStream_t s) {
   const BLevel &L = lv_[k];
+  if constexpr (std::is_same<BT, VT>::value) {
+    if (k > 0 && L.cluster && cluster_passes(L, steps, 0).total() <= kClusterMaxPasses) {
+      cluster_smooth(L, &b->v[0], &x->v[0], steps, zero, 0, s);
+      return;
+    }
+  }
   const bool skip = VT(opt_.omega) == VT(1);
   for (int step = 0; step < steps; ++step) {
     for (size_t j = skip && step > 0 ? 1 : 0; j < L.fwd.size(); ++j)
@@ -687,6 +719,102 @@ void Batch<VT, R>::smooth(int k, const Rv<BT, R> *b, RV *x, int steps, bool zero
     for (size_t j = skip ? 1 : 0; j < L.bwd.size(); ++j)
       gs_pass<BT>(L, items_ + L.bwd[j].off, L.bwd[j].count, b, x, false, s);
   }
+}
+
+// The steps of every system of the level, one cluster each; the same iterates
+// as the CSR-vector passes with the same lanes per row, bit for bit.
+template <typename VT, int R>
+void Batch<VT, R>::cluster_smooth(const BLevel &L, const VT *b, VT *x, int steps, bool zero, int dir, cudaStream_t s) {
+  ClusterLaunch l(L.cncta, L.csystems, kClusterThreads, L.csmem, pdl_, s);
+  with_lanes(L.cg, [&](auto G) {
+    BCK(cudaLaunchKernelEx(&l.cfg, cluster_gs_batch_kernel<ClusterScalar<VT, VT, decltype(G)::value, R>>, L.views, L.csys,
+                           L.cncta, cluster_passes(L, steps, dir), b, x, zero ? 1 : 0, VT(opt_.omega), sys_done_,
+                           &sh_->sync_fault));
+  });
+  BKL("batched cluster Gauss-Seidel step");
+}
+
+// A cluster's wait that gave up: reported once, the batch stays usable.
+// host_sh_[0] holds the state of the finished work.
+template <typename VT, int R>
+void Batch<VT, R>::check_fault() {
+  if (host_sh_[0].sync_fault == 0) return;
+  BCK(cudaMemset(sh_, 0, sizeof(BCgShared)));
+  throw CudaError("batched cluster Gauss-Seidel step: a wait timed out");
+}
+
+// A symmetric step of level k (below the finest) with one cluster per system
+// against the colour passes of the whole batch; the faster is kept. Many small
+// systems get clusters of 8 CTAs, so that more of them run at once; up to nine
+// systems, or large ones, get 16 (11 systems of up to 51 k entries a colour, 4
+// FP32 right-hand sides, a step: 246 us with 8 CTAs, 147 with 16, 156 by
+// passes; 5 systems of up to 8 k, FP64: 84 us by passes, 36 with 16). Tried
+// where the largest system has at most kBatchClusterEntries entries a colour:
+// above, its cluster alone takes longer than the passes.
+constexpr long long kBatchClusterEntries = 60000;
+constexpr long long kBatchClusterWide = 20000;
+
+template <typename VT, int R>
+void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
+  BLevel &L = lv_[k];
+  L.cluster = false;
+  if (k == 0 || ly_.whole[k].empty()) return;
+  long long nnz = 0, largest = 0;
+  int rows = 0;
+  for (const Seg &g : ly_.whole[k]) {
+    const SysLevel &v = sp[g.sys].lv[k];
+    largest = std::max(largest, v.A.nnz() / std::max<long long>(1, static_cast<long long>(v.cf.size()) - 1));
+    nnz += v.A.nnz();
+    rows += v.A.rows;
+  }
+  if (largest > kBatchClusterEntries) return;
+  const int S = static_cast<int>(ly_.whole[k].size()), g = cluster_lanes(nnz, rows, false);
+  int ncta = 0;
+  const auto fit = [&](size_t smem, int most) {
+    int n = 0;
+    with_lanes(g, [&](auto G) {
+      n = cluster_fit(cluster_gs_batch_kernel<ClusterScalar<VT, VT, decltype(G)::value, R>>, kClusterThreads, smem, most,
+                      device_);
+    });
+    return n;
+  };
+  ncta = fit(0, S <= 9 || largest > kBatchClusterWide ? 16 : 8);
+  if (ncta == 0) return;
+  std::vector<ClusterView<VT>> views;
+  std::vector<int> systems;
+  int max_slots = 0, colors = 0;
+  std::vector<HostCluster<VT>> hc(S);
+  for (int i = 0; i < S; ++i) {
+    const Seg &q = ly_.whole[k][i];
+    const SysLevel &v = sp[q.sys].lv[k];
+    if (!make_cluster<VT>(v.A, v.cf, g, ncta, false, cluster_slots(static_cast<int>(sizeof(RV)), false, device_), hc[i]))
+      return;
+    max_slots = std::max(max_slots, hc[i].max_slots);
+    colors = std::max(colors, hc[i].ncolors);
+  }
+  const size_t smem = (static_cast<size_t>(max_slots) + 1) * sizeof(RV);
+  if (fit(smem, ncta) != ncta) return;
+  std::unique_ptr<Arena> arena(new Arena);
+  // the largest systems first: their clusters bound the step
+  std::vector<int> order(S);
+  std::iota(order.begin(), order.end(), 0);
+  std::sort(order.begin(), order.end(), [&](int p, int q) { return hc[p].val.size() > hc[q].val.size(); });
+  for (int i : order) {
+    const Seg &q = ly_.whole[k][i];
+    views.push_back(upload_cluster<VT>(*arena, hc[i], nullptr, q.r0).v);
+    systems.push_back(q.sys);
+  }
+  L.cncta = ncta, L.cg = g, L.csystems = S, L.ccolors = colors, L.csmem = smem;
+  L.views = arena->upload(views);
+  L.csys = arena->upload(systems);
+  BCK(cudaDeviceSynchronize());
+  const auto step = [&] { smooth<VT>(k, L.b, L.x, 1, false, stream_); };
+  const float t_pass = time_ms(step, 5);
+  L.cluster = true;
+  L.cluster = time_ms(step, 5) < t_pass;
+  BCK(cudaMemcpy(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost));
+  check_fault();
+  if (L.cluster) kept_.push_back(std::move(arena));
 }
 
 template <typename VT, int R>
@@ -804,7 +932,9 @@ double Batch<VT, R>::time_level(int level, int op, int lanes, int reps, cudaStre
   BCK(cudaStreamWaitEvent(stream_, ev_[0], 0));
   BCK(cudaMemsetAsync(sys_done_, 0, sizeof(int) * S_, stream_));
   const long long saved = launches_;
-  const float ms = time_level_op(level, op, g, std::max(1, reps));
+  const bool steps = lanes == 0 && op == 0 && L.cluster && cluster_passes(L, 1, 1).total() <= kClusterMaxPasses;
+  const float ms = steps ? time_ms([&] { cluster_smooth(L, &L.b->v[0], &L.x->v[0], 1, false, 1, stream_); }, std::max(1, reps))
+                         : time_level_op(level, op, g, std::max(1, reps));
   launches_ = saved;
   BCK(cudaEventRecord(ev_[1], stream_));
   BCK(cudaStreamWaitEvent(stream, ev_[1], 0));
@@ -937,9 +1067,11 @@ void Batch<VT, R>::run(std::vector<SolveStats> &out) {
     }
   }
   BCK(cudaEventRecord(ev_[3], stream_));
-  BCK(cudaEventSynchronize(ev_[3]));
+  BCK(cudaMemcpyAsync(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost, stream_));
+  BCK(cudaStreamSynchronize(stream_));
   float ms = 0.f;
   BCK(cudaEventElapsedTime(&ms, ev_[2], ev_[3]));
+  check_fault();
   std::vector<BPair> hp(static_cast<size_t>(S_) * R);
   BCK(cudaMemcpy(hp.data(), pairs_, sizeof(BPair) * hp.size(), cudaMemcpyDeviceToHost));
   out.assign(static_cast<size_t>(S_) * nrhs_, SolveStats{});

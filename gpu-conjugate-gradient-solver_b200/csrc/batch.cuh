@@ -420,6 +420,7 @@ struct BCgShared {
   int max_iter;
   int flexible;
   int active;  // systems with at least one pair still running (after the last convergence test)
+  int sync_fault;  // a bounded wait of a cluster step gave up
 };
 
 // Deterministic block sum of kN values per thread into smem-backed totals;

@@ -135,6 +135,26 @@ __device__ __forceinline__ void send_value(unsigned addr, float v, unsigned bar)
                "r"(__float_as_uint(v)), "r"(bar)
                : "memory");
 }
+// The W values of a row: 16 bytes a message where they fill it.
+template <typename T, int W>
+__device__ __forceinline__ void send_row(unsigned addr, const T (&v)[W], unsigned bar) {
+  if constexpr (W == 4 && sizeof(T) == 4) {
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
+                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+                 "r"(__float_as_uint(v[3])), "r"(bar)
+                 : "memory");
+  } else if constexpr (W == 4) {
+#pragma unroll
+    for (int j = 0; j < 4; j += 2)
+      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr + 8 * j),
+                   "l"(__double_as_longlong(v[j])), "l"(__double_as_longlong(v[j + 1])), "r"(bar)
+                   : "memory");
+  } else {
+#pragma unroll
+    for (int j = 0; j < W; ++j) send_value(addr + j * static_cast<unsigned>(sizeof(T)), v[j], bar);
+  }
+}
+
 // Read-only loads that keep their place: the operands of the next row are
 // requested before the wait on the current pass (a plain load is moved down to
 // its first use, which exposes its latency: 770 of 3000 cycles a pass).
@@ -237,12 +257,33 @@ struct ClusterScalar {
     u.d = load_early(reinterpret_cast<const P2 *>(A.diag) + row);
   }
   static __device__ __forceinline__ void load_b(const BT *b, int row, Unit &u) {
+    if constexpr (R == 4 && sizeof(BT) == 4) {
+      const float2 *q = reinterpret_cast<const float2 *>(b) + 2 * static_cast<size_t>(row);
+      const float2 lo = cluster_detail::load_early(q), hi = cluster_detail::load_early(q + 1);
+      u.b[0] = lo.x, u.b[1] = lo.y, u.b[2] = hi.x, u.b[3] = hi.y;
+    } else if constexpr (R == 4) {
+      const double2 *q = reinterpret_cast<const double2 *>(b) + 2 * static_cast<size_t>(row);
+      const double2 lo = cluster_detail::load_early(q), hi = cluster_detail::load_early(q + 1);
+      u.b[0] = lo.x, u.b[1] = lo.y, u.b[2] = hi.x, u.b[3] = hi.y;
+    } else {
 #pragma unroll
-    for (int j = 0; j < R; ++j) u.b[j] = cluster_detail::load_early(b + static_cast<size_t>(row) * R + j);
+      for (int j = 0; j < R; ++j) u.b[j] = cluster_detail::load_early(b + static_cast<size_t>(row) * R + j);
+    }
   }
   static __device__ __forceinline__ void add(T v, const T *xs, unsigned slot, T (&sum)[R]) {
+    if constexpr (R == 4 && sizeof(T) == 4) {
+      const float4 q = *reinterpret_cast<const float4 *>(xs + 4 * slot);
+      sum[0] = fma(v, q.x, sum[0]), sum[1] = fma(v, q.y, sum[1]);
+      sum[2] = fma(v, q.z, sum[2]), sum[3] = fma(v, q.w, sum[3]);
+    } else if constexpr (R == 4) {
+      const double2 q0 = *reinterpret_cast<const double2 *>(xs + 4 * slot);
+      const double2 q1 = *reinterpret_cast<const double2 *>(xs + 4 * slot + 2);
+      sum[0] = fma(v, q0.x, sum[0]), sum[1] = fma(v, q0.y, sum[1]);
+      sum[2] = fma(v, q1.x, sum[2]), sum[3] = fma(v, q1.y, sum[3]);
+    } else {
 #pragma unroll
-    for (int j = 0; j < R; ++j) sum[j] = fma(v, xs[slot * R + j], sum[j]);
+      for (int j = 0; j < R; ++j) sum[j] = fma(v, xs[slot * R + j], sum[j]);
+    }
   }
   // neighbour sums of the row (in every lane of its group)
   static __device__ __forceinline__ void sums(const ClusterView<T> &A, const ClusterSeg &sg, int t, int tid,
@@ -451,17 +492,12 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
 #pragma unroll
           for (int j = 0; j < W; ++j) xn[j] = fma(T(1) - w, xs[own + j], w * xn[j]);
         }
-        if (cur.send != kNoSend)
-#pragma unroll
-          for (int j = 0; j < W; ++j) send_value(to_x + j * static_cast<unsigned>(sizeof(T)), xn[j], to_bar);
+        if (cur.send != kNoSend) send_row(to_x, xn, to_bar);
         for (int q = 1; q < sg.schunks; ++q) {
           const unsigned to = __ldg(A.send + sg.sbase + (t * sg.schunks + q) * sg.stride + tid);
-          if (to != kNoSend) {
-            const unsigned rx = remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (to & 0xffffu), to >> 16);
-            const unsigned rb = remote(bar_addr + 8 * p, to >> 16);
-#pragma unroll
-            for (int j = 0; j < W; ++j) send_value(rx + j * static_cast<unsigned>(sizeof(T)), xn[j], rb);
-          }
+          if (to != kNoSend)
+            send_row(remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (to & 0xffffu), to >> 16), xn,
+                     remote(bar_addr + 8 * p, to >> 16));
         }
         if (p >= keep && (tid & (G - 1)) == 0)
 #pragma unroll
@@ -503,6 +539,21 @@ __global__ void __launch_bounds__(Row::kThreads, 1)
                       typename Row::V *__restrict__ x, int zero, const typename Row::V *__restrict__ wts,
                       const typename Row::V *__restrict__ nw, typename Row::V omega, CgState *st) {
   cluster_steps<Row>(A, P, b, x, zero, wts, nw, omega, ClusterStatus{&st->done, &st->sync_fault});
+}
+
+// One cluster per system of a batch level: views[i] belongs to system
+// systems[i], whose rows start at its row0 in b and x.
+template <typename Row>
+__global__ void __launch_bounds__(Row::kThreads, 1)
+    cluster_gs_batch_kernel(const ClusterView<typename Row::V> *__restrict__ views, const int *__restrict__ systems,
+                            int ncta, ClusterPasses P, const typename Row::B *__restrict__ b,
+                            typename Row::V *__restrict__ x, int zero, typename Row::V omega, int *sys_done,
+                            int *fault) {
+  const int i = blockIdx.x / ncta;
+  const ClusterView<typename Row::V> A = views[i];
+  P.ncolors = A.ncolors;
+  const size_t at = static_cast<size_t>(A.row0) * Row::kW;
+  cluster_steps<Row>(A, P, b + at, x + at, zero, nullptr, nullptr, omega, ClusterStatus{sys_done + systems[i], fault});
 }
 
 }  // namespace gsb

@@ -4,6 +4,7 @@
 #pragma once
 
 #include <algorithm>
+#include <type_traits>
 #include <vector>
 
 #include "cluster.cuh"
@@ -262,6 +263,82 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
   if (diag == nullptr) diag = d.diag = ar.upload(h.diag);
   d.v.diag = diag;
   return d;
+}
+
+// Lanes per row: about five entries, or two 3x3 blocks, a lane (what a thread
+// loads ahead). Fewer lanes leave the loaded-ahead slots (5,103 rows, 70
+// entries a row: 125 us a step with 8 lanes, 86 with 16, 90 with 32).
+inline int cluster_lanes(long long nnz, int rows, bool block) {
+  const double len = static_cast<double>(nnz) / std::max(1, rows) / (block ? 3.0 : 1.0) - 1.0;
+  int g = 4;
+  while (g < 32 && g * (block ? 2.0 : 5.0) < len) g *= 2;
+  return g;
+}
+
+// Lanes per row of the cluster layout's kernels.
+template <typename F>
+void with_lanes(int g, F &&f) {
+  switch (g) {
+    case 4: f(std::integral_constant<int, 4>()); break;
+    case 8: f(std::integral_constant<int, 8>()); break;
+    case 16: f(std::integral_constant<int, 16>()); break;
+    default: f(std::integral_constant<int, 32>()); break;
+  }
+}
+
+// Launch of clusters of ncta CTAs, with programmatic stream serialization
+// when `overlap` (launch_pass).
+struct ClusterLaunch {
+  cudaLaunchAttribute attr[2];
+  cudaLaunchConfig_t cfg = {};
+  ClusterLaunch(int ncta, int clusters, int threads, size_t smem, bool overlap, cudaStream_t s) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ncta;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
+    cfg.gridDim = dim3(static_cast<unsigned>(ncta * clusters));
+    cfg.blockDim = dim3(static_cast<unsigned>(threads));
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = attr;
+    cfg.numAttrs = overlap ? 2 : 1;
+  }
+  ClusterLaunch(const ClusterLaunch &) = delete;
+};
+
+// Shared memory that a CTA of the cluster kernels has for x.
+inline int cluster_smem_bytes(int device) {
+  int optin = 0;
+  GSB_CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device));
+  return optin - static_cast<int>(sizeof(ClusterSeg) * kClusterMaxColors + 8 * kClusterMaxPasses +
+                                  2 * (kClusterMaxPasses + 8)) - 1024;
+}
+
+// Slots of `bytes` each that fit it.
+inline int cluster_slots(int bytes, bool relaxed, int device) {
+  return std::min(kClusterMaxSlots, cluster_smem_bytes(device) / (bytes * (relaxed ? 2 : 1)) - 1);
+}
+
+// Largest cluster of at most `most` CTAs (16 or 8) of `kernel` the device
+// co-schedules with `smem` bytes per CTA, or 0. Raises the kernel's shared
+// memory limit to what the device has (a limit only, the same for every solver
+// of the process).
+template <typename K>
+int cluster_fit(K kernel, int threads, size_t smem, int most, int device) {
+  const int limit = cluster_smem_bytes(device);
+  GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+  GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  if (smem > static_cast<size_t>(limit)) return 0;
+  for (int want : {16, 8}) {
+    if (want > most) continue;
+    ClusterLaunch l(want, 1, threads, smem, false, nullptr);
+    int n = 0;
+    if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) return want;
+    cudaGetLastError();
+  }
+  return 0;
 }
 
 }  // namespace gsb

@@ -538,7 +538,6 @@ class AmgPcg final : public Solver {
   bool in_cluster(const Level &L, int steps, int dir) const {
     return L.cluster && cluster_passes(L, steps, dir).total() <= kClusterMaxPasses;
   }
-  int cluster_limit(bool relaxed);
   int cluster_ctas(int g, size_t smem);
   bool build_cluster(Level &L, int k, Arena &where);
   void tune_cluster(Level &L, int k);
@@ -1418,45 +1417,12 @@ void AmgPcg<VT>::coop_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero
   CKL("cooperative Gauss-Seidel sweep");
 }
 
-// Lanes per row of the cluster layout's kernels.
-template <typename F>
-void with_lanes(int g, F &&f) {
-  switch (g) {
-    case 4: f(std::integral_constant<int, 4>()); break;
-    case 8: f(std::integral_constant<int, 8>()); break;
-    case 16: f(std::integral_constant<int, 16>()); break;
-    default: f(std::integral_constant<int, 32>()); break;
-  }
-}
-
-// Launch of one cluster of ncta CTAs, with programmatic stream serialization
-// when `overlap` (launch_pass).
-struct ClusterLaunch {
-  cudaLaunchAttribute attr[2];
-  cudaLaunchConfig_t cfg = {};
-  ClusterLaunch(int ncta, int threads, size_t smem, bool overlap, cudaStream_t s) {
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = ncta;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[1].val.programmaticStreamSerializationAllowed = 1;
-    cfg.gridDim = dim3(static_cast<unsigned>(ncta));
-    cfg.blockDim = dim3(static_cast<unsigned>(threads));
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = s;
-    cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 2 : 1;
-  }
-  ClusterLaunch(const ClusterLaunch &) = delete;
-};
-
 // Smoothing steps of a level in one cluster (cluster.cuh); the same iterate
 // as the per-colour passes with the same lanes per row, bit for bit.
 template <typename VT>
 template <typename BT>
 void AmgPcg<VT>::cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool zero, int dir, cudaStream_t s) {
-  ClusterLaunch l(L.K.ncta, L.K.threads, L.K.smem(block_ ? 3 : 1), pdl_, s);
+  ClusterLaunch l(L.K.ncta, 1, L.K.threads, L.K.smem(block_ ? 3 : 1), pdl_, s);
   const VT *w = L.wts.empty() ? nullptr : L.wts[0];
   const VT *nw = L.nwts;
   with_lanes(L.K.g, [&](auto G) {
@@ -1471,48 +1437,19 @@ void AmgPcg<VT>::cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool z
   CKL("cluster Gauss-Seidel step");
 }
 
-// Slots of x that one CTA's shared memory holds.
-template <typename VT>
-int AmgPcg<VT>::cluster_limit(bool relaxed) {
-  int optin = 0;
-  CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-  cudaFuncAttributes fa{};
-  CK(cudaFuncGetAttributes(&fa, cluster_gs_kernel<ClusterScalar<VT, VT, 8, 1>>));
-  const long long bytes = optin - static_cast<long long>(fa.sharedSizeBytes) - 1024;
-  const long long slot = static_cast<long long>(sizeof(VT)) * (block_ ? 3 : 1) * (relaxed ? 2 : 1);
-  return static_cast<int>(std::min<long long>(kClusterMaxSlots, bytes / slot - 1));
-}
-
-// Largest cluster (16 or 8 CTAs) the device co-schedules with `smem` bytes per
-// CTA, or 0. Raises the kernels' shared memory limit to the device's maximum
-// (a limit only, the same for every solver of the process).
+// Largest cluster (16 or 8 CTAs) both of the level's kernels can run as with
+// `smem` bytes per CTA, or 0.
 template <typename VT>
 int AmgPcg<VT>::cluster_ctas(int g, size_t smem) {
   int best = 0;
   with_lanes(g, [&](auto G) {
-    auto setup = [&](auto kernel) {
-      int optin = 0;
-      CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, device_));
-      cudaFuncAttributes fa{};
-      CK(cudaFuncGetAttributes(&fa, kernel));
-      const int most = optin - static_cast<int>(fa.sharedSizeBytes);
-      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, most));
-      CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-      if (smem > static_cast<size_t>(most)) return 0;
-      for (int want : {16, 8}) {
-        ClusterLaunch l(want, block_ ? kClusterBlockThreads : kClusterThreads, smem, false, nullptr);
-        int n = 0;
-        if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) return want;
-        cudaGetLastError();
-      }
-      return 0;
-    };
-    constexpr int g = decltype(G)::value;
+    constexpr int n = decltype(G)::value;
     if (block_)
-      best = std::min(setup(cluster_gs_kernel<ClusterBlock<VT, VT, g>>), setup(cluster_gs_kernel<ClusterBlock<VT, double, g>>));
+      best = std::min(cluster_fit(cluster_gs_kernel<ClusterBlock<VT, VT, n>>, kClusterBlockThreads, smem, 16, device_),
+                      cluster_fit(cluster_gs_kernel<ClusterBlock<VT, double, n>>, kClusterBlockThreads, smem, 16, device_));
     else
-      best = std::min(setup(cluster_gs_kernel<ClusterScalar<VT, VT, g, 1>>),
-                      setup(cluster_gs_kernel<ClusterScalar<VT, double, g, 1>>));
+      best = std::min(cluster_fit(cluster_gs_kernel<ClusterScalar<VT, VT, n, 1>>, kClusterThreads, smem, 16, device_),
+                      cluster_fit(cluster_gs_kernel<ClusterScalar<VT, double, n, 1>>, kClusterThreads, smem, 16, device_));
   });
   return best;
 }
@@ -1982,38 +1919,28 @@ void AmgPcg<VT>::autotune() {
   }
 }
 
-// Entries per colour pass up to which a level is tried in one cluster, and
-// the lanes per row there. One cluster's 16 SMs beat a launch per pass while a
+// Entries per colour pass up to which a level is tried in one cluster. One
+// cluster's 16 SMs beat a launch per pass while a
 // pass is latency: FP64 symmetric steps, cluster / launches: 9.8 k entries a
 // pass (5,103 rows, 37 colours) 86 / 183 us, 8.2 k (4,143, 23) 53 / 108,
 // 13.5 k (4,096, 2) 7.7 / 9.4; above, the 16 SMs' gathers bound it: 58 k
-// (32,768, 8) 58 / 37, 66 k (37,505, 18) 120 / 95. About five entries a lane:
-// fewer lanes leave the loaded-ahead slots (5,103 rows, 70 entries a row: 125
-// us with 8 lanes, 86 with 16, 90 with 32).
+// (32,768, 8) 58 / 37, 66 k (37,505, 18) 120 / 95.
 constexpr long long kClusterPassEntries = 40000;
 // 3x3 levels stream nine values per gathered slot: they are tried up to three
 // times as many entries.
 constexpr long long kClusterPassBlockEntries = 120000;
-inline int cluster_lanes(const Csr &a, bool block) {
-  // blocks: two a lane, what a thread loads ahead
-  const double len = static_cast<double>(a.nnz()) / std::max(1, a.rows) / (block ? 3.0 : 1.0) - 1.0;
-  int g = 4;
-  while (g < 32 && g * (block ? 2.0 : 5.0) < len) g *= 2;
-  return g;
-}
-
 // The cluster layout of level k (cluster_layout.h), built into `where`; false
 // when the level or the device does not qualify.
 template <typename VT>
 bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
   const Csr &a = host_A_.at(k);
-  const int g = cluster_lanes(a, block_), ncta = cluster_ctas(g, 0);
+  const int g = cluster_lanes(a.nnz(), a.rows, block_), ncta = cluster_ctas(g, 0);
   HostCluster<VT> h;
   if (ncta == 0) return false;
   if (block_) {
-    if (!make_cluster_blocks<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_limit(L.relaxed), h)) return false;
+    if (!make_cluster_blocks<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_slots(static_cast<int>(sizeof(VT)) * (block_ ? 3 : 1), L.relaxed, device_), h)) return false;
   } else {
-    if (!make_cluster<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_limit(L.relaxed), h)) return false;
+    if (!make_cluster<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_slots(static_cast<int>(sizeof(VT)) * (block_ ? 3 : 1), L.relaxed, device_), h)) return false;
   }
   L.K = upload_cluster<VT>(where, h, block_ ? L.B1.dinv : nullptr);
   return cluster_ctas(g, L.K.smem(block_ ? 3 : 1)) >= ncta;
