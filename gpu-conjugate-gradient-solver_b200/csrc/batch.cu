@@ -770,15 +770,10 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
   if (largest > kBatchClusterEntries) return;
   const int S = static_cast<int>(ly_.whole[k].size()), g = cluster_lanes(nnz, rows, false);
   int ncta = 0;
-  const auto fit = [&](size_t smem, int most) {
-    int n = 0;
-    with_lanes(g, [&](auto G) {
-      n = cluster_fit(cluster_gs_batch_kernel<ClusterScalar<VT, VT, decltype(G)::value, R>>, kClusterThreads, smem, most,
-                      device_);
-    });
-    return n;
-  };
-  ncta = fit(0, S <= 9 || largest > kBatchClusterWide ? 16 : 8);
+  with_lanes(g, [&](auto G) {
+    ncta = cluster_fit(cluster_gs_batch_kernel<ClusterScalar<VT, VT, decltype(G)::value, R>>, kClusterThreads,
+                       S <= 9 || largest > kBatchClusterWide ? 16 : 8, device_);
+  });
   if (ncta == 0) return;
   std::vector<ClusterView<VT>> views;
   std::vector<int> systems;
@@ -793,7 +788,6 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
     colors = std::max(colors, hc[i].ncolors);
   }
   const size_t smem = (static_cast<size_t>(max_slots) + 1) * sizeof(RV);
-  if (fit(smem, ncta) != ncta) return;
   std::unique_ptr<Arena> arena(new Arena);
   // the largest systems first: their clusters bound the step
   std::vector<int> order(S);

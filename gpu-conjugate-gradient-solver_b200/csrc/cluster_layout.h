@@ -4,7 +4,11 @@
 #pragma once
 
 #include <algorithm>
+#include <cstring>
+#include <mutex>
 #include <type_traits>
+#include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "cluster.cuh"
@@ -252,15 +256,26 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
   d.v.ncta = h.ncta, d.v.ncolors = h.ncolors, d.v.threads = h.threads, d.v.max_slots = h.max_slots;
   d.v.relaxed = h.relaxed;
   d.v.row0 = row0;
-  d.v.seg = ar.upload(h.seg);
-  d.v.expect = ar.upload(h.expect);
-  d.v.slot_ptr = ar.upload(h.slot_ptr);
-  d.v.slot_row = ar.upload(h.slot_row);
-  d.v.val = d.val = ar.upload(h.val);
-  d.v.col = reinterpret_cast<const unsigned *>(ar.upload(h.col));
-  d.v.send = ar.upload(h.send);
-  d.v.own = ar.upload(h.own);
-  if (diag == nullptr) diag = d.diag = ar.upload(h.diag);
+  // one allocation and one copy for the whole layout
+  std::vector<unsigned char> pack;
+  const auto put = [&](const auto &v) {
+    const size_t at = (pack.size() + 255) / 256 * 256;
+    pack.resize(at + sizeof(v[0]) * v.size());
+    if (!v.empty()) std::memcpy(pack.data() + at, v.data(), sizeof(v[0]) * v.size());
+    return at;
+  };
+  const size_t seg = put(h.seg), expect = put(h.expect), slot_ptr = put(h.slot_ptr), slot_row = put(h.slot_row),
+               val = put(h.val), col = put(h.col), send = put(h.send), own = put(h.own), dd = put(h.diag);
+  unsigned char *base = ar.upload(pack);
+  d.v.seg = reinterpret_cast<const ClusterSeg *>(base + seg);
+  d.v.expect = reinterpret_cast<const unsigned *>(base + expect);
+  d.v.slot_ptr = reinterpret_cast<const int *>(base + slot_ptr);
+  d.v.slot_row = reinterpret_cast<const int *>(base + slot_row);
+  d.v.val = d.val = reinterpret_cast<T *>(base + val);
+  d.v.col = reinterpret_cast<const unsigned *>(base + col);
+  d.v.send = reinterpret_cast<const unsigned *>(base + send);
+  d.v.own = reinterpret_cast<const unsigned short *>(base + own);
+  if (diag == nullptr) diag = d.diag = reinterpret_cast<T *>(base + dd);
   d.v.diag = diag;
   return d;
 }
@@ -321,23 +336,35 @@ inline int cluster_slots(int bytes, bool relaxed, int device) {
   return std::min(kClusterMaxSlots, cluster_smem_bytes(device) / (bytes * (relaxed ? 2 : 1)) - 1);
 }
 
-// Largest cluster of at most `most` CTAs (16 or 8) of `kernel` the device
-// co-schedules with `smem` bytes per CTA, or 0. Raises the kernel's shared
-// memory limit to what the device has (a limit only, the same for every solver
-// of the process).
+// Whether the device co-schedules clusters of 16 and of 8 CTAs of `kernel`
+// with all the shared memory the CTAs may ask for (asked once per kernel and
+// device). Raises the kernel's shared memory limit to what the device has (a
+// limit only, the same for every solver of the process). Returns the largest
+// size of at most `most`, or 0.
 template <typename K>
-int cluster_fit(K kernel, int threads, size_t smem, int most, int device) {
-  const int limit = cluster_smem_bytes(device);
-  GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
-  GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
-  if (smem > static_cast<size_t>(limit)) return 0;
-  for (int want : {16, 8}) {
-    if (want > most) continue;
-    ClusterLaunch l(want, 1, threads, smem, false, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) return want;
-    cudaGetLastError();
+int cluster_fit(K kernel, int threads, int most, int device) {
+  static std::mutex mu;
+  static std::unordered_map<const void *, std::vector<std::pair<int, int>>> cache;  // device, sizes (bit mask)
+  std::lock_guard<std::mutex> lock(mu);
+  auto &known = cache[reinterpret_cast<const void *>(kernel)];
+  int sizes = -1;
+  for (const auto &k : known)
+    if (k.first == device) sizes = k.second;
+  if (sizes < 0) {
+    const int limit = cluster_smem_bytes(device);
+    GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, limit));
+    GSB_CK(cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    sizes = 0;
+    for (int want : {16, 8}) {
+      ClusterLaunch l(want, 1, threads, static_cast<size_t>(limit), false, nullptr);
+      int n = 0;
+      if (cudaOccupancyMaxActiveClusters(&n, kernel, &l.cfg) == cudaSuccess && n >= 1) sizes |= want;
+      else cudaGetLastError();
+    }
+    known.emplace_back(device, sizes);
   }
+  for (int want : {16, 8})
+    if (want <= most && (sizes & want) != 0) return want;
   return 0;
 }
 

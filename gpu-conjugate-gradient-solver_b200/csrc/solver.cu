@@ -538,9 +538,9 @@ class AmgPcg final : public Solver {
   bool in_cluster(const Level &L, int steps, int dir) const {
     return L.cluster && cluster_passes(L, steps, dir).total() <= kClusterMaxPasses;
   }
-  int cluster_ctas(int g, size_t smem);
+  int cluster_ctas(int g);
   bool build_cluster(Level &L, int k, Arena &where);
-  void tune_cluster(Level &L, int k);
+  void tune_cluster(Level &L, int k, float t_now);
   // omega 1 and no learned weight: the update of a row does not depend on
   // its own value, so a colour pass repeated right after itself (where the
   // sweep turns) reproduces its input bit for bit and is skipped
@@ -1437,19 +1437,18 @@ void AmgPcg<VT>::cluster_sweep(Level &L, const BT *rhs, VT *x, int steps, bool z
   CKL("cluster Gauss-Seidel step");
 }
 
-// Largest cluster (16 or 8 CTAs) both of the level's kernels can run as with
-// `smem` bytes per CTA, or 0.
+// Largest cluster (16 or 8 CTAs) both of the level's kernels can run as, or 0.
 template <typename VT>
-int AmgPcg<VT>::cluster_ctas(int g, size_t smem) {
+int AmgPcg<VT>::cluster_ctas(int g) {
   int best = 0;
   with_lanes(g, [&](auto G) {
     constexpr int n = decltype(G)::value;
     if (block_)
-      best = std::min(cluster_fit(cluster_gs_kernel<ClusterBlock<VT, VT, n>>, kClusterBlockThreads, smem, 16, device_),
-                      cluster_fit(cluster_gs_kernel<ClusterBlock<VT, double, n>>, kClusterBlockThreads, smem, 16, device_));
+      best = std::min(cluster_fit(cluster_gs_kernel<ClusterBlock<VT, VT, n>>, kClusterBlockThreads, 16, device_),
+                      cluster_fit(cluster_gs_kernel<ClusterBlock<VT, double, n>>, kClusterBlockThreads, 16, device_));
     else
-      best = std::min(cluster_fit(cluster_gs_kernel<ClusterScalar<VT, VT, n, 1>>, kClusterThreads, smem, 16, device_),
-                      cluster_fit(cluster_gs_kernel<ClusterScalar<VT, double, n, 1>>, kClusterThreads, smem, 16, device_));
+      best = std::min(cluster_fit(cluster_gs_kernel<ClusterScalar<VT, VT, n, 1>>, kClusterThreads, 16, device_),
+                      cluster_fit(cluster_gs_kernel<ClusterScalar<VT, double, n, 1>>, kClusterThreads, 16, device_));
   });
   return best;
 }
@@ -1851,6 +1850,7 @@ void AmgPcg<VT>::autotune() {
         set_layout(L, static_cast<int>(k), best_sliced, bestg, ar_);
       }
       L.staged = best_staged;
+      float t_now = 0.f;
       // then one launch per colour pass against one cooperative launch per
       // symmetric step, on the chosen layout (the iterates are identical)
       // (half sweeps run one direction per smoothing call, as per-colour
@@ -1879,8 +1879,9 @@ void AmgPcg<VT>::autotune() {
           t_coop = 1e30f;
         }
         L.coop = t_coop < t_pass;
+        t_now = std::min(t_pass, t_coop);
       }
-      if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k));
+      if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k), t_now);
     }
     if (k + 1 < lv_.size()) {
       Level &Cn = lv_[k + 1];
@@ -1934,7 +1935,7 @@ constexpr long long kClusterPassBlockEntries = 120000;
 template <typename VT>
 bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
   const Csr &a = host_A_.at(k);
-  const int g = cluster_lanes(a.nnz(), a.rows, block_), ncta = cluster_ctas(g, 0);
+  const int g = cluster_lanes(a.nnz(), a.rows, block_), ncta = cluster_ctas(g);
   HostCluster<VT> h;
   if (ncta == 0) return false;
   if (block_) {
@@ -1943,13 +1944,14 @@ bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
     if (!make_cluster<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_slots(static_cast<int>(sizeof(VT)) * (block_ ? 3 : 1), L.relaxed, device_), h)) return false;
   }
   L.K = upload_cluster<VT>(where, h, block_ ? L.B1.dinv : nullptr);
-  return cluster_ctas(g, L.K.smem(block_ ? 3 : 1)) >= ncta;
+  return true;
 }
 
 // One smoothing step of the level as the solve runs it, per-colour (or
-// cooperative) launches against one cluster; the faster is kept.
+// cooperative) launches (t_now ms when already timed, else 0) against one
+// cluster; the faster is kept.
 template <typename VT>
-void AmgPcg<VT>::tune_cluster(Level &L, int k) {
+void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
   L.cluster = false;
   if (host_A_.at(k).nnz() > (block_ ? kClusterPassBlockEntries : kClusterPassEntries) * L.ncolors) return;
   auto step = [&] {
@@ -1962,9 +1964,9 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k) {
   };
   std::unique_ptr<Arena> arena(new Arena);
   if (!build_cluster(L, k, *arena)) return;
-  const float t_pass = time_segment(step, 10, 2);
+  const float t_pass = t_now > 0.f ? t_now : time_segment(step, 10);
   L.cluster = true;
-  L.cluster = time_segment(step, 10, 2) < t_pass;
+  L.cluster = time_segment(step, 10) < t_pass;
   CK(cudaStreamSynchronize(stream_));
   if (L.cluster) kept_layouts_.push_back(std::move(arena));
 }
