@@ -20,10 +20,12 @@
 //     (values and 16-bit slot numbers, slot pairs, threads contiguous), and
 //     every thread loads its next row's operands before it waits.
 // Measured (one B200, FP64, level 2 of a 61 x 47 x 83 Poisson: 5,103 rows, 37
-// colours, 361 k entries): a symmetric step of 73 passes 183 -> 86 us, 1.0 us
-// a pass. What is left of a pass: 0.78 us with next to no rows (message,
-// mbarrier wake-up, shuffles, quotient), the rest shared memory gathers (bank
-// conflicts) and the issue of the 16 warps.
+// colours, 361 k entries): a symmetric step of 73 passes 183 -> 71 us, 0.84 us
+// a pass, of which 0.74 us are there with next to no rows. A pass is bound by
+// the instructions between two messages (clock: loads issued 360 cycles, wait
+// 190, gathers, sums and shuffles 640, quotient 190, messages 300), not by the
+// message, so the operands of the next row stay in place (two units change
+// roles from pass to pass) and the way to the messages has no branch.
 //
 // No race. Row j of colour c' is overwritten in CTA B's slots only after the
 // owner A of j has waited for every earlier pass of the sweep, and A receives
@@ -125,33 +127,41 @@ __device__ __forceinline__ unsigned remote(unsigned addr, unsigned cta) {
   asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(cta));
   return r;
 }
-__device__ __forceinline__ void send_value(unsigned addr, double v, unsigned bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(addr),
-               "l"(__double_as_longlong(v)), "r"(bar)
-               : "memory");
+__device__ __forceinline__ void send_value(unsigned addr, double v, unsigned bar, bool on) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];\n}" ::"r"(addr),
+      "l"(__double_as_longlong(v)), "r"(bar), "r"(static_cast<unsigned>(on))
+      : "memory");
 }
-__device__ __forceinline__ void send_value(unsigned addr, float v, unsigned bar) {
-  asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];" ::"r"(addr),
-               "r"(__float_as_uint(v)), "r"(bar)
-               : "memory");
+__device__ __forceinline__ void send_value(unsigned addr, float v, unsigned bar, bool on) {
+  asm volatile(
+      "{\n .reg .pred p;\n setp.ne.u32 p, %3, 0;\n"
+      " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b32 [%0], %1, [%2];\n}" ::"r"(addr),
+      "r"(__float_as_uint(v)), "r"(bar), "r"(static_cast<unsigned>(on))
+      : "memory");
 }
-// The W values of a row: 16 bytes a message where they fill it.
+// The W values of a row, if `on`: 16 bytes a message where they fill it.
 template <typename T, int W>
-__device__ __forceinline__ void send_row(unsigned addr, const T (&v)[W], unsigned bar) {
+__device__ __forceinline__ void send_row(unsigned addr, const T (&v)[W], unsigned bar, bool on) {
   if constexpr (W == 4 && sizeof(T) == 4) {
-    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];" ::"r"(addr),
-                 "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
-                 "r"(__float_as_uint(v[3])), "r"(bar)
-                 : "memory");
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.u32 p, %6, 0;\n"
+        " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v4.b32 [%0], {%1, %2, %3, %4}, [%5];\n}" ::"r"(addr),
+        "r"(__float_as_uint(v[0])), "r"(__float_as_uint(v[1])), "r"(__float_as_uint(v[2])),
+        "r"(__float_as_uint(v[3])), "r"(bar), "r"(static_cast<unsigned>(on))
+        : "memory");
   } else if constexpr (W == 4) {
 #pragma unroll
     for (int j = 0; j < 4; j += 2)
-      asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(addr + 8 * j),
-                   "l"(__double_as_longlong(v[j])), "l"(__double_as_longlong(v[j + 1])), "r"(bar)
-                   : "memory");
+      asm volatile(
+          "{\n .reg .pred p;\n setp.ne.u32 p, %4, 0;\n"
+          " @p st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];\n}" ::"r"(addr + 8 * j),
+          "l"(__double_as_longlong(v[j])), "l"(__double_as_longlong(v[j + 1])), "r"(bar), "r"(static_cast<unsigned>(on))
+          : "memory");
   } else {
 #pragma unroll
-    for (int j = 0; j < W; ++j) send_value(addr + j * static_cast<unsigned>(sizeof(T)), v[j], bar);
+    for (int j = 0; j < W; ++j) send_value(addr + j * static_cast<unsigned>(sizeof(T)), v[j], bar, on);
   }
 }
 
@@ -435,16 +445,16 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
   // the first row's matrix operands do not change during a solve
   constexpr int kLog = G == 4 ? 2 : (G == 8 ? 3 : (G == 16 ? 4 : 5));
   const int grp = tid >> kLog, groups = nthr >> kLog;
-  typename Row::Unit cur, nxt;
+  typename Row::Unit unit0, unit1;
   unsigned code = plist[0];
   ClusterSeg sg = seg[code & 0x7fffu];
   if (tid < sg.stride) {
-    Row::load(A, sg, 0, tid, sg.row0 + min(grp, sg.rows - 1), cur);
-    cur.send = load_early(A.send + sg.sbase + tid);
+    Row::load(A, sg, 0, tid, sg.row0 + min(grp, sg.rows - 1), unit0);
+    unit0.send = load_early(A.send + sg.sbase + tid);
   }
   const bool stop = pass_entry(status.stop);  // the same in every CTA: only a finished kernel writes it
   if (!stop) {
-    if (tid < sg.stride) Row::load_b(b, sg.row0 + min(grp, sg.rows - 1), cur);
+    if (tid < sg.stride) Row::load_b(b, sg.row0 + min(grp, sg.rows - 1), unit0);
     for (int i = tid; i < (A.max_slots + 1) * W; i += nthr) {
       const int slot = i / W;
       const T v = zero || slot >= nslots ? T(0) : x[static_cast<size_t>(__ldg(A.slot_row + s0 + slot)) * W + i % W];
@@ -459,7 +469,11 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
   const int keep = npass - (P.dir == 0 ? P.count(P.sweeps() - 1) + P.count(P.sweeps() - 2) : A.ncolors);
   int p = 0, t = 0;
   bool fresh = true, dead = false;  // first pass of a sweep; a wait gave up
-  for (;;) {
+  const bool weighted = nw != nullptr || wts != nullptr || omega != T(1);
+  // One unit (a trip of a pass) from `cur`, the next one's operands into
+  // `nxt`; true at the end. The two change places from call to call: moved
+  // instead, the operands would have to arrive a unit early.
+  const auto step = [&](typename Row::Unit &cur, typename Row::Unit &nxt) __attribute__((always_inline)) {
     // the next unit's operands, before this one waits
     const bool last_trip = t + 1 == sg.trips;
     const int tn = last_trip ? 0 : t + 1;
@@ -482,27 +496,28 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     if (tid < sg.stride) {
       T sum[W], xn[W];
       Row::sums(A, sg, t, tid, xs, cur, sum);
-      const int local = t * groups + grp;
-      if (local < sg.rows) {
-        Row::update(cur, sum, xn);
-        const T w = nw != nullptr ? __ldg(nw + sg.row0 + local)
-                                  : (wts != nullptr ? __ldg(wts + (code & 0x7fffu)) : omega);
+      // lanes past the piece's rows compute along (their sums are zero and
+      // they send nothing): no branch on the way to the messages
+      Row::update(cur, sum, xn);
+      const int local = t * groups + grp, row = sg.row0 + min(local, sg.rows - 1);
+      if (weighted) {
+        const T w = nw != nullptr ? __ldg(nw + row) : (wts != nullptr ? __ldg(wts + (code & 0x7fffu)) : omega);
         if (w != T(1)) {
-          const unsigned own = W * __ldg(A.own + sg.row0 + local);
+          const unsigned own = W * __ldg(A.own + row);
 #pragma unroll
           for (int j = 0; j < W; ++j) xn[j] = fma(T(1) - w, xs[own + j], w * xn[j]);
         }
-        if (cur.send != kNoSend) send_row(to_x, xn, to_bar);
+      }
+      send_row(to_x, xn, to_bar, cur.send != kNoSend);
+      if (sg.schunks > 1)
         for (int q = 1; q < sg.schunks; ++q) {
           const unsigned to = __ldg(A.send + sg.sbase + (t * sg.schunks + q) * sg.stride + tid);
-          if (to != kNoSend)
-            send_row(remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (to & 0xffffu), to >> 16), xn,
-                     remote(bar_addr + 8 * p, to >> 16));
+          send_row(remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (to & 0xffffu), (to >> 16) & 15u), xn,
+                   remote(bar_addr + 8 * p, (to >> 16) & 15u), to != kNoSend);
         }
-        if (p >= keep && (tid & (G - 1)) == 0)
+      if (p >= keep && (tid & (G - 1)) == 0 && local < sg.rows)
 #pragma unroll
-          for (int j = 0; j < W; ++j) x[static_cast<size_t>(sg.row0 + local) * W + j] = xn[j];
-      }
+        for (int j = 0; j < W; ++j) x[static_cast<size_t>(row) * W + j] = xn[j];
     }
     fresh = false;
     if (last_trip) {
@@ -515,7 +530,7 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
           for (int k = tid; k < nslots * W; k += nthr) xp[k] = xs[k];
         }
         cluster_barrier();
-        if (next_code == 0xffffu) break;
+        if (next_code == 0xffffu) return true;
         fresh = true;
       }
       ++p;
@@ -523,7 +538,11 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     code = next_code;
     t = tn;
     sg = sn;
-    cur = nxt;
+    return false;
+  };
+  for (;;) {
+    if (step(unit0, unit1)) break;
+    if (step(unit1, unit0)) break;
   }
   if (dead) {
     *status.fault = 1;

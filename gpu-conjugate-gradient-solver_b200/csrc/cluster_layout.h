@@ -282,7 +282,7 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
 
 // Lanes per row: about five entries, or two 3x3 blocks, a lane (what a thread
 // loads ahead). Fewer lanes leave the loaded-ahead slots (5,103 rows, 70
-// entries a row: 125 us a step with 8 lanes, 86 with 16, 90 with 32).
+// entries a row: 111 us a step with 8 lanes, 71 with 16, 80 with 32).
 inline int cluster_lanes(long long nnz, int rows, bool block) {
   const double len = static_cast<double>(nnz) / std::max(1, rows) / (block ? 3.0 : 1.0) - 1.0;
   int g = 4;

@@ -1923,7 +1923,7 @@ void AmgPcg<VT>::autotune() {
 // Entries per colour pass up to which a level is tried in one cluster. One
 // cluster's 16 SMs beat a launch per pass while a
 // pass is latency: FP64 symmetric steps, cluster / launches: 9.8 k entries a
-// pass (5,103 rows, 37 colours) 86 / 183 us, 8.2 k (4,143, 23) 53 / 108,
+// pass (5,103 rows, 37 colours) 71 / 183 us, 8.2 k (4,143, 23) 53 / 108,
 // 13.5 k (4,096, 2) 7.7 / 9.4; above, the 16 SMs' gathers bound it: 58 k
 // (32,768, 8) 58 / 37, 66 k (37,505, 18) 120 / 95.
 constexpr long long kClusterPassEntries = 40000;
