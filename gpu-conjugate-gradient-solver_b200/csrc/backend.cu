@@ -220,10 +220,10 @@ void spmv(const DeviceCsr *m, const void *x, void *y, cudaStream_t s) {
   const int gb = std::min((m->rows * 8 + 255) / 256, 148 * 16);
   if (m->dtype == GS_F32) {
     CsrvView<float> v{m->rows, m->rp, m->ci, static_cast<const float *>(m->v), nullptr, m->rp + 1};
-    csrv_spmv_kernel<float, float, kSpmvSet, 8><<<gb, 256, 0, s>>>(v, static_cast<const float *>(x), static_cast<float *>(y), nullptr, nullptr, 0, m->rows, FirstColour<float>{});
+    csrv_spmv_kernel<float, float, kSpmvSet, 8><<<gb, 256, 0, s>>>(v, static_cast<const float *>(x), static_cast<float *>(y), nullptr, nullptr, 0, m->rows, FirstColour<float>{}, static_cast<float *>(nullptr));
   } else {
     CsrvView<double> v{m->rows, m->rp, m->ci, static_cast<const double *>(m->v), nullptr, m->rp + 1};
-    csrv_spmv_kernel<double, double, kSpmvSet, 8><<<gb, 256, 0, s>>>(v, static_cast<const double *>(x), static_cast<double *>(y), nullptr, nullptr, 0, m->rows, FirstColour<double>{});
+    csrv_spmv_kernel<double, double, kSpmvSet, 8><<<gb, 256, 0, s>>>(v, static_cast<const double *>(x), static_cast<double *>(y), nullptr, nullptr, 0, m->rows, FirstColour<double>{}, static_cast<double *>(nullptr));
   }
   check(cudaGetLastError(), "spmv");
 }

@@ -258,7 +258,8 @@ struct FirstColour {
   }
 };
 
-// y = A x (kSpmvSet), y = b - A x (kSpmvResid), y += A x (kSpmvAdd).
+// y = A x (kSpmvSet), y = b - A x (kSpmvResid), y += A x (kSpmvAdd, a copy of
+// the result to y2 when given).
 // One warp per slice, grid-stride over slices. G lanes per row: a slice holds
 // 32 / G rows, lane l serves row l / G and the group adds its partial sums.
 template <typename T, typename BT, int kMode, int G = 1>
@@ -266,7 +267,7 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
                                                         const int *done, int s_begin, int s_end,
-                                                        FirstColour<T> fc = FirstColour<T>{}) {
+                                                        FirstColour<T> fc = FirstColour<T>{}, T *y2 = nullptr) {
   if (pass_entry(done)) return;
   const int lane = threadIdx.x & 31;
   const int warps = (gridDim.x * blockDim.x) >> 5;
@@ -284,7 +285,11 @@ __global__ void __launch_bounds__(256) sell_spmv_kernel(SellView<T> A, const T *
         if (fc.x != nullptr) fc(row, sum);
       } else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
-      else y[row] += sum;
+      else {
+        const T v = y[row] + sum;
+        y[row] = v;
+        if (y2 != nullptr) y2[row] = v;
+      }
     }
   }
 }
@@ -482,7 +487,7 @@ __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *
                                                         T *__restrict__ y,
                                                         const BT *__restrict__ b,
                                                         const int *done, int row_begin, int row_end,
-                                                        FirstColour<T> fc = FirstColour<T>{}) {
+                                                        FirstColour<T> fc = FirstColour<T>{}, T *y2 = nullptr) {
   const int sub = threadIdx.x & (G - 1);
   const int groups = (gridDim.x * blockDim.x) / G;
   // every lane of a warp runs the same number of trips so the shuffles
@@ -511,7 +516,11 @@ __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *
       } else if (kMode == kSpmvResid) y[row] = T(b[row]) - sum;
       else if (kMode == kSpmvTwice) y[row] = sum + sum;
       else if (kMode == kSpmvNeg) y[row] = -sum;
-      else y[row] += sum;
+      else {
+        const T v = y[row] + sum;
+        y[row] = v;
+        if (y2 != nullptr) y2[row] = v;
+      }
     }
   }
 }

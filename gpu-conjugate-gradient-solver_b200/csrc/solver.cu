@@ -522,9 +522,10 @@ class AmgPcg final : public Solver {
 
   // dir: 0 symmetric steps (forward then backward colours), 1 forward
   // sweeps only, 2 backward sweeps only (half_sweeps pre / post smoothing)
-  // first_done: the first colour of a sweep from zero is already in x
+  // ready: what the first sweep begins with is there already -- from zero, its
+  // first colour in x; else, on a relaxed level, the copy of x it reads
   template <typename BT>
-  void smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir = 0, bool first_done = false);
+  void smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir = 0, bool ready = false);
   FirstColour<VT> first_colour(int k, VT *x);
   template <typename BT>
   void gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaStream_t s);
@@ -580,11 +581,11 @@ class AmgPcg final : public Solver {
   void level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, Part part, cudaStream_t s);
   void restrict_residual(Level &L, Part part, VT *y, cudaStream_t s, FirstColour<VT> fc = FirstColour<VT>{});
   template <int kMode>
-  void prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s);
+  void prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s, VT *copy = nullptr);
   void precondition(const double *r, VT *z, cudaStream_t s, bool first_done = false);
   template <int kMode, typename BT>
   void transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g, const VT *x, VT *y,
-                const BT *b, cudaStream_t s, FirstColour<VT> fc = FirstColour<VT>{});
+                const BT *b, cudaStream_t s, FirstColour<VT> fc = FirstColour<VT>{}, VT *y2 = nullptr);
   void autotune();
   float time_ms(const std::function<void()> &f, int reps);
   void cg_iteration(int parity, cudaStream_t s);
@@ -1278,7 +1279,7 @@ void AmgPcg<VT>::gs_pass(Level &L, int c, const BT *rhs, VT *x, bool zero, cudaS
 // each step is a forward sweep over colours 0..C-1 then a backward sweep.
 template <typename VT>
 template <typename BT>
-void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir, bool first_done) {
+void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cudaStream_t s, int dir, bool ready) {
   const int *done = &st_->done;
   if (L.kind == 4) {  // IdentityPreconditioner::apply
     launch_pass(pdl_, convert_kernel<VT, BT>, blocks_for(L.n, cap_blocks_), s, L.n, rhs, x, done);
@@ -1315,10 +1316,10 @@ void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cu
     // one direction per step: consecutive passes never repeat a colour
     for (int step = 0; step < steps; ++step) {
       const bool zs = zero && step == 0 && dir == 1;
-      if (!zs) sweep_start(L, x, s);  // from zero the own colour is skipped anyway
+      if (!zs && !(ready && step == 0)) sweep_start(L, x, s);  // from zero the own colour is skipped anyway
       for (int i = 0; i < L.ncolors; ++i) {
         const int c = dir == 1 ? i : L.ncolors - 1 - i;
-        if (first_done && step == 0 && i == 0) continue;
+        if (zs && ready && i == 0) continue;
         // from a zero iterate the first forward sweep skips the later colours'
         // gathers; a backward sweep from zero has no such shortcut
         gs_pass(L, c, rhs, x, zs, s);
@@ -1332,10 +1333,10 @@ void AmgPcg<VT>::smooth(Level &L, const BT *rhs, VT *x, int steps, bool zero, cu
   }
   const bool skip = skip_repeats(L);
   for (int step = 0; step < steps; ++step) {
-    if (!(zero && step == 0)) sweep_start(L, x, s);
+    if (step > 0 || !(zero || ready)) sweep_start(L, x, s);
     for (int c = 0; c < L.ncolors; ++c) {
       if (skip && step > 0 && c == 0) continue;  // the backward sweep just ended with colour 0
-      if (first_done && step == 0 && c == 0) continue;
+      if (zero && ready && step == 0 && c == 0) continue;
       gs_pass(L, c, rhs, x, zero && step == 0, s);
     }
     sweep_start(L, x, s);
@@ -1546,7 +1547,7 @@ void AmgPcg<VT>::level_spmv_resid(Level &L, const BT *rhs, const VT *x, VT *r, P
     const int gb = blocks_for(32LL * (s1 - s0), cap_blocks_);
 #define RES_SELL(G)                                                                                      \
   if (part.upper) launch_pass(pdl_, sell_upper_kernel<VT, G>, gb, s, L.A.view(), x, r, done, s0, s1);     \
-  else launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.A.view(), x, r, rhs, done, s0, s1, FirstColour<VT>{});
+  else launch_pass(pdl_, sell_spmv_kernel<VT, BT, kSpmvResid, G>, gb, s, L.A.view(), x, r, rhs, done, s0, s1, FirstColour<VT>{}, static_cast<VT *>(nullptr));
     switch (L.g) {
       case 1: RES_SELL(1) break;
       case 2: RES_SELL(2) break;
@@ -1575,11 +1576,11 @@ void AmgPcg<VT>::restrict_residual(Level &L, Part part, VT *y, cudaStream_t s, F
 // x += P xc (kSpmvAdd; kSpmvTwice as the mode says) on the rows of `part`.
 template <typename VT>
 template <int kMode>
-void AmgPcg<VT>::prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s) {
+void AmgPcg<VT>::prolong(Level &L, Part part, const VT *xc, VT *x, cudaStream_t s, VT *copy) {
   const int u = block_ ? 3 : 1, r0 = u * L.color_first[part.c0], r1 = u * L.color_first[part.c1];
   if (r1 <= r0) return;
   transfer<kMode, VT>(L.P.view(), L.P.slice_of(r0), L.P.slice_of(r1), L.Pc.view(), r0, r1, L.pg, xc, x,
-                      (const VT *)nullptr, s);
+                      (const VT *)nullptr, s, FirstColour<VT>{}, copy);
   CKL("prolongation");
 }
 
@@ -1670,9 +1671,14 @@ void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s, 
   const FirstColour<VT> fc = first_colour(k + 1, C.x);
   restrict_residual(L, part, C.b, s, fc);
   vcycle<VT>(k + 1, C.b, C.x, true, s, fc.x != nullptr);
+  const int dir = opt_.half_sweeps ? 2 : 0;
+  // relaxed passes read their own colour as their sweep found it: the
+  // prolongation writes that copy along (a copy of its own is a node between
+  // kernels, 4 us with the overlap it interrupts)
+  const bool copied = L.relaxed && !opt_.reference_vcycle && !in_cluster(L, opt_.post, dir);
   if (opt_.reference_vcycle && k > 0) prolong<kSpmvTwice>(L, swept_part(L), C.x, x, s);
-  else prolong<kSpmvAdd>(L, swept_part(L), C.x, x, s);
-  smooth(L, rhs, x, opt_.post, false, s, opt_.half_sweeps ? 2 : 0);
+  else prolong<kSpmvAdd>(L, swept_part(L), C.x, x, s, copied ? L.xprev : nullptr);
+  smooth(L, rhs, x, opt_.post, false, s, dir, copied);
 }
 
 // y (op)= M x on rows [r0, r1) of M in SELL-32 (g == 1, slices [s0, s1)) or
@@ -1680,19 +1686,19 @@ void AmgPcg<VT>::vcycle(int k, const BT *rhs, VT *x, bool zero, cudaStream_t s, 
 template <typename VT>
 template <int kMode, typename BT>
 void AmgPcg<VT>::transfer(const SellView<VT> &S, int s0, int s1, const CsrvView<VT> &Cm, int r0, int r1, int g,
-                          const VT *x, VT *y, const BT *b, cudaStream_t s, FirstColour<VT> fc) {
+                          const VT *x, VT *y, const BT *b, cudaStream_t s, FirstColour<VT> fc, VT *y2) {
   const int *done = &st_->done;
   if (g == 1) {
     launch_pass(pdl_, sell_spmv_kernel<VT, BT, kMode>, blocks_for(32LL * (s1 - s0), cap_blocks_), s, S, x, y, b, done, s0,
-                s1, fc);
+                s1, fc, y2);
     return;
   }
   const int gb = blocks_for(static_cast<long long>(r1 - r0) * g, cap_blocks_);
   switch (g) {
-    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
-    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
-    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
-    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm, x, y, b, done, r0, r1, fc); break;
+    case 4: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 4>, gb, s, Cm, x, y, b, done, r0, r1, fc, y2); break;
+    case 8: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 8>, gb, s, Cm, x, y, b, done, r0, r1, fc, y2); break;
+    case 16: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 16>, gb, s, Cm, x, y, b, done, r0, r1, fc, y2); break;
+    default: launch_pass(pdl_, csrv_spmv_kernel<VT, BT, kMode, 32>, gb, s, Cm, x, y, b, done, r0, r1, fc, y2); break;
   }
 }
 
