@@ -1624,7 +1624,7 @@ void AmgPcg<VT>::dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s) {
     }
     CKL("coarse solve (reduce)");
   } else {
-    launch_pass(pdl_, dense_solve_kernel<BT, VT>, (L.n + 7) / 8, s, L.n, L.ainv, rhs, x, done);
+    launch_pass(pdl_, dense_solve_kernel<BT, VT>, (L.n + kDenseRows - 1) / kDenseRows, s, L.n, L.ainv, rhs, x, done);
     CKL("coarse solve");
   }
 }
