@@ -645,7 +645,7 @@ class AmgPcg final : public Solver {
   size_t tail_smem_ = 0;         // dynamic shared memory of the tail launch (x replicas)
   bool tail_on_ = false;
   int tail_cluster_size(size_t smem, int want);
-  float time_segment(const std::function<void()> &f, int reps, int trials = 1);
+  float time_segment(const std::function<void()> &f, int reps, int trials = 1, bool as_issued = false);
   void upload_tail_table(int k0);
   TailLevel<VT> *tail_lv_ = nullptr;
   void setup_tail();
@@ -955,7 +955,8 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
     info_[k].tail_ctas = info_[k].in_tail ? tail_cluster_ : 0;
     info_[k].lanes = lv_[k].g;
     info_[k].sliced = lv_[k].sliced ? 1 : 0;
-    info_[k].launch = lv_[k].coop || lv_[k].cluster ? 1 : (lv_[k].staged ? 2 : 0);
+    // block levels tell their colour passes apart (0, 2), in a cluster or not
+    info_[k].launch = lv_[k].coop || (lv_[k].cluster && !block_) ? 1 : (lv_[k].staged ? 2 : 0);
     info_[k].p_lanes = lv_[k].pg;
     info_[k].r_lanes = lv_[k].rg;
   }
@@ -1864,11 +1865,11 @@ void AmgPcg<VT>::autotune() {
       if (L.kind == 0 && !block_ && !L.relaxed && !opt_.half_sweeps && opt_.sweep_launch == 1) {
         auto step = [&] { smooth<VT>(L, L.b, L.x, 1, false, stream_); };
         L.coop = false;
-        const float t_pass = time_segment(step, 10);
+        const float t_pass = time_segment(step, 10, 1, true);
         L.coop = true;
         float t_coop = 1e30f;
         try {
-          t_coop = time_segment(step, 10);
+          t_coop = time_segment(step, 10, 1, true);
           CgState hs{};
           CK(cudaMemcpy(&hs, st_, sizeof(CgState), cudaMemcpyDeviceToHost));
           check_sync_fault(hs);
@@ -1884,8 +1885,10 @@ void AmgPcg<VT>::autotune() {
           cudaGetLastError();
           t_coop = 1e30f;
         }
-        L.coop = t_coop < t_pass;
-        t_now = std::min(t_pass, t_coop);
+        // timed back to back the host's issue counts in full; in a solve it runs
+        // ahead for part of the time: a tenth in favour of the passes
+        L.coop = t_coop < 0.9f * t_pass;
+        t_now = L.coop ? t_coop : t_pass;
       }
       if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k), t_now);
     }
@@ -1970,9 +1973,9 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
   };
   std::unique_ptr<Arena> arena(new Arena);
   if (!build_cluster(L, k, *arena)) return;
-  const float t_pass = t_now > 0.f ? t_now : time_segment(step, 10);
+  const float t_pass = t_now > 0.f ? t_now : time_segment(step, 10, 1, true);
   L.cluster = true;
-  L.cluster = time_segment(step, 10) < t_pass;
+  L.cluster = time_segment(step, 10, 1, true) < t_pass;
   CK(cudaStreamSynchronize(stream_));
   if (L.cluster) kept_layouts_.push_back(std::move(arena));
 }
@@ -2079,16 +2082,21 @@ void AmgPcg<VT>::upload_tail_table(int k0) {
   tail_k0_ = k0;
 }
 
-// Times f() as the solve will run it: replayed from a captured CUDA graph
-// in graph mode, launched on the stream otherwise.
+// Times f() as the GPU will run it in the solve, replayed from a captured CUDA
+// graph, or as an eager solve issues it.
 template <typename VT>
-float AmgPcg<VT>::time_segment(const std::function<void()> &f, int reps, int trials) {
+float AmgPcg<VT>::time_segment(const std::function<void()> &f, int reps, int trials, bool as_issued) {
   // A pass reads its matrix before it waits on the launch ahead of it: the
   // uploads of a new layout have landed, and the first launch follows an
   // operation of the stream that is not a kernel, so it starts in plain order
   CK(cudaDeviceSynchronize());
   CK(cudaMemsetAsync(sync_, 0, sizeof(SweepSync), stream_));
-  if (!opt_.graph) {
+  // Layouts of eager solves are timed from a graph too: the host issues the
+  // repeated passes of a small level more slowly than the GPU runs them, so
+  // that every layout would seem to take the same time. Not with
+  // overlap_launch 1, whose graphs have other edges than its stream, nor where
+  // candidates differ in their number of launches (as_issued).
+  if (!opt_.graph && (as_issued || opt_.overlap_launch == 1)) {
     float t = time_ms(f, reps);
     for (int i = 1; i < trials; ++i) t = std::min(t, time_ms(f, reps));
     return t;
@@ -2163,7 +2171,7 @@ void AmgPcg<VT>::setup_tail() {
   auto segment = [&] { vcycle<VT>(kmin, T0.b, T0.x, true, stream_); };
   float best = 1e30f;
   int best_k0 = -1, best_cl = 0;
-  if (opt_.tail == 1) best = time_segment(segment, 3);
+  if (opt_.tail == 1) best = time_segment(segment, 3, 1, true);
   for (int k0 : cands) {
     if (opt_.tail == 2 && k0 != kmin) continue;
     upload_tail_table(k0);
@@ -2174,7 +2182,7 @@ void AmgPcg<VT>::setup_tail() {
       prev = cl;
       tail_cluster_ = cl;
       tail_on_ = true;
-      const float t = time_segment(segment, 3);
+      const float t = time_segment(segment, 3, 1, true);
       tail_on_ = false;
       if (t < best || (opt_.tail == 2 && best_k0 < 0)) best = t, best_k0 = k0, best_cl = cl;
     }

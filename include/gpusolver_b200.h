@@ -344,8 +344,9 @@ int gs_solver_level_layout(const gs_solver *s, int level);
 /* How `level`'s colour passes are launched: 0 one kernel per colour pass,
  * 1 one kernel per smoothing step (grid barriers between the colours, or one
  * thread-block cluster), 2 one kernel per colour pass that bulk-copies each BELL-1
- * slice's blocks to shared memory (gs_solver_options.sweep_launch chooses);
- * -1 on a bad argument. No reference counterpart. */
+ * slice's blocks to shared memory (gs_solver_options.sweep_launch chooses;
+ * a 3x3 block level whose steps run in a cluster reports what its colour
+ * passes would use); -1 on a bad argument. No reference counterpart. */
 int gs_solver_level_launch(const gs_solver *s, int level);
 /* Average device milliseconds of one launch of a kernel, CUDA events on
  * `stream`: kind 0 outer SpMV (+ p.Ap), 1 one forward GS sweep of the finest
