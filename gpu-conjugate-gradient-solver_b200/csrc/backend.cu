@@ -18,6 +18,7 @@
 #include <vector>
 
 #include "backend.h"
+#include "formats.cuh"
 #include "kernels.cuh"
 
 namespace gsb {
@@ -54,6 +55,15 @@ DotScratch &dot_scratch() {
   return s;
 }
 
+// Entry of the kernels below. They are launched with programmatic stream
+// serialization, so that a chain of Backend calls does not start each kernel
+// cold, and read nothing before the wait: what a call is given may be the
+// output of whatever precedes it on the caller's stream.
+__device__ __forceinline__ void backend_entry() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+
 // result = x . y, sequential-order partials per block, the last block adds
 // the partials in block order (deterministic for a given n).
 template <typename T>
@@ -61,6 +71,7 @@ __global__ void __launch_bounds__(256) dot_kernel(int n, const T *__restrict__ x
                                                   const T *__restrict__ y, T *result,
                                                   double *partials, unsigned int *ticket) {
   __shared__ double smem[32];
+  backend_entry();
   double acc[1] = {0.0};
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride)
@@ -68,61 +79,101 @@ __global__ void __launch_bounds__(256) dot_kernel(int n, const T *__restrict__ x
   if (grid_sum<1>(acc, partials, ticket, smem) && threadIdx.x == 0) *result = T(acc[0]);
 }
 
+// 8 lanes per listed row, 4 entries per lane and trip: their columns, then
+// the gathers and values, then the FMAs.
 template <typename T>
-__global__ void gs_color_indirect_kernel(int n, const int *__restrict__ rp, const int *__restrict__ ci,
-                                         const T *__restrict__ v, const int *__restrict__ order,
-                                         long long start, long long count, const T *__restrict__ rhs,
-                                         T *__restrict__ x, T omega) {
-  // 8 lanes per listed row
+__global__ void __launch_bounds__(256) gs_color_indirect_kernel(const int *rp, const int *ci, const T *v, const int *order,
+                                                                long long start, long long count, const T *rhs, T *x,
+                                                                T omega) {
+  backend_entry();
   const int sub = threadIdx.x & 7;
   const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 3;
   const bool valid = i < count;
   const int row = valid ? order[start + i] : 0;
-  T off = T(0), diag = T(0);
-  if (valid)
-    for (int k = rp[row] + sub; k < rp[row + 1]; k += 8) {
-      const int c = ci[k];
-      if (c == row) diag = v[k];
-      else off = fma(v[k], x[c], off);
+  T off = T(0), diag = T(0), b = T(0), own = T(0);
+  if (valid) {
+    b = rhs[row];
+    own = x[row];
+    const int k1 = rp[row + 1];
+    for (int k = rp[row] + sub; k < k1; k += 32) {
+      int c[4];
+      T a[4], xv[4];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) c[u] = k + 8 * u < k1 ? ci[k + 8 * u] : -1;
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        a[u] = c[u] >= 0 ? v[k + 8 * u] : T(0);
+        xv[u] = c[u] >= 0 && c[u] != row ? x[c[u]] : T(0);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        if (c[u] == row) diag = a[u];
+        else off = fma(a[u], xv[u], off);
+      }
     }
+  }
   for (int o = 4; o > 0; o >>= 1) {
     off += __shfl_xor_sync(0xffffffffu, off, o, 8);
     diag += __shfl_xor_sync(0xffffffffu, diag, o, 8);
   }
-  if (valid && sub == 0) x[row] = (T(1) - omega) * x[row] + omega * ((rhs[row] - off) / diag);
+  if (valid && sub == 0) x[row] = (T(1) - omega) * own + omega * ((b - off) / diag);
 }
 
+// 16 lanes per listed node, each taking every 16th entry of the node's three
+// rows.
 template <typename T>
-__global__ void block_gs_indirect_kernel(const int *__restrict__ rp, const int *__restrict__ ci,
-                                         const T *__restrict__ v, const int *__restrict__ order,
-                                         long long start, long long count,
-                                         const T *__restrict__ dinv, const T *__restrict__ rhs,
-                                         T *__restrict__ x, T omega) {
-  const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
-  if (i >= count) return;
-  const int blk = order[start + i], r0 = 3 * blk;
-  T res[3];
-  for (int l = 0; l < 3; ++l) {
-    T s = T(0);
-    for (int k = rp[r0 + l]; k < rp[r0 + l + 1]; ++k) {
-      const int c = ci[k];
-      if (c >= r0 && c < r0 + 3) continue;
-      s = fma(v[k], x[c], s);
+__global__ void __launch_bounds__(256) block_gs_indirect_kernel(const int *rp, const int *ci, const T *v, const int *order,
+                                                                long long start, long long count, const T *dinv,
+                                                                const T *rhs, T *x, T omega) {
+  backend_entry();
+  const int sub = threadIdx.x & 15;
+  const long long i = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) >> 4;
+  const bool valid = i < count;
+  const int blk = valid ? order[start + i] : 0, r0 = 3 * blk;
+  T res[3] = {T(0), T(0), T(0)};
+  if (valid) {
+    int k0[3], k1[3], len = 0;
+#pragma unroll
+    for (int l = 0; l < 3; ++l) {
+      k0[l] = rp[r0 + l] + sub;
+      k1[l] = rp[r0 + l + 1];
+      len = max(len, k1[l] - k0[l]);
     }
-    res[l] = rhs[r0 + l] - s;
+    for (int k = 0; k < len; k += 16) {
+      int c[3];
+      T a[3], xv[3];
+#pragma unroll
+      for (int l = 0; l < 3; ++l) c[l] = k0[l] + k < k1[l] ? ci[k0[l] + k] : r0;
+#pragma unroll
+      for (int l = 0; l < 3; ++l) {
+        const bool use = c[l] < r0 || c[l] >= r0 + 3;  // not the node's own block
+        a[l] = use ? v[k0[l] + k] : T(0);
+        xv[l] = use ? x[c[l]] : T(0);
+      }
+#pragma unroll
+      for (int l = 0; l < 3; ++l) res[l] = fma(a[l], xv[l], res[l]);
+    }
   }
-  const T *bi = dinv + 9 * static_cast<size_t>(blk);
-  for (int l = 0; l < 3; ++l) {
-    T nv = bi[3 * l] * res[0];
-    nv = fma(bi[3 * l + 1], res[1], nv);
-    nv = fma(bi[3 * l + 2], res[2], nv);
-    x[r0 + l] = (T(1) - omega) * x[r0 + l] + omega * nv;
+  for (int o = 8; o > 0; o >>= 1)
+#pragma unroll
+    for (int l = 0; l < 3; ++l) res[l] += __shfl_xor_sync(0xffffffffu, res[l], o, 16);
+  if (valid && sub == 0) {
+#pragma unroll
+    for (int l = 0; l < 3; ++l) res[l] = rhs[r0 + l] - res[l];
+    const T *bi = dinv + 9 * static_cast<size_t>(blk);
+    for (int l = 0; l < 3; ++l) {
+      T nv = bi[3 * l] * res[0];
+      nv = fma(bi[3 * l + 1], res[1], nv);
+      nv = fma(bi[3 * l + 2], res[2], nv);
+      x[r0 + l] = (T(1) - omega) * x[r0 + l] + omega * nv;
+    }
   }
 }
 
 template <typename T>
 __global__ void block_inverse_apply_kernel(long long nblocks, const T *__restrict__ dinv,
                                            const T *__restrict__ r, T *__restrict__ c) {
+  backend_entry();
   const long long b = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
   const T *bi = dinv + 9 * b;
@@ -134,6 +185,7 @@ __global__ void block_inverse_apply_kernel(long long nblocks, const T *__restric
 template <typename T>
 __global__ void vec_kernel(int op, long long n, const T *__restrict__ x, T *__restrict__ y, T alpha,
                            const T *alpha_dev) {
+  backend_entry();
   const T a = alpha_dev != nullptr ? *alpha_dev : alpha;
   const long long stride = static_cast<long long>(gridDim.x) * blockDim.x;
   for (long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -150,6 +202,7 @@ __global__ void vec_kernel(int op, long long n, const T *__restrict__ x, T *__re
 
 template <typename T>
 __global__ void scalar_kernel(int op, const T *a, const T *b, T *out, T value) {
+  backend_entry();
   switch (op) {
     case GS_SCALAR_DIVIDE: *out = *a / *b; break;
     case GS_SCALAR_MULTIPLY: *out = *a * *b; break;
@@ -234,9 +287,9 @@ void gauss_seidel_color(const DeviceCsr *m, const int *order, long long start, l
   if (count <= 0) return;
   const int gb = static_cast<int>((count * 8 + 255) / 256);
   if (m->dtype == GS_F32)
-    gs_color_indirect_kernel<float><<<gb, 256, 0, s>>>(m->rows, m->rp, m->ci, static_cast<const float *>(m->v), order, start, count, static_cast<const float *>(rhs), static_cast<float *>(x), float(omega));
+    launch_pass(true, gs_color_indirect_kernel<float>, gb, s, m->rp, m->ci, static_cast<const float *>(m->v), order, start, count, static_cast<const float *>(rhs), static_cast<float *>(x), float(omega));
   else
-    gs_color_indirect_kernel<double><<<gb, 256, 0, s>>>(m->rows, m->rp, m->ci, static_cast<const double *>(m->v), order, start, count, static_cast<const double *>(rhs), static_cast<double *>(x), omega);
+    launch_pass(true, gs_color_indirect_kernel<double>, gb, s, m->rp, m->ci, static_cast<const double *>(m->v), order, start, count, static_cast<const double *>(rhs), static_cast<double *>(x), omega);
   check(cudaGetLastError(), "gauss-seidel colour");
 }
 
@@ -244,11 +297,11 @@ void block_gauss_seidel_color3x3(const DeviceCsr *m, const int *order, long long
                                  const void *dinv, const void *rhs, void *x, double omega, cudaStream_t s) {
   if (m->rows % 3 != 0) throw std::runtime_error("3x3 block smoother requires number of DOFs divisible by 3.");
   if (count <= 0) return;
-  const int gb = static_cast<int>((count + 255) / 256);
+  const int gb = static_cast<int>((count * 16 + 255) / 256);
   if (m->dtype == GS_F32)
-    block_gs_indirect_kernel<float><<<gb, 256, 0, s>>>(m->rp, m->ci, static_cast<const float *>(m->v), order, start, count, static_cast<const float *>(dinv), static_cast<const float *>(rhs), static_cast<float *>(x), float(omega));
+    launch_pass(true, block_gs_indirect_kernel<float>, gb, s, m->rp, m->ci, static_cast<const float *>(m->v), order, start, count, static_cast<const float *>(dinv), static_cast<const float *>(rhs), static_cast<float *>(x), float(omega));
   else
-    block_gs_indirect_kernel<double><<<gb, 256, 0, s>>>(m->rp, m->ci, static_cast<const double *>(m->v), order, start, count, static_cast<const double *>(dinv), static_cast<const double *>(rhs), static_cast<double *>(x), omega);
+    launch_pass(true, block_gs_indirect_kernel<double>, gb, s, m->rp, m->ci, static_cast<const double *>(m->v), order, start, count, static_cast<const double *>(dinv), static_cast<const double *>(rhs), static_cast<double *>(x), omega);
   check(cudaGetLastError(), "block gauss-seidel colour");
 }
 
@@ -259,9 +312,9 @@ void apply_block_inverses3x3(long long n, const void *dinv, const void *r, void 
   if (nb == 0) return;
   const int gb = static_cast<int>((nb + 255) / 256);
   if (dtype == GS_F32)
-    block_inverse_apply_kernel<float><<<gb, 256, 0, s>>>(nb, static_cast<const float *>(dinv), static_cast<const float *>(r), static_cast<float *>(c));
+    launch_pass(true, block_inverse_apply_kernel<float>, gb, s, nb, static_cast<const float *>(dinv), static_cast<const float *>(r), static_cast<float *>(c));
   else
-    block_inverse_apply_kernel<double><<<gb, 256, 0, s>>>(nb, static_cast<const double *>(dinv), static_cast<const double *>(r), static_cast<double *>(c));
+    launch_pass(true, block_inverse_apply_kernel<double>, gb, s, nb, static_cast<const double *>(dinv), static_cast<const double *>(r), static_cast<double *>(c));
   check(cudaGetLastError(), "apply block inverses");
 }
 
@@ -270,9 +323,9 @@ void launch_dot(long long n, const void *x, const void *y, void *result, int dty
   if (n < 0 || n > 0x7fffffffLL) throw std::runtime_error("encodeDot: bad size");
   const int gb = std::min(grid_for(n), kDotBlocks);
   if (dtype == GS_F32)
-    dot_kernel<float><<<gb, 256, 0, s>>>(static_cast<int>(n), static_cast<const float *>(x), static_cast<const float *>(y), static_cast<float *>(result), partials, ticket);
+    launch_pass(true, dot_kernel<float>, gb, s, static_cast<int>(n), static_cast<const float *>(x), static_cast<const float *>(y), static_cast<float *>(result), partials, ticket);
   else
-    dot_kernel<double><<<gb, 256, 0, s>>>(static_cast<int>(n), static_cast<const double *>(x), static_cast<const double *>(y), static_cast<double *>(result), partials, ticket);
+    launch_pass(true, dot_kernel<double>, gb, s, static_cast<int>(n), static_cast<const double *>(x), static_cast<const double *>(y), static_cast<double *>(result), partials, ticket);
   check(cudaGetLastError(), "dot");
 }
 
@@ -339,17 +392,17 @@ void vector_op(int op, long long n, const void *x, void *y, double alpha, const 
   if (n <= 0) return;
   const int gb = grid_for(n);
   if (dtype == GS_F32)
-    vec_kernel<float><<<gb, 256, 0, s>>>(op, n, static_cast<const float *>(x), static_cast<float *>(y), float(alpha), static_cast<const float *>(alpha_dev));
+    launch_pass(true, vec_kernel<float>, gb, s, op, n, static_cast<const float *>(x), static_cast<float *>(y), float(alpha), static_cast<const float *>(alpha_dev));
   else
-    vec_kernel<double><<<gb, 256, 0, s>>>(op, n, static_cast<const double *>(x), static_cast<double *>(y), alpha, static_cast<const double *>(alpha_dev));
+    launch_pass(true, vec_kernel<double>, gb, s, op, n, static_cast<const double *>(x), static_cast<double *>(y), alpha, static_cast<const double *>(alpha_dev));
   check(cudaGetLastError(), "vector op");
 }
 
 void scalar_op(int op, const void *a, const void *b, void *out, double value, int dtype, cudaStream_t s) {
   if (dtype == GS_F32)
-    scalar_kernel<float><<<1, 1, 0, s>>>(op, static_cast<const float *>(a), static_cast<const float *>(b), static_cast<float *>(out), float(value));
+    launch_pass_n(true, scalar_kernel<float>, 1, 1, s, op, static_cast<const float *>(a), static_cast<const float *>(b), static_cast<float *>(out), float(value));
   else
-    scalar_kernel<double><<<1, 1, 0, s>>>(op, static_cast<const double *>(a), static_cast<const double *>(b), static_cast<double *>(out), value);
+    launch_pass_n(true, scalar_kernel<double>, 1, 1, s, op, static_cast<const double *>(a), static_cast<const double *>(b), static_cast<double *>(out), value);
   check(cudaGetLastError(), "scalar op");
 }
 

@@ -287,24 +287,29 @@ inline int sm_count(int device) {
   return v;
 }
 
-// Launches a V-cycle kernel (256 threads per block) on stream s. With
+// Launches a kernel on stream s (V-cycle kernels: 256 threads per block). With
 // `overlap` the launch carries programmatic stream serialization: its CTAs may
 // become resident while the previous kernel in the stream drains, and the
 // kernel's pass_entry holds them until that kernel's writes are visible. Under
 // stream capture this becomes a programmatic edge of the CUDA graph.
 template <typename... P, typename... A>
-void launch_pass(bool overlap, void (*kernel)(P...), int grid, cudaStream_t s, A &&...args) {
+void launch_pass_n(bool overlap, void (*kernel)(P...), int grid, int block, cudaStream_t s, A &&...args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(static_cast<unsigned>(grid));
-  cfg.blockDim = dim3(256);
+  cfg.blockDim = dim3(static_cast<unsigned>(block));
   cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cfg.attrs = overlap ? attr : nullptr;
   cfg.numAttrs = overlap ? 1 : 0;
   GSB_CK(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
+
+template <typename... P, typename... A>
+void launch_pass(bool overlap, void (*kernel)(P...), int grid, cudaStream_t s, A &&...args) {
+  launch_pass_n(overlap, kernel, grid, 256, s, std::forward<A>(args)...);
 }
 
 inline int blocks_for(long long threads, int cap) {

@@ -163,6 +163,7 @@ def lib() -> C.CDLL:
                                         C.c_void_p]
         _lib.gs_vector_op.argtypes = [C.c_int, C.c_longlong, C.c_void_p, C.c_void_p, C.c_double,
                                       C.c_void_p, C.c_int, C.c_void_p]
+        _lib.gs_spmv.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p]
         _lib.gs_mlp_adam.argtypes = [C.c_void_p, C.c_void_p, C.c_void_p, C.c_void_p, C.c_int,
                                      C.c_double, C.c_double, C.c_double, C.c_double, C.c_int,
                                      C.c_void_p]
@@ -877,56 +878,64 @@ class DeviceCsr:
             self._h = None
 
 
+# Addresses go to ctypes as plain integers (the argument types are declared):
+# a Backend call's cost is its host side, and a chain of them is as fast as the
+# binding.
 def spmv(A: DeviceCsr, x_ptr: int, y_ptr: int, stream: int = 0) -> None:
-    _check(lib().gs_spmv(A._h, C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(stream)))
+    rc = lib().gs_spmv(A._h, x_ptr, y_ptr, stream)
+    if rc:
+        _check(rc)
 
 
 def gauss_seidel_color(A: DeviceCsr, order_ptr: int, start: int, count: int, rhs_ptr: int,
                        x_ptr: int, omega: float, stream: int = 0) -> None:
-    _check(lib().gs_gauss_seidel_color(A._h, C.c_void_p(order_ptr), start, count,
-                                       C.c_void_p(rhs_ptr), C.c_void_p(x_ptr), omega,
-                                       C.c_void_p(stream)))
+    rc = lib().gs_gauss_seidel_color(A._h, order_ptr, start, count, rhs_ptr, x_ptr, omega, stream)
+    if rc:
+        _check(rc)
 
 
 def block_gauss_seidel_color3x3(A: DeviceCsr, order_ptr: int, start: int, count: int,
                                 dinv_ptr: int, rhs_ptr: int, x_ptr: int, omega: float,
                                 stream: int = 0) -> None:
-    _check(lib().gs_block_gauss_seidel_color3x3(A._h, C.c_void_p(order_ptr), start, count,
-                                                C.c_void_p(dinv_ptr), C.c_void_p(rhs_ptr),
-                                                C.c_void_p(x_ptr), omega, C.c_void_p(stream)))
+    rc = lib().gs_block_gauss_seidel_color3x3(A._h, order_ptr, start, count, dinv_ptr, rhs_ptr, x_ptr, omega, stream)
+    if rc:
+        _check(rc)
 
 
 def apply_block_inverses3x3(n: int, dinv_ptr: int, r_ptr: int, c_ptr: int, dtype: int,
                             stream: int = 0) -> None:
-    _check(lib().gs_apply_block_inverses3x3(n, C.c_void_p(dinv_ptr), C.c_void_p(r_ptr),
-                                            C.c_void_p(c_ptr), dtype, C.c_void_p(stream)))
+    rc = lib().gs_apply_block_inverses3x3(n, dinv_ptr, r_ptr, c_ptr, dtype, stream)
+    if rc:
+        _check(rc)
 
 
 def dot(n: int, x_ptr: int, y_ptr: int, result_ptr: int, dtype: int, stream: int = 0) -> None:
-    _check(lib().gs_dot(n, C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(result_ptr), dtype,
-                        C.c_void_p(stream)))
+    rc = lib().gs_dot(n, x_ptr, y_ptr, result_ptr, dtype, stream)
+    if rc:
+        _check(rc)
 
 
 def dot_noalloc(n: int, x_ptr: int, y_ptr: int, result_ptr: int, dtype: int,
                 stream: int = 0) -> None:
     """gs_dot without allocating: scratch in a fixed array of the library
     (n <= 8,388,608; calls that overlap on the GPU race on that array)."""
-    _check(lib().gs_dot_noalloc(n, C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(result_ptr),
-                                dtype, C.c_void_p(stream)))
+    rc = lib().gs_dot_noalloc(n, x_ptr, y_ptr, result_ptr, dtype, stream)
+    if rc:
+        _check(rc)
 
 
 def vector_op(op: int, n: int, x_ptr: int, y_ptr: int, alpha: float = 0.0,
               alpha_ptr: Optional[int] = None, dtype: int = F64, stream: int = 0) -> None:
-    _check(lib().gs_vector_op(op, n, C.c_void_p(x_ptr), C.c_void_p(y_ptr), alpha,
-                              None if alpha_ptr is None else C.c_void_p(alpha_ptr), dtype,
-                              C.c_void_p(stream)))
+    rc = lib().gs_vector_op(op, n, x_ptr, y_ptr, alpha, alpha_ptr, dtype, stream)
+    if rc:
+        _check(rc)
 
 
 def scalar_op(op: int, a_ptr: Optional[int], b_ptr: Optional[int], out_ptr: int,
               value: float = 0.0, dtype: int = F64, stream: int = 0) -> None:
-    _check(lib().gs_scalar_op(op, None if a_ptr is None else C.c_void_p(a_ptr),
-                              None if b_ptr is None else C.c_void_p(b_ptr), C.c_void_p(out_ptr),
-                              value, dtype, C.c_void_p(stream)))
+    rc = lib().gs_scalar_op(op, a_ptr, b_ptr, out_ptr, value, dtype, stream)
+    if rc:
+        _check(rc)
 
 
 # ---- learned relaxation weights: MLP kernels (device arrays by address) ------

@@ -175,3 +175,54 @@ def test_zero_diagonal_is_rejected(gs, torch_mod):
     v = dev([1.0, 1.0], "float64")
     with pytest.raises(gs.SolverError, match="zero diagonal"):
         gs.gauss_seidel_color(A, order.data_ptr(), 0, 2, v.data_ptr(), v.data_ptr(), 1.0)
+
+
+@pytest.mark.parametrize("dt", ["float32", "float64"])
+@pytest.mark.parametrize("rows,width", [(1, 1), (33, 7), (257, 40), (64, 95)])
+def test_colour_passes_on_ragged_rows(gs, torch_mod, dt, rows, width):
+    """Scalar and 3x3 colour passes (all rows listed at once, i.e. one Jacobi
+    pass on a copy of x) on rows of 1 to `width` entries around the trip sizes,
+    chained with vector operations on one stream, against numpy in FP64."""
+    torch = torch_mod
+    kind = gs.F32 if dt == "float32" else gs.F64
+    r = np.random.default_rng(rows)
+    # off-diagonal columns in a second half of the unknowns that no listed row owns
+    for block in (1, 3):
+        n, m = rows * block, rows * block
+        cols = max(3, width)
+        dense = np.zeros((n + cols, n + cols))
+        for i in range(rows):
+            own = slice(block * i, block * (i + 1))
+            g = r.standard_normal((block, block))
+            dense[own, own] = g @ g.T + 3.0 * np.eye(block)
+            k = r.integers(0, cols + 1)
+            dense[own, n + r.permutation(cols)[:k]] = r.standard_normal((block, k))
+        dense[n:, n:] = np.eye(cols)
+        pad = (-dense.shape[0]) % 3 if block == 3 else 0
+        full = np.eye(dense.shape[0] + pad)
+        full[:dense.shape[0], :dense.shape[0]] = dense
+        a = gs.Csr.from_scipy(sp.csr_matrix(full))
+        A = gs.DeviceCsr(a, kind)
+        x0, b = r.standard_normal(a.rows), r.standard_normal(a.rows)
+        x, rhs, y = dev(x0, dt), dev(b, dt), dev(np.zeros(a.rows), dt)
+        order = dev(np.arange(rows), "int32")
+        if block == 3:
+            dinv = dev(np.concatenate([np.linalg.inv(full[3 * i:3 * i + 3, 3 * i:3 * i + 3]).ravel()
+                                       for i in range(a.rows // 3)]), dt)
+            gs.block_gauss_seidel_color3x3(A, order.data_ptr(), 0, rows, dinv.data_ptr(), rhs.data_ptr(), x.data_ptr(), 0.8)
+        else:
+            gs.gauss_seidel_color(A, order.data_ptr(), 0, rows, rhs.data_ptr(), x.data_ptr(), 0.8)
+        gs.spmv(A, x.data_ptr(), y.data_ptr())
+        gs.vector_op(gs.VEC_AXPY, a.rows, x.data_ptr(), y.data_ptr(), alpha=-2.0, dtype=kind)
+        torch.cuda.synchronize()
+        want = x0.copy()
+        for i in range(rows):
+            own = slice(block * i, block * (i + 1))
+            res = b[own] - full[own] @ x0 + full[own, own] @ x0[own]
+            want[own] = 0.2 * x0[own] + 0.8 * np.linalg.solve(full[own, own], res)
+        # rows of `width` products in T's rounding, conditioned by the small diagonal blocks
+        eps = 1.2e-7 if dt == "float32" else 2.3e-16
+        scale = np.abs(full) @ np.abs(x0) + np.abs(b) + np.abs(x0)
+        tol = 64 * (width + 8) * eps * scale.max()
+        assert np.abs(x.double().cpu().numpy() - want).max() <= tol
+        assert np.abs(y.double().cpu().numpy() - (full @ want - 2.0 * want)).max() <= 64 * tol
