@@ -1164,10 +1164,14 @@ __global__ void __launch_bounds__(256, 2) cg_bell_spmv_pap_kernel(BellView<doubl
   }
 }
 
-// What the host polls: 2 * (iterations whose convergence test has run) + stop
-// flag, in pinned memory.
+// What the host polls in pinned memory. Word 0: 2 * (iterations whose
+// convergence test has run) + stop flag, the status (CgStatus) in the top four
+// bits once stopped. Word 1: the start's outcome, before any of that.
+enum CgStartCode : unsigned { kStartRuns = 1, kStartZeroRhs = 2 };
+
 __device__ __forceinline__ void publish_state(const CgState *st, volatile unsigned *host) {
-  *host = 2u * static_cast<unsigned>(st->iter) + (st->done != 0 ? 1u : 0u);
+  const unsigned n = 2u * (static_cast<unsigned>(st->iter) & 0x03ffffffu);
+  host[0] = st->done != 0 ? n | 1u | static_cast<unsigned>(st->status) << 28 : n;
 }
 
 // x += alpha p; r -= alpha Ap; rr = r . r; convergence test on rr / bb, its
@@ -1276,14 +1280,17 @@ __global__ void __launch_bounds__(256) cg_update_p_kernel(int n, const ZT *__res
   }
 }
 
-// Start of the solve: p = z; bb = b.b, rho = r.z, rr = r.r.
+// Start of the solve: p = z; bb = b.b, rho = r.z, rr = r.r; the solver state,
+// cleared before, gets the solve's parameters.
 template <typename ZT>
 __global__ void __launch_bounds__(256) cg_init_kernel(int n, const double *__restrict__ b,
                                                       const double *__restrict__ r,
-                                                      const ZT *__restrict__ z,
+                                                      const ZT *z,
                                                       double *__restrict__ p, CgState *st,
-                                                      double *partials) {
+                                                      double *partials, double tol2, int max_iter, int flexible,
+                                                      volatile unsigned *host) {
   __shared__ double smem[96];
+  pass_entry(nullptr);
   double acc[3] = {0.0, 0.0, 0.0};
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
@@ -1298,6 +1305,9 @@ __global__ void __launch_bounds__(256) cg_init_kernel(int n, const double *__res
     st->rho = acc[1];
     st->rr = acc[2];
     st->ratio = acc[2] / acc[0];
+    st->tol2 = tol2;
+    st->max_iter = max_iter;
+    st->flexible = flexible;
     st->iter = 0;
     st->done = 0;
     st->status = kCgRunning;
@@ -1309,6 +1319,8 @@ __global__ void __launch_bounds__(256) cg_init_kernel(int n, const double *__res
       st->status = kCgInitialConverged;
       st->done = 1;
     }
+    // a zero right-hand side: whatever else is found, the host returns x = 0
+    host[1] = finite_d(acc[0]) && !(sqrt(acc[0]) >= 1e-12) ? kStartZeroRhs : kStartRuns;
   }
 }
 

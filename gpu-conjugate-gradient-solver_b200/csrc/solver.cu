@@ -591,7 +591,7 @@ class AmgPcg final : public Solver {
   void cg_iteration(int parity, cudaStream_t s);
   void cg_start(cudaStream_t s);
   void ensure_graphs();
-  void run(cudaStream_t user, SolveStats *st);
+  void run(double *x, SolveStats *st);
 
   SolverOptions opt_;
   int device_ = 0, sms_ = 148, cap_blocks_ = 148 * 8;
@@ -630,7 +630,7 @@ class AmgPcg final : public Solver {
   CgState *st_ = nullptr, *scratch_st_ = nullptr;
   double *partials_ = nullptr;
   CgState *host_st_ = nullptr;                  // pinned
-  volatile unsigned *host_seq_ = nullptr;       // pinned, written by the convergence test (publish_state)
+  volatile unsigned *host_seq_ = nullptr;       // pinned, two words written by the kernels (publish_state)
   bool wait_published(int it);
   SweepSync *sync_ = nullptr;                   // grid-barrier state of the cooperative sweeps
   VT *wbuf_ = nullptr;
@@ -2311,16 +2311,12 @@ void AmgPcg<VT>::cg_iteration(int parity, cudaStream_t s) {
 // r = b - A x; z = M r; p = z; bb, rho, rr.
 template <typename VT>
 void AmgPcg<VT>::cg_start(cudaStream_t s) {
-  CgState init{};
-  init.tol2 = opt_.tol * opt_.tol;
-  init.max_iter = opt_.max_iter;
-  init.flexible = opt_.flexible;
-  // pageable source: staged by the runtime before the call returns
-  CK(cudaMemcpyAsync(st_, &init, sizeof(CgState), cudaMemcpyHostToDevice, s));
+  CK(cudaMemsetAsync(st_, 0, sizeof(CgState), s));
   outer_resid(s);
   CKL("initial residual");
   precondition(r_, z_[0], s);
-  cg_init_kernel<VT><<<blocks_for(n0_, cap_blocks_), 256, 0, s>>>(n0_, b_, r_, z_[0], p_, st_, partials_);
+  launch_pass(pdl_, cg_init_kernel<VT>, blocks_for(n0_, cap_blocks_), s, n0_, b_, r_, z_[0], p_, st_, partials_,
+              opt_.tol * opt_.tol, opt_.max_iter, opt_.flexible ? 1 : 0, host_seq_);
   CKL("cg init");
 }
 
@@ -2345,62 +2341,61 @@ void AmgPcg<VT>::ensure_graphs() {
 // stopped there (or before, on a breakdown or a fault).
 template <typename VT>
 bool AmgPcg<VT>::wait_published(int it) {
+  const unsigned want = 2u * static_cast<unsigned>(it + 1);
   for (unsigned spins = 0;; ++spins) {
-    const unsigned v = *host_seq_;
+    const unsigned v = host_seq_[0];
     if (v & 1u) return true;
-    if (v >= 2u * static_cast<unsigned>(it + 1)) return false;
+    if (v >= want) return false;
     if ((spins & 1023u) == 1023u) {
       // an idle stream that published nothing: the solve was stopped elsewhere
       const cudaError_t e = cudaStreamQuery(stream_);
-      if (e == cudaSuccess) return *host_seq_ < 2u * static_cast<unsigned>(it + 1) || (*host_seq_ & 1u) != 0;
+      if (e == cudaSuccess) return host_seq_[0] < want || (host_seq_[0] & 1u) != 0;
       if (e != cudaErrorNotReady) CK(e);
     }
   }
 }
 
+// Queues the whole solve on the solver's stream and, where it has an answer,
+// the answer's way back to the caller's order; returns when it has finished.
 template <typename VT>
-void AmgPcg<VT>::run(cudaStream_t user, SolveStats *out) {
-  // Order after the caller's stream, work on the solver's own stream.
-  CK(cudaEventRecord(ev_[0], user));
-  CK(cudaStreamWaitEvent(stream_, ev_[0], 0));
+void AmgPcg<VT>::run(double *x, SolveStats *out) {
+  host_seq_[0] = host_seq_[1] = 0u;  // the stream is idle
   CK(cudaEventRecord(ev_[2], stream_));
   cg_start(stream_);
+  // One iteration at a time, as CGSolver::solve; its convergence test runs
+  // before its V-cycle and tells the host through pinned memory, so the next
+  // iteration is queued while the V-cycle runs (and the V-cycle of the last one
+  // returns at once: its kernels see the stop flag). The first iteration is
+  // queued without waiting for the start; if there was nothing to do, its
+  // kernels return at once as well.
+  if (opt_.graph) ensure_graphs();
+  for (int it = 0; it < opt_.max_iter; ++it) {
+    if (opt_.graph) {
+      CK(cudaGraphLaunch(exec_[it & 1], stream_));
+      launches_ += graph_kernels_;
+    } else {
+      cg_iteration(it & 1, stream_);
+    }
+    if (wait_published(it) || host_seq_[1] == kStartZeroRhs) break;
+  }
   CK(cudaMemcpyAsync(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
+  unsigned status = host_seq_[0] >> 28;
+  if (opt_.max_iter == 0) {  // nothing was published but the start
+    CK(cudaStreamSynchronize(stream_));
+    status = host_st_[0].status == kCgNotFinite ? kCgNotFinite : kCgMaxIter;
+  }
+  const bool zero_rhs = host_seq_[1] == kStartZeroRhs;
+  // no answer: NaN/Inf, or a fault (stopped without a status)
+  const bool answer = zero_rhs || (status != kCgNotFinite && status != kCgRunning);
+  if (zero_rhs) CK(cudaMemsetAsync(x_, 0, sizeof(double) * n0_, stream_));  // CGSolver::solve: x = 0
+  CK(cudaEventRecord(ev_[3], stream_));
+  if (answer) {
+    gather_kernel<double, double><<<blocks_for(n0_, cap_blocks_), 256, 0, stream_>>>(n0_, q0_, x_, x);
+    CKL("permute out");
+  }
   CK(cudaStreamSynchronize(stream_));
   CgState hs = host_st_[0];
-  int spmv = 0;
-  if (!(std::sqrt(hs.bb) >= 1e-12)) {
-    // CGSolver::solve: a zero right-hand side returns x = 0.
-    if (std::isfinite(hs.bb)) {
-      CK(cudaMemsetAsync(x_, 0, sizeof(double) * n0_, stream_));
-      hs.status = kCgZeroRhs;
-      hs.iterations = 0;
-    }
-  } else if (!hs.done) {
-    // One iteration at a time, as CGSolver::solve; its convergence test runs
-    // before its V-cycle and tells the host through pinned memory, so the next
-    // iteration is queued while the V-cycle runs (and the V-cycle of the last
-    // one returns at once: its kernels see the stop flag).
-    if (opt_.graph) ensure_graphs();
-    *host_seq_ = 0u;
-    for (int it = 0; it < opt_.max_iter; ++it) {
-      if (opt_.graph) {
-        CK(cudaGraphLaunch(exec_[it & 1], stream_));
-        launches_ += graph_kernels_;
-      } else {
-        cg_iteration(it & 1, stream_);
-      }
-      if (wait_published(it)) break;
-    }
-    CK(cudaMemcpyAsync(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost, stream_));
-    CK(cudaStreamSynchronize(stream_));
-    hs = host_st_[0];
-    spmv = hs.iter;
-  }
-  CK(cudaEventRecord(ev_[3], stream_));
-  CK(cudaEventRecord(ev_[1], stream_));
-  CK(cudaStreamWaitEvent(user, ev_[1], 0));
-  CK(cudaEventSynchronize(ev_[3]));
+  if (zero_rhs) hs.status = kCgZeroRhs, hs.iterations = 0, hs.iter = 0;
   float ms = 0.f;
   CK(cudaEventElapsedTime(&ms, ev_[2], ev_[3]));
   check_sync_fault(hs);
@@ -2409,7 +2404,7 @@ void AmgPcg<VT>::run(cudaStream_t user, SolveStats *out) {
     out->status = hs.status;
     out->ratio = hs.ratio;
     out->bb = hs.bb;
-    out->spmv = spmv;
+    out->spmv = hs.iter;
     out->solve_ms = ms;
   }
   if (hs.status == kCgNotFinite)
@@ -2419,6 +2414,7 @@ void AmgPcg<VT>::run(cudaStream_t user, SolveStats *out) {
 template <typename VT>
 void AmgPcg<VT>::solve_device(const double *b, double *x, cudaStream_t stream, SolveStats *st) {
   CK(cudaSetDevice(device_));
+  // ordered after the caller's stream, on the solver's own
   CK(cudaEventRecord(ev_[0], stream));
   CK(cudaStreamWaitEvent(stream_, ev_[0], 0));
   const int blocks = blocks_for(n0_, cap_blocks_);
@@ -2426,16 +2422,7 @@ void AmgPcg<VT>::solve_device(const double *b, double *x, cudaStream_t stream, S
   scatter_kernel<double, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, x, x_);
   CKL("permute in");
   ++launches_;
-  CK(cudaEventRecord(ev_[1], stream_));
-  CK(cudaStreamWaitEvent(stream, ev_[1], 0));
-  run(stream, st);
-  CK(cudaEventRecord(ev_[0], stream));
-  CK(cudaStreamWaitEvent(stream_, ev_[0], 0));
-  gather_kernel<double, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, x_, x);
-  CKL("permute out");
-  CK(cudaEventRecord(ev_[1], stream_));
-  CK(cudaStreamWaitEvent(stream, ev_[1], 0));
-  CK(cudaStreamSynchronize(stream));
+  run(x, st);
 }
 
 template <typename VT>
