@@ -347,7 +347,8 @@ class Batch final : public BatchSolver {
   void cg_start(cudaStream_t s);
   void cg_iteration(int parity, cudaStream_t s);
   void ensure_graphs();
-  void run(std::vector<SolveStats> &st);
+  bool wait_published(int it);
+  void run(double *x, std::vector<SolveStats> &st);
   void build_items();
   std::vector<std::unique_ptr<Arena>> kept_;  // cluster layouts in use
   void autotune();
@@ -383,7 +384,9 @@ class Batch final : public BatchSolver {
   double *partials_ = nullptr;
   BPair *pairs_ = nullptr;
   int *sys_done_ = nullptr;
-  BCgShared *sh_ = nullptr, *host_sh_ = nullptr;
+  BCgShared *sh_ = nullptr, *host_sh_ = nullptr;  // host, pinned: the state read back, the state of the start
+  BPair *host_pairs_ = nullptr;                   // pinned
+  volatile unsigned *host_seq_ = nullptr;         // pinned, two words written by the convergence test
   double *ub_ = nullptr, *ux_ = nullptr;  // caller-layout staging of host solves
   // caller layout
   long long *uoff_ = nullptr, *qoff_ = nullptr;
@@ -523,8 +526,11 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
   sys_done_ = ar_.alloc<int>(S_);
   BCK(cudaMemset(sys_done_, 0, sizeof(int) * S_));
   sh_ = ar_.alloc<BCgShared>(1);
-  BCK(cudaMallocHost(&host_sh_, 2 * sizeof(BCgShared)));
-  std::memset(host_sh_, 0, 2 * sizeof(BCgShared));
+  const size_t host_bytes = sizeof(BPair) * S_ * R + 2 * sizeof(BCgShared) + 2 * sizeof(unsigned);
+  BCK(cudaMallocHost(&host_pairs_, host_bytes));
+  std::memset(host_pairs_, 0, host_bytes);
+  host_sh_ = reinterpret_cast<BCgShared *>(host_pairs_ + static_cast<size_t>(S_) * R);
+  host_seq_ = reinterpret_cast<volatile unsigned *>(host_sh_ + 2);
   ub_ = ar_.alloc<double>(static_cast<size_t>(unknowns_) * nrhs_);
   ux_ = ar_.alloc<double>(static_cast<size_t>(unknowns_) * nrhs_);
 
@@ -602,7 +608,7 @@ Batch<VT, R>::~Batch() {
   }
   if (items_) cudaFree(items_);
   if (tmp_) cudaFree(tmp_);
-  if (host_sh_) cudaFreeHost(host_sh_);
+  if (host_pairs_) cudaFreeHost(host_pairs_);
   for (auto &e : ev_)
     if (e) cudaEventDestroy(e);
   if (stream_) cudaStreamDestroy(stream_);
@@ -975,17 +981,17 @@ void Batch<VT, R>::cg_iteration(int parity, cudaStream_t s) {
   const int nc = cg_range_.count, gb = grid(nc);
   launch_pass(pdl_, bcg_spmv_pap_kernel<R>, gb, s, cgA_.view(), ci, nc, p_, ap_, sys_done_, partials_);
   BKL("batched cg spmv");
-  bcg_finalize_kernel<R, kBFinPap><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
+  launch_pass_n(pdl_, bcg_finalize_kernel<R, kBFinPap>, S_, 32 * R, s, cg_first_, partials_, pairs_, sys_done_, sh_, host_seq_);
   BKL("batched cg alpha");
   launch_pass(pdl_, bcg_update_xr_kernel<R>, gb, s, cgA_.srow, ci, nc, x_, r_, p_, ap_, pairs_, sys_done_, partials_);
   BKL("batched cg update");
-  bcg_finalize_kernel<R, kBFinXr><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
+  launch_pass_n(pdl_, bcg_finalize_kernel<R, kBFinXr>, S_, 32 * R, s, cg_first_, partials_, pairs_, sys_done_, sh_, host_seq_);
   BKL("batched cg convergence");
   precondition(r_, z_new, s);
   launch_pass(pdl_, bcg_dot_rz_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, r_, z_new, opt_.flexible ? z_old : nullptr,
                                               sys_done_, partials_);
   BKL("batched cg dot");
-  bcg_finalize_kernel<R, kBFinRz><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
+  launch_pass_n(pdl_, bcg_finalize_kernel<R, kBFinRz>, S_, 32 * R, s, cg_first_, partials_, pairs_, sys_done_, sh_, host_seq_);
   BKL("batched cg beta");
   launch_pass(pdl_, bcg_update_p_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, z_new, p_, pairs_, sys_done_);
   BKL("batched cg p update");
@@ -994,22 +1000,21 @@ void Batch<VT, R>::cg_iteration(int parity, cudaStream_t s) {
 // r = b - A x; z = M r; p = z; bb, rho, rr per pair.
 template <typename VT, int R>
 void Batch<VT, R>::cg_start(cudaStream_t s) {
-  BCgShared init{};
+  BCgShared &init = host_sh_[1];  // pinned, and not written again before this solve has ended
+  init = BCgShared{};
   init.tol2 = opt_.tol * opt_.tol;
   init.max_iter = opt_.max_iter;
   init.flexible = opt_.flexible;
-  init.active = 0;
-  // pageable source: staged by the runtime before the call returns
   BCK(cudaMemcpyAsync(sh_, &init, sizeof(BCgShared), cudaMemcpyHostToDevice, s));
   BCK(cudaMemsetAsync(sys_done_, 0, sizeof(int) * S_, s));
   const BItem *ci = items_ + cg_range_.off;
   const int nc = cg_range_.count, gb = grid(nc);
-  bsell_spmv_kernel<double, double, R, kSpmvResid><<<gb, 256, 0, s>>>(cgA_.view(), ci, nc, x_, r_, b_, nullptr);
+  launch_pass(pdl_, bsell_spmv_kernel<double, double, R, kSpmvResid>, gb, s, cgA_.view(), ci, nc, x_, r_, b_, nullptr);
   BKL("batched initial residual");
   precondition(r_, z_[0], s);
-  bcg_init_kernel<VT, R><<<gb, 256, 0, s>>>(cgA_.srow, ci, nc, b_, r_, z_[0], p_, partials_);
+  launch_pass(pdl_, bcg_init_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, b_, r_, z_[0], p_, partials_);
   BKL("batched cg init");
-  bcg_finalize_kernel<R, kBFinInit><<<S_, 32 * R, 0, s>>>(cg_first_, partials_, pairs_, sys_done_, sh_);
+  launch_pass_n(pdl_, bcg_finalize_kernel<R, kBFinInit>, S_, 32 * R, s, cg_first_, partials_, pairs_, sys_done_, sh_, host_seq_);
   BKL("batched cg init scalars");
 }
 
@@ -1030,48 +1035,62 @@ void Batch<VT, R>::ensure_graphs() {
   }
 }
 
+// Waits until iteration `it`'s convergence test has run; whether the solve ends
+// with it.
 template <typename VT, int R>
-void Batch<VT, R>::run(std::vector<SolveStats> &out) {
+bool Batch<VT, R>::wait_published(int it) {
+  const unsigned want = 2u * static_cast<unsigned>(it + 1);
+  for (unsigned spins = 0;; ++spins) {
+    const unsigned v = host_seq_[0];
+    if ((v & 1u) != 0) return true;
+    if (v >= want) return false;
+    if ((spins & 1023u) == 1023u) {
+      const cudaError_t e = cudaStreamQuery(stream_);
+      if (e == cudaSuccess) return host_seq_[0] < want || (host_seq_[0] & 1u) != 0;
+      if (e != cudaErrorNotReady) BCK(e);
+    }
+  }
+}
+
+// Queues the whole solve on the batch's stream and, unless a wait gave up, the
+// way of x back to the caller's order; returns when it has finished. The first
+// iteration is queued without waiting for the start: if every system was done
+// there, its kernels skip all their items.
+template <typename VT, int R>
+void Batch<VT, R>::run(double *x, std::vector<SolveStats> &out) {
+  host_seq_[0] = host_seq_[1] = 0u;  // the stream is idle
   BCK(cudaEventRecord(ev_[2], stream_));
   cg_start(stream_);
-  BCK(cudaMemcpyAsync(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost, stream_));
-  BCK(cudaStreamSynchronize(stream_));
-  if (host_sh_[0].active > 0) {
+  if (opt_.graph) ensure_graphs();
+  for (int it = 0; it < opt_.max_iter; ++it) {
     if (opt_.graph) {
-      ensure_graphs();
-      // One iteration queued ahead of the host check; the kernels of an
-      // iteration queued after every system finished skip all their items.
-      for (int it = 0; it < opt_.max_iter; ++it) {
-        BCK(cudaGraphLaunch(exec_[it & 1], stream_));
-        launches_ += graph_kernels_;
-        BCK(cudaMemcpyAsync(&host_sh_[it & 1], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost, stream_));
-        BCK(cudaEventRecord(ev_[it & 1], stream_));
-        if (it >= 1) {
-          BCK(cudaEventSynchronize(ev_[(it - 1) & 1]));
-          if (host_sh_[(it - 1) & 1].active == 0) break;
-        }
-      }
+      BCK(cudaGraphLaunch(exec_[it & 1], stream_));
+      launches_ += graph_kernels_;
     } else {
-      for (int it = 0; it < opt_.max_iter; ++it) {
-        cg_iteration(it & 1, stream_);
-        BCK(cudaMemcpyAsync(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost, stream_));
-        BCK(cudaStreamSynchronize(stream_));
-        if (host_sh_[0].active == 0) break;
-      }
+      cg_iteration(it & 1, stream_);
     }
+    if (wait_published(it)) break;
   }
   BCK(cudaEventRecord(ev_[3], stream_));
   BCK(cudaMemcpyAsync(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost, stream_));
+  BCK(cudaMemcpyAsync(host_pairs_, pairs_, sizeof(BPair) * S_ * R, cudaMemcpyDeviceToHost, stream_));
+  if (opt_.max_iter == 0) {  // nothing was published
+    BCK(cudaStreamSynchronize(stream_));
+    check_fault();
+  }
+  if (host_seq_[1] == 0u) {
+    const dim3 g(std::max(1, std::min(256, (maxn_ + 255) / 256)), S_);
+    bgather_kernel<R><<<g, 256, 0, stream_>>>(uoff_, n_dev_, off0_, qoff_, q0_, nrhs_, x_, pairs_, x);
+    BKL("batched permute out");
+  }
   BCK(cudaStreamSynchronize(stream_));
   float ms = 0.f;
   BCK(cudaEventElapsedTime(&ms, ev_[2], ev_[3]));
   check_fault();
-  std::vector<BPair> hp(static_cast<size_t>(S_) * R);
-  BCK(cudaMemcpy(hp.data(), pairs_, sizeof(BPair) * hp.size(), cudaMemcpyDeviceToHost));
   out.assign(static_cast<size_t>(S_) * nrhs_, SolveStats{});
   for (int s = 0; s < S_; ++s)
     for (int j = 0; j < nrhs_; ++j) {
-      const BPair &p = hp[static_cast<size_t>(s) * R + j];
+      const BPair &p = host_pairs_[static_cast<size_t>(s) * R + j];
       SolveStats &o = out[static_cast<size_t>(s) * nrhs_ + j];
       o.iterations = p.iterations;
       o.status = p.status;
@@ -1092,12 +1111,7 @@ void Batch<VT, R>::solve_device(const double *b, double *x, cudaStream_t stream,
   bscatter_kernel<R><<<g, 256, 0, stream_>>>(uoff_, n_dev_, off0_, qoff_, q0_, nrhs_, x, x_);
   BKL("batched permute in");
   ++launches_;
-  run(st);
-  bgather_kernel<R><<<g, 256, 0, stream_>>>(uoff_, n_dev_, off0_, qoff_, q0_, nrhs_, x_, pairs_, x);
-  BKL("batched permute out");
-  BCK(cudaEventRecord(ev_[1], stream_));
-  BCK(cudaStreamWaitEvent(stream, ev_[1], 0));
-  BCK(cudaStreamSynchronize(stream));
+  run(x, st);
 }
 
 template <typename VT, int R>

@@ -2,6 +2,8 @@
 stops after a given number of iterations, a zero right-hand side, a start that
 has converged already, and values that are not finite, through the host and
 the device entry points."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -58,3 +60,43 @@ def test_device_solves_that_end_at_the_start(gs, device, prob, graph):
         x.zero_()
         st = s.solve_device(bd.data_ptr(), x.data_ptr(), stream.cuda_stream)
         assert st.status == gs.STATUS_CONVERGED and np.array_equal(x.cpu().numpy(), own)
+
+
+@pytest.mark.parametrize("overlap", [0, 1, 2])
+@pytest.mark.parametrize("graph", [0, 1])
+def test_batch_ends(gs, orc, device, graph, overlap):
+    mats = [gs.varcoef_loguniform(x, y, z, seed=7 + i) for i, (x, y, z) in enumerate([(9, 5, 7), (13, 13, 13), (5, 7, 11)])]
+    hs = [gs.Hierarchy.build(m, 1, 0.1, 10, 60) for m in mats]
+    n = [m.rows for m in mats]
+    at = np.concatenate([[0], np.cumsum(n)])
+
+    def batch(**kw):
+        return gs.Batch(hs, 1, gs.SolverOptions(use_graph=graph, overlap_launch=overlap, **kw), device=device)
+
+    b = np.concatenate([gs.uniform_rhs(m, i) for i, m in enumerate(n)])
+    for max_iter in (1, 2, 5):
+        x, st = batch(tol=1e-14, max_iter=max_iter).solve(b)
+        for i, H in enumerate(hs):
+            L = H.levels
+            xo, _, _, _ = orc.amg_pcg([H.A(k) for k in range(L)], [H.P(k) for k in range(L - 1)],
+                                      [H.R(k) for k in range(L - 1)], b[at[i]:at[i + 1]], tol=1e-14, max_iter=max_iter)
+            assert st[i].status == gs.STATUS_MAX_ITER and st[i].iterations == max_iter
+            # FP64, the same operations up to the order of a row's sum
+            assert np.linalg.norm(x[at[i]:at[i + 1]] - xo) <= 1e-11 * np.linalg.norm(xo)
+    B = batch(tol=1e-8, max_iter=200)
+    own, st = B.solve(b)
+    assert all(s.status == gs.STATUS_CONVERGED for s in st)
+    # every system done at the start, then one of three, then none
+    x, st = B.solve(np.zeros_like(b), np.ones_like(b))
+    assert all(s.status == gs.STATUS_ZERO_RHS for s in st) and not x.any()
+    part = b.copy()
+    part[at[1]:at[2]] = 0.0
+    x, st = B.solve(part, np.zeros_like(b))
+    assert [s.status for s in st] == [gs.STATUS_CONVERGED, gs.STATUS_ZERO_RHS, gs.STATUS_CONVERGED]
+    assert not x[at[1]:at[2]].any() and np.array_equal(x[:at[1]], own[:at[1]]) and np.array_equal(x[at[2]:], own[at[2]:])
+    x, st = B.solve(b)
+    assert np.array_equal(x, own)
+    x0 = np.linspace(-1.0, 1.0, b.size)
+    assert gs.lib().gs_batch_set_tolerance(B._b, ctypes.c_double(1e-8), 0) == 0
+    x, st = B.solve(b, x0)
+    assert np.array_equal(x, x0) and all(s.iterations == 0 for s in st)
