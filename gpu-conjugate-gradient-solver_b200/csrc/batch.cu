@@ -148,10 +148,27 @@ struct Layout {
   std::vector<int> maxc;                               // [k] colour passes per sweep
   std::vector<std::vector<std::vector<Seg>>> fwd, bwd; // [k][pass]
   std::vector<std::vector<Seg>> whole;                 // [k] smoothed systems, all their rows
+  std::vector<std::vector<Seg>> rest;                  // [k] the same without colour 0 (where there is another)
   std::vector<std::vector<Seg>> below;                 // [k] systems on level k + 1, their rows there
   std::vector<std::vector<int>> bounds;                // [k] system and colour boundaries
   std::vector<std::vector<int>> sys_bounds;            // [k] system boundaries
 };
+
+// First row of a level's colours past the first; 0 if it has no other.
+int first_rest(const SysLevel &lv) { return lv.cf.size() > 2 ? lv.cf[1] : 0; }
+
+// `a` without its columns below c0.
+Csr drop_columns(const Csr &a, int c0) {
+  Csr m;
+  m.rows = a.rows, m.cols = a.cols;
+  m.rp.assign(a.rows + 1, 0);
+  for (int r = 0; r < a.rows; ++r) {
+    for (int e = a.rp[r]; e < a.rp[r + 1]; ++e)
+      if (a.ci[e] >= c0) m.ci.push_back(a.ci[e]), m.v.push_back(a.v[e]);
+    m.rp[r + 1] = static_cast<int>(m.ci.size());
+  }
+  return m;
+}
 
 Layout make_layout(const std::vector<SysPrep> &sp) {
   Layout ly;
@@ -167,6 +184,7 @@ Layout make_layout(const std::vector<SysPrep> &sp) {
   ly.fwd.resize(K);
   ly.bwd.resize(K);
   ly.whole.resize(K);
+  ly.rest.resize(K);
   ly.below.resize(K);
   ly.bounds.resize(K);
   ly.sys_bounds.resize(K);
@@ -193,6 +211,8 @@ Layout make_layout(const std::vector<SysPrep> &sp) {
       if (ly.L[s] - 1 > k) {  // smoothed on this level
         ly.maxc[k] = std::max(ly.maxc[k], C);
         ly.whole[k].push_back(Seg{s, o, o + lv.A.rows, o});
+        const int r0 = o + first_rest(lv);
+        ly.rest[k].push_back(Seg{s, r0, o + lv.A.rows, r0});
       }
     }
     std::sort(bd.begin(), bd.end());
@@ -302,7 +322,7 @@ class Batch final : public BatchSolver {
     const ClusterView<VT> *views = nullptr;
     const int *csys = nullptr;
     std::vector<Range> fwd, bwd;
-    Range whole_a, whole_p, below_r;
+    Range resid_a, corr_p, below_r;
   };
 
  public:
@@ -354,7 +374,17 @@ class Batch final : public BatchSolver {
   void autotune();
   float time_ms(const std::function<void()> &f, int reps);
 
+  // Rows of level k that the residual and the prolongation visit. With omega 1
+  // a step leaves no residual on colour 0, which its backward sweep solves
+  // last, and the step after the prolongation overwrites colour 0 first: both
+  // leave its rows out, and R has no columns there. Half of a two-colour level
+  // drops out of all three (one B200, 12 systems of 16^3 to 56^3, 4 FP32
+  // right-hand sides, level 0: residual 17.3 -> 8.3 us, restriction
+  // 17.3 -> 9.4, prolongation 15.3 -> 8.5; with the heads loaded before the wait).
+  const std::vector<Seg> &parts(int k) const { return exact_ ? ly_.rest[k] : ly_.whole[k]; }
+
   SolverOptions opt_;
+  bool exact_ = false;  // omega 1: a colour pass solves its rows whatever they held
   int device_ = 0, sms_ = 148, cap_blocks_ = 148 * 8;
   int S_ = 0, nrhs_ = 1, K_ = 0, n0_ = 0, maxn_ = 0;
   long long unknowns_ = 0;
@@ -417,6 +447,7 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
       opt.lanes != 32)
     throw std::runtime_error("lanes must be 1, 2, 4, 8, 16 or 32");
   pdl_ = opt.overlap_launch >= 1;
+  exact_ = VT(opt.omega) == VT(1);
   S_ = static_cast<int>(h.size());
   nrhs_ = nrhs;
   BCK(cudaSetDevice(device_));
@@ -458,15 +489,18 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
     info_[k].max_colors = ly_.maxc[k];
     if (k + 1 < K_) {
       std::vector<const Csr *> pp, rr;
+      std::vector<Csr> cut;
+      cut.reserve(S_);
       std::vector<int> ro, co, rro, rco;
       for (int s = 0; s < S_; ++s) {
         if (ly_.L[s] - 1 <= k) continue;
         pp.push_back(&sp[s].lv[k].P), ro.push_back(ly_.off[k][s]), co.push_back(ly_.off[k + 1][s]);
-        rr.push_back(&sp[s].lv[k].R), rro.push_back(ly_.off[k + 1][s]), rco.push_back(ly_.off[k][s]);
+        if (exact_) cut.push_back(drop_columns(sp[s].lv[k].R, first_rest(sp[s].lv[k])));
+        rr.push_back(exact_ ? &cut.back() : &sp[s].lv[k].R), rro.push_back(ly_.off[k + 1][s]), rco.push_back(ly_.off[k][s]);
       }
       const Csr P = block_diag(pp, ro, co, L.n, ly_.rows[k + 1]);
       const Csr Rm = block_diag(rr, rro, rco, ly_.rows[k + 1], L.n);
-      L.P = upload_sell(ar_, make_sell<VT>(P, ly_.sys_bounds[k], false));
+      L.P = upload_sell(ar_, make_sell<VT>(P, ly_.bounds[k], false));
       L.Rs = upload_sell(ar_, make_sell<VT>(Rm, ly_.sys_bounds[k + 1], false));
       L.Pc = upload_csrv<VT>(ar_, P, false);
       L.Rc = upload_csrv<VT>(ar_, Rm, false);
@@ -553,14 +587,23 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
     n_dev_ = ar_.upload(n_host_);
   }
 
-  // CG work list: level-0 slices of one system, kCgItemSlices per item
+  // CG work list: level-0 slices of one system, as many per item (a multiple
+  // of the block's warps) as let the product's blocks fill the device once. One
+  // B200, the product: 5 systems of 14^3 to 30^3 with 8 slices an item instead
+  // of 32, 8.3 -> 6.3 us; 12 systems of 16^3 to 56^3, 4 right-hand sides, keep
+  // 32 (25.7 us; 24 start a second wave, 32.1).
   {
     std::vector<int> first(S_ + 1, 0);
     std::vector<BItem> cgi;
+    const int slices = static_cast<int>(cgA_.h_srow.size()) - 1;
+    int resident = 1;
+    BCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, bcg_spmv_pap_kernel<R>, 256, 0));
+    const int wave = std::max(1, resident) * sms_, each = (slices + wave - 1) / wave;
+    const int per = std::min(kCgItemSlices, std::max(1, (each + kSellItemSlices - 1) / kSellItemSlices) * kSellItemSlices);
     for (int s = 0; s < S_; ++s) {
       first[s] = static_cast<int>(cgi.size());
       const int o = ly_.off[0][s];
-      sell_items({Seg{s, o, o + n_host_[s], o}}, cgA_.h_srow, kCgItemSlices, cgi);
+      sell_items({Seg{s, o, o + n_host_[s], o}}, cgA_.h_srow, per, cgi);
     }
     first[S_] = static_cast<int>(cgi.size());
     cg_first_ = ar_.upload(first);
@@ -633,9 +676,9 @@ void Batch<VT, R>::build_items() {
       L.fwd.push_back(add(ly_.fwd[k][j], L.g, L.A.h_srow));
       L.bwd.push_back(add(ly_.bwd[k][j], L.g, L.A.h_srow));
     }
-    L.whole_a = add(ly_.whole[k], L.g, L.A.h_srow);
+    L.resid_a = add(parts(k), L.g, L.A.h_srow);
     if (k + 1 < K_) {
-      L.whole_p = add(ly_.whole[k], L.pg, L.P.h_srow);
+      L.corr_p = add(parts(k), L.pg, L.P.h_srow);
       L.below_r = add(ly_.below[k], L.rg, L.Rs.h_srow);
     }
   }
@@ -718,7 +761,7 @@ void Batch<VT, R>::smooth(int k, const Rv<BT, R> *b, RV *x, int steps, bool zero
       return;
     }
   }
-  const bool skip = VT(opt_.omega) == VT(1);
+  const bool skip = exact_;
   for (int step = 0; step < steps; ++step) {
     for (size_t j = skip && step > 0 ? 1 : 0; j < L.fwd.size(); ++j)
       gs_pass<BT>(L, items_ + L.fwd[j].off, L.fwd[j].count, b, x, zero && step == 0, s);
@@ -823,10 +866,10 @@ void Batch<VT, R>::vcycle(const RD *r0, RV *z, bool zero0, cudaStream_t s) {
     BLevel &L = lv_[k];
     if (k == 0) {
       smooth<double>(0, r0, z, opt_.pre, zero0, s);
-      spmv<kSpmvResid, double>(L.A, L.C, L.g, items_ + L.whole_a.off, L.whole_a.count, z, L.r, r0, s);
+      spmv<kSpmvResid, double>(L.A, L.C, L.g, items_ + L.resid_a.off, L.resid_a.count, z, L.r, r0, s);
     } else {
       smooth<VT>(k, L.b, L.x, opt_.pre, true, s);
-      spmv<kSpmvResid, VT>(L.A, L.C, L.g, items_ + L.whole_a.off, L.whole_a.count, L.x, L.r, L.b, s);
+      spmv<kSpmvResid, VT>(L.A, L.C, L.g, items_ + L.resid_a.off, L.resid_a.count, L.x, L.r, L.b, s);
     }
     spmv<kSpmvSet, VT>(L.Rs, L.Rc, L.rg, items_ + L.below_r.off, L.below_r.count, L.r, lv_[k + 1].b,
                        static_cast<const RV *>(nullptr), s);
@@ -838,7 +881,7 @@ void Batch<VT, R>::vcycle(const RD *r0, RV *z, bool zero0, cudaStream_t s) {
   for (int k = K_ - 2; k >= 0; --k) {
     BLevel &L = lv_[k];
     RV *x = k == 0 ? z : L.x;
-    spmv<kSpmvAdd, VT>(L.P, L.Pc, L.pg, items_ + L.whole_p.off, L.whole_p.count, lv_[k + 1].x, x,
+    spmv<kSpmvAdd, VT>(L.P, L.Pc, L.pg, items_ + L.corr_p.off, L.corr_p.count, lv_[k + 1].x, x,
                        static_cast<const RV *>(nullptr), s);
     if (k == 0) smooth<double>(0, r0, z, opt_.post, false, s);
     else smooth<VT>(k, L.b, L.x, opt_.post, false, s);
@@ -876,11 +919,11 @@ float Batch<VT, R>::time_level_op(int k, int op, int g, int reps) {
       cnt.push_back(static_cast<int>(v.size() - before));
     }
   } else if (op == 1) {
-    items_for(ly_.whole[k], g, L.A.h_srow, v);
+    items_for(parts(k), g, L.A.h_srow, v);
   } else if (op == 2) {
     items_for(ly_.below[k], g, L.Rs.h_srow, v);
   } else {
-    items_for(ly_.whole[k], g, L.P.h_srow, v);
+    items_for(parts(k), g, L.P.h_srow, v);
   }
   if (v.size() > tmp_cap_) {
     if (tmp_) BCK(cudaFree(tmp_));

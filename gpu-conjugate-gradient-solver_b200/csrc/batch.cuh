@@ -172,8 +172,27 @@ __global__ void __launch_bounds__(256) bsell_gs_kernel(SellView<T> A, const BIte
   }
 }
 
-// y = A x (kSpmvSet), y = b - A x (kSpmvResid), y += A x (kSpmvAdd); items
-// are slice ranges.
+// One row of y = A x (kSpmvSet), b - A x (kSpmvResid) or y + A x (kSpmvAdd)
+// from its off-diagonal sum.
+template <typename T, typename BT, int R, int kMode>
+__device__ __forceinline__ void bspmv_store(const T *__restrict__ diag, int row, Rv<T, R> sum,
+                                            const Rv<T, R> *__restrict__ x, Rv<T, R> *__restrict__ y,
+                                            const Rv<BT, R> *__restrict__ b) {
+  if (diag != nullptr) fma_rv<T, R>(__ldg(diag + row), x[row], sum);
+  if (kMode == kSpmvResid) {
+    const Rv<BT, R> bv = b[row];
+#pragma unroll
+    for (int j = 0; j < R; ++j) sum.v[j] = T(bv.v[j]) - sum.v[j];
+  } else if (kMode == kSpmvAdd) {
+    const Rv<T, R> old = y[row];
+#pragma unroll
+    for (int j = 0; j < R; ++j) sum.v[j] = old.v[j] + sum.v[j];
+  }
+  y[row] = sum;
+}
+
+// Items are slice ranges. The first slice's head is loaded before the wait on
+// the predecessor, as in the colour passes.
 template <typename T, typename BT, int R, int kMode>
 __global__ void __launch_bounds__(256) bsell_spmv_kernel(SellView<T> A, const BItem *__restrict__ items,
                                                          int nitems, const Rv<T, R> *__restrict__ x,
@@ -181,55 +200,28 @@ __global__ void __launch_bounds__(256) bsell_spmv_kernel(SellView<T> A, const BI
                                                          const Rv<BT, R> *__restrict__ b,
                                                          const int *__restrict__ sys_done) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+  BItem q = __ldg(items + blockIdx.x);
+  SellHead<T> h;
+  if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h);
   bpass_entry();
+  x = after_wait(x);
+  b = after_wait(b);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const BItem q = items[it];
+    const bool first = it == static_cast<int>(blockIdx.x);
+    if (!first) q = __ldg(items + it);
     if (item_skipped(sys_done, q.x)) continue;
     for (int s = q.y + warp; s < q.z; s += nw) {
-      Rv<T, R> sum = bsell_offdiag<T, R, false>(A, s, lane, x, 0);
-      const int row = A.srow[s] + lane;
-      if (row < A.srow[s + 1]) {
-        if (A.diag != nullptr) fma_rv<T, R>(A.diag[row], x[row], sum);
-        Rv<T, R> out;
-        if (kMode == kSpmvResid) {
-          const Rv<BT, R> bv = b[row];
-#pragma unroll
-          for (int j = 0; j < R; ++j) out.v[j] = T(bv.v[j]) - sum.v[j];
-        } else if (kMode == kSpmvAdd) {
-          out = y[row];
-#pragma unroll
-          for (int j = 0; j < R; ++j) out.v[j] += sum.v[j];
-        } else {
-          out = sum;
-        }
-        y[row] = out;
-      }
+      if (!first || s != q.y + warp) sell_head_ops(A, s, lane, h);
+      const Rv<T, R> sum = bsell_offdiag_head<T, R, false>(A, h, lane, x, 0);
+      const int row = h.r0 + lane;
+      if (row < h.r1) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
     }
   }
 }
 
 // ---- CSR-vector, G lanes per row -----------------------------------------
-template <typename T, int R, bool kSkip, int G>
-__device__ __forceinline__ Rv<T, R> bcsrv_offdiag(const CsrvView<T> &A, int row, bool valid, int sub,
-                                                  const Rv<T, R> *__restrict__ x, int skip_from) {
-  Rv<T, R> sum = rv_zero<T, R>();
-  if (valid) {
-    const int k1 = A.rp[row + 1];
-#pragma unroll 4
-    for (int k = A.rp[row] + sub; k < k1; k += G) {
-      const int c = __ldg(A.ci + k);
-      if (!kSkip || c < skip_from) fma_rv<T, R>(__ldg(A.v + k), ldg_rv<T, R>(x + c), sum);
-    }
-  }
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1)
-#pragma unroll
-    for (int j = 0; j < R; ++j) sum.v[j] += __shfl_xor_sync(0xffffffffu, sum.v[j], o, G);
-  return sum;
-}
-
-// bcsrv_offdiag from a loaded head: the same sums in the same order, the
-// gathers of four entries requested together.
+// A row's off-diagonal sum from a loaded head, the gathers of four entries
+// requested together.
 template <typename T, int R, bool kSkip, int G, int kE>
 __device__ __forceinline__ Rv<T, R> bcsrv_offdiag_head(const CsrvView<T> &A, const CsrvHead<T, kE> &h,
                                                        const Rv<T, R> *__restrict__ x, int skip_from) {
@@ -305,39 +297,30 @@ __global__ void __launch_bounds__(256) bcsrv_gs_kernel(CsrvView<T> A, const BIte
   }
 }
 
+// Items are row ranges, at most one row per group of G lanes; the head as in
+// the colour passes.
 template <typename T, typename BT, int R, int kMode, int G>
 __global__ void __launch_bounds__(256) bcsrv_spmv_kernel(CsrvView<T> A, const BItem *__restrict__ items,
                                                          int nitems, const Rv<T, R> *__restrict__ x,
                                                          Rv<T, R> *__restrict__ y,
                                                          const Rv<BT, R> *__restrict__ b,
                                                          const int *__restrict__ sys_done) {
-  const int sub = threadIdx.x & (G - 1), grp = threadIdx.x / G, ngrp = blockDim.x / G;
+  const int sub = threadIdx.x & (G - 1), grp = threadIdx.x / G;
+  BItem q = __ldg(items + blockIdx.x);
+  CsrvHead<T, 8> h;
+  csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
   bpass_entry();
+  x = after_wait(x);
+  b = after_wait(b);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    const BItem q = items[it];
-    if (item_skipped(sys_done, q.x)) continue;
-    const int trips = (q.z - q.y + ngrp - 1) / ngrp;
-    for (int t = 0; t < trips; ++t) {
-      const int row = q.y + grp + t * ngrp;
-      const bool valid = row < q.z;
-      Rv<T, R> sum = bcsrv_offdiag<T, R, false, G>(A, row, valid, sub, x, 0);
-      if (valid && sub == 0) {
-        if (A.diag != nullptr) fma_rv<T, R>(A.diag[row], x[row], sum);
-        Rv<T, R> out;
-        if (kMode == kSpmvResid) {
-          const Rv<BT, R> bv = b[row];
-#pragma unroll
-          for (int j = 0; j < R; ++j) out.v[j] = T(bv.v[j]) - sum.v[j];
-        } else if (kMode == kSpmvAdd) {
-          out = y[row];
-#pragma unroll
-          for (int j = 0; j < R; ++j) out.v[j] += sum.v[j];
-        } else {
-          out = sum;
-        }
-        y[row] = out;
-      }
+    if (it != static_cast<int>(blockIdx.x)) {
+      q = __ldg(items + it);
+      csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
     }
+    if (item_skipped(sys_done, q.x)) continue;
+    const int row = q.y + grp;
+    const Rv<T, R> sum = bcsrv_offdiag_head<T, R, false, G>(A, h, x, 0);
+    if (row < q.z && sub == 0) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
   }
 }
 
