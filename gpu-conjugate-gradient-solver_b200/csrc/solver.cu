@@ -1613,14 +1613,14 @@ void AmgPcg<VT>::dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s) {
                             static_cast<const float *>(L.ainv_scale), static_cast<const uint4 *>(L.dense_frag),
                             static_cast<const float *>(L.dense_inv), L.dense_partial_f, st_));
       CKL("coarse solve (tensor-core tiles)");
-      launch_pass(pdl_, dense_reduce_kernel<VT, float>, tiles, s, L.n, tiles, static_cast<const float *>(L.dense_partial_f),
+      launch_pass_n(pdl_, dense_reduce_kernel<VT, float>, tiles, kReduceThreads, s, L.n, tiles, static_cast<const float *>(L.dense_partial_f),
                   x, done);
     } else {
       constexpr int kT = dense_tiles_per_cta<VT>();
       launch_pass(pdl_, dense_tile_kernel<BT, VT, VT>, static_cast<int>((total + kT - 1) / kT), s, L.n, tiles, L.ainv,
                   rhs, L.dense_partial, done, static_cast<const float *>(nullptr));
       CKL("coarse solve (tiles)");
-      launch_pass(pdl_, dense_reduce_kernel<VT>, tiles, s, L.n, tiles, static_cast<const double *>(L.dense_partial), x,
+      launch_pass_n(pdl_, dense_reduce_kernel<VT>, tiles, kReduceThreads, s, L.n, tiles, static_cast<const double *>(L.dense_partial), x,
                   done);
     }
     CKL("coarse solve (reduce)");
