@@ -2011,11 +2011,12 @@ void AmgPcg<VT>::launch_tail(cudaStream_t s) {
 
 // Largest cluster of at most `want` CTAs (16, 8, 4, 2 or 1, 1024 threads
 // each) the device co-schedules with `smem` bytes of dynamic shared memory
-// per CTA; 0 if none.
+// per CTA; 0 if none. The kernel's limit is one for the process: it is set to
+// what the device allows, so that it holds for every solver alive.
 template <typename VT>
 int AmgPcg<VT>::tail_cluster_size(size_t smem, int want) {
   if (cudaFuncSetAttribute(coarse_tail_kernel<VT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           static_cast<int>(smem)) != cudaSuccess) {
+                           cluster_smem_bytes(device_)) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
