@@ -390,34 +390,6 @@ struct CsrvView {
   const int *__restrict__ re;  // end of each row (rp + 1 for whole rows)
 };
 
-template <typename T, bool kSkip, int G>
-__device__ __forceinline__ T csrv_offdiag(const CsrvView<T> &A, int row, bool valid, int sub,
-                                          const T *__restrict__ x, int skip_from) {
-  T sum = T(0);
-  if (valid) {
-    const int k1 = A.re[row];
-    // chunks of 4 entries per lane: the 4 column loads, then their 4 gathers
-    // and values, then the FMAs, so a chunk costs two dependent round trips
-    for (int k0 = A.rp[row] + sub; k0 < k1; k0 += 4 * G) {
-      int c[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) c[u] = k0 + u * G < k1 ? __ldg(A.ci + k0 + u * G) : -1;
-      T xv[4], v[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const bool use = c[u] >= 0 && (!kSkip || c[u] < skip_from);
-        xv[u] = use ? __ldg(x + c[u]) : T(0);
-        v[u] = c[u] >= 0 ? __ldg(A.v + k0 + u * G) : T(0);
-      }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) sum = fma(v[u], xv[u], sum);
-    }
-  }
-#pragma unroll
-  for (int o = G / 2; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o, G);
-  return sum;
-}
-
 // Operands of a row's first kE entries per lane that do not depend on the
 // iterate. The size changes only how many entries are loaded before the wait
 // on the predecessor: every lane still sums its entries in increasing order
@@ -447,7 +419,9 @@ __device__ __forceinline__ void csrv_head(const CsrvView<T> &A, int row, bool va
   }
 }
 
-// csrv_offdiag from a loaded head: the same chunks in the same order.
+// A row's off-diagonal sum from a loaded head, then in chunks of 4 entries per
+// lane: the 4 column loads, then their 4 gathers and values, then the FMAs, so
+// a chunk costs two dependent round trips.
 template <typename T, bool kSkip, int G, int kE, bool kRel = false>
 __device__ __forceinline__ T csrv_offdiag_head(const CsrvView<T> &A, const CsrvHead<T, kE> &h, int sub,
                                                const T *__restrict__ x, int skip_from,
@@ -496,7 +470,7 @@ __global__ void __launch_bounds__(256) csrv_spmv_kernel(CsrvView<T> A, const T *
   const int trips = (row_end - row_begin + groups - 1) / groups;
   // The first row's head (64 entries per row from 8 lanes up) is loaded
   // before the wait on the predecessor, and every trip loads the next row's
-  // while its own gathers are in flight. Same sums as csrv_offdiag.
+  // while its own gathers are in flight. The same sums in the same order.
   CsrvHead<T, (G >= 8 ? 8 : 64 / G)> h;
   csrv_head<T, G>(A, first, first < row_end, sub, h);
   if (pass_entry(done)) return;

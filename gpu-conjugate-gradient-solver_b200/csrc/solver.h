@@ -89,10 +89,11 @@ struct SolverOptions {
   // (relaxed_coloring) whose passes read their own colour's neighbours from
   // the iterate the sweep started with. A value refresh keeps the colouring.
   int coloring = 0;
-  // Symmetric Gauss-Seidel sweeps of a scalar level: 0 one launch per colour
-  // pass (the reference's structure), 1 the whole smoothing step as one
-  // cooperative launch with grid barriers between colours where that is
-  // timed faster at setup, 2 cooperative on every such level. Colour passes
+  // Symmetric Gauss-Seidel sweeps: 0 one launch per colour pass (the
+  // reference's structure), 1 the whole smoothing step in one launch where that
+  // is timed faster at setup, by one thread-block cluster (cluster.cuh; scalar
+  // and 3x3 block levels) or, on a scalar level, cooperatively with grid
+  // barriers between colours, 2 cooperative on every scalar level. Colour passes
   // of a 3x3 block level in the BELL-1 layout: 1 with each slice's blocks
   // bulk-copied to shared memory where timed faster, 2 on every such level
   // whose widest slice fits, 0 never. The iterates are the same bit for bit.

@@ -410,7 +410,10 @@ int gs_dense_spd_inverse(int n, const int *row_ptr, const int *col_idx, const do
  * iteration is one CUDA graph. The systems' R right-hand sides share each
  * matrix read.
  * Options: pre/post_steps, vcycles, omega, precision, flexible, use_graph,
- * tol, max_iter, autotune, lanes (1, 2, 4, 8, 16 or 32 here). Required:
+ * tol, max_iter, autotune, lanes (1, 2, 4, 8, 16 or 32 here), overlap_launch,
+ * sweep_launch (1: the smoothing steps of levels below the finest run in one
+ * thread-block cluster per system where timed faster; needs autotune and
+ * lanes 0). Required:
  * smoother 0, coarse_solver 1, reference_vcycle 0, and at least two levels
  * per hierarchy.
  * --------------------------------------------------------------------- */
