@@ -1637,7 +1637,10 @@ void AmgPcg<VT>::dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s) {
 
 // The first pass of level k's pre-smoothing from zero, for the kernel that
 // writes its right-hand side; none where the level is not smoothed by
-// per-colour launches of scalar Gauss-Seidel passes.
+// per-colour launches of scalar Gauss-Seidel passes. A single level of one
+// colour keeps the pass as well: it is the only launch of that preconditioner,
+// and the dot kernel behind it loads r before it waits, which is safe because
+// a launch lies between it and the update that writes r.
 template <typename VT>
 FirstColour<VT> AmgPcg<VT>::first_colour(int k, VT *x) {
   const Level &L = lv_[k];
@@ -1645,7 +1648,7 @@ FirstColour<VT> AmgPcg<VT>::first_colour(int k, VT *x) {
   const int steps = k + 1 < static_cast<int>(lv_.size()) ? opt_.pre : opt_.coarse_steps;
   const int dir = k + 1 < static_cast<int>(lv_.size()) && opt_.half_sweeps ? 1 : 0;
   if (!smoothed || L.kind != 0 || block_ || (tail_on_ && k >= tail_k0_) || in_cluster(L, steps, dir) ||
-      (L.coop && dir == 0 && !L.relaxed))
+      (L.coop && dir == 0 && !L.relaxed) || (lv_.size() == 1 && L.ncolors < 2))
     return FirstColour<VT>{};
   return FirstColour<VT>{x, L.C.diag, L.color_first[1], L.wts[0], VT(opt_.omega)};
 }

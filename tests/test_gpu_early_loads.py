@@ -1,0 +1,33 @@
+"""Kernels that load operands before they wait on the launch ahead of them: the
+same bits whether launches overlap or not, where only few launches lie between
+a vector's writer and its reader."""
+import numpy as np
+import pytest
+import scipy.sparse as sp
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 33, 70001])
+@pytest.mark.parametrize("flexible", [0, 1])
+def test_one_level_of_one_colour(gs, device, n, flexible):
+    """A diagonal matrix: one level, one colour, so the whole preconditioner is
+    one pass. FP32 passes and a tight tolerance keep the solve going past its
+    first iteration."""
+    r = np.random.default_rng(n)
+    d = r.uniform(0.5, 3.0, n) if n > 1 else np.array([3.0])
+    H = gs.Hierarchy.from_levels([gs.Csr.from_scipy(sp.diags(d).tocsr())], [], [])
+    b = gs.uniform_rhs(n, 5)
+    out = []
+    for graph in (0, 1):
+        for overlap in (0, 1, 2):
+            o = gs.SolverOptions(tol=1e-13, precision=1, flexible=flexible, coarse_solver=0, coarse_tail=0,
+                                 use_graph=graph, overlap_launch=overlap)
+            s = gs.Solver(H, o, device=device)
+            for _ in range(3):
+                x, st = s.solve(b)
+                out.append((x, st.iterations, st.status))
+            # FP32 relaxation: 24 bits an iteration at least
+            assert st.status == gs.STATUS_CONVERGED and np.linalg.norm(d * x - b) <= 2e-13 * np.linalg.norm(b)
+    for x, it, status in out[1:]:
+        assert it == out[0][1] and status == out[0][2] and np.array_equal(x, out[0][0])
