@@ -30,7 +30,8 @@
 // No race. Row j of colour c' is overwritten in CTA B's slots only after the
 // owner A of j has waited for every earlier pass of the sweep, and A receives
 // every row i that reads j (checked when the layout is built): B's read of j
-// for i happened before B sent i. Two writes of one row to one slot are
+// for i happened before B sent i. A weighted update also reads the row's own
+// slot, in every lane of its group, before any lane sends. Two writes of one row to one slot are
 // separated by a direction change or a step's end, where every CTA first
 // waits for all its passes and then meets the others at the cluster barrier,
 // so the earlier write has landed. Rows of one colour do not read each other
@@ -507,6 +508,9 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
 #pragma unroll
           for (int j = 0; j < W; ++j) xn[j] = fma(T(1) - w, xs[own + j], w * xn[j]);
         }
+        // every lane of a row has read its old value before one of them
+        // sends the new one into the same slot
+        __syncwarp();
       }
       send_row(to_x, xn, to_bar, cur.send != kNoSend);
       if (sg.schunks > 1)

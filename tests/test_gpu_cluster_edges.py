@@ -1,0 +1,25 @@
+"""Edges of the cluster-resident smoothing steps (cluster.cuh), against colour
+passes with the same lanes per row: the same bits."""
+import numpy as np
+import pytest
+
+from test_gpu_cluster import solver_with
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_own_values_are_read_before_they_are_replaced(gs, device, tmp_path, precision):
+    """Weights that differ from row to row, some exactly 1: the rows of a warp
+    part ways around the read of their old values."""
+    a = gs.elasticity(9)
+    H = gs.Hierarchy.build(a, 3, 0.1, 10, 60)
+    out = []
+    for cluster in (False, True):
+        o = gs.SolverOptions(smoother=1, tol=1e-9, coarse_tail=0, precision=precision, flexible=precision)
+        s = solver_with(gs, device, tmp_path, H, o, cluster)
+        n = len(s.node_features())
+        s.set_node_weights(np.where(np.arange(n) % 3 == 0, 1.0, 0.8 + 0.4 * (np.arange(n) % 7) / 6))
+        out.append([s.solve(a.rhs)[0] for _ in range(4)])
+    for p in out[0] + out[1]:
+        assert np.array_equal(p, out[0][0])
