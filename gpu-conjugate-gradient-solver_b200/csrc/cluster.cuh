@@ -91,7 +91,9 @@ struct ClusterView {
   int row0;                                    // first row of this system in the level's vectors (batches)
 };
 
-constexpr unsigned kNoSend = 0xffffffffu;
+// No message. Its CTA and slot read 0, which every cluster has: the addresses
+// are formed ahead of the test whether to send.
+constexpr unsigned kNoSend = 0x80000000u;
 
 // The passes of one call: dir 0 symmetric steps, 1 forward sweeps, 2
 // backward sweeps; skip drops the colour repeated where a sweep turns.
@@ -447,6 +449,7 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
   constexpr int kLog = G == 4 ? 2 : (G == 8 ? 3 : (G == 16 ? 4 : 5));
   const int grp = tid >> kLog, groups = nthr >> kLog;
   typename Row::Unit unit0, unit1;
+  unit0.send = unit1.send = kNoSend;  // threads without a row
   unsigned code = plist[0];
   ClusterSeg sg = seg[code & 0x7fffu];
   if (tid < sg.stride) {
@@ -481,6 +484,7 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     const unsigned next_code = plist[last_trip ? p + 1 : p];
     ClusterSeg sn;
     sn.stride = 0;
+    nxt.send = kNoSend;
     if (next_code != 0xffffu) {
       sn = seg[next_code & 0x7fffu];
       if (tid < sn.stride) {
