@@ -733,6 +733,11 @@ int gs_set_tune_cache(const char *path) {
   return GS_OK;
 }
 
+int gs_debug_withhold_cluster_message(int on) {
+  gsb::cluster_message_withheld() = on != 0;
+  return GS_OK;
+}
+
 int gs_solver_create(const gs_hierarchy *h, const int *const *o2n, const int *const *n2o,
                      const gs_solver_options *opt, int device, gs_solver **out) {
   return guarded([&] {

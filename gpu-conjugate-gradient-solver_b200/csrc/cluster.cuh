@@ -45,7 +45,8 @@
 //
 // Waits on mbarriers are bounded: a wait that gives up records
 // CgState::sync_fault and stops the solve; the kernel then runs to its end
-// without waiting.
+// without waiting, sends all its messages, and before it leaves waits (bounded
+// as well) for those that are on their way to it.
 #pragma once
 
 #include "bulk.cuh"
@@ -60,6 +61,7 @@ constexpr int kClusterBlocks = 2;       // 3x3 blocks per lane loaded ahead
 constexpr int kClusterMaxPasses = 512;  // mbarriers
 constexpr int kClusterMaxSlots = 32760; // two copies of the slots in 16 bits
 constexpr int kClusterMaxColors = 128;
+constexpr long long kClusterWaitClocks = 2000000000LL;  // about a second
 
 // One CTA's piece of one colour.
 struct __align__(16) ClusterSeg {
@@ -88,6 +90,7 @@ struct ClusterView {
   const T *__restrict__ diag;                  // scalar: {d, 1 / d} per row, the latter 0 where it is not safe to
                                                // use; 3x3: the inverse diagonal block per node
   int relaxed;                                 // own-colour reads from the sweep's start
+  long long wait_clocks;                       // bound of a wait
   int row0;                                    // first row of this system in the level's vectors (batches)
 };
 
@@ -216,8 +219,7 @@ __device__ __forceinline__ T quotient(T n, T d, T r) {
 }
 
 // Bounded wait for the values of a pass (written by other CTAs: acquire at
-// cluster scope); false after about a second of clocks.
-constexpr long long kClusterWaitClocks = 2000000000LL;
+// cluster scope); false after `clocks`.
 
 __device__ __forceinline__ bool pass_ready(unsigned bar) {
   unsigned ok;
@@ -229,12 +231,21 @@ __device__ __forceinline__ bool pass_ready(unsigned bar) {
       : "memory");
   return ok != 0;
 }
-__device__ __forceinline__ bool pass_wait(unsigned bar) {
+__device__ __forceinline__ bool pass_wait(unsigned bar, long long clocks) {
   if (pass_ready(bar)) return true;
   const long long t0 = clock64();
-  while (clock64() - t0 < kClusterWaitClocks)
+  while (clock64() - t0 < clocks)
     if (pass_ready(bar)) return true;
   return false;
+}
+// After a wait gave up, ahead of the last cluster barrier: what is on its way
+// to this CTA lands before it leaves. What is still missing after `clocks` in
+// all was not sent.
+__device__ __forceinline__ void drain_passes(unsigned bars, int npass, long long clocks) {
+  const long long t0 = clock64();
+  for (int p = 0; p < npass; ++p)
+    while (!pass_ready(bars + 8 * p) && clock64() - t0 < clocks) {
+    }
 }
 
 }  // namespace cluster_detail
@@ -497,7 +508,7 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     const unsigned to_cta = (cur.send >> 16) & 15u;
     const unsigned to_x = remote(xs_addr + static_cast<unsigned>(W * sizeof(T)) * (cur.send & 0xffffu), to_cta);
     const unsigned to_bar = remote(bar_addr + 8 * p, to_cta);
-    if (t == 0 && !fresh && !dead) dead = !pass_wait(bar_addr + 8 * (p - 1));
+    if (t == 0 && !fresh && !dead) dead = !pass_wait(bar_addr + 8 * (p - 1), A.wait_clocks);
     if (tid < sg.stride) {
       T sum[W], xn[W];
       Row::sums(A, sg, t, tid, xs, cur, sum);
@@ -532,7 +543,8 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
       if (code & 0x8000u) {
         // every value of this sweep has arrived before the next one starts
         // (or before the CTAs leave)
-        if (!dead) dead = !pass_wait(bar_addr + 8 * p);
+        if (!dead) dead = !pass_wait(bar_addr + 8 * p, A.wait_clocks);
+        if (dead && next_code == 0xffffu) drain_passes(bar_addr, npass, A.wait_clocks);
         if (A.relaxed) {
           __syncthreads();
           for (int k = tid; k < nslots * W; k += nthr) xp[k] = xs[k];

@@ -13,12 +13,14 @@
 
 #include "cluster.cuh"
 #include "formats.cuh"
+#include "solver.h"
 
 namespace gsb {
 
 template <typename T>
 struct HostCluster {
   int ncta = 0, ncolors = 0, g = 0, threads = 0, max_slots = 0, relaxed = 0;
+  long long wait_clocks = kClusterWaitClocks;
   std::vector<ClusterSeg> seg;
   std::vector<unsigned> expect;
   std::vector<int> slot_ptr, slot_row;
@@ -131,6 +133,10 @@ bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci
       h.expect[static_cast<size_t>(q) * nc + c] = static_cast<unsigned>(
           std::lower_bound(rq.begin(), rq.end(), first[c + 1]) - std::lower_bound(rq.begin(), rq.end(), first[c]));
     }
+  if (cluster_message_withheld()) {  // tests: the wait for the first colour runs out
+    ++h.expect[0];
+    h.wait_clocks = 2000000;
+  }
   h.val.assign(static_cast<size_t>(values) * words, T(0));
   h.col.assign(static_cast<size_t>(per) * words, zero_slot);
   h.send.assign(static_cast<size_t>(send_total), kNoSend);
@@ -255,6 +261,7 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
   d.values = h.val.size();
   d.v.ncta = h.ncta, d.v.ncolors = h.ncolors, d.v.threads = h.threads, d.v.max_slots = h.max_slots;
   d.v.relaxed = h.relaxed;
+  d.v.wait_clocks = h.wait_clocks;
   d.v.row0 = row0;
   // one allocation and one copy for the whole layout
   std::vector<unsigned char> pack;

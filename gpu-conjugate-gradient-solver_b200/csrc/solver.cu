@@ -2657,6 +2657,11 @@ double AmgPcg<VT>::error_reduction(const double *e0, cudaStream_t stream) {
 
 }  // namespace
 
+bool &cluster_message_withheld() {
+  static thread_local bool on = false;
+  return on;
+}
+
 std::unique_ptr<Solver> Solver::create(const Hierarchy &h, const std::vector<const int *> &o2n,
                                        const std::vector<const int *> &n2o,
                                        const SolverOptions &opt, int device) {

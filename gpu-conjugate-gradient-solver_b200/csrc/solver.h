@@ -20,6 +20,10 @@ struct CudaError : std::runtime_error {
 };
 void cuda_check(cudaError_t e, const char *what);
 
+// Whether cluster layouts built on this thread expect a message that nobody
+// sends (gs_debug_withhold_cluster_message).
+bool &cluster_message_withheld();
+
 struct SolverOptions {
   // Smoother of the finest level (and of every level unless coarse_smoother
   // is set): 0 multicolour SGS, 1 3x3 block SGS, 2 damped Jacobi, 3 3x3 block

@@ -47,7 +47,7 @@ EXPORTED_SYMBOLS = [
     "gs_permute_matrix", "gs_ell_build", "gs_block_graph", "gs_block_inverses3x3",
     "gs_expand_block_permutation", "gs_problem_create", "gs_host_csr_create",
     "gs_host_csr_info", "gs_host_csr_copy", "gs_host_csr_rhs", "gs_host_csr_destroy",
-    "gs_uniform_rhs", "gs_set_tune_cache", "gs_hierarchy_build", "gs_hierarchy_from_levels",
+    "gs_uniform_rhs", "gs_set_tune_cache", "gs_debug_withhold_cluster_message", "gs_hierarchy_build", "gs_hierarchy_from_levels",
     "gs_hierarchy_num_levels", "gs_hierarchy_matrix_info", "gs_hierarchy_matrix",
     "gs_hierarchy_aggregates", "gs_hierarchy_build_ex", "gs_solver_setup_times", "gs_hierarchy_destroy", "gs_hierarchical_reordering", "gs_solver_options_default",
     "gs_solver_create", "gs_solver_solve", "gs_solver_solve_f32", "gs_solver_solve_device",

@@ -304,6 +304,11 @@ void gs_solver_options_default(gs_solver_options *opt);
 /* Path of the autotuner's decision cache used by solvers created afterwards
  * on this thread (NULL or "" = no cache). The reference has no autotuner. */
 int gs_set_tune_cache(const char *path);
+/* For tests of the failure path: while on, smoothing steps in one thread-block
+ * cluster of solvers and batches created on this thread expect a message that
+ * nobody sends, so that a wait of theirs gives up (after about a millisecond)
+ * and the call that runs them reports an error. */
+int gs_debug_withhold_cluster_message(int on);
 /* old_to_new / new_to_old: one permutation per level (the reference's
  * std::vector<Permutation>), or NULL for identity on every level. */
 int gs_solver_create(const gs_hierarchy *h, const int *const *old_to_new,

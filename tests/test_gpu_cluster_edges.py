@@ -23,3 +23,34 @@ def test_own_values_are_read_before_they_are_replaced(gs, device, tmp_path, prec
         out.append([s.solve(a.rhs)[0] for _ in range(4)])
     for p in out[0] + out[1]:
         assert np.array_equal(p, out[0][0])
+
+
+@pytest.fixture
+def withheld(gs):
+    """While the returned function is on, cluster steps wait for a message that nobody sends."""
+    yield gs.lib().gs_debug_withhold_cluster_message
+    gs.lib().gs_debug_withhold_cluster_message(0)
+
+
+@pytest.fixture(scope="module")
+def kuhn(gs):
+    a = gs.kuhn_laplacian(15)
+    return a, gs.Hierarchy.build(a, 1, 0.1, 10, 20), gs.uniform_rhs(a.rows, 5)
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("kw", [dict(), dict(pre_steps=2, post_steps=2), dict(half_sweeps=1, coloring=2)],
+                         ids=lambda kw: "-".join(f"{k}{v}" for k, v in kw.items()) or "default")
+def test_a_wait_that_gives_up_is_an_error(gs, device, tmp_path, withheld, kuhn, graph, kw):
+    """The step returns, the solve reports the failure, and the device goes on."""
+    a, H, b = kuhn
+    o = gs.SolverOptions(tol=1e-9, coarse_tail=0, use_graph=graph, **kw)
+    good = solver_with(gs, device, tmp_path, H, o, True)
+    x, _ = good.solve(b)
+    withheld(1)
+    s = solver_with(gs, device, tmp_path, H, o, True)
+    withheld(0)
+    for _ in range(2):
+        with pytest.raises(gs.SolverError, match="timed out"):
+            s.solve(b)
+    assert np.array_equal(good.solve(b)[0], x)
