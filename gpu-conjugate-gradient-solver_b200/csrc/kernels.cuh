@@ -1293,6 +1293,7 @@ __global__ void __launch_bounds__(256) cg_init_kernel(int n, const double *__res
       st->status = kCgInitialConverged;
       st->done = 1;
     }
+    if (st->sync_fault != 0) st->done = 1;  // a wait of the start's V-cycle gave up: nothing to go on from
     // a zero right-hand side: whatever else is found, the host returns x = 0
     host[1] = finite_d(acc[0]) && !(sqrt(acc[0]) >= 1e-12) ? kStartZeroRhs : kStartRuns;
   }
@@ -1640,9 +1641,12 @@ __global__ void convert_kernel(int n, const BT *__restrict__ v, T *__restrict__ 
 }
 
 // ---- permutation between the caller's order and the internal colour order.
+// fault: CgState::sync_fault; after a fault there is no answer and the caller's
+// array stays as it is.
 template <typename T, typename U>
 __global__ void gather_kernel(int n, const int *__restrict__ src_of, const T *__restrict__ in,
-                              U *__restrict__ out) {
+                              U *__restrict__ out, const int *fault) {
+  if (*fault != 0) return;
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = U(in[src_of[i]]);
 }

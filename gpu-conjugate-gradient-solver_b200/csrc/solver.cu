@@ -2399,7 +2399,7 @@ void AmgPcg<VT>::run(double *x, SolveStats *out) {
   if (zero_rhs) CK(cudaMemsetAsync(x_, 0, sizeof(double) * n0_, stream_));  // CGSolver::solve: x = 0
   CK(cudaEventRecord(ev_[3], stream_));
   if (answer) {
-    gather_kernel<double, double><<<blocks_for(n0_, cap_blocks_), 256, 0, stream_>>>(n0_, q0_, x_, x);
+    gather_kernel<double, double><<<blocks_for(n0_, cap_blocks_), 256, 0, stream_>>>(n0_, q0_, x_, x, &st_->sync_fault);
     CKL("permute out");
   }
   CK(cudaStreamSynchronize(stream_));
@@ -2453,7 +2453,7 @@ void AmgPcg<VT>::apply_preconditioner(const double *r, double *z, cudaStream_t s
   const int blocks = blocks_for(n0_, cap_blocks_);
   scatter_kernel<double, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, r, r_);
   precondition(r_, z_[0], stream_);
-  gather_kernel<VT, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, z_[0], z);
+  gather_kernel<VT, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, z_[0], z, &st_->sync_fault);
   CKL("apply preconditioner");
   ++launches_;  // the scatter before the V-cycle
   CK(cudaEventRecord(ev_[1], stream_));

@@ -54,3 +54,20 @@ def test_a_wait_that_gives_up_is_an_error(gs, device, tmp_path, withheld, kuhn, 
         with pytest.raises(gs.SolverError, match="timed out"):
             s.solve(b)
     assert np.array_equal(good.solve(b)[0], x)
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+@pytest.mark.parametrize("max_iter", [1, 50])
+def test_x_is_left_alone_after_a_fault(gs, device, tmp_path, withheld, kuhn, graph, max_iter):
+    """The wait gives up in the V-cycle that starts the solve."""
+    torch = pytest.importorskip("torch")
+    a, H, b = kuhn
+    o = gs.SolverOptions(tol=1e-9, coarse_tail=0, use_graph=graph, max_iter=max_iter)
+    withheld(1)
+    s = solver_with(gs, device, tmp_path, H, o, True)
+    bd = torch.from_numpy(np.asarray(b)).cuda()
+    x = torch.full_like(bd, 2.0)
+    torch.cuda.synchronize()
+    with pytest.raises(gs.SolverError, match="timed out"):
+        s.solve_device(bd.data_ptr(), x.data_ptr(), 0)
+    assert bool((x == 2.0).all())
