@@ -1642,11 +1642,14 @@ __global__ void convert_kernel(int n, const BT *__restrict__ v, T *__restrict__ 
 
 // ---- permutation between the caller's order and the internal colour order.
 // fault: CgState::sync_fault; after a fault there is no answer and the caller's
-// array stays as it is.
+// array stays as it is. host (or nullptr): told of the fault.
 template <typename T, typename U>
 __global__ void gather_kernel(int n, const int *__restrict__ src_of, const T *__restrict__ in,
-                              U *__restrict__ out, const int *fault) {
-  if (*fault != 0) return;
+                              U *__restrict__ out, const int *fault, volatile unsigned *host) {
+  if (*fault != 0) {
+    if (host != nullptr && blockIdx.x == 0 && threadIdx.x == 0) *host = 1u;
+    return;
+  }
   const int stride = gridDim.x * blockDim.x;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = U(in[src_of[i]]);
 }

@@ -554,6 +554,11 @@ class AmgPcg final : public Solver {
   }
   void forward_sweep(Level &L, cudaStream_t s);
   void check_sync_fault(const CgState &hs);
+  void report_fault() {
+    CgState hs{};
+    CK(cudaMemcpy(&hs, st_, sizeof(CgState), cudaMemcpyDeviceToHost));
+    check_sync_fault(hs);
+  }
   void drop_graphs();
   template <typename BT>
   void dense_coarse(Level &L, const BT *rhs, VT *x, cudaStream_t s);
@@ -630,7 +635,8 @@ class AmgPcg final : public Solver {
   CgState *st_ = nullptr, *scratch_st_ = nullptr;
   double *partials_ = nullptr;
   CgState *host_st_ = nullptr;                  // pinned
-  volatile unsigned *host_seq_ = nullptr;       // pinned, two words written by the kernels (publish_state)
+  volatile unsigned *host_seq_ = nullptr;       // pinned, written by the kernels: two words of a solve (publish_state),
+                                                // then whether applying the preconditioner met a fault
   bool wait_published(int it);
   SweepSync *sync_ = nullptr;                   // grid-barrier state of the cooperative sweeps
   VT *wbuf_ = nullptr;
@@ -2399,7 +2405,7 @@ void AmgPcg<VT>::run(double *x, SolveStats *out) {
   if (zero_rhs) CK(cudaMemsetAsync(x_, 0, sizeof(double) * n0_, stream_));  // CGSolver::solve: x = 0
   CK(cudaEventRecord(ev_[3], stream_));
   if (answer) {
-    gather_kernel<double, double><<<blocks_for(n0_, cap_blocks_), 256, 0, stream_>>>(n0_, q0_, x_, x, &st_->sync_fault);
+    gather_kernel<double, double><<<blocks_for(n0_, cap_blocks_), 256, 0, stream_>>>(n0_, q0_, x_, x, &st_->sync_fault, nullptr);
     CKL("permute out");
   }
   CK(cudaStreamSynchronize(stream_));
@@ -2453,12 +2459,14 @@ void AmgPcg<VT>::apply_preconditioner(const double *r, double *z, cudaStream_t s
   const int blocks = blocks_for(n0_, cap_blocks_);
   scatter_kernel<double, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, r, r_);
   precondition(r_, z_[0], stream_);
-  gather_kernel<VT, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, z_[0], z, &st_->sync_fault);
+  host_seq_[2] = 0u;  // the stream was idle when this call began
+  gather_kernel<VT, double><<<blocks, 256, 0, stream_>>>(n0_, q0_, z_[0], z, &st_->sync_fault, host_seq_ + 2);
   CKL("apply preconditioner");
   ++launches_;  // the scatter before the V-cycle
   CK(cudaEventRecord(ev_[1], stream_));
   CK(cudaStreamWaitEvent(stream, ev_[1], 0));
   CK(cudaStreamSynchronize(stream));
+  if (host_seq_[2] != 0u) report_fault();
 }
 
 template <typename VT>
@@ -2650,7 +2658,9 @@ double AmgPcg<VT>::error_reduction(const double *e0, cudaStream_t stream) {
   precondition(ap_, z_[0], s);             // z = M A e0
   sub_kernel<VT><<<blocks, 256, 0, s>>>(n0_, x_, z_[0], p_);  // e1 = e0 - z
   CKL("error update");
+  CK(cudaMemcpyAsync(&host_st_[0], st_, sizeof(CgState), cudaMemcpyDeviceToHost, s));
   const double e1a = energy(p_);
+  check_sync_fault(host_st_[0]);
   if (!(e0a > 0.0)) throw std::runtime_error("error_reduction: e0 has zero energy");
   return std::sqrt(std::max(e1a, 0.0) / e0a);
 }

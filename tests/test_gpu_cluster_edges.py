@@ -71,3 +71,24 @@ def test_x_is_left_alone_after_a_fault(gs, device, tmp_path, withheld, kuhn, gra
     with pytest.raises(gs.SolverError, match="timed out"):
         s.solve_device(bd.data_ptr(), x.data_ptr(), 0)
     assert bool((x == 2.0).all())
+
+
+@pytest.mark.parametrize("precision", [0, 1])
+def test_applying_the_preconditioner_reports_a_fault(gs, device, tmp_path, withheld, kuhn, precision):
+    torch = pytest.importorskip("torch")
+    a, H, b = kuhn
+    o = gs.SolverOptions(coarse_tail=0, precision=precision)
+    good = solver_with(gs, device, tmp_path, H, o, True)
+    withheld(1)
+    s = solver_with(gs, device, tmp_path, H, o, True)
+    r = torch.from_numpy(np.asarray(b)).cuda()
+    z = torch.full_like(r, 2.0)
+    torch.cuda.synchronize()
+    for _ in range(2):
+        with pytest.raises(gs.SolverError, match="timed out"):
+            s.apply_preconditioner_device(r.data_ptr(), z.data_ptr(), 0)
+        assert bool((z == 2.0).all())
+        with pytest.raises(gs.SolverError, match="timed out"):
+            s.error_reduction(r.data_ptr(), 0)
+    good.apply_preconditioner_device(r.data_ptr(), z.data_ptr(), 0)
+    assert bool(torch.isfinite(z).all()) and good.error_reduction(r.data_ptr(), 0) < 1.0
