@@ -865,9 +865,13 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
     L.cluster = true;
     t_cluster = std::min(t_cluster, time_ms(step, 5));
   }
-  L.cluster = t_cluster < 1.1f * t_pass;
   BCK(cudaMemcpy(&host_sh_[0], sh_, sizeof(BCgShared), cudaMemcpyDeviceToHost));
-  check_fault();
+  if (host_sh_[0].sync_fault != 0) {  // a wait gave up and stopped its system: the passes stay
+    BCK(cudaMemset(sh_, 0, sizeof(BCgShared)));
+    BCK(cudaMemset(sys_done_, 0, sizeof(int) * S_));
+    t_cluster = 1e30f;
+  }
+  L.cluster = t_cluster < 1.1f * t_pass;
   if (L.cluster) kept_.push_back(std::move(arena));
 }
 

@@ -1989,7 +1989,13 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
   if (!build_cluster(L, k, *arena)) return;
   const float t_pass = t_now > 0.f ? t_now : time_segment(step, 10, kIssuedTrials, true);
   L.cluster = true;
-  L.cluster = time_segment(step, 10, kIssuedTrials, true) < t_pass;
+  float t_cluster = time_segment(step, 10, kIssuedTrials, true);
+  try {
+    report_fault();
+  } catch (const CudaError &) {
+    t_cluster = 1e30f;  // a wait gave up, after which every launch returned at once: the passes stay
+  }
+  L.cluster = t_cluster < t_pass;
   CK(cudaStreamSynchronize(stream_));
   if (L.cluster) kept_layouts_.push_back(std::move(arena));
 }

@@ -92,3 +92,34 @@ def test_applying_the_preconditioner_reports_a_fault(gs, device, tmp_path, withh
             s.error_reduction(r.data_ptr(), 0)
     good.apply_preconditioner_device(r.data_ptr(), z.data_ptr(), 0)
     assert bool(torch.isfinite(z).all()) and good.error_reduction(r.data_ptr(), 0) < 1.0
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_the_tuner_drops_a_cluster_whose_wait_gives_up(gs, device, tmp_path, withheld, kuhn, graph):
+    """After a fault every launch returns at once: such a step would time as the fastest."""
+    a, H, b = kuhn
+    o = gs.SolverOptions(tol=1e-9, coarse_tail=0, use_graph=graph)
+    path = tmp_path / "decisions"
+    gs.set_tune_cache(str(path))
+    withheld(1)
+    try:
+        s = gs.Solver(H, o, device=device)
+    finally:
+        gs.set_tune_cache(None)
+    fields = [int(v) for v in path.read_text().split()[1:]]
+    assert not any(fields[6::7])
+    x, st = s.solve(b)
+    assert st.status == gs.STATUS_CONVERGED and np.linalg.norm(b - a.to_scipy() @ x) <= 2e-9 * np.linalg.norm(b)
+
+
+def test_the_batch_tuner_drops_a_cluster_whose_wait_gives_up(gs, device, withheld):
+    mats = [gs.varcoef_loguniform(x, y, z, seed=3 + i) for i, (x, y, z) in enumerate([(17, 19, 15), (21, 9, 23), (14, 14, 14)])]
+    hs = [gs.Hierarchy.build(m, 1, 0.1, 10, 60) for m in mats]
+    b = np.concatenate([gs.uniform_rhs(m.rows, i) for i, m in enumerate(mats)])
+    withheld(1)
+    B = gs.Batch(hs, 1, gs.SolverOptions(tol=1e-9), device=device)
+    x, st = B.solve(b)
+    assert all(s.status == gs.STATUS_CONVERGED for s in st)
+    for m, xi, bi in zip(mats, np.split(x, np.cumsum([m.rows for m in mats])[:-1]),
+                         np.split(b, np.cumsum([m.rows for m in mats])[:-1])):
+        assert np.linalg.norm(bi - m.to_scipy() @ xi) <= 2e-9 * np.linalg.norm(bi)
