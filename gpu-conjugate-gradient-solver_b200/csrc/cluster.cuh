@@ -565,7 +565,7 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     if (step(unit1, unit0)) break;
   }
   if (dead) {
-    *status.fault = 1;
+    *status.fault = kFaultCluster;
     *status.stop = 1;
   }
 }

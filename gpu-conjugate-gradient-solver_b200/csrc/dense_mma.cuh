@@ -241,7 +241,7 @@ static __global__ void __launch_bounds__(32 * kMmaWarps) dense_mma_kernel(int ti
     }
     if (!__all_sync(0xffffffffu, mbar_wait_bounded(&bars[k], static_cast<unsigned>((i / kMmaStages) & 1)))) {
       if (lane == 0) {
-        atomicExch(&st->sync_fault, 1);
+        atomicExch(&st->sync_fault, kFaultBulkCopy);
         atomicExch(&st->done, 1);
       }
       drain(i);  // this tile's copy and the two after it

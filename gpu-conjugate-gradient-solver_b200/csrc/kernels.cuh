@@ -56,6 +56,8 @@ struct BellView {
   const int *__restrict__ up;
 };
 
+enum SyncFault : int { kFaultNone = 0, kFaultGridBarrier = 1, kFaultCluster = 2, kFaultBulkCopy = 3 };
+
 // State of one preconditioned CG solve, resident on the device. Scalars are
 // produced by the last block of each reduction kernel; the host reads
 // `done`/`status` only when it has to.
@@ -63,7 +65,7 @@ struct CgState {
   double rho, rho_new, rz_old, pAp, alpha, beta, rr, bb, ratio, tol2;
   int iter, max_iter, done, status, iterations, flexible;
   unsigned int ticket;
-  int sync_fault;  // a bounded grid-barrier wait gave up (cooperative sweeps)
+  int sync_fault;  // SyncFault: which bounded wait gave up
 };
 
 enum CgStatus : int {

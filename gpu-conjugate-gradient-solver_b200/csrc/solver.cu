@@ -1480,15 +1480,18 @@ void AmgPcg<VT>::forward_sweep(Level &L, cudaStream_t s) {
   for (int c = 0; c < L.ncolors; ++c) gs_pass<VT>(L, c, L.b, L.x, false, s);
 }
 
-// A grid-barrier wait that gave up leaves the barrier state undefined: it is
-// cleared before the error is reported, so the solver stays usable.
+// A wait that gave up. One at a grid barrier leaves the barrier state
+// undefined: it is cleared before the error is reported, so the solver stays
+// usable.
 template <typename VT>
 void AmgPcg<VT>::check_sync_fault(const CgState &hs) {
   if (hs.sync_fault == 0) return;
   CK(cudaStreamSynchronize(stream_));
   CK(cudaMemset(sync_, 0, sizeof(SweepSync)));
   CK(cudaMemset(st_, 0, sizeof(CgState)));
-  throw CudaError("cooperative Gauss-Seidel sweep: a grid-barrier wait timed out");
+  throw CudaError(hs.sync_fault == kFaultCluster    ? "cluster Gauss-Seidel step: a wait timed out"
+                  : hs.sync_fault == kFaultBulkCopy ? "bulk copy of matrix entries: a wait timed out"
+                                                    : "cooperative Gauss-Seidel sweep: a grid-barrier wait timed out");
 }
 
 // Rows whose residual is not zero after pre-smoothing. The colour updated

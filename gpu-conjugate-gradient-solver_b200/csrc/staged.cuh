@@ -94,7 +94,7 @@ __global__ void __launch_bounds__(32 * kStagedWarps) bell_gs_staged_kernel(
   if (active) ok = __all_sync(0xffffffffu, mbar_wait_bounded(bar));
   if (!ok) {
     if (lane == 0) {
-      atomicExch(&st->sync_fault, 1);
+      atomicExch(&st->sync_fault, kFaultBulkCopy);
       atomicExch(&st->done, 1);
       mbar_wait_bounded(bar);  // let the copy in flight finish before the block can leave
     }

@@ -109,7 +109,7 @@ __device__ __forceinline__ void sweep_barrier(SweepSync *sy, CgState *st, unsign
       unsigned spins = 0;
       while (ld_relaxed_gpu(&sy->arrive) < target) {
         if (++spins >= kSweepSpinLimit) {
-          atomicExch(&st->sync_fault, 1);
+          atomicExch(&st->sync_fault, kFaultGridBarrier);
           atomicExch(&st->done, 1);
           break;
         }

@@ -123,3 +123,11 @@ def test_the_batch_tuner_drops_a_cluster_whose_wait_gives_up(gs, device, withhel
     for m, xi, bi in zip(mats, np.split(x, np.cumsum([m.rows for m in mats])[:-1]),
                          np.split(b, np.cumsum([m.rows for m in mats])[:-1])):
         assert np.linalg.norm(bi - m.to_scipy() @ xi) <= 2e-9 * np.linalg.norm(bi)
+
+
+def test_the_error_names_the_cluster_step(gs, device, tmp_path, withheld, kuhn):
+    a, H, b = kuhn
+    withheld(1)
+    s = solver_with(gs, device, tmp_path, H, gs.SolverOptions(coarse_tail=0), True)
+    with pytest.raises(gs.SolverError, match="cluster Gauss-Seidel step: a wait timed out"):
+        s.solve(b)
