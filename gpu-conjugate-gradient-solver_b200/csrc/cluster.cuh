@@ -205,16 +205,29 @@ __device__ __forceinline__ unsigned short load_early(const unsigned short *p) {
   return v;
 }
 
+// Finite, and large enough that a residual n - q d has all its bits: at least
+// 2^(emin + p), emin the smallest normal exponent and p the digits (one binade
+// more here).
+__device__ __forceinline__ bool full_residual(double v) {
+  constexpr unsigned lo = (1023u - 968u) << 20;
+  return (static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu) - lo < 0x7ff00000u - lo;
+}
+__device__ __forceinline__ bool full_residual(float v) {
+  constexpr unsigned lo = (127u - 101u) << 23;
+  return (__float_as_uint(v) & 0x7fffffffu) - lo < 0x7f800000u - lo;
+}
+
 // The quotient n / d from r = 1 / d: two residual corrections of n r
 // (Markstein, IBM J. Res. Dev. 34, 1990), after which it is correctly rounded.
 // The plain division (370 cycles in FP64 on the critical path of every pass)
-// where r is 0 (1 / d may not be a normal number) or the result not finite.
+// where r is 0 (1 / d may not be a normal number), or n or the result is not
+// finite or so small that a residual loses bits; zeros need neither.
 template <typename T>
 __device__ __forceinline__ T quotient(T n, T d, T r) {
   T q = n * r;
   q = fma(fma(-q, d, n), r, q);
   q = fma(fma(-q, d, n), r, q);
-  if (r == T(0) || !isfinite(q)) q = n / d;
+  if (r == T(0) || !full_residual(n) || !full_residual(q)) q = n == T(0) && r != T(0) ? n * r : n / d;
   return q;
 }
 

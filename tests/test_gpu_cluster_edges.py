@@ -131,3 +131,22 @@ def test_the_error_names_the_cluster_step(gs, device, tmp_path, withheld, kuhn):
     s = solver_with(gs, device, tmp_path, H, gs.SolverOptions(coarse_tail=0), True)
     with pytest.raises(gs.SolverError, match="cluster Gauss-Seidel step: a wait timed out"):
         s.solve(b)
+
+
+@pytest.mark.parametrize("precision,exponents", [(0, [-300, -290, -200, 0, 300]), (1, [-37, -34, -31, -20, 0, 37])])
+def test_quotients_near_the_ends_of_the_range(gs, device, tmp_path, kuhn, precision, exponents):
+    """One V-cycle of right-hand sides whose quotients or their residuals leave
+    the normal range, and one with zeros: the bits of the passes' division."""
+    torch = pytest.importorskip("torch")
+    a, H, b = kuhn
+    o = gs.SolverOptions(coarse_tail=0, precision=precision)
+    pair = [solver_with(gs, device, tmp_path, H, o, cluster) for cluster in (False, True)]
+    for e in exponents + ["zeros"]:
+        r = np.where(np.arange(a.rows) % 5 == 0, b, 0.0) if e == "zeros" else b * 10.0 ** e
+        rd = torch.from_numpy(r).cuda()
+        z = [torch.zeros_like(rd) for _ in pair]
+        torch.cuda.synchronize()
+        for s, zd in zip(pair, z):
+            s.apply_preconditioner_device(rd.data_ptr(), zd.data_ptr(), 0)
+        assert np.array_equal(z[0].cpu().numpy(), z[1].cpu().numpy(), equal_nan=True), e
+        assert e in (-37, -300) or bool(z[0].any())
