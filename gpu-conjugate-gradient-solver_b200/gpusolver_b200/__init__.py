@@ -878,10 +878,14 @@ class DeviceCsr:
             self._h = None
 
 
-# Addresses go to ctypes as plain integers (the argument types are declared):
-# a Backend call's cost is its host side, and a chain of them is as fast as the
-# binding.
+# A Backend call's cost is its host side, and a chain of them is as fast as the
+# binding: integer addresses go to ctypes as they are (the argument types are
+# declared). Anything else goes through C.c_void_p, which takes None for the
+# null address and refuses the rest; a declared c_void_p argument alone would
+# also take bytes, strings and host arrays.
 def spmv(A: DeviceCsr, x_ptr: int, y_ptr: int, stream: int = 0) -> None:
+    if not type(x_ptr) is type(y_ptr) is type(stream) is int:
+        x_ptr, y_ptr, stream = C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(stream)
     rc = lib().gs_spmv(A._h, x_ptr, y_ptr, stream)
     if rc:
         _check(rc)
@@ -889,6 +893,9 @@ def spmv(A: DeviceCsr, x_ptr: int, y_ptr: int, stream: int = 0) -> None:
 
 def gauss_seidel_color(A: DeviceCsr, order_ptr: int, start: int, count: int, rhs_ptr: int,
                        x_ptr: int, omega: float, stream: int = 0) -> None:
+    if not type(order_ptr) is type(rhs_ptr) is type(x_ptr) is type(stream) is int:
+        order_ptr, rhs_ptr, x_ptr, stream = (C.c_void_p(order_ptr), C.c_void_p(rhs_ptr), C.c_void_p(x_ptr),
+                                             C.c_void_p(stream))
     rc = lib().gs_gauss_seidel_color(A._h, order_ptr, start, count, rhs_ptr, x_ptr, omega, stream)
     if rc:
         _check(rc)
@@ -897,6 +904,9 @@ def gauss_seidel_color(A: DeviceCsr, order_ptr: int, start: int, count: int, rhs
 def block_gauss_seidel_color3x3(A: DeviceCsr, order_ptr: int, start: int, count: int,
                                 dinv_ptr: int, rhs_ptr: int, x_ptr: int, omega: float,
                                 stream: int = 0) -> None:
+    if not type(order_ptr) is type(dinv_ptr) is type(rhs_ptr) is type(x_ptr) is type(stream) is int:
+        order_ptr, dinv_ptr, rhs_ptr, x_ptr, stream = (C.c_void_p(order_ptr), C.c_void_p(dinv_ptr),
+                                                       C.c_void_p(rhs_ptr), C.c_void_p(x_ptr), C.c_void_p(stream))
     rc = lib().gs_block_gauss_seidel_color3x3(A._h, order_ptr, start, count, dinv_ptr, rhs_ptr, x_ptr, omega, stream)
     if rc:
         _check(rc)
@@ -904,12 +914,17 @@ def block_gauss_seidel_color3x3(A: DeviceCsr, order_ptr: int, start: int, count:
 
 def apply_block_inverses3x3(n: int, dinv_ptr: int, r_ptr: int, c_ptr: int, dtype: int,
                             stream: int = 0) -> None:
+    if not type(dinv_ptr) is type(r_ptr) is type(c_ptr) is type(stream) is int:
+        dinv_ptr, r_ptr, c_ptr, stream = C.c_void_p(dinv_ptr), C.c_void_p(r_ptr), C.c_void_p(c_ptr), C.c_void_p(stream)
     rc = lib().gs_apply_block_inverses3x3(n, dinv_ptr, r_ptr, c_ptr, dtype, stream)
     if rc:
         _check(rc)
 
 
 def dot(n: int, x_ptr: int, y_ptr: int, result_ptr: int, dtype: int, stream: int = 0) -> None:
+    if not type(x_ptr) is type(y_ptr) is type(result_ptr) is type(stream) is int:
+        x_ptr, y_ptr, result_ptr, stream = (C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(result_ptr),
+                                            C.c_void_p(stream))
     rc = lib().gs_dot(n, x_ptr, y_ptr, result_ptr, dtype, stream)
     if rc:
         _check(rc)
@@ -919,6 +934,9 @@ def dot_noalloc(n: int, x_ptr: int, y_ptr: int, result_ptr: int, dtype: int,
                 stream: int = 0) -> None:
     """gs_dot without allocating: scratch in a fixed array of the library
     (n <= 8,388,608; calls that overlap on the GPU race on that array)."""
+    if not type(x_ptr) is type(y_ptr) is type(result_ptr) is type(stream) is int:
+        x_ptr, y_ptr, result_ptr, stream = (C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(result_ptr),
+                                            C.c_void_p(stream))
     rc = lib().gs_dot_noalloc(n, x_ptr, y_ptr, result_ptr, dtype, stream)
     if rc:
         _check(rc)
@@ -926,6 +944,10 @@ def dot_noalloc(n: int, x_ptr: int, y_ptr: int, result_ptr: int, dtype: int,
 
 def vector_op(op: int, n: int, x_ptr: int, y_ptr: int, alpha: float = 0.0,
               alpha_ptr: Optional[int] = None, dtype: int = F64, stream: int = 0) -> None:
+    if not type(x_ptr) is type(y_ptr) is type(stream) is int:
+        x_ptr, y_ptr, stream = C.c_void_p(x_ptr), C.c_void_p(y_ptr), C.c_void_p(stream)
+    if alpha_ptr is not None:
+        alpha_ptr = C.c_void_p(alpha_ptr)
     rc = lib().gs_vector_op(op, n, x_ptr, y_ptr, alpha, alpha_ptr, dtype, stream)
     if rc:
         _check(rc)
@@ -933,6 +955,8 @@ def vector_op(op: int, n: int, x_ptr: int, y_ptr: int, alpha: float = 0.0,
 
 def scalar_op(op: int, a_ptr: Optional[int], b_ptr: Optional[int], out_ptr: int,
               value: float = 0.0, dtype: int = F64, stream: int = 0) -> None:
+    if not type(a_ptr) is type(b_ptr) is type(out_ptr) is type(stream) is int:
+        a_ptr, b_ptr, out_ptr, stream = C.c_void_p(a_ptr), C.c_void_p(b_ptr), C.c_void_p(out_ptr), C.c_void_p(stream)
     rc = lib().gs_scalar_op(op, a_ptr, b_ptr, out_ptr, value, dtype, stream)
     if rc:
         _check(rc)
