@@ -58,7 +58,9 @@ DotScratch &dot_scratch() {
 // Entry of the kernels below. They are launched with programmatic stream
 // serialization, so that a chain of Backend calls does not start each kernel
 // cold, and read nothing before the wait: what a call is given may be the
-// output of whatever precedes it on the caller's stream.
+// output of whatever precedes it on the caller's stream. For the same reason
+// no input is const __restrict__: such a pointer promises that nobody writes
+// the data while the kernel runs, and its loads need not stay behind the wait.
 __device__ __forceinline__ void backend_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -67,8 +69,7 @@ __device__ __forceinline__ void backend_entry() {
 // result = x . y, sequential-order partials per block, the last block adds
 // the partials in block order (deterministic for a given n).
 template <typename T>
-__global__ void __launch_bounds__(256) dot_kernel(int n, const T *__restrict__ x,
-                                                  const T *__restrict__ y, T *result,
+__global__ void __launch_bounds__(256) dot_kernel(int n, const T *x, const T *y, T *result,
                                                   double *partials, unsigned int *ticket) {
   __shared__ double smem[32];
   backend_entry();
@@ -171,8 +172,7 @@ __global__ void __launch_bounds__(256) block_gs_indirect_kernel(const int *rp, c
 }
 
 template <typename T>
-__global__ void block_inverse_apply_kernel(long long nblocks, const T *__restrict__ dinv,
-                                           const T *__restrict__ r, T *__restrict__ c) {
+__global__ void block_inverse_apply_kernel(long long nblocks, const T *dinv, const T *r, T *__restrict__ c) {
   backend_entry();
   const long long b = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (b >= nblocks) return;
@@ -183,7 +183,7 @@ __global__ void block_inverse_apply_kernel(long long nblocks, const T *__restric
 
 // y op= alpha x, alpha from the host (alpha_dev == nullptr) or the device
 template <typename T>
-__global__ void vec_kernel(int op, long long n, const T *__restrict__ x, T *__restrict__ y, T alpha,
+__global__ void vec_kernel(int op, long long n, const T *x, T *__restrict__ y, T alpha,
                            const T *alpha_dev) {
   backend_entry();
   const T a = alpha_dev != nullptr ? *alpha_dev : alpha;

@@ -68,7 +68,9 @@ using BItem = int4;
 // Entry of every kernel of an iteration (kernels.cuh: pass_entry, without the
 // stop flag: a finished system's items are skipped one by one). Whatever an
 // earlier kernel of the iteration writes -- vectors, pair scalars, sys_done --
-// is read after it; items and matrices never change during a solve.
+// is read after it, through pointers that are not const __restrict__ (which
+// would promise that nobody writes the data while the kernel runs) or that
+// after_wait holds back; items and matrices never change during a solve.
 __device__ __forceinline__ void bpass_entry() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -437,13 +439,14 @@ __device__ __forceinline__ void bblock_sum(double (&v)[kN], double *smem) {
 // Ap = A p and the per-item partials of p . Ap (R values per item).
 template <int R>
 __global__ void __launch_bounds__(256) bcg_spmv_pap_kernel(SellView<double> A, const BItem *__restrict__ items,
-                                                           int nitems, const Rv<double, R> *__restrict__ p,
+                                                           int nitems, const Rv<double, R> *p,
                                                            Rv<double, R> *__restrict__ ap,
                                                            const int *__restrict__ sys_done,
                                                            double *__restrict__ partials) {
   __shared__ double smem[32 * R];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
   bpass_entry();
+  p = after_wait(p);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const BItem q = items[it];
     if (item_skipped(sys_done, q.x)) continue;
@@ -474,8 +477,8 @@ __global__ void __launch_bounds__(256) bcg_update_xr_kernel(const int *__restric
                                                             const BItem *__restrict__ items, int nitems,
                                                             Rv<double, R> *__restrict__ x,
                                                             Rv<double, R> *__restrict__ r,
-                                                            const Rv<double, R> *__restrict__ p,
-                                                            const Rv<double, R> *__restrict__ ap,
+                                                            const Rv<double, R> *p,
+                                                            const Rv<double, R> *ap,
                                                             const BPair *__restrict__ pairs,
                                                             const int *__restrict__ sys_done,
                                                             double *__restrict__ partials) {
@@ -519,9 +522,9 @@ __global__ void __launch_bounds__(256) bcg_update_xr_kernel(const int *__restric
 template <typename ZT, int R>
 __global__ void __launch_bounds__(256) bcg_dot_rz_kernel(const int *__restrict__ srow,
                                                          const BItem *__restrict__ items, int nitems,
-                                                         const Rv<double, R> *__restrict__ r,
-                                                         const Rv<ZT, R> *__restrict__ z,
-                                                         const Rv<ZT, R> *__restrict__ z_old,
+                                                         const Rv<double, R> *r,
+                                                         const Rv<ZT, R> *z,
+                                                         const Rv<ZT, R> *z_old,
                                                          const int *__restrict__ sys_done,
                                                          double *__restrict__ partials) {
   __shared__ double smem[32 * 2 * R];
@@ -556,7 +559,7 @@ __global__ void __launch_bounds__(256) bcg_dot_rz_kernel(const int *__restrict__
 template <typename ZT, int R>
 __global__ void __launch_bounds__(256) bcg_update_p_kernel(const int *__restrict__ srow,
                                                            const BItem *__restrict__ items, int nitems,
-                                                           const Rv<ZT, R> *__restrict__ z,
+                                                           const Rv<ZT, R> *z,
                                                            Rv<double, R> *__restrict__ p,
                                                            const BPair *__restrict__ pairs,
                                                            const int *__restrict__ sys_done) {
@@ -588,9 +591,9 @@ __global__ void __launch_bounds__(256) bcg_update_p_kernel(const int *__restrict
 template <typename ZT, int R>
 __global__ void __launch_bounds__(256) bcg_init_kernel(const int *__restrict__ srow,
                                                        const BItem *__restrict__ items, int nitems,
-                                                       const Rv<double, R> *__restrict__ b,
-                                                       const Rv<double, R> *__restrict__ r,
-                                                       const Rv<ZT, R> *__restrict__ z,
+                                                       const Rv<double, R> *b,
+                                                       const Rv<double, R> *r,
+                                                       const Rv<ZT, R> *z,
                                                        Rv<double, R> *__restrict__ p,
                                                        double *__restrict__ partials) {
   __shared__ double smem[32 * 3 * R];
@@ -646,7 +649,7 @@ enum BFinal : int { kBFinInit = 0, kBFinPap = 1, kBFinXr = 2, kBFinRz = 3 };
 
 template <int R, int kWhich>
 __global__ void __launch_bounds__(128) bcg_finalize_kernel(const int *__restrict__ item_first,
-                                                           const double *__restrict__ partials,
+                                                           const double *partials,
                                                            BPair *__restrict__ pairs, int *__restrict__ sys_done,
                                                            BCgShared *__restrict__ sh,
                                                            volatile unsigned *host) {
