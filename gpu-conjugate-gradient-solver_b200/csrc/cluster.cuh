@@ -217,18 +217,28 @@ __device__ __forceinline__ bool full_residual(float v) {
   return (__float_as_uint(v) & 0x7fffffffu) - lo < 0x7f800000u - lo;
 }
 
-// The quotient n / d from r = 1 / d: two residual corrections of n r
-// (Markstein, IBM J. Res. Dev. 34, 1990), after which it is correctly rounded.
-// The plain division (370 cycles in FP64 on the critical path of every pass)
-// where r is 0 (1 / d may not be a normal number), or n or the result is not
-// finite or so small that a residual loses bits; zeros need neither.
-template <typename T>
-__device__ __forceinline__ T quotient(T n, T d, T r) {
-  T q = n * r;
-  q = fma(fma(-q, d, n), r, q);
-  q = fma(fma(-q, d, n), r, q);
-  if (r == T(0) || !full_residual(n) || !full_residual(q)) q = n == T(0) && r != T(0) ? n * r : n / d;
-  return q;
+// The quotients n / d from r = 1 / d: two residual corrections of n r
+// (Markstein, IBM J. Res. Dev. 34, 1990), after which they are correctly
+// rounded. The plain division (370 cycles in FP64 on the critical path of every
+// pass) where r is 0 (1 / d may not be a normal number), or n or the result is
+// not finite or so small that a residual loses bits; zeros need neither. One
+// test for the row's R quotients.
+template <typename T, int R>
+__device__ __forceinline__ void quotients(const T (&n)[R], T d, T r, T (&q)[R]) {
+  bool exact = r != T(0);
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    q[j] = n[j] * r;
+    q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
+    q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
+    exact = exact && full_residual(n[j]) && full_residual(q[j]);
+  }
+  if (!exact) {
+#pragma unroll
+    for (int j = 0; j < R; ++j)
+      if (r == T(0) || !full_residual(n[j]) || !full_residual(q[j]))
+        q[j] = n[j] == T(0) && r != T(0) ? n[j] * r : n[j] / d;
+  }
 }
 
 // Bounded wait for the values of a pass (written by other CTAs: acquire at
@@ -349,8 +359,10 @@ struct ClusterScalar {
       for (int j = 0; j < R; ++j) sum[j] += __shfl_xor_sync(0xffffffffu, sum[j], o, G);
   }
   static __device__ __forceinline__ void update(const Unit &u, const T (&sum)[R], T (&xn)[R]) {
+    T n[R];
 #pragma unroll
-    for (int j = 0; j < R; ++j) xn[j] = cluster_detail::quotient(T(u.b[j]) - sum[j], u.d.x, u.d.y);
+    for (int j = 0; j < R; ++j) n[j] = T(u.b[j]) - sum[j];
+    cluster_detail::quotients(n, u.d.x, u.d.y, xn);
   }
 };
 
