@@ -1296,8 +1296,11 @@ __global__ void __launch_bounds__(256) cg_init_kernel(int n, const double *__res
       st->done = 1;
     }
     if (st->sync_fault != 0) st->done = 1;  // a wait of the start's V-cycle gave up: nothing to go on from
-    // a zero right-hand side: whatever else is found, the host returns x = 0
-    host[1] = finite_d(acc[0]) && !(sqrt(acc[0]) >= 1e-12) ? kStartZeroRhs : kStartRuns;
+    // a zero right-hand side: whatever else is found, the host returns x = 0;
+    // the iteration queued behind the start has nothing to do
+    const bool zero = finite_d(acc[0]) && !(sqrt(acc[0]) >= 1e-12);
+    if (zero) st->done = 1;
+    host[1] = zero ? kStartZeroRhs : kStartRuns;
   }
 }
 

@@ -31,3 +31,19 @@ def test_one_level_of_one_colour(gs, device, n, flexible):
             assert st.status == gs.STATUS_CONVERGED and np.linalg.norm(d * x - b) <= 2e-13 * np.linalg.norm(b)
     for x, it, status in out[1:]:
         assert it == out[0][1] and status == out[0][2] and np.array_equal(x, out[0][0])
+
+
+@pytest.mark.parametrize("graph", [0, 1])
+def test_a_zero_right_hand_side_stops_at_the_start(gs, device, graph):
+    """The iteration queued behind the start does not run: the statistics are
+    those of the start, x0 = 1 and b below the bound of a zero right-hand side."""
+    a = gs.varcoef_loguniform(9, 10, 11, seed=3)
+    s = gs.Solver(gs.Hierarchy.build(a, 1, 0.1, 10, 40), gs.SolverOptions(tol=1e-8, coarse_tail=0, use_graph=graph),
+                  device=device)
+    b, x0 = np.full(a.rows, 1e-18), np.ones(a.rows)
+    x, st = s.solve(b, x0)
+    assert st.status == gs.STATUS_ZERO_RHS and st.iterations == 0 and st.spmv == 0 and not x.any()
+    # sums of 990 squares in FP64
+    assert st.rhs_norm2 == pytest.approx(float(b @ b), rel=1e-12)
+    r = b - a.to_scipy() @ x0
+    assert st.ratio == pytest.approx(float(r @ r) / float(b @ b), rel=1e-10)
