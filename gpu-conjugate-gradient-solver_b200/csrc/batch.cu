@@ -360,6 +360,12 @@ class Batch final : public BatchSolver {
   void cluster_smooth(const BLevel &L, const VT *b, VT *x, int steps, bool zero, int dir, cudaStream_t s);
   void tune_cluster(int k, const std::vector<SysPrep> &sp);
   void check_fault();
+  // The setup's copies and clears run on the legacy default stream. The device
+  // as a whole is not waited for: another thread may be capturing a stream.
+  void wait_uploads() {
+    BCK(cudaStreamSynchronize(nullptr));
+    BCK(cudaStreamSynchronize(stream_));
+  }
   void vcycle(const RD *r0, RV *z, bool zero0, cudaStream_t s);
   void precondition(const RD *r, RV *z, cudaStream_t s) {
     for (int v = 0; v < opt_.vcycles; ++v) vcycle(r, z, v == 0, s);
@@ -612,14 +618,14 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
     cg_range_ = Range{0, static_cast<int>(cgi.size())};
   }
 
-  BCK(cudaDeviceSynchronize());  // uploads precede the kernels of stream_
+  wait_uploads();  // before the kernels of stream_
   if (opt_.lanes > 0) {
     for (BLevel &L : lv_) L.g = L.pg = L.rg = opt_.lanes;
   } else if (opt_.autotune) {
     autotune();
   }
   build_items();
-  BCK(cudaDeviceSynchronize());  // every upload has landed
+  wait_uploads();
   if (opt_.lanes == 0 && opt_.autotune && opt_.sweep_launch == 1) {
     const long long saved = launches_;
     BCK(cudaMemset(sh_, 0, sizeof(BCgShared)));
@@ -628,7 +634,7 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
       BCK(cudaMemset(L.x, 0, sizeof(RV) * L.n));
       BCK(cudaMemset(L.b, 0, sizeof(RV) * L.n));
     }
-    BCK(cudaDeviceSynchronize());
+    wait_uploads();
     launches_ = saved;
   }
   for (int k = 0; k < K_; ++k) {
@@ -850,7 +856,7 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
   L.cncta = ncta, L.cg = g, L.csystems = S, L.ccolors = colors, L.csmem = smem;
   L.views = arena->upload(views);
   L.csys = arena->upload(systems);
-  BCK(cudaDeviceSynchronize());
+  wait_uploads();
   const auto step = [&] { smooth<VT>(k, L.b, L.x, 1, false, stream_); };
   // the fastest of a few trials each, in turn: one alone can meet a pause of the
   // host. Timed back to back the level stays in L2; in a solve every pass first

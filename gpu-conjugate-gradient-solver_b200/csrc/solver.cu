@@ -553,6 +553,12 @@ class AmgPcg final : public Solver {
     if (L.relaxed) CK(cudaMemcpyAsync(L.xprev, x, sizeof(VT) * L.n, cudaMemcpyDeviceToDevice, s));
   }
   void forward_sweep(Level &L, cudaStream_t s);
+  // The setup's copies and clears run on the legacy default stream. The device
+  // as a whole is not waited for: another thread may be capturing a stream.
+  void wait_uploads() {
+    CK(cudaStreamSynchronize(nullptr));
+    CK(cudaStreamSynchronize(stream_));
+  }
   void check_sync_fault(const CgState &hs);
   void report_fault() {
     CgState hs{};
@@ -1098,7 +1104,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
   }
   features_ = features;
   node_features_ = node_features;
-  CK(cudaDeviceSynchronize());  // the new values have landed before the next solve reads them
+  wait_uploads();  // the next solve reads the new values
 }
 
 template <typename VT>
@@ -2113,7 +2119,7 @@ float AmgPcg<VT>::time_segment(const std::function<void()> &f, int reps, int tri
   // A pass reads its matrix before it waits on the launch ahead of it: the
   // uploads of a new layout have landed, and the first launch follows an
   // operation of the stream that is not a kernel, so it starts in plain order
-  CK(cudaDeviceSynchronize());
+  wait_uploads();
   CK(cudaMemsetAsync(sync_, 0, sizeof(SweepSync), stream_));
   // Layouts of eager solves are timed from a graph too: the host issues the
   // repeated passes of a small level more slowly than the GPU runs them, so
