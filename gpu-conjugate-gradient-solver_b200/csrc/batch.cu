@@ -34,6 +34,12 @@ namespace {
 
 #define BCK(x) cuda_check((x), #x)
 
+template <typename F>
+void with_flag(bool on, F &&f) {
+  if (on) f(std::true_type());
+  else f(std::false_type());
+}
+
 constexpr int kSellItemSlices = 8;  // GS / SpMV items: one slice per warp of a 256-thread block (CSR-vector: 256 / G rows)
 constexpr int kCgItemSlices = 32;   // CG items: up to 1024 rows, one partial sum each
 constexpr int kDenseItemRows = 32;  // coarsest-level items: 32 rows of one system
@@ -347,6 +353,8 @@ class Batch final : public BatchSolver {
  private:
   float time_level_op(int k, int op, int g, int reps);
   int grid(int count) const { return std::max(1, std::min(count, cap_blocks_)); }
+  // whether a list of items takes the kernels that load their first entries early
+  bool head(int lanes, int count) const { return count <= (lanes == 1 ? kHeadSliceItems : kHeadRowItems) * cap_blocks_; }
   template <typename BT>
   void gs_pass(const BLevel &L, const BItem *it, int cnt, const Rv<BT, R> *b, RV *x, bool zero, cudaStream_t s);
   template <int kMode, typename BT>
@@ -708,23 +716,18 @@ void Batch<VT, R>::gs_pass(const BLevel &L, const BItem *it, int cnt, const Rv<B
   if (cnt <= 0) return;
   const VT w = VT(opt_.omega);
   const int gb = grid(cnt);
-  if (L.g == 1) {
-    if (zero) launch_pass(pdl_, bsell_gs_kernel<VT, BT, R, true>, gb, s, L.A.view(), it, cnt, b, x, w, sys_done_);
-    else launch_pass(pdl_, bsell_gs_kernel<VT, BT, R, false>, gb, s, L.A.view(), it, cnt, b, x, w, sys_done_);
-  } else {
+  with_flag(zero, [&](auto Z) { with_flag(head(L.g, cnt), [&](auto H) {
+    constexpr bool kZero = decltype(Z)::value, kHead = decltype(H)::value;
     const CsrvView<VT> v = L.C.view();
-#define BGS(G)                                                                                       \
-  if (zero) launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, true, G>, gb, s, v, it, cnt, b, x, w, sys_done_);  \
-  else launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, false, G>, gb, s, v, it, cnt, b, x, w, sys_done_);
     switch (L.g) {
-      case 2: BGS(2) break;
-      case 4: BGS(4) break;
-      case 8: BGS(8) break;
-      case 16: BGS(16) break;
-      default: BGS(32) break;
+      case 1: launch_pass(pdl_, bsell_gs_kernel<VT, BT, R, kZero, kHead>, gb, s, L.A.view(), it, cnt, b, x, w, sys_done_); break;
+      case 2: launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, kZero, 2, kHead>, gb, s, v, it, cnt, b, x, w, sys_done_); break;
+      case 4: launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, kZero, 4, kHead>, gb, s, v, it, cnt, b, x, w, sys_done_); break;
+      case 8: launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, kZero, 8, kHead>, gb, s, v, it, cnt, b, x, w, sys_done_); break;
+      case 16: launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, kZero, 16, kHead>, gb, s, v, it, cnt, b, x, w, sys_done_); break;
+      default: launch_pass(pdl_, bcsrv_gs_kernel<VT, BT, R, kZero, 32, kHead>, gb, s, v, it, cnt, b, x, w, sys_done_); break;
     }
-#undef BGS
-  }
+  }); });
   BKL("batched gauss-seidel colour pass");
 }
 
@@ -734,18 +737,18 @@ void Batch<VT, R>::spmv(const DevSell<VT> &Sm, const DevCsrv<VT> &Cm, int g, con
                         const RV *x, RV *y, const Rv<BT, R> *b, cudaStream_t s) {
   if (cnt <= 0) return;
   const int gb = grid(cnt);
-  if (g == 1) {
-    launch_pass(pdl_, bsell_spmv_kernel<VT, BT, R, kMode>, gb, s, Sm.view(), it, cnt, x, y, b, sys_done_);
-  } else {
+  with_flag(head(g, cnt), [&](auto H) {
+    constexpr bool kHead = decltype(H)::value;
     const CsrvView<VT> v = Cm.view();
     switch (g) {
-      case 2: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 2>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
-      case 4: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 4>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
-      case 8: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 8>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
-      case 16: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 16>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
-      default: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 32>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 1: launch_pass(pdl_, bsell_spmv_kernel<VT, BT, R, kMode, kHead>, gb, s, Sm.view(), it, cnt, x, y, b, sys_done_); break;
+      case 2: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 2, kHead>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 4: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 4, kHead>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 8: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 8, kHead>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      case 16: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 16, kHead>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
+      default: launch_pass(pdl_, bcsrv_spmv_kernel<VT, BT, R, kMode, 32, kHead>, gb, s, v, it, cnt, x, y, b, sys_done_); break;
     }
-  }
+  });
   BKL("batched spmv");
 }
 
@@ -1073,7 +1076,10 @@ void Batch<VT, R>::cg_start(cudaStream_t s) {
   BCK(cudaMemsetAsync(sys_done_, 0, sizeof(int) * S_, s));
   const BItem *ci = items_ + cg_range_.off;
   const int nc = cg_range_.count, gb = grid(nc);
-  launch_pass(pdl_, bsell_spmv_kernel<double, double, R, kSpmvResid>, gb, s, cgA_.view(), ci, nc, x_, r_, b_, nullptr);
+  with_flag(head(1, nc), [&](auto H) {
+    launch_pass(pdl_, bsell_spmv_kernel<double, double, R, kSpmvResid, decltype(H)::value>, gb, s, cgA_.view(), ci, nc, x_,
+                r_, b_, nullptr);
+  });
   BKL("batched initial residual");
   precondition(r_, z_[0], s);
   launch_pass(pdl_, bcg_init_kernel<VT, R>, gb, s, cgA_.srow, ci, nc, b_, r_, z_[0], p_, partials_);

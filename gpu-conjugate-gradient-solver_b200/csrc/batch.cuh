@@ -81,11 +81,27 @@ __device__ __forceinline__ bool item_skipped(const int *sys_done, int sys) {
 }
 
 // ---- SELL-32, one lane per row -------------------------------------------
+// kHead of the kernels below: with it the first item's matrix entries are loaded
+// before the wait on the predecessor and held in registers, which is what a
+// short list of items waits for; on a long list, bound by bandwidth, the
+// registers halve the warps in flight (FP32, 4 right-hand sides: 64 a thread
+// against 32 in the colour pass, 48 against 32 in the product). The lists are
+// told apart by their items in blocks that fill the device (148 SMs x 8): up to
+// 4 times as many slice items or 8 times as many row items take the head.
+// Measured (one B200, 64 systems of 16^3 to 96^3, 4 FP32 right-hand sides, head /
+// no head): slices: sweep of 31,600 items a pass 397 / 331 us, product of 9,300
+// 61 / 47, product of 1,300 8.6 / 10.5, sweep of 585 a pass 541 / 565; rows: sweep
+// of 2,300 a pass 482 / 516, of 4,700 505 / 514, product of 5,300 48 / 52, of
+// 10,500 102 / 91, of 39,700 369 / 325. The solve: 176.3 ms with the head
+// throughout, 182.7 without, 169.5 by this rule.
+constexpr int kHeadSliceItems = 4;
+constexpr int kHeadRowItems = 8;
+
 template <typename T, int R, bool kSkip>
 __device__ __forceinline__ Rv<T, R> bsell_offdiag(const SellView<T> &A, int s, int lane,
                                                   const Rv<T, R> *__restrict__ x, int skip_from) {
   using P2 = typename Pair<T>::type;
-  const int p0 = A.sptr[s], p1 = A.sptr[s + 1];
+  const int p0 = A.sptr[s], p1 = kSkip && A.lo != nullptr ? A.lo[s] : A.sptr[s + 1];
   Rv<T, R> sum = rv_zero<T, R>();
 #pragma unroll 2
   for (int p = p0 + 2 * lane; p < p1; p += 64) {
@@ -126,50 +142,67 @@ __device__ __forceinline__ Rv<T, R> bsell_offdiag_head(const SellView<T> &A, con
   return sum;
 }
 
+// One row of a colour pass from its off-diagonal sum.
+template <typename T, typename BT, int R, bool kZero>
+__device__ __forceinline__ Rv<T, R> bgs_row(const Rv<T, R> &off, const Rv<BT, R> &b, const Rv<T, R> &old, T d, T w) {
+  Rv<T, R> xn;
+#pragma unroll
+  for (int j = 0; j < R; ++j) {
+    const T gs = (T(b.v[j]) - off.v[j]) / d;
+    xn.v[j] = kZero ? w * gs : (T(1) - w) * old.v[j] + w * gs;
+  }
+  return xn;
+}
+
 // Gauss-Seidel colour pass, items = slice ranges of one colour of one system
 // (aux = first row of that colour), at most one slice per warp:
 //     x_i <- (1 - w) x_i + w (b_i - sum_{j != i} a_ij x_j) / a_ii
 // for each of the R right-hand sides. kZero: x is an implicit zero vector
-// before this forward sweep (columns >= aux hold zero and are not read). The
-// first item and its slice's first slot pairs are loaded before the wait on
-// the predecessor.
-template <typename T, typename BT, int R, bool kZero>
+// before this forward sweep (columns >= aux hold zero and are not read).
+template <typename T, typename BT, int R, bool kZero, bool kHead>
 __global__ void __launch_bounds__(256) bsell_gs_kernel(SellView<T> A, const BItem *__restrict__ items,
                                                        int nitems, const Rv<BT, R> *__restrict__ b,
                                                        Rv<T, R> *__restrict__ x, T w,
                                                        const int *__restrict__ sys_done) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  BItem q = __ldg(items + blockIdx.x);
   SellHead<T> h;
-  if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
+  BItem q;
+  if constexpr (kHead) {
+    q = __ldg(items + blockIdx.x);
+    if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
+  }
   bpass_entry();
   b = after_wait(b);
   x = after_wait(x);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    if (it != static_cast<int>(blockIdx.x)) {
+    if (!kHead || it != static_cast<int>(blockIdx.x)) {
       q = __ldg(items + it);
-      if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
+      if constexpr (kHead)
+        if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h, kZero);
     }
     if (item_skipped(sys_done, q.x) || q.y + warp >= q.z) continue;
-    const int row = h.r0 + lane;
-    const bool valid = row < h.r1;
-    T d = T(1);
-    Rv<BT, R> bv;
-    Rv<T, R> xo = rv_zero<T, R>();
-    if (valid) {
-      d = __ldg(A.diag + row);
-      bv = b[row];
-      if (!kZero) xo = x[row];
-    }
-    const Rv<T, R> off = bsell_offdiag_head<T, R, kZero>(A, h, lane, x, q.w);
-    if (valid) {
-      Rv<T, R> xn;
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const T gs = (T(bv.v[j]) - off.v[j]) / d;
-        xn.v[j] = kZero ? w * gs : (T(1) - w) * xo.v[j] + w * gs;
+    if constexpr (kHead) {
+      const int row = h.r0 + lane;
+      const bool valid = row < h.r1;
+      T d = T(1);
+      Rv<BT, R> bv;
+      Rv<T, R> xo = rv_zero<T, R>();
+      if (valid) {
+        d = __ldg(A.diag + row);
+        bv = b[row];
+        if (!kZero) xo = x[row];
       }
-      x[row] = xn;
+      const Rv<T, R> off = bsell_offdiag_head<T, R, kZero>(A, h, lane, x, q.w);
+      if (valid) x[row] = bgs_row<T, BT, R, kZero>(off, bv, xo, d, w);
+    } else {
+      const int s = q.y + warp;
+      const Rv<T, R> off = bsell_offdiag<T, R, kZero>(A, s, lane, x, q.w);
+      const int row = A.srow[s] + lane;
+      if (row < A.srow[s + 1]) {
+        Rv<T, R> xo = rv_zero<T, R>();
+        if (!kZero) xo = x[row];
+        x[row] = bgs_row<T, BT, R, kZero>(off, b[row], xo, A.diag[row], w);
+      }
     }
   }
 }
@@ -195,28 +228,37 @@ __device__ __forceinline__ void bspmv_store(const T *__restrict__ diag, int row,
 
 // Items are slice ranges. The first slice's head is loaded before the wait on
 // the predecessor, as in the colour passes.
-template <typename T, typename BT, int R, int kMode>
+template <typename T, typename BT, int R, int kMode, bool kHead>
 __global__ void __launch_bounds__(256) bsell_spmv_kernel(SellView<T> A, const BItem *__restrict__ items,
                                                          int nitems, const Rv<T, R> *__restrict__ x,
                                                          Rv<T, R> *__restrict__ y,
                                                          const Rv<BT, R> *__restrict__ b,
                                                          const int *__restrict__ sys_done) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-  BItem q = __ldg(items + blockIdx.x);
+  BItem q;
   SellHead<T> h;
-  if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h);
+  if constexpr (kHead) {
+    q = __ldg(items + blockIdx.x);
+    if (q.y + warp < q.z) sell_head_ops(A, q.y + warp, lane, h);
+  }
   bpass_entry();
   x = after_wait(x);
   b = after_wait(b);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
     const bool first = it == static_cast<int>(blockIdx.x);
-    if (!first) q = __ldg(items + it);
+    if (!kHead || !first) q = __ldg(items + it);
     if (item_skipped(sys_done, q.x)) continue;
     for (int s = q.y + warp; s < q.z; s += nw) {
-      if (!first || s != q.y + warp) sell_head_ops(A, s, lane, h);
-      const Rv<T, R> sum = bsell_offdiag_head<T, R, false>(A, h, lane, x, 0);
-      const int row = h.r0 + lane;
-      if (row < h.r1) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
+      if constexpr (kHead) {
+        if (!first || s != q.y + warp) sell_head_ops(A, s, lane, h);
+        const Rv<T, R> sum = bsell_offdiag_head<T, R, false>(A, h, lane, x, 0);
+        const int row = h.r0 + lane;
+        if (row < h.r1) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
+      } else {
+        const Rv<T, R> sum = bsell_offdiag<T, R, false>(A, s, lane, x, 0);
+        const int row = A.srow[s] + lane;
+        if (row < A.srow[s + 1]) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
+      }
     }
   }
 }
@@ -251,6 +293,25 @@ __device__ __forceinline__ Rv<T, R> bcsrv_offdiag_head(const CsrvView<T> &A, con
   return sum;
 }
 
+template <typename T, int R, bool kSkip, int G>
+__device__ __forceinline__ Rv<T, R> bcsrv_offdiag(const CsrvView<T> &A, int row, bool valid, int sub,
+                                                  const Rv<T, R> *__restrict__ x, int skip_from) {
+  Rv<T, R> sum = rv_zero<T, R>();
+  if (valid) {
+    const int k1 = A.re[row];
+#pragma unroll 4
+    for (int k = A.rp[row] + sub; k < k1; k += G) {
+      const int c = __ldg(A.ci + k);
+      if (!kSkip || c < skip_from) fma_rv<T, R>(__ldg(A.v + k), ldg_rv<T, R>(x + c), sum);
+    }
+  }
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1)
+#pragma unroll
+    for (int j = 0; j < R; ++j) sum.v[j] += __shfl_xor_sync(0xffffffffu, sum.v[j], o, G);
+  return sum;
+}
+
 // Items are row ranges of one colour of one system (aux = first row of the
 // colour), at most one row per group of G lanes. Coarse passes are
 // latency-bound: the first item, its rows' first 8 entries per lane and their
@@ -258,70 +319,82 @@ __device__ __forceinline__ Rv<T, R> bcsrv_offdiag_head(const CsrvView<T> &A, con
 // B200, a forward sweep of level 1): 12 systems of 16^3 to 56^3, 4 FP32
 // right-hand sides, 17 passes, 105 -> 69 us; 5 systems of 14^3 to 30^3, one
 // FP64 right-hand side, 18 passes, 92 -> 43 us.
-template <typename T, typename BT, int R, bool kZero, int G>
+template <typename T, typename BT, int R, bool kZero, int G, bool kHead>
 __global__ void __launch_bounds__(256) bcsrv_gs_kernel(CsrvView<T> A, const BItem *__restrict__ items,
                                                        int nitems, const Rv<BT, R> *__restrict__ b,
                                                        Rv<T, R> *__restrict__ x, T w,
                                                        const int *__restrict__ sys_done) {
   const int sub = threadIdx.x & (G - 1), grp = threadIdx.x / G;
-  BItem q = __ldg(items + blockIdx.x);
+  BItem q;
   CsrvHead<T, 8> h;
-  csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
-  T d = q.y + grp < q.z ? __ldg(A.diag + q.y + grp) : T(1);
+  T d = T(1);
+  if constexpr (kHead) {
+    q = __ldg(items + blockIdx.x);
+    csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
+    if (q.y + grp < q.z) d = __ldg(A.diag + q.y + grp);
+  }
   bpass_entry();
   b = after_wait(b);
   x = after_wait(x);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    if (it != static_cast<int>(blockIdx.x)) {
+    if (!kHead || it != static_cast<int>(blockIdx.x)) {
       q = __ldg(items + it);
-      csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
-      d = q.y + grp < q.z ? __ldg(A.diag + q.y + grp) : T(1);
+      if constexpr (kHead) {
+        csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
+        d = q.y + grp < q.z ? __ldg(A.diag + q.y + grp) : T(1);
+      }
     }
     if (item_skipped(sys_done, q.x)) continue;
     const int row = q.y + grp;
     const bool mine = row < q.z && sub == 0;
-    Rv<BT, R> bv;
-    Rv<T, R> xo = rv_zero<T, R>();
-    if (mine) {
-      bv = b[row];
-      if (!kZero) xo = x[row];
-    }
-    const Rv<T, R> off = bcsrv_offdiag_head<T, R, kZero, G>(A, h, x, q.w);
-    if (mine) {
-      Rv<T, R> xn;
-#pragma unroll
-      for (int j = 0; j < R; ++j) {
-        const T gs = (T(bv.v[j]) - off.v[j]) / d;
-        xn.v[j] = kZero ? w * gs : (T(1) - w) * xo.v[j] + w * gs;
+    if constexpr (kHead) {
+      Rv<BT, R> bv;
+      Rv<T, R> xo = rv_zero<T, R>();
+      if (mine) {
+        bv = b[row];
+        if (!kZero) xo = x[row];
       }
-      x[row] = xn;
+      const Rv<T, R> off = bcsrv_offdiag_head<T, R, kZero, G>(A, h, x, q.w);
+      if (mine) x[row] = bgs_row<T, BT, R, kZero>(off, bv, xo, d, w);
+    } else {
+      const Rv<T, R> off = bcsrv_offdiag<T, R, kZero, G>(A, row, row < q.z, sub, x, q.w);
+      if (mine) {
+        Rv<T, R> xo = rv_zero<T, R>();
+        if (!kZero) xo = x[row];
+        x[row] = bgs_row<T, BT, R, kZero>(off, b[row], xo, A.diag[row], w);
+      }
     }
   }
 }
 
 // Items are row ranges, at most one row per group of G lanes; the head as in
 // the colour passes.
-template <typename T, typename BT, int R, int kMode, int G>
+template <typename T, typename BT, int R, int kMode, int G, bool kHead>
 __global__ void __launch_bounds__(256) bcsrv_spmv_kernel(CsrvView<T> A, const BItem *__restrict__ items,
                                                          int nitems, const Rv<T, R> *__restrict__ x,
                                                          Rv<T, R> *__restrict__ y,
                                                          const Rv<BT, R> *__restrict__ b,
                                                          const int *__restrict__ sys_done) {
   const int sub = threadIdx.x & (G - 1), grp = threadIdx.x / G;
-  BItem q = __ldg(items + blockIdx.x);
+  BItem q;
   CsrvHead<T, 8> h;
-  csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
+  if constexpr (kHead) {
+    q = __ldg(items + blockIdx.x);
+    csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
+  }
   bpass_entry();
   x = after_wait(x);
   b = after_wait(b);
   for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
-    if (it != static_cast<int>(blockIdx.x)) {
+    if (!kHead || it != static_cast<int>(blockIdx.x)) {
       q = __ldg(items + it);
-      csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
+      if constexpr (kHead) csrv_head<T, G>(A, q.y + grp, q.y + grp < q.z, sub, h);
     }
     if (item_skipped(sys_done, q.x)) continue;
     const int row = q.y + grp;
-    const Rv<T, R> sum = bcsrv_offdiag_head<T, R, false, G>(A, h, x, 0);
+    Rv<T, R> sum;
+    if constexpr (kHead) sum = bcsrv_offdiag_head<T, R, false, G>(A, h, x, 0);
+    else sum = bcsrv_offdiag<T, R, false, G>(A, row, row < q.z, sub, x, 0);
     if (row < q.z && sub == 0) bspmv_store<T, BT, R, kMode>(A.diag, row, sum, x, y, b);
   }
 }
