@@ -17,6 +17,14 @@
 
 namespace gsb {
 
+// Where the layout has the off-diagonal entries of its matrix: what a refresh
+// of the values needs.
+struct ClusterEntries {
+  std::vector<unsigned> at;          // entry e (scalar levels: rows in order; else blocks): its place in val
+  std::vector<unsigned short> step;  // 3x3 levels: distance of the block's components
+  BlockRows blocks;                  // 3x3 levels
+};
+
 template <typename T>
 struct HostCluster {
   int ncta = 0, ncolors = 0, g = 0, threads = 0, max_slots = 0, relaxed = 0;
@@ -29,6 +37,7 @@ struct HostCluster {
   std::vector<unsigned> send;
   std::vector<unsigned short> own;
   std::vector<T> diag;               // scalar levels: {d, 1 / d} per row
+  ClusterEntries entries;
 };
 
 // Rows [lo, hi) of colour piece q of ncta over [r0, r1).
@@ -41,15 +50,14 @@ inline int cluster_cut(int r0, int r1, int q, int ncta) {
 // (rp, ci), columns ascending, for ncta CTAs of `threads` threads and g lanes
 // per row: the k-th entry of a row goes to lane k % g, as the CSR-vector
 // kernels read it, as that lane's entry k / g; `per` entries share a slot word
-// (2 on scalar levels, 1 on 3x3 ones). put(e, at, step) stores entry e's values
-// (scalar: at `at`; 3x3: component c at at + c * step). False when the level
-// does not qualify: a CTA needs more than `slot_limit` slots, a single colour,
+// (2 on scalar levels, 1 on 3x3 ones). The values are left zero, their places
+// in h.entries. False when the level does not qualify: a CTA needs more than `slot_limit` slots, a single colour,
 // too many colours, or a row is read by a row that its own owner does not
 // read (the pattern is not structurally symmetric; see the race argument in
 // cluster.cuh).
-template <typename T, typename F>
+template <typename T>
 bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci, const std::vector<int> &first, int per,
-                   int g, int ncta, int threads, bool relaxed, int slot_limit, HostCluster<T> &h, F put) {
+                   int g, int ncta, int threads, bool relaxed, int slot_limit, HostCluster<T> &h) {
   const int nc = static_cast<int>(first.size()) - 1, values = per == 2 ? 2 : 9;  // values per slot word
   if (nc < 2 || nc > kClusterMaxColors || n < 1) return false;
   const int limit = std::min(slot_limit, kClusterMaxSlots);
@@ -138,6 +146,8 @@ bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci
     h.wait_clocks = 2000000;
   }
   h.val.assign(static_cast<size_t>(values) * words, T(0));
+  h.entries.at.assign(ci.size(), 0u);
+  if (per == 1) h.entries.step.assign(ci.size(), 0);
   h.col.assign(static_cast<size_t>(per) * words, zero_slot);
   h.send.assign(static_cast<size_t>(send_total), kNoSend);
   parallel_for(ncta, [&](long long q0, long long q1) {
@@ -158,10 +168,11 @@ bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci
             if (per == 2) {
               const size_t at = 2 * (s.base + word * s.stride + lane) + (kk & 1);
               h.col[at] = sl;
-              put(e, at, 0);
+              h.entries.at[e] = static_cast<unsigned>(at);
             } else {
               h.col[s.base + word * s.stride + lane] = sl;
-              put(e, 9 * static_cast<size_t>(s.base) + 9 * word * s.stride + lane, s.stride);
+              h.entries.at[e] = static_cast<unsigned>(9 * static_cast<size_t>(s.base) + 9 * word * s.stride + lane);
+              h.entries.step[e] = static_cast<unsigned short>(s.stride);
             }
           }
           int d = 0;
@@ -179,32 +190,66 @@ bool cluster_build(int n, const std::vector<int> &rp, const std::vector<int> &ci
   return true;
 }
 
-// The layout of a square scalar matrix (sorted columns), with {d, 1 / d} of
-// every row; the reciprocal is 0 where d or 1 / d is too close to the ends of
-// T's range for the kernel's quotient.
+// First off-diagonal entry of each row.
+inline std::vector<int> off_diagonal_rows(const Csr &a) {
+  std::vector<int> rp(a.rows + 1, 0);
+  parallel_for(a.rows, [&](long long r0, long long r1) {
+    for (long long r = r0; r < r1; ++r)
+      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) rp[r + 1] += a.ci[k] != r ? 1 : 0;
+  }, row_grain(a.rows, a.nnz()));
+  for (int r = 0; r < a.rows; ++r) rp[r + 1] += rp[r];
+  return rp;
+}
+
+// The values of a scalar matrix in the layout, and {d, 1 / d} of every row; the
+// reciprocal is 0 where d or 1 / d is too close to the ends of T's range for
+// the kernel's quotient. False when the matrix is not the layout's.
+template <typename T>
+bool cluster_values(const Csr &a, const ClusterEntries &where, std::vector<T> &val, std::vector<T> &diag) {
+  const std::vector<int> rp = off_diagonal_rows(a);
+  if (static_cast<size_t>(rp[a.rows]) != where.at.size()) return false;
+  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p60f);
+  diag.assign(2 * static_cast<size_t>(a.rows), T(0));
+  parallel_for(a.rows, [&](long long r0, long long r1) {
+    for (long long r = r0; r < r1; ++r) {
+      int e = rp[r];
+      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) {
+        if (a.ci[k] != r) {
+          val[where.at[e++]] = T(a.v[k]);
+          continue;
+        }
+        const T d = T(a.v[k]);
+        diag[2 * r] = d;
+        diag[2 * r + 1] = std::fabs(d) < big && std::fabs(d) > T(1) / big ? T(1) / d : T(0);
+      }
+    }
+  }, row_grain(a.rows, a.nnz()));
+  return true;
+}
+
+// The same for a 3x3-blocked matrix, whose inverse diagonal blocks are the
+// level's own.
+template <typename T>
+bool cluster_block_values(const Csr &a, const ClusterEntries &where, std::vector<T> &val) {
+  return for_block_entries(a, where.blocks,
+                           [&](size_t e, int c, double v) { val[where.at[e] + static_cast<size_t>(c) * where.step[e]] = T(v); });
+}
+
+// The layout of a square scalar matrix (sorted columns).
 template <typename T>
 bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, bool relaxed, int slot_limit,
                   HostCluster<T> &h) {
-  std::vector<int> rp(a.rows + 1, 0), ci, from;
-  ci.reserve(a.ci.size());
-  from.reserve(a.ci.size());
-  const T big = sizeof(T) == 8 ? T(0x1p500) : T(0x1p60f);
-  h.diag.assign(2 * static_cast<size_t>(a.rows), T(0));
-  for (int r = 0; r < a.rows; ++r) {
-    for (int k = a.rp[r]; k < a.rp[r + 1]; ++k) {
-      if (a.ci[k] != r) {
-        ci.push_back(a.ci[k]);
-        from.push_back(k);
-        continue;
-      }
-      const T d = T(a.v[k]);
-      h.diag[2 * static_cast<size_t>(r)] = d;
-      h.diag[2 * static_cast<size_t>(r) + 1] = std::fabs(d) < big && std::fabs(d) > T(1) / big ? T(1) / d : T(0);
+  const std::vector<int> rp = off_diagonal_rows(a);
+  std::vector<int> ci(rp[a.rows]);
+  parallel_for(a.rows, [&](long long r0, long long r1) {
+    for (long long r = r0; r < r1; ++r) {
+      int e = rp[r];
+      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
+        if (a.ci[k] != r) ci[e++] = a.ci[k];
     }
-    rp[r + 1] = static_cast<int>(ci.size());
-  }
-  return cluster_build<T>(a.rows, rp, ci, first, 2, g, ncta, kClusterThreads, relaxed, slot_limit, h,
-                          [&](int e, size_t at, int) { h.val[at] = T(a.v[from[e]]); });
+  }, row_grain(a.rows, a.nnz()));
+  return cluster_build<T>(a.rows, rp, ci, first, 2, g, ncta, kClusterThreads, relaxed, slot_limit, h) &&
+         cluster_values<T>(a, h.entries, h.val, h.diag);
 }
 
 // The layout of a 3x3-blocked matrix, `first` in nodes; the inverse diagonal
@@ -212,33 +257,10 @@ bool make_cluster(const Csr &a, const std::vector<int> &first, int g, int ncta, 
 template <typename T>
 bool make_cluster_blocks(const Csr &a, const std::vector<int> &first, int g, int ncta, bool relaxed, int slot_limit,
                          HostCluster<T> &h) {
-  const int nn = a.rows / 3;
-  std::vector<int> rp(nn + 1, 0), ci, cols;
-  std::vector<T> v;  // 9 per block, row-major
-  for (int I = 0; I < nn; ++I) {
-    cols.clear();
-    for (int r = 3 * I; r < 3 * I + 3; ++r)
-      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
-        if (a.ci[k] / 3 != I) cols.push_back(a.ci[k] / 3);
-    std::sort(cols.begin(), cols.end());
-    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-    const size_t base = v.size();
-    v.resize(base + 9 * cols.size(), T(0));
-    for (int r = 0; r < 3; ++r)
-      for (int k = a.rp[3 * I + r]; k < a.rp[3 * I + r + 1]; ++k) {
-        const int J = a.ci[k] / 3;
-        if (J == I) continue;
-        const size_t q = std::lower_bound(cols.begin(), cols.end(), J) - cols.begin();
-        v[base + 9 * q + 3 * r + a.ci[k] % 3] = T(a.v[k]);
-      }
-    ci.insert(ci.end(), cols.begin(), cols.end());
-    rp[I + 1] = static_cast<int>(ci.size());
-  }
-  return cluster_build<T>(nn, rp, ci, first, 1, g, ncta, kClusterBlockThreads, relaxed, slot_limit, h,
-                          [&](int e, size_t at, int step) {
-                            for (int c = 0; c < 9; ++c)
-                              h.val[at + static_cast<size_t>(c) * step] = v[9 * static_cast<size_t>(e) + c];
-                          });
+  h.entries.blocks = block_rows(a);
+  return cluster_build<T>(a.rows / 3, h.entries.blocks.rp, h.entries.blocks.ci, first, 1, g, ncta, kClusterBlockThreads,
+                          relaxed, slot_limit, h) &&
+         cluster_block_values<T>(a, h.entries, h.val);
 }
 
 template <typename T>
@@ -246,6 +268,7 @@ struct DevCluster {
   int g = 0, ncta = 0, threads = 0, max_slots = 0;
   T *val = nullptr, *diag = nullptr;  // what a value refresh overwrites
   size_t values = 0;
+  ClusterEntries entries;  // kept by levels whose values can be refreshed
   ClusterView<T> v{};
   // dynamic shared memory of a CTA, `width` values a slot
   size_t smem(int width) const {

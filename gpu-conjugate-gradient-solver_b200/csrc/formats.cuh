@@ -6,6 +6,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <stdexcept>
 #include <utility>
@@ -52,6 +53,58 @@ class Arena {
 // ---------------------------------------------------------------------------
 // host construction of SELL-32 / BELL-32
 // ---------------------------------------------------------------------------
+// Off-diagonal 3x3 blocks of a blocked matrix by node row, columns ascending.
+struct BlockRows {
+  std::vector<int> rp, ci;
+};
+
+inline BlockRows block_rows(const Csr &a) {
+  const int nn = a.rows / 3;
+  std::vector<std::vector<int>> cols(nn);
+  const long long grain = row_grain(nn, a.nnz());
+  parallel_for(nn, [&](long long I0, long long I1) {
+    for (long long I = I0; I < I1; ++I) {
+      auto &c = cols[I];
+      for (long long r = 3 * I; r < 3 * I + 3; ++r)
+        for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
+          if (a.ci[k] / 3 != I) c.push_back(a.ci[k] / 3);
+      std::sort(c.begin(), c.end());
+      c.erase(std::unique(c.begin(), c.end()), c.end());
+    }
+  }, grain);
+  BlockRows b;
+  b.rp.assign(nn + 1, 0);
+  for (int I = 0; I < nn; ++I) b.rp[I + 1] = b.rp[I] + static_cast<int>(cols[I].size());
+  b.ci.resize(b.rp[nn]);
+  parallel_for(nn, [&](long long I0, long long I1) {
+    for (long long I = I0; I < I1; ++I) std::copy(cols[I].begin(), cols[I].end(), b.ci.begin() + b.rp[I]);
+  }, grain);
+  return b;
+}
+
+// put(e, c, v): component c (row-major) of block e of `b`, from the entries of
+// `a`, in parallel over node rows; false where `a` has a block that `b` has not.
+template <typename F>
+bool for_block_entries(const Csr &a, const BlockRows &b, F put) {
+  const int nn = a.rows / 3;
+  if (static_cast<int>(b.rp.size()) != nn + 1) return false;
+  std::atomic<bool> ok{true};
+  parallel_for(nn, [&](long long I0, long long I1) {
+    for (long long I = I0; I < I1; ++I) {
+      const auto c0 = b.ci.begin() + b.rp[I], c1 = b.ci.begin() + b.rp[I + 1];
+      for (int r = 0; r < 3; ++r)
+        for (int k = a.rp[3 * I + r]; k < a.rp[3 * I + r + 1]; ++k) {
+          const int J = a.ci[k] / 3;
+          if (J == I) continue;
+          const auto q = std::lower_bound(c0, c1, J);
+          if (q == c1 || *q != J) ok = false;
+          else put(q - b.ci.begin(), 3 * r + a.ci[k] % 3, a.v[k]);
+        }
+    }
+  }, row_grain(nn, a.nnz()));
+  return ok;
+}
+
 template <typename T>
 struct HostSell {
   int rows = 0, cols = 0, g = 1;

@@ -221,35 +221,20 @@ struct DevBsrv {
 template <typename T>
 DevBsrv<T> upload_bsrv(Arena &ar, const Csr &a, const DevBell<T> &bell, const std::vector<int> &node_bounds) {
   const int nn = a.rows / 3;
-  std::vector<int> rp(nn + 1, 0), bc, mid(nn, 0);
+  const BlockRows b = block_rows(a);
+  std::vector<T> v(9 * b.ci.size(), T(0));
+  for_block_entries(a, b, [&](size_t e, int c, double x) { v[9 * e + c] = T(x); });
+  std::vector<int> mid(nn, 0);
   size_t colour = 0;
-  std::vector<T> v;
-  std::vector<int> cols;
   for (int I = 0; I < nn; ++I) {
-    cols.clear();
-    for (int r = 3 * I; r < 3 * I + 3; ++r)
-      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
-        if (a.ci[k] / 3 != I) cols.push_back(a.ci[k] / 3);
-    std::sort(cols.begin(), cols.end());
-    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-    const size_t base = v.size();
-    v.resize(base + 9 * cols.size(), T(0));
-    for (int r = 0; r < 3; ++r)
-      for (int k = a.rp[3 * I + r]; k < a.rp[3 * I + r + 1]; ++k) {
-        const int J = a.ci[k] / 3;
-        if (J == I) continue;
-        const size_t q = std::lower_bound(cols.begin(), cols.end(), J) - cols.begin();
-        v[base + 9 * q + 3 * r + a.ci[k] % 3] = T(a.v[k]);
-      }
     while (node_bounds[colour + 1] <= I) ++colour;
-    mid[I] = rp[I] + static_cast<int>(std::lower_bound(cols.begin(), cols.end(), node_bounds[colour]) - cols.begin());
-    bc.insert(bc.end(), cols.begin(), cols.end());
-    rp[I + 1] = static_cast<int>(bc.size());
+    mid[I] = static_cast<int>(std::lower_bound(b.ci.begin() + b.rp[I], b.ci.begin() + b.rp[I + 1], node_bounds[colour]) -
+                              b.ci.begin());
   }
   DevBsrv<T> d;
   d.nodes = nn;
-  d.rp = ar.upload(rp);
-  d.bc = ar.upload(bc);
+  d.rp = ar.upload(b.rp);
+  d.bc = ar.upload(b.ci);
   d.mid = ar.upload(mid);
   d.v = ar.upload(v);
   d.diag = bell.diag;
@@ -375,16 +360,13 @@ void refresh_sell(const DevSell<T> &d, const Csr &a, const std::vector<int> &bou
 }
 
 template <typename T>
-void refresh_cluster(const DevCluster<T> &d, const Csr &a, const std::vector<int> &bounds, bool block) {
-  HostCluster<T> h;
-  const bool relaxed = d.v.relaxed != 0;
-  const bool built = block ? make_cluster_blocks<T>(a, bounds, d.g, d.ncta, relaxed, kClusterMaxSlots, h)
-                           : make_cluster<T>(a, bounds, d.g, d.ncta, relaxed, kClusterMaxSlots, h);
-  if (!built || h.val.size() != d.values || h.max_slots != d.max_slots)
+void refresh_cluster(const DevCluster<T> &d, const Csr &a, bool block) {
+  std::vector<T> val(d.values, T(0)), diag;
+  if (!(block ? cluster_block_values<T>(a, d.entries, val) : cluster_values<T>(a, d.entries, val, diag)))
     throw std::runtime_error("update_values: the matrix sparsity changed");
-  GSB_CK(cudaMemcpy(d.val, h.val.data(), sizeof(T) * h.val.size(), cudaMemcpyHostToDevice));
+  GSB_CK(cudaMemcpy(d.val, val.data(), sizeof(T) * val.size(), cudaMemcpyHostToDevice));
   if (d.diag != nullptr)  // scalar levels; the inverse blocks are the level's own
-    GSB_CK(cudaMemcpy(d.diag, h.diag.data(), sizeof(T) * h.diag.size(), cudaMemcpyHostToDevice));
+    GSB_CK(cudaMemcpy(d.diag, diag.data(), sizeof(T) * diag.size(), cudaMemcpyHostToDevice));
 }
 
 template <typename T>
@@ -420,26 +402,9 @@ void refresh_bell(const DevBell<T> &d, const Csr &a, const std::vector<int> &nod
 template <typename T>
 void refresh_bsrv(const DevBsrv<T> &d, const Csr &a) {
   if (d.v == nullptr) return;
-  const int nn = a.rows / 3;
-  std::vector<T> v;
-  std::vector<int> cols;
-  for (int I = 0; I < nn; ++I) {
-    cols.clear();
-    for (int r = 3 * I; r < 3 * I + 3; ++r)
-      for (int k = a.rp[r]; k < a.rp[r + 1]; ++k)
-        if (a.ci[k] / 3 != I) cols.push_back(a.ci[k] / 3);
-    std::sort(cols.begin(), cols.end());
-    cols.erase(std::unique(cols.begin(), cols.end()), cols.end());
-    const size_t base = v.size();
-    v.resize(base + 9 * cols.size(), T(0));
-    for (int r = 0; r < 3; ++r)
-      for (int k = a.rp[3 * I + r]; k < a.rp[3 * I + r + 1]; ++k) {
-        const int J = a.ci[k] / 3;
-        if (J == I) continue;
-        const size_t q = std::lower_bound(cols.begin(), cols.end(), J) - cols.begin();
-        v[base + 9 * q + 3 * r + a.ci[k] % 3] = T(a.v[k]);
-      }
-  }
+  const BlockRows b = block_rows(a);
+  std::vector<T> v(9 * b.ci.size(), T(0));
+  for_block_entries(a, b, [&](size_t e, int c, double x) { v[9 * e + c] = T(x); });
   if (!v.empty()) GSB_CK(cudaMemcpy(d.v, v.data(), sizeof(T) * v.size(), cudaMemcpyHostToDevice));
 }
 
@@ -1076,7 +1041,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
       refresh_bell(lv.B1, Ai, lv.color_first);
       if (lv.B.val != lv.B1.val) refresh_bell(lv.B, Ai, lv.color_first);
       refresh_bsrv(lv.Bv, Ai);
-      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first, true);
+      if (lv.cluster) refresh_cluster(lv.K, Ai, true);
       if (k == 0) refresh_bell(cgB_, Ai, lv.color_first);
     } else {
       for (int r = 0; r < Ai.rows; ++r) {
@@ -1088,7 +1053,7 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
       refresh_sell(lv.A1, Ai, lv.color_first, true);
       if (lv.A.val != lv.A1.val) refresh_sell(lv.A, Ai, lv.color_first, true);
       refresh_csrv(lv.C, Ai, true);
-      if (lv.cluster) refresh_cluster(lv.K, Ai, lv.color_first, false);
+      if (lv.cluster) refresh_cluster(lv.K, Ai, false);
       if (k == 0) refresh_sell(cgA_, Ai, lv.color_first, true);
       if (lv.kind == 2) {
         std::vector<VT> jd(Ai.rows, VT(0));
@@ -1976,6 +1941,7 @@ bool AmgPcg<VT>::build_cluster(Level &L, int k, Arena &where) {
     if (!make_cluster<VT>(a, L.color_first, g, ncta, L.relaxed, cluster_slots(static_cast<int>(sizeof(VT)) * (block_ ? 3 : 1), L.relaxed, device_), h)) return false;
   }
   L.K = upload_cluster<VT>(where, h, block_ ? L.B1.dinv : nullptr);
+  L.K.entries = std::move(h.entries);
   return true;
 }
 

@@ -55,8 +55,51 @@ static int check(const HostCluster<T> &h) {
   return bad;
 }
 
+// `a` with every entry replaced by a 3x3 block.
+static Csr blocked(const Csr &a) {
+  Csr m;
+  m.rows = m.cols = 3 * a.rows;
+  m.rp.assign(1, 0);
+  for (int r = 0; r < m.rows; ++r) {
+    for (int k = a.rp[r / 3]; k < a.rp[r / 3 + 1]; ++k)
+      for (int c = 0; c < 3; ++c)
+        if (a.ci[k] == r / 3 || c != r % 3 || (k & 1)) {  // blocks with holes
+          m.ci.push_back(3 * a.ci[k] + c);
+          m.v.push_back(a.v[k] + 0.001 * r + 0.01 * c);
+        }
+    m.rp.push_back(static_cast<int>(m.ci.size()));
+  }
+  return m;
+}
+
+// New values put into a kept layout against the layout built from them.
+template <typename T>
+static int refreshed(const Csr &a, const std::vector<int> &first, int g, int ncta, bool block) {
+  HostCluster<T> h, fresh;
+  Csr b = a;
+  for (size_t k = 0; k < b.v.size(); ++k) b.v[k] = 1.0 / (3.0 + static_cast<double>(k % 1001));
+  const auto make = [&](const Csr &m, HostCluster<T> &out) {
+    return block ? make_cluster_blocks<T>(m, first, g, ncta, false, 20000, out) : make_cluster<T>(m, first, g, ncta, false, 20000, out);
+  };
+  if (!make(a, h) || !make(b, fresh)) return 1;
+  std::vector<T> val(h.val.size(), T(0)), diag;
+  if (!(block ? cluster_block_values<T>(b, h.entries, val) : cluster_values<T>(b, h.entries, val, diag))) return 1;
+  int bad = val != fresh.val || (!block && diag != fresh.diag);
+  // another pattern is refused
+  const int u = block ? 3 : 1;
+  Csr c = b;
+  for (int r = 0; r < u; ++r) {
+    const int at = c.rp[r + 1];
+    c.ci.insert(c.ci.begin() + at, a.cols - 1);
+    c.v.insert(c.v.begin() + at, 1.0);
+    for (int q = r + 1; q <= c.rows; ++q) ++c.rp[q];
+  }
+  bad += block ? cluster_block_values<T>(c, h.entries, val) : cluster_values<T>(c, h.entries, val, diag);
+  return bad;
+}
+
 int main() {
-  int bad = 0;
+  int bad = 0, stale = 0;
   for (int ncta : {8, 16})
     for (int g : {4, 8, 16, 32})
       for (int side : {3, 17, 40}) {
@@ -68,7 +111,10 @@ int main() {
           continue;
         }
         bad += check(h);
+        stale += refreshed<double>(a, first, g, ncta, false) + refreshed<float>(a, first, g, ncta, false);
+        const Csr b = blocked(a);
+        stale += refreshed<double>(b, first, g, ncta, true) + refreshed<float>(b, first, g, ncta, true);
       }
-  std::printf("bad %d\n", bad);
+  std::printf("bad %d\nstale %d\n", bad, stale);
   return 0;
 }

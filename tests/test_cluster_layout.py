@@ -26,3 +26,9 @@ def program(tmp_path_factory):
 def test_messages_stay_inside_the_cluster(program):
     out = subprocess.run([program], check=True, capture_output=True, text=True, timeout=120).stdout
     assert out.split("\n")[0] == "bad 0"
+
+
+def test_new_values_go_to_their_places(program):
+    """Refreshed in place, the layout equals one built from the new values."""
+    out = subprocess.run([program], check=True, capture_output=True, text=True, timeout=120).stdout
+    assert out.split("\n")[1] == "stale 0"
