@@ -286,7 +286,7 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
   d.v.relaxed = h.relaxed;
   d.v.wait_clocks = h.wait_clocks;
   d.v.row0 = row0;
-  // one allocation and one copy for the whole layout
+  // the values, and one allocation and one copy for the rest of the layout
   std::vector<unsigned char> pack;
   const auto put = [&](const auto &v) {
     const size_t at = (pack.size() + 255) / 256 * 256;
@@ -295,13 +295,13 @@ DevCluster<T> upload_cluster(Arena &ar, const HostCluster<T> &h, const T *diag, 
     return at;
   };
   const size_t seg = put(h.seg), expect = put(h.expect), slot_ptr = put(h.slot_ptr), slot_row = put(h.slot_row),
-               val = put(h.val), col = put(h.col), send = put(h.send), own = put(h.own), dd = put(h.diag);
+               col = put(h.col), send = put(h.send), own = put(h.own), dd = put(h.diag);
   unsigned char *base = ar.upload(pack);
   d.v.seg = reinterpret_cast<const ClusterSeg *>(base + seg);
   d.v.expect = reinterpret_cast<const unsigned *>(base + expect);
   d.v.slot_ptr = reinterpret_cast<const int *>(base + slot_ptr);
   d.v.slot_row = reinterpret_cast<const int *>(base + slot_row);
-  d.v.val = d.val = reinterpret_cast<T *>(base + val);
+  d.v.val = d.val = ar.upload(h.val);
   d.v.col = reinterpret_cast<const unsigned *>(base + col);
   d.v.send = reinterpret_cast<const unsigned *>(base + send);
   d.v.own = reinterpret_cast<const unsigned short *>(base + own);

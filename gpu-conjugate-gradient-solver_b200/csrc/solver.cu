@@ -625,8 +625,16 @@ class AmgPcg final : public Solver {
   // Trials of a step timed as it is issued, the fastest counts: the host's pace
   // is part of the time, and with one trial a pause of the host chose the
   // cooperative step of a 37,505-row level in 1 of 6 solvers (504 us an
-  // iteration of the 61 x 47 x 83 Poisson instead of 422).
+  // iteration of the 61 x 47 x 83 Poisson instead of 422). The trials after the
+  // first are run where the first could change the choice.
   static constexpr int kIssuedTrials = 3;
+  // Replays a timing of a captured candidate, behind one that warms up: its
+  // graph costs more to build than to replay.
+  static constexpr int kTuneReps = 6;
+  // A sliced layout this many times slower than one with fewer lanes a row ends
+  // the search over more lanes, which would be slower still: on a fine level
+  // their host layouts cost more than all timing.
+  static constexpr float kHopeless = 1.5f;
   float time_segment(const std::function<void()> &f, int reps, int trials = 1, bool as_issued = false);
   void upload_tail_table(int k0);
   TailLevel<VT> *tail_lv_ = nullptr;
@@ -1811,10 +1819,11 @@ void AmgPcg<VT>::autotune() {
       DevSell<VT> bestA;
       DevBell<VT> bestB;
       bool best_staged = false;
+      float fewer = 1e30f;  // the best with fewer lanes
       for (int g : {1, 2, 4, 8}) {
         std::unique_ptr<Arena> trial(new Arena);
         set_layout(L, static_cast<int>(k), true, g, *trial);
-        const float t = time_segment(sweep, 10);
+        const float t = time_segment(sweep, kTuneReps);
         if (t < best) {
           best = t, best_sliced = true, bestg = g, best_staged = false;
           if (g > 1) best_arena = std::move(trial), bestA = L.A, bestB = L.B;
@@ -1822,16 +1831,18 @@ void AmgPcg<VT>::autotune() {
         // block levels: BELL-1 also with the slices bulk-copied to shared memory
         if (g == 1 && block_ && opt_.sweep_launch == 1 && prepare_staged<VT>(L.B.max_slots, device_)) {
           L.staged = true;
-          const float ts = time_segment(sweep, 10);
+          const float ts = time_segment(sweep, kTuneReps);
           L.staged = false;
           if (ts < best) best = ts, best_sliced = true, bestg = 1, best_staged = true;
         }
+        if (t > kHopeless * fewer) break;
+        fewer = std::min(fewer, t);
       }
       CK(cudaStreamSynchronize(stream_));
       set_layout(L, static_cast<int>(k), true, 1, ar_);
       for (int g : {4, 8, 16, 32}) {
         set_layout(L, static_cast<int>(k), false, g, ar_);
-        const float t = time_segment(sweep, 10);
+        const float t = time_segment(sweep, kTuneReps);
         if (t < best) best = t, best_sliced = false, bestg = g;
       }
       if (best_sliced && bestg > 1) {
@@ -1853,14 +1864,20 @@ void AmgPcg<VT>::autotune() {
       if (L.kind == 0 && !block_ && !L.relaxed && !opt_.half_sweeps && opt_.sweep_launch == 1) {
         auto step = [&] { smooth<VT>(L, L.b, L.x, 1, false, stream_); };
         L.coop = false;
-        const float t_pass = time_segment(step, 10, kIssuedTrials, true);
+        // timed back to back the host's issue counts in full; in a solve it runs
+        // ahead for part of the time: a tenth in favour of the passes
+        constexpr float kBias = 0.9f;
+        float t_pass = time_segment(step, 10, 1, true);
         L.coop = true;
         float t_coop = 1e30f;
         try {
-          t_coop = time_segment(step, 10, kIssuedTrials, true);
-          CgState hs{};
-          CK(cudaMemcpy(&hs, st_, sizeof(CgState), cudaMemcpyDeviceToHost));
-          check_sync_fault(hs);
+          t_coop = time_segment(step, 10, 1, true);
+          if (t_coop < kBias * t_pass) {
+            t_coop = std::min(t_coop, time_segment(step, 10, kIssuedTrials - 1, true));
+            L.coop = false;
+            t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
+          }
+          report_fault();
         } catch (const CudaError &) {
           // a launch the device refused: close a capture left open, keep the
           // per-colour passes
@@ -1873,9 +1890,7 @@ void AmgPcg<VT>::autotune() {
           cudaGetLastError();
           t_coop = 1e30f;
         }
-        // timed back to back the host's issue counts in full; in a solve it runs
-        // ahead for part of the time: a tenth in favour of the passes
-        L.coop = t_coop < 0.9f * t_pass;
+        L.coop = t_coop < kBias * t_pass;
         t_now = L.coop ? t_coop : t_pass;
       }
       if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k), t_now);
@@ -1894,8 +1909,8 @@ void AmgPcg<VT>::autotune() {
         const float tr = time_segment([&] {
           level_spmv_resid<VT>(L, L.b, L.x, L.r, rpart, stream_);
           restrict_residual(L, rpart, Cn.b, stream_);
-        }, 10, 2);
-        const float tp = time_segment([&] { prolong<kSpmvAdd>(L, swept_part(L), Cn.x, L.x, stream_); }, 10, 2);
+        }, kTuneReps, 2);
+        const float tp = time_segment([&] { prolong<kSpmvAdd>(L, swept_part(L), Cn.x, L.x, stream_); }, kTuneReps, 2);
         if (tr < br) br = tr, gr = g;
         if (tp < bp) bp = tp, gp = g;
       }
@@ -1962,14 +1977,17 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
   };
   std::unique_ptr<Arena> arena(new Arena);
   if (!build_cluster(L, k, *arena)) return;
-  const float t_pass = t_now > 0.f ? t_now : time_segment(step, 10, kIssuedTrials, true);
+  float t_pass = t_now > 0.f ? t_now : time_segment(step, 10, 1, true);
   L.cluster = true;
-  float t_cluster = time_segment(step, 10, kIssuedTrials, true);
+  float t_cluster = time_segment(step, 10, 1, true);
+  if (t_cluster < 2.f * t_pass) t_cluster = std::min(t_cluster, time_segment(step, 10, kIssuedTrials - 1, true));
   try {
     report_fault();
   } catch (const CudaError &) {
     t_cluster = 1e30f;  // a wait gave up, after which every launch returned at once: the passes stay
   }
+  L.cluster = false;
+  if (t_cluster < t_pass) t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
   L.cluster = t_cluster < t_pass;
   CK(cudaStreamSynchronize(stream_));
   if (L.cluster) kept_layouts_.push_back(std::move(arena));
