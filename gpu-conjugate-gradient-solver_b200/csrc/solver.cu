@@ -475,6 +475,7 @@ class AmgPcg final : public Solver {
     bool coop = false;      // symmetric sweeps as one cooperative launch (scalar SGS levels)
     bool cluster = false;   // smoothing steps in one thread-block cluster (cluster.cuh), layout K
     DevCluster<VT> K;
+    std::unique_ptr<Arena> cluster_arena;  // what K points to
     // colouring of the strong couplings only (coloring 2): a pass reads its
     // own colour's neighbours from `xprev`, the iterate its sweep started with
     bool relaxed = false;
@@ -937,6 +938,12 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
   for (const Level &l : lv_) all_sgs = all_sgs && l.kind == 0 && !l.relaxed;
   // the cluster-resident tail runs symmetric multicolour SGS steps only
   if (!block_ && all_sgs && !opt_.half_sweeps) setup_tail();
+  for (size_t k = 0; tail_on_ && k < lv_.size(); ++k)
+    if (static_cast<int>(k) >= tail_k0_) {  // the tail smooths these levels itself
+      lv_[k].cluster = false;
+      lv_[k].K = DevCluster<VT>{};
+      lv_[k].cluster_arena.reset();
+    }
   CK(cudaDeviceSynchronize());
   setup_ms_[2] = ms_since(t_tail);
   setup_ms_[3] = ms_since(t_setup);
@@ -1790,8 +1797,9 @@ void AmgPcg<VT>::autotune() {
         L.pg = v[7 * k + 3];
         set_layout(L, static_cast<int>(k), v[7 * k] != 0, v[7 * k + 1], ar_);
         L.coop = v[7 * k + 4] != 0 && opt_.sweep_launch != 0 && !L.relaxed && !opt_.half_sweeps;
+        L.cluster_arena.reset(new Arena);
         L.cluster = v[7 * k + 6] != 0 && opt_.sweep_launch == 1 && L.kind == (block_ ? 1 : 0) &&
-                    build_cluster(L, static_cast<int>(k), ar_);
+                    build_cluster(L, static_cast<int>(k), *L.cluster_arena);
         L.staged = v[7 * k + 5] != 0 && opt_.sweep_launch != 0 && block_ && L.sliced && L.g == 1 &&
                    prepare_staged<VT>(L.B.max_slots, device_);
       }
@@ -1990,7 +1998,7 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
   if (t_cluster < t_pass) t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
   L.cluster = t_cluster < t_pass;
   CK(cudaStreamSynchronize(stream_));
-  if (L.cluster) kept_layouts_.push_back(std::move(arena));
+  if (L.cluster) L.cluster_arena = std::move(arena);
 }
 
 template <typename VT>
@@ -2183,9 +2191,9 @@ void AmgPcg<VT>::setup_tail() {
   fill_kernel<VT><<<blocks_for(T0.n, cap_blocks_), 256, 0, stream_>>>(T0.n, T0.b, VT(1));
   CKL("tail timing fill");
   auto segment = [&] { vcycle<VT>(kmin, T0.b, T0.x, true, stream_); };
-  float best = 1e30f;
+  float t_none = 1e30f, best = 1e30f;
   int best_k0 = -1, best_cl = 0;
-  if (opt_.tail == 1) best = time_segment(segment, 3, 1, true);
+  if (opt_.tail == 1) best = t_none = time_segment(segment, 3, 1, true);
   for (int k0 : cands) {
     if (opt_.tail == 2 && k0 != kmin) continue;
     upload_tail_table(k0);
@@ -2201,6 +2209,10 @@ void AmgPcg<VT>::setup_tail() {
       if (t < best || (opt_.tail == 2 && best_k0 < 0)) best = t, best_k0 = k0, best_cl = cl;
     }
   }
+  // a tail that beat one trial of the launches has to beat their fastest (kIssuedTrials)
+  if (opt_.tail == 1 && best_k0 >= 0 &&
+      std::min(t_none, time_segment(segment, 3, kIssuedTrials - 1, true)) <= best)
+    best_k0 = -1;
   if (best_k0 >= 0) {
     upload_tail_table(best_k0);
     tail_cluster_ = best_cl;
