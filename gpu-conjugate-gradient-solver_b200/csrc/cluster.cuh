@@ -205,39 +205,40 @@ __device__ __forceinline__ unsigned short load_early(const unsigned short *p) {
   return v;
 }
 
-// Finite, and large enough that a residual n - q d has all its bits: at least
+// Whether the quotient q of n and a d that has a reciprocal here is finite and
+// large enough that the residuals n - q d have all their bits: |n| of at least
 // 2^(emin + p), emin the smallest normal exponent and p the digits (one binade
-// more here).
-__device__ __forceinline__ bool full_residual(double v) {
-  constexpr unsigned lo = (1023u - 968u) << 20;
-  return (static_cast<unsigned>(__double2hiint(v)) & 0x7fffffffu) - lo < 0x7ff00000u - lo;
+// more here). FP64 asks q alone, 1 / d being above 2^-500 (make_cluster).
+__device__ __forceinline__ bool full_residuals(double, double q) {
+  constexpr unsigned lo = (1023u - 968u + 500u) << 20;
+  return (static_cast<unsigned>(__double2hiint(q)) & 0x7fffffffu) - lo < 0x7ff00000u - lo;
 }
-__device__ __forceinline__ bool full_residual(float v) {
+__device__ __forceinline__ bool full_residuals(float n, float q) {
   constexpr unsigned lo = (127u - 101u) << 23;
-  return (__float_as_uint(v) & 0x7fffffffu) - lo < 0x7f800000u - lo;
+  return (__float_as_uint(n) & 0x7fffffffu) - lo < 0x7f800000u - lo &&
+         (__float_as_uint(q) & 0x7fffffffu) - lo < 0x7f800000u - lo;
 }
 
 // The quotients n / d from r = 1 / d: two residual corrections of n r
 // (Markstein, IBM J. Res. Dev. 34, 1990), after which they are correctly
 // rounded. The plain division (370 cycles in FP64 on the critical path of every
-// pass) where r is 0 (1 / d may not be a normal number), or n or the result is
-// not finite or so small that a residual loses bits; zeros need neither. One
-// test for the row's R quotients.
+// pass) where r is 0 (1 / d may not be a normal number; the result is 0 or NaN
+// then), or n or the result is not finite or so small that a residual loses
+// bits; zeros need neither. One test for the row's R quotients.
 template <typename T, int R>
 __device__ __forceinline__ void quotients(const T (&n)[R], T d, T r, T (&q)[R]) {
-  bool exact = r != T(0);
+  bool exact = true;
 #pragma unroll
   for (int j = 0; j < R; ++j) {
     q[j] = n[j] * r;
     q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
     q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
-    exact = exact && full_residual(n[j]) && full_residual(q[j]);
+    exact = exact && full_residuals(n[j], q[j]);
   }
   if (!exact) {
 #pragma unroll
     for (int j = 0; j < R; ++j)
-      if (r == T(0) || !full_residual(n[j]) || !full_residual(q[j]))
-        q[j] = n[j] == T(0) && r != T(0) ? n[j] * r : n[j] / d;
+      if (!full_residuals(n[j], q[j])) q[j] = n[j] == T(0) && r != T(0) ? n[j] * r : n[j] / d;
   }
 }
 
