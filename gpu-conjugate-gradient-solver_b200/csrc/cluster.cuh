@@ -570,13 +570,12 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
         // every value of this sweep has arrived before the next one starts
         // (or before the CTAs leave)
         if (!dead) dead = !pass_wait(bar_addr + 8 * p, A.wait_clocks);
-        if (dead && next_code == 0xffffu) drain_passes(bar_addr, npass, A.wait_clocks);
+        if (next_code == 0xffffu) return true;
         if (A.relaxed) {
           __syncthreads();
           for (int k = tid; k < nslots * W; k += nthr) xp[k] = xs[k];
         }
         cluster_barrier();
-        if (next_code == 0xffffu) return true;
         fresh = true;
       }
       ++p;
@@ -590,6 +589,8 @@ __device__ __forceinline__ void cluster_steps(const ClusterView<typename Row::V>
     if (step(unit0, unit1)) break;
     if (step(unit1, unit0)) break;
   }
+  if (dead) drain_passes(bar_addr, npass, A.wait_clocks);
+  cluster_barrier();
   if (dead) {
     *status.fault = kFaultCluster;
     *status.stop = 1;
