@@ -366,7 +366,7 @@ class Batch final : public BatchSolver {
     return ClusterPasses{L.ccolors, steps, dir, VT(opt_.omega) == VT(1) ? 1 : 0};
   }
   void cluster_smooth(const BLevel &L, const VT *b, VT *x, int steps, bool zero, int dir, cudaStream_t s);
-  void tune_cluster(int k, const std::vector<SysPrep> &sp);
+  void tune_cluster(int k, const std::vector<SysPrep> &sp, bool forced);
   void check_fault();
   // The setup's copies and clears run on the legacy default stream. The device
   // as a whole is not waited for: another thread may be capturing a stream.
@@ -634,10 +634,11 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
   }
   build_items();
   wait_uploads();
-  if (opt_.lanes == 0 && opt_.autotune && opt_.sweep_launch == 1) {
+  const bool forced = batch_clusters_forced() && opt_.lanes >= 4;
+  if (((opt_.lanes == 0 && opt_.autotune) || forced) && opt_.sweep_launch == 1) {
     const long long saved = launches_;
     BCK(cudaMemset(sh_, 0, sizeof(BCgShared)));
-    for (int k = 1; k + 1 < K_; ++k) tune_cluster(k, sp);
+    for (int k = 1; k + 1 < K_; ++k) tune_cluster(k, sp, forced);
     for (BLevel &L : lv_) {  // the timed steps left values in the level vectors
       BCK(cudaMemset(L.x, 0, sizeof(RV) * L.n));
       BCK(cudaMemset(L.b, 0, sizeof(RV) * L.n));
@@ -649,6 +650,7 @@ Batch<VT, R>::Batch(const std::vector<const Hierarchy *> &h, int nrhs, const Sol
     info_[k].lanes = lv_[k].g;
     info_[k].p_lanes = lv_[k].pg;
     info_[k].r_lanes = lv_[k].rg;
+    info_[k].cluster = lv_[k].cluster ? lv_[k].cncta : 0;
     long long it = 0;
     for (const Range &r : lv_[k].fwd) it += r.count;
     info_[k].sweep_items = it;
@@ -813,7 +815,7 @@ constexpr long long kBatchClusterEntries = 60000;
 constexpr long long kBatchClusterWide = 20000;
 
 template <typename VT, int R>
-void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
+void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp, bool forced) {
   BLevel &L = lv_[k];
   L.cluster = false;
   if (k == 0 || ly_.whole[k].empty()) return;
@@ -826,7 +828,7 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
     rows += v.A.rows;
   }
   if (largest > kBatchClusterEntries) return;
-  const int S = static_cast<int>(ly_.whole[k].size()), g = cluster_lanes(nnz, rows, false);
+  const int S = static_cast<int>(ly_.whole[k].size()), g = forced ? opt_.lanes : cluster_lanes(nnz, rows, false);
   int ncta = 0;
   with_lanes(g, [&](auto G) {
     ncta = cluster_fit(cluster_gs_batch_kernel<ClusterScalar<VT, VT, decltype(G)::value, R>>, kClusterThreads,
@@ -860,6 +862,11 @@ void Batch<VT, R>::tune_cluster(int k, const std::vector<SysPrep> &sp) {
   L.views = arena->upload(views);
   L.csys = arena->upload(systems);
   wait_uploads();
+  if (forced) {
+    L.cluster = true;
+    kept_.push_back(std::move(arena));
+    return;
+  }
   const auto step = [&] { smooth<VT>(k, L.b, L.x, 1, false, stream_); };
   // the fastest of a few trials each, in turn: one alone can meet a pause of the
   // host. Timed back to back the level stays in L2; in a solve every pass first

@@ -24,6 +24,7 @@ struct BatchLevelInfo {
   int max_colors = 0;    // colour passes per sweep
   int lanes = 1, p_lanes = 1, r_lanes = 1;  // threads per row (1 = SELL-32)
   long long sweep_items = 0;  // work-list items of one forward sweep
+  int cluster = 0;            // CTAs of the clusters that run the smoothing steps, or 0
 };
 
 class BatchSolver {

@@ -738,6 +738,11 @@ int gs_debug_withhold_cluster_message(int on) {
   return GS_OK;
 }
 
+int gs_debug_force_batch_clusters(int on) {
+  gsb::batch_clusters_forced() = on != 0;
+  return GS_OK;
+}
+
 int gs_solver_create(const gs_hierarchy *h, const int *const *o2n, const int *const *n2o,
                      const gs_solver_options *opt, int device, gs_solver **out) {
   return guarded([&] {
@@ -865,6 +870,13 @@ int gs_solver_level_launch(const gs_solver *s, int level) {
   const auto info = s->s->level_info();
   if (level < 0 || level >= static_cast<int>(info.size())) return -1;
   return info[level].launch;
+}
+
+int gs_solver_level_cluster(const gs_solver *s, int level) {
+  if (s == nullptr) return -1;
+  const auto info = s->s->level_info();
+  if (level < 0 || level >= static_cast<int>(info.size())) return -1;
+  return info[level].cluster;
 }
 
 int gs_solver_level_in_tail(const gs_solver *s, int level) {
@@ -1045,6 +1057,12 @@ int gs_batch_level_info(const gs_batch *b, int level, int *rows, long long *nnz,
   if (p_lanes) *p_lanes = l.p_lanes;
   if (r_lanes) *r_lanes = l.r_lanes;
   return GS_OK;
+}
+
+int gs_batch_level_cluster(const gs_batch *b, int level) {
+  if (b == nullptr) return -1;
+  const auto &li = b->b->level_info();
+  return level < 0 || level >= static_cast<int>(li.size()) ? -1 : li[level].cluster;
 }
 
 int gs_batch_launch_count(const gs_batch *b, long long *count) {

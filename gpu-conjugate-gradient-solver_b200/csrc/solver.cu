@@ -954,6 +954,7 @@ AmgPcg<VT>::AmgPcg(const Hierarchy &h, const std::vector<const int *> &o2n,
     info_[k].sliced = lv_[k].sliced ? 1 : 0;
     // block levels tell their colour passes apart (0, 2), in a cluster or not
     info_[k].launch = lv_[k].coop || (lv_[k].cluster && !block_) ? 1 : (lv_[k].staged ? 2 : 0);
+    info_[k].cluster = lv_[k].cluster ? lv_[k].K.ncta : 0;
     info_[k].p_lanes = lv_[k].pg;
     info_[k].r_lanes = lv_[k].rg;
   }
@@ -2679,6 +2680,11 @@ double AmgPcg<VT>::error_reduction(const double *e0, cudaStream_t stream) {
 }  // namespace
 
 bool &cluster_message_withheld() {
+  static thread_local bool on = false;
+  return on;
+}
+
+bool &batch_clusters_forced() {
   static thread_local bool on = false;
   return on;
 }

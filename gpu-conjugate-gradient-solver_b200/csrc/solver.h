@@ -23,6 +23,9 @@ void cuda_check(cudaError_t e, const char *what);
 // Whether cluster layouts built on this thread expect a message that nobody
 // sends (gs_debug_withhold_cluster_message).
 bool &cluster_message_withheld();
+// Whether batches created on this thread take clusters of their forced lanes
+// (gs_debug_force_batch_clusters).
+bool &batch_clusters_forced();
 
 struct SolverOptions {
   // Smoother of the finest level (and of every level unless coarse_smoother
@@ -142,6 +145,7 @@ struct LevelInfo {
   int tail_ctas = 0;                        // CTAs of that kernel's cluster
   int launch = 0;                           // colour passes: 0 one launch each, 1 one cooperative
                                             // launch per smoothing step, 2 bulk-copy staged (BELL-1)
+  int cluster = 0;                          // CTAs of the cluster that runs the smoothing steps, or 0
 };
 
 class Solver {

@@ -47,13 +47,15 @@ EXPORTED_SYMBOLS = [
     "gs_permute_matrix", "gs_ell_build", "gs_block_graph", "gs_block_inverses3x3",
     "gs_expand_block_permutation", "gs_problem_create", "gs_host_csr_create",
     "gs_host_csr_info", "gs_host_csr_copy", "gs_host_csr_rhs", "gs_host_csr_destroy",
-    "gs_uniform_rhs", "gs_set_tune_cache", "gs_debug_withhold_cluster_message", "gs_hierarchy_build", "gs_hierarchy_from_levels",
+    "gs_uniform_rhs", "gs_set_tune_cache", "gs_debug_withhold_cluster_message",
+    "gs_debug_force_batch_clusters", "gs_hierarchy_build", "gs_hierarchy_from_levels",
     "gs_hierarchy_num_levels", "gs_hierarchy_matrix_info", "gs_hierarchy_matrix",
     "gs_hierarchy_aggregates", "gs_hierarchy_build_ex", "gs_solver_setup_times", "gs_hierarchy_destroy", "gs_hierarchical_reordering", "gs_solver_options_default",
     "gs_solver_create", "gs_solver_solve", "gs_solver_solve_f32", "gs_solver_solve_device",
     "gs_solver_apply_preconditioner", "gs_solver_set_tolerance",
     "gs_solver_set_colour_weights", "gs_solver_num_levels", "gs_solver_level_info",
     "gs_solver_level_format", "gs_solver_level_in_tail", "gs_solver_level_layout", "gs_solver_level_launch",
+    "gs_solver_level_cluster", "gs_batch_level_cluster",
     "gs_solver_setup_phases",
     "gs_solver_time_kernel", "gs_solver_time_level", "gs_solver_launch_count", "gs_solver_destroy", "gs_dense_spd_inverse",
     "gs_solver_update_matrix",
@@ -535,7 +537,8 @@ class SolverOptions:
     packed_rows: int = 8192     # dense coarsest levels above this size store a tiled lower triangle of the inverse
     coloring: int = 0           # 0 the reference's greedy colouring, 1 smallest-last order where it has fewer
                                 # colours, 2 and the strong couplings only on the coarse levels
-    sweep_launch: int = 1       # SGS steps: 0 a launch per colour, 1 cooperative where faster, 2 always cooperative
+    sweep_launch: int = 1       # SGS steps: 0 a launch per colour, 1 one cluster or cooperative launch where faster,
+                                # 2 always cooperative
     half_sweeps: int = 0        # 1: forward sweeps before, backward sweeps after the coarse correction
     coarse_half: int = 0        # 1: packed dense coarsest inverse in FP16 tiles with a scale per tile
 
@@ -644,7 +647,8 @@ class Solver:
                             stored=st.value, lanes=ln.value, p_lanes=pl.value, r_lanes=rl.value,
                             in_tail=L.gs_solver_level_in_tail(self._s, k),
                             sliced=L.gs_solver_level_layout(self._s, k),
-                            launch=L.gs_solver_level_launch(self._s, k)))
+                            launch=L.gs_solver_level_launch(self._s, k),
+                            cluster=L.gs_solver_level_cluster(self._s, k)))
         return out
 
     def launch_count(self) -> int:
@@ -826,7 +830,8 @@ class Batch:
             _check(lib().gs_batch_level_info(self._b, k, C.byref(r), C.byref(nz), C.byref(sy),
                                              C.byref(mc), C.byref(ln), C.byref(pl), C.byref(rl)))
             out.append(dict(rows=r.value, nnz=nz.value, systems=sy.value, max_colors=mc.value,
-                            lanes=ln.value, p_lanes=pl.value, r_lanes=rl.value))
+                            lanes=ln.value, p_lanes=pl.value, r_lanes=rl.value,
+                            cluster=lib().gs_batch_level_cluster(self._b, k)))
         return out
 
     def launch_count(self) -> int:

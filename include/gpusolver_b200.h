@@ -309,6 +309,11 @@ int gs_set_tune_cache(const char *path);
  * nobody sends, so that a wait of theirs gives up (after about a millisecond)
  * and the call that runs them reports an error. */
 int gs_debug_withhold_cluster_message(int on);
+/* For tests: while on, batches created on this thread with `lanes` of 4 to 32
+ * and sweep_launch 1 run the smoothing steps of every level below the finest
+ * in clusters with that many lanes a row, without timing, where the level's
+ * layout fits. */
+int gs_debug_force_batch_clusters(int on);
 /* old_to_new / new_to_old: one permutation per level (the reference's
  * std::vector<Permutation>), or NULL for identity on every level. */
 int gs_solver_create(const gs_hierarchy *h, const int *const *old_to_new,
@@ -353,6 +358,10 @@ int gs_solver_level_layout(const gs_solver *s, int level);
  * a 3x3 block level whose steps run in a cluster reports what its colour
  * passes would use); -1 on a bad argument. No reference counterpart. */
 int gs_solver_level_launch(const gs_solver *s, int level);
+/* CTAs of the thread-block cluster that runs the smoothing steps of `level`
+ * (scalar and 3x3 block levels); 0 where they run otherwise, -1 on a bad
+ * argument. No reference counterpart. */
+int gs_solver_level_cluster(const gs_solver *s, int level);
 /* Average device milliseconds of one launch of a kernel, CUDA events on
  * `stream`: kind 0 outer SpMV (+ p.Ap), 1 one forward GS sweep of the finest
  * level over all colours, 2 its V-cycle residual, 3 the dense coarsest solve
@@ -446,6 +455,9 @@ int gs_batch_system_rows(const gs_batch *b, int *rows);
  * systems, colour passes per sweep, threads per row of A, P and R. */
 int gs_batch_level_info(const gs_batch *b, int level, int *rows, long long *nnz, int *systems,
                         int *max_colors, int *lanes, int *p_lanes, int *r_lanes);
+/* CTAs of the thread-block clusters (one per system) that run the smoothing
+ * steps of `level`; 0 where they run as colour passes, -1 on a bad argument. */
+int gs_batch_level_cluster(const gs_batch *b, int level);
 int gs_batch_launch_count(const gs_batch *b, long long *count);
 /* Average device milliseconds of: kind 0 the outer FP64 SpMV (+ p.Ap) over
  * every system and right-hand side, 1 one forward Gauss-Seidel sweep of
