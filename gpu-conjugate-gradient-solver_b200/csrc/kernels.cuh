@@ -1141,13 +1141,23 @@ __global__ void __launch_bounds__(256, 2) cg_bell_spmv_pap_kernel(BellView<doubl
 }
 
 // What the host polls in pinned memory. Word 0: 2 * (iterations whose
-// convergence test has run) + stop flag, the status (CgStatus) in the top four
-// bits once stopped. Word 1: the start's outcome, before any of that.
+// convergence test has run, modulo 2^26) + stop flag, the status (CgStatus) in
+// the top four bits once stopped. Word 1: the start's outcome, before any of
+// that.
 enum CgStartCode : unsigned { kStartRuns = 1, kStartZeroRhs = 2 };
 
+__host__ __device__ __forceinline__ unsigned published_word(int iter, bool done, int status) {
+  const unsigned n = 2u * (static_cast<unsigned>(iter) & 0x03ffffffu);
+  return done ? n | 1u | static_cast<unsigned>(status) << 28 : n;
+}
+// Whether `iterations` tests have run when the word of a solve that goes on is
+// w; the two are never more than a few iterations apart.
+inline bool published_reached(unsigned w, unsigned iterations) {
+  return (((w >> 1) - iterations) & 0x03ffffffu) < 0x02000000u;
+}
+
 __device__ __forceinline__ void publish_state(const CgState *st, volatile unsigned *host) {
-  const unsigned n = 2u * (static_cast<unsigned>(st->iter) & 0x03ffffffu);
-  host[0] = st->done != 0 ? n | 1u | static_cast<unsigned>(st->status) << 28 : n;
+  host[0] = published_word(st->iter, st->done != 0, st->status);
 }
 
 // x += alpha p; r -= alpha Ap; rr = r . r; convergence test on rr / bb, its

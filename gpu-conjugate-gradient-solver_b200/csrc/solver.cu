@@ -2368,15 +2368,15 @@ void AmgPcg<VT>::ensure_graphs() {
 // stopped there (or before, on a breakdown or a fault).
 template <typename VT>
 bool AmgPcg<VT>::wait_published(int it) {
-  const unsigned want = 2u * static_cast<unsigned>(it + 1);
+  const unsigned want = static_cast<unsigned>(it) + 1u;
   for (unsigned spins = 0;; ++spins) {
     const unsigned v = host_seq_[0];
     if (v & 1u) return true;
-    if (v >= want) return false;
+    if (published_reached(v, want)) return false;
     if ((spins & 1023u) == 1023u) {
       // an idle stream that published nothing: the solve was stopped elsewhere
       const cudaError_t e = cudaStreamQuery(stream_);
-      if (e == cudaSuccess) return host_seq_[0] < want || (host_seq_[0] & 1u) != 0;
+      if (e == cudaSuccess) return (host_seq_[0] & 1u) != 0 || !published_reached(host_seq_[0], want);
       if (e != cudaErrorNotReady) CK(e);
     }
   }
