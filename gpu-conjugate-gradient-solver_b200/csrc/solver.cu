@@ -519,8 +519,11 @@ class AmgPcg final : public Solver {
     if (L.relaxed) CK(cudaMemcpyAsync(L.xprev, x, sizeof(VT) * L.n, cudaMemcpyDeviceToDevice, s));
   }
   void forward_sweep(Level &L, cudaStream_t s);
-  // The setup's copies and clears run on the legacy default stream. The device
-  // as a whole is not waited for: another thread may be capturing a stream.
+  // The copies and clears of setups, refreshes and weights run on the legacy
+  // default stream, and a copy from pageable memory may return before its last
+  // bytes have landed; the solves' stream does not wait for that one by itself.
+  // The device as a whole is not waited for: another thread may be capturing a
+  // stream.
   void wait_uploads() {
     CK(cudaStreamSynchronize(nullptr));
     CK(cudaStreamSynchronize(stream_));
@@ -1091,11 +1094,13 @@ void AmgPcg<VT>::update_values(const double *a0_values) {
 template <typename VT>
 void AmgPcg<VT>::set_weights(const ColourWeights &w) {
   if (w.w.empty()) {
+    CK(cudaSetDevice(device_));
     for (auto &l : lv_) std::fill(l.wts.begin(), l.wts.end(), nullptr);
-    if (tail_on_) upload_tail_table(tail_k0_);
+    if (tail_on_) upload_tail_table(tail_k0_), wait_uploads();
     drop_graphs();  // the captured kernels carry the weight pointers
     return;
   }
+  CK(cudaSetDevice(device_));
   const int L = static_cast<int>(lv_.size());
   if (static_cast<int>(w.level_offset.size()) != L + 1)
     throw std::runtime_error("colour weights: level offsets do not match the hierarchy");
@@ -1118,6 +1123,7 @@ void AmgPcg<VT>::set_weights(const ColourWeights &w) {
     for (int c = 0; c < lv_[k].ncolors; ++c) lv_[k].wts[c] = wbuf_ + w.level_offset[k] + c;
   if (tail_on_) upload_tail_table(tail_k0_);  // the table carries the weight pointers
   drop_graphs();  // graphs bake the pointers in: rebuild on next use
+  wait_uploads();
 }
 
 // Learned scaling per node of the 3x3 block smoother, every level's nodes in
@@ -1150,6 +1156,7 @@ void AmgPcg<VT>::set_node_weights(const std::vector<double> &w) {
     base += nn;
   }
   drop_graphs();
+  wait_uploads();
 }
 
 template <typename VT>

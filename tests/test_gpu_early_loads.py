@@ -47,3 +47,21 @@ def test_a_zero_right_hand_side_stops_at_the_start(gs, device, graph):
     assert st.rhs_norm2 == pytest.approx(float(b @ b), rel=1e-12)
     r = b - a.to_scipy() @ x0
     assert st.ratio == pytest.approx(float(r @ r) / float(b @ b), rel=1e-10)
+
+
+@pytest.mark.parametrize("tail", [0, 2])
+def test_weights_count_from_the_next_solve(gs, device, tail):
+    """Weights of two kinds in turn, each solved with at once."""
+    a = gs.varcoef_loguniform(17, 16, 15, seed=3)
+    s = gs.Solver(gs.Hierarchy.build(a, 1, 0.1, 10, 60), gs.SolverOptions(tol=1e-9, coarse_tail=tail), device=device)
+    b = gs.uniform_rhs(a.rows, 2)
+    n = [lv["colors"] for lv in s.level_info()]
+    kinds = [[np.linspace(0.9, 1.1, c) for c in n], [np.full(c, 0.85) for c in n], None]
+    want = [None] * 3
+    for i in range(24):
+        s.set_colour_weights(kinds[i % 3])
+        x, st = s.solve(b)
+        assert st.status == gs.STATUS_CONVERGED
+        want[i % 3] = x if want[i % 3] is None else want[i % 3]
+        assert np.array_equal(x, want[i % 3])
+    assert not np.array_equal(want[0], want[1])
