@@ -1782,8 +1782,8 @@ void AmgPcg<VT>::set_layout(Level &L, int k, bool sliced, int g, Arena &where) {
 // operator: each candidate -- sliced (SELL-32 / BELL-32 with 1, 2, 4 or 8
 // lanes per row or node) and CSR-vector with 4, 8, 16 or 32 lanes -- runs a
 // full forward Gauss-Seidel sweep (one SpMV for P and R) on the solver's own
-// buffers, 10 times, launched as the solve launches it (replayed from a
-// captured graph in graph mode), timed with CUDA events; the fastest wins.
+// buffers, replayed kTuneReps times from a captured graph (time_segment) and
+// timed with CUDA events; the fastest wins.
 template <typename VT>
 void AmgPcg<VT>::autotune() {
   static const int cands[] = {1, 4, 8, 16, 32};

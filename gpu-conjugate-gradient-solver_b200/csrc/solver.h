@@ -103,7 +103,8 @@ struct SolverOptions {
   // barriers between colours, 2 cooperative on every scalar level. Colour passes
   // of a 3x3 block level in the BELL-1 layout: 1 with each slice's blocks
   // bulk-copied to shared memory where timed faster, 2 on every such level
-  // whose widest slice fits, 0 never. The iterates are the same bit for bit.
+  // whose widest slice fits, 0 never. The iterates are the same bit for bit
+  // with the same lanes per row and layout (a cluster chooses its own lanes).
   int sweep_launch = 1;
   // 1: pre-smoothing is `pre` forward colour sweeps and post-smoothing `post`
   // backward sweeps (the symmetric pair S, S^T of a textbook V-cycle: half the

@@ -279,12 +279,15 @@ typedef struct {
                          grid barriers on every such level. Colour passes of
                          a 3x3 block level in the BELL-1 layout: 1 with each slice's blocks
                          bulk-copied to shared memory where timed faster, 2 on every such
-                         level whose widest slice fits, 0 never. Same iterates bit for bit
-                         (no reference counterpart) */
+                         level whose widest slice fits, 0 never. The same iterates bit for bit
+                         with the same lanes per row and layout; a cluster chooses its own
+                         lanes, which adds a row's terms in another order (no reference
+                         counterpart) */
   int half_sweeps;    /* 1: pre-smoothing is pre_steps forward colour sweeps and post-smoothing
                          post_steps backward sweeps (the symmetric pair S, S^T: half the colour
                          passes, still symmetric positive definite; no reference counterpart;
-                         one launch per colour pass, whatever sweep_launch says);
+                         small levels in a cluster as sweep_launch says, else one launch per
+                         colour pass, never a cooperative step);
                          0 (default): symmetric Gauss-Seidel steps on both sides (the reference) */
   int coarse_half;    /* 1 (FP32 V-cycle, packed dense coarsest level): its inverse stored in FP16
                          tiles with one FP32 scale each (half the bytes of the coarse solve; no
