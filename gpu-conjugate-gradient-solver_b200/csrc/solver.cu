@@ -1888,12 +1888,13 @@ void AmgPcg<VT>::autotune() {
         float t_coop = 1e30f;
         try {
           t_coop = time_segment(step, 10, 1, true);
+          report_fault();  // after a fault every launch returns at once: nothing more is timed
           if (t_coop < kBias * t_pass) {
             t_coop = std::min(t_coop, time_segment(step, 10, kIssuedTrials - 1, true));
+            report_fault();
             L.coop = false;
             t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
           }
-          report_fault();
         } catch (const CudaError &) {
           // a launch the device refused: close a capture left open, keep the
           // per-colour passes
