@@ -36,7 +36,7 @@
 // waits for all its passes and then meets the others at the cluster barrier,
 // so the earlier write has landed. Rows of one colour do not read each other
 // (or, on a level whose colouring is of the strong couplings only, read the
-// copy of x taken where the sweep starts: slot numbers with bit 15 set).
+// copy of x taken where the sweep starts: slot numbers past the zero slot).
 // All CTAs meet at the cluster barrier before any of them exits.
 //
 // Each row is updated with the arithmetic of csrv_gs_kernel with the same
@@ -208,7 +208,8 @@ __device__ __forceinline__ unsigned short load_early(const unsigned short *p) {
 // Whether the quotient q of n and a d that has a reciprocal here is finite and
 // large enough that the residuals n - q d have all their bits: |n| of at least
 // 2^(emin + p), emin the smallest normal exponent and p the digits (one binade
-// more here). FP64 asks q alone, 1 / d being above 2^-500 (make_cluster).
+// more here). FP64 asks q alone: a d with a reciprocal is above 2^-500
+// (cluster_values), so n is above 2^-968 when q is above 2^-468.
 __device__ __forceinline__ bool full_residuals(double, double q) {
   constexpr unsigned lo = (1023u - 968u + 500u) << 20;
   return (static_cast<unsigned>(__double2hiint(q)) & 0x7fffffffu) - lo < 0x7ff00000u - lo;
