@@ -205,41 +205,44 @@ __device__ __forceinline__ unsigned short load_early(const unsigned short *p) {
   return v;
 }
 
-// Whether the quotient q of n and a d that has a reciprocal here is finite and
-// large enough that the residuals n - q d have all their bits: |n| of at least
-// 2^(emin + p), emin the smallest normal exponent and p the digits (one binade
-// more here). FP64 asks q alone: a d with a reciprocal is above 2^-500
-// (cluster_values), so n is above 2^-968 when q is above 2^-468.
-__device__ __forceinline__ bool full_residuals(double, double q) {
+// Whether the quotient q of an n and a d that has a reciprocal here is finite
+// and large enough that the residuals n - q d have all their bits: |n| of at
+// least 2^-969. Such a d is above 2^-500 (cluster_values), so n is above 2^-968
+// when q is above 2^-468.
+__device__ __forceinline__ bool full_residuals(double q) {
   constexpr unsigned lo = (1023u - 968u + 500u) << 20;
   return (static_cast<unsigned>(__double2hiint(q)) & 0x7fffffffu) - lo < 0x7ff00000u - lo;
 }
-__device__ __forceinline__ bool full_residuals(float n, float q) {
-  constexpr unsigned lo = (127u - 101u) << 23;
-  return (__float_as_uint(n) & 0x7fffffffu) - lo < 0x7f800000u - lo &&
-         (__float_as_uint(q) & 0x7fffffffu) - lo < 0x7f800000u - lo;
-}
 
-// The quotients n / d from r = 1 / d: two residual corrections of n r
-// (Markstein, IBM J. Res. Dev. 34, 1990), after which they are correctly
-// rounded. The plain division (370 cycles in FP64 on the critical path of every
-// pass) where r is 0 (1 / d may not be a normal number; the result is 0 or NaN
-// then), or n or the result is not finite or so small that a residual loses
-// bits; zeros need neither. One test for the row's R quotients.
+// The quotients n / d of a row's R right-hand sides. FP64: from r = 1 / d, two
+// residual corrections of n r (Markstein, IBM J. Res. Dev. 34, 1990), after
+// which they are correctly rounded; the division (370 cycles on the critical
+// path of every pass) where r is 0 (1 / d may not be a normal number; the result
+// is 0 or NaN then), or n or the result is not finite or so small that a residual
+// loses bits. Zeros need neither: a batch of two or three right-hand sides is
+// padded with them (9 systems of 20^3 to 34^3, two right-hand sides, a sweep: 46
+// us, 62 where zeros divide), and only there the test for them pays ahead of the
+// branch. FP32: the division itself, which is as fast (two
+// right-hand sides: 43 us either way).
 template <typename T, int R>
 __device__ __forceinline__ void quotients(const T (&n)[R], T d, T r, T (&q)[R]) {
-  bool exact = true;
+  if constexpr (sizeof(T) == 4) {
 #pragma unroll
-  for (int j = 0; j < R; ++j) {
-    q[j] = n[j] * r;
-    q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
-    q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
-    exact = exact && full_residuals(n[j], q[j]);
-  }
-  if (!exact) {
+    for (int j = 0; j < R; ++j) q[j] = n[j] / d;
+  } else {
+    bool exact = true;
 #pragma unroll
-    for (int j = 0; j < R; ++j)
-      if (!full_residuals(n[j], q[j])) q[j] = n[j] == T(0) && r != T(0) ? n[j] * r : n[j] / d;
+    for (int j = 0; j < R; ++j) {
+      q[j] = n[j] * r;
+      q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
+      q[j] = fma(fma(-q[j], d, n[j]), r, q[j]);
+      exact = exact && (full_residuals(q[j]) || (R > 1 && n[j] == T(0)));
+    }
+    if (!exact) {
+#pragma unroll
+      for (int j = 0; j < R; ++j)
+        if (!full_residuals(q[j]) && n[j] != T(0)) q[j] = n[j] / d;
+    }
   }
 }
 
