@@ -632,6 +632,15 @@ class AmgPcg final : public Solver {
   // iteration of the 61 x 47 x 83 Poisson instead of 422). The trials after the
   // first are run where the first could change the choice.
   static constexpr int kIssuedTrials = 3;
+  // Steps timed back to back favour one launch over passes: the host's issue
+  // counts in full, while in a solve it runs ahead for part of the time, and on a
+  // scalar level the solve does not launch the first colour from zero (first_colour).
+  // A tenth in favour of the passes of a scalar level, against the cooperative
+  // step and against the cluster (level 0 of a 20^3 Poisson, within a tenth of
+  // each other: the solve 1.95 ms with passes, 2.01 with the cluster, which 6 of
+  // 24 solvers chose without it). None on 3x3 levels, which launch every pass
+  // (level 0 of 17^3 elasticity, as close: 7.80 ms with passes, 7.30 with it).
+  static constexpr float kPassBias = 0.9f;
   // Replays a timing of a captured candidate, behind one that warms up: its
   // graph costs more to build than to replay.
   static constexpr int kTuneReps = 6;
@@ -1880,16 +1889,13 @@ void AmgPcg<VT>::autotune() {
       if (L.kind == 0 && !block_ && !L.relaxed && !opt_.half_sweeps && opt_.sweep_launch == 1) {
         auto step = [&] { smooth<VT>(L, L.b, L.x, 1, false, stream_); };
         L.coop = false;
-        // timed back to back the host's issue counts in full; in a solve it runs
-        // ahead for part of the time: a tenth in favour of the passes
-        constexpr float kBias = 0.9f;
         float t_pass = time_segment(step, 10, 1, true);
         L.coop = true;
         float t_coop = 1e30f;
         try {
           t_coop = time_segment(step, 10, 1, true);
           report_fault();  // after a fault every launch returns at once: nothing more is timed
-          if (t_coop < kBias * t_pass) {
+          if (t_coop < kPassBias * t_pass) {
             t_coop = std::min(t_coop, time_segment(step, 10, kIssuedTrials - 1, true));
             report_fault();
             L.coop = false;
@@ -1907,7 +1913,7 @@ void AmgPcg<VT>::autotune() {
           cudaGetLastError();
           t_coop = 1e30f;
         }
-        L.coop = t_coop < kBias * t_pass;
+        L.coop = t_coop < kPassBias * t_pass;
         t_now = L.coop ? t_coop : t_pass;
       }
       if (L.kind == (block_ ? 1 : 0) && opt_.sweep_launch == 1) tune_cluster(L, static_cast<int>(k), t_now);
@@ -2004,8 +2010,9 @@ void AmgPcg<VT>::tune_cluster(Level &L, int k, float t_now) {
     t_cluster = 1e30f;  // a wait gave up, after which every launch returned at once: the passes stay
   }
   L.cluster = false;
-  if (t_cluster < t_pass) t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
-  L.cluster = t_cluster < t_pass;
+  const float bias = block_ ? 1.f : kPassBias;
+  if (t_cluster < bias * t_pass) t_pass = std::min(t_pass, time_segment(step, 10, kIssuedTrials - 1, true));
+  L.cluster = t_cluster < bias * t_pass;
   CK(cudaStreamSynchronize(stream_));
   if (L.cluster) L.cluster_arena = std::move(arena);
 }
